@@ -41,20 +41,20 @@ int cuda_fail(sgnb_ctx* c, cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
   } while (0)
 
-// One fused launch: mode 0 rhs (in -> out), 1 stage (u + coef dt k -> K2 or K3),
-// 2 end-point stage. Dispatches on the arithmetic mode of the context.
+// One fused launch: mode 0 rhs (in -> out), 1 second stage (u + dt/2 k1 -> K2), 2 end-point
+// stage, 3 third stage with the candidate. Dispatches on the arithmetic mode of the context.
 struct Launch {
   int mode = 0;
   const double* in = nullptr;  // mode 0
   double* out = nullptr;       // mode 0
-  int stage = 2;               // mode 1: 2 (k1 -> K2) or 3 (k2 -> K3)
+  int stage = 2;               // 2 (adds k1) or 3 (adds k2)
 };
 
 static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
                              CUtensorMapDataType type, size_t elem, cuuint32_t nz);
 
 cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
-  if (c->mixed) {
+  if (c->k32) {
     StageArgsM A{};
     A.U[0] = c->U[0]; A.U[1] = c->U[1];
     A.K1[0] = (float*)c->K1[0]; A.K1[1] = (float*)c->K1[1];
@@ -66,8 +66,8 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
     A.kin_k2 = L.stage == 3;
     A.coef = L.stage == 3 ? 0.75 : 0.5;
     if (L.mode == 0) A.out = L.out ? nullptr : A.K1[c->cur];  // no FP64 output: the FSAL head
-    else A.out = L.stage == 3 ? A.K3 : A.K2;
-    return dev::launch_fused_mixed(L.mode, c->C, A, s, c->mapsM.ok ? &c->mapsM : nullptr);
+    else A.out = A.K2;
+    return dev::launch_line(L.mode, c->C, A, s);
   }
   StageArgs A{};
   A.U[0] = c->U[0]; A.U[1] = c->U[1];
@@ -78,7 +78,8 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
   A.in = L.in;
   A.kin_k2 = L.stage == 3;
   A.coef = L.stage == 3 ? 0.75 : 0.5;
-  A.out = L.mode == 0 ? L.out : (L.stage == 3 ? A.K3 : A.K2);
+  A.out = L.mode == 0 ? L.out : A.K2;
+  if (c->precision != SGNB_FP64_EXACT) return dev::launch_fused_fast(L.mode, c->C, A, s);
   // tile copies by the tensor-memory accelerator: A names the context's buffers; the
   // right-hand side's input gets its own map, encoded for this launch
   const TileMaps* M = nullptr;
@@ -94,8 +95,7 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
       }
     }
   }
-  return c->precision == SGNB_FP64_FAST ? dev::launch_fused_fast(L.mode, c->C, A, s, M)
-                                        : dev::launch_fused_exact(L.mode, c->C, A, s, M);
+  return dev::launch_fused_exact(L.mode, c->C, A, s, M);
 }
 
 Launch rhs_launch(const double* in, double* out) {
@@ -105,7 +105,7 @@ Launch rhs_launch(const double* in, double* out) {
 }
 Launch stage_launch(int stage) {
   Launch L;
-  if (stage == 4) { L.mode = 2; } else { L.mode = 1; L.stage = stage; }
+  if (stage == 4) { L.mode = 2; } else { L.mode = stage == 3 ? 3 : 1; L.stage = stage; }
   return L;
 }
 
@@ -226,8 +226,8 @@ static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
 static void build_tile_maps(sgnb_ctx* c) {
   c->maps.ok = 0;
   c->maps.inOk = 0;
-  c->mapsM.ok = 0;
   c->encode_tiled = nullptr;
+  if (c->precision != SGNB_FP64_EXACT) return;  // the other modes' kernels copy rows
   if (c->desc.Nx % 8 != 0 || c->desc.Ny % 4 != 0) return;
   const char* sw = std::getenv("SGNB_TMA");
   if (sw && sw[0] == '0') return;
@@ -252,15 +252,7 @@ static void build_tile_maps(sgnb_ctx* c) {
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
            CUDA_SUCCESS;
   };
-  const auto F64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64, F32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  if (c->mixed) {
-    const bool okm = encode_state_map(c, &c->mapsM.K1[0], c->K1[0], F32, 4, 1) &&
-                     encode_state_map(c, &c->mapsM.K1[1], c->K1[1], F32, 4, 1) &&
-                     encode_state_map(c, &c->mapsM.K2, c->K2, F32, 4, 1) &&
-                     encode_state_map(c, &c->mapsM.K3, c->K3, F32, 4, 1) && mapH(&c->mapsM.H);
-    c->mapsM.ok = okm ? 1 : 0;
-    return;
-  }
+  const auto F64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
   const bool ok = encode_state_map(c, &c->maps.U[0], c->U[0], F64, 8, 5) &&
                   encode_state_map(c, &c->maps.U[1], c->U[1], F64, 8, 5) &&
                   encode_state_map(c, &c->maps.K1[0], c->K1[0], F64, 8, 5) &&
@@ -302,6 +294,35 @@ void fill_consts(sgnb_ctx* c) {
   }
   C.gauss = c->tab.gauss;
   C.tr = c->trbuf;
+  // the fast mode's split tables (LineTables), and whether the tables have the symmetry
+  const double *D = C.D, *gl = C.gLp, *gr = C.gRp;
+  double dmax = 0.0, gmax = 0.0;
+  for (int k = 0; k < 25; ++k) dmax = std::fmax(dmax, std::fabs(D[k]));
+  for (int k = 0; k < 5; ++k) gmax = std::fmax(gmax, std::fmax(std::fabs(gl[k]), std::fabs(gr[k])));
+  C.sym = 1;
+  auto zero = [&](double x, double scale) {
+    if (!(std::fabs(x) <= 1e-13 * scale)) C.sym = 0;  // also where a table is not finite
+  };
+  for (int m = 0; m < 5; ++m) {
+    double row = 0.0;
+    for (int k = 0; k < 5; ++k) {
+      row += D[5 * m + k];
+      zero(D[5 * m + k] + D[24 - 5 * m - k], dmax);
+    }
+    zero(row, dmax);
+    zero(gl[m] + gr[4 - m], gmax);
+  }
+  for (int m = 0; m < 3; ++m) {
+    for (int k = 0; k < 2; ++k) {
+      if (m < 2) C.eo.A[2 * m + k] = 0.5 * (D[5 * m + k] + D[5 * m + 4 - k]);
+      C.eo.B[2 * m + k] = 0.5 * (D[5 * m + k] - D[5 * m + 4 - k]);
+    }
+    C.eo.a[m] = 0.5 * (gl[m] + gl[4 - m]);
+    if (m < 2) C.eo.b[m] = 0.5 * (gl[m] - gl[4 - m]);
+  }
+  const char* sw = std::getenv("SGNB_TMA");
+  C.bulk = (sw && sw[0] == '0') ? 0 : (d.Nx % 4 == 0 ? 2 : (d.Nx % 2 == 0 ? 1 : 0));
+  c->k32 = c->mixed && C.sym;
 }
 
 // The device-side loop: a CUDA graph whose one node is a WHILE conditional node; its body
@@ -367,7 +388,7 @@ int run_loop(sgnb_ctx* c) {
   const long long per_rhs = c->tab.gauss ? 2 : 1, per_attempt = 3 * per_rhs + 1;
   const long long attempts0 = h.attempts;
   // FSAL head: k1 = R(u) into K1[cur] (FP32 in the mixed mode)
-  SGNB_CU(c, launch(c, rhs_launch(c->U[c->cur], c->mixed ? nullptr : (double*)c->K1[c->cur]),
+  SGNB_CU(c, launch(c, rhs_launch(c->U[c->cur], c->k32 ? nullptr : (double*)c->K1[c->cur]),
                     c->stream));
   long long host_attempts = 0;  // attempts launched by the host loop (finished runs' exit at entry)
   for (;;) {
@@ -511,9 +532,7 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   if ((rc = set_device(c))) { g_create_error = c->err; delete c; return rc; }
   e = dev::prepare_fused_exact();
   if (e == cudaSuccess) e = dev::prepare_fused_fast();
-  if (e == cudaSuccess) e = dev::prepare_fused_mixed();
   if (e == cudaSuccess) e = dev::prepare_fused_batch();
-  if (e == cudaSuccess) e = dev::prepare_mixed_batch();
   if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
 
   // statics: Hnod, Hx, Hy (Nd each), HfX, HfY (5 ne each), HfXEnd (5 Ny), HfYEnd (5 Nx)
@@ -568,7 +587,7 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   const size_t sbytes = (size_t)c->ntot * sizeof(double);
   // stage derivatives are FP32 in the mixed mode; K2 and K3 are allocated as one block so
   // that together they always hold an FP64 state (scratch for sgnb_rhs_host)
-  const size_t kbytes = (size_t)c->ntot * (c->mixed ? sizeof(float) : sizeof(double));
+  const size_t kbytes = (size_t)c->ntot * (c->k32 ? sizeof(float) : sizeof(double));
   for (double** bp : {&c->U[0], &c->U[1]}) {
     e = cudaMalloc(bp, sbytes);
     if (e != cudaSuccess) { cuda_fail(c, e, "cudaMalloc(state)"); g_create_error = c->err; return bail(SGNB_ERR_NOMEM); }
@@ -660,7 +679,7 @@ int sgnb_rhs_host(sgnb_ctx* c, const double* U, double* dU) {
   // is not allowed, so the input goes to U[cur ^ 1] and the output to the FP64 view of the
   // stage buffers (K2, K3 together hold one FP64 state in every precision mode)
   double* in = c->U[c->cur ^ 1];
-  double* out = c->mixed ? (double*)c->K2 : (double*)c->K3;
+  double* out = c->k32 ? (double*)c->K2 : (double*)c->K3;
   SGNB_CU(c, cudaMemcpyAsync(in, U, c->ntot * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (int rc = sgnb_rhs_device(c, in, out, c->stream)) return rc;
   SGNB_CU(c, cudaMemcpyAsync(dU, out, c->ntot * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -970,6 +989,7 @@ BatchArgs batch_args(sgnb_batch* b, int shape, int kin_k2, double coef) {
     B.tables.gLp[k] = C0.gLp[k]; B.tables.gRp[k] = C0.gRp[k];
     B.tables.gLpf[k] = C0.gLpf[k]; B.tables.gRpf[k] = C0.gRpf[k];
   }
+  B.tables.eo = C0.eo;
   B.consts = b->dconsts;
   B.args = b->dargs;
   B.tile_inst = b->dtile_inst[shape];
@@ -1003,7 +1023,7 @@ int batch_build_graph(sgnb_batch* b) {
                                       cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
       e = batch_launch(b, 1, b->shape, b->blocks, 0, 0.5);
-      if (e == cudaSuccess) e = batch_launch(b, 1, b->shape, b->blocks, 1, 0.75);
+      if (e == cudaSuccess) e = batch_launch(b, 3, b->shape, b->blocks, 1, 0.75);
       if (e == cudaSuccess) e = batch_launch(b, 2, b->shape, b->blocks, 0, 0.0);
       if (e == cudaSuccess)
         e = dev::launch_controller_batch_loop(b->dctrl, b->dpart, b->dnblk[b->shape], b->dntot,
@@ -1087,6 +1107,18 @@ int batch_prepare(sgnb_batch* b) {
 // graph launch up to 4096 attempts (a bound on one launch; the host then relaunches).
 int batch_run(sgnb_batch* b) {
   constexpr long long kAttemptsPerLaunch = 4096;
+  if (!b->ctx[0]->C.sym) {
+    // caller-given FR tables without the reflection symmetry that the batched kernels need:
+    // one instance after the other, each through its own loop
+    for (int i = 0; i < b->n; ++i) {
+      sgnb_ctx* c = b->ctx[i];
+      *c->hctrl = b->hctrl[i];
+      if (int rc = run_loop(c)) return bfail(b, rc, c->err);
+      b->hctrl[i] = *c->hctrl;
+      b->launches = c->launches;
+    }
+    return SGNB_OK;
+  }
   if (int rc = batch_build_graph(b)) return rc;
   long long a0 = 0;
   for (int i = 0; i < b->n; ++i) {
@@ -1119,13 +1151,14 @@ int sgnb_checked_oob(int device, long long* count, int reset) {
   *count = 0;
 #ifdef SGNB_CHECKED
   cudaError_t e = cudaSetDevice(device);
-  unsigned long long a = 0, b = 0, m = 0, j = 0;
+  unsigned long long a = 0, b = 0, l = 0, k = 0, j = 0;
   if (e == cudaSuccess) e = dev::read_oob_exact(&a, reset != 0);
   if (e == cudaSuccess) e = dev::read_oob_fast(&b, reset != 0);
-  if (e == cudaSuccess) e = dev::read_oob_mixed(&m, reset != 0);
+  if (e == cudaSuccess) e = dev::read_oob_line(&l, reset != 0);
+  if (e == cudaSuccess) e = dev::read_oob_batch(&k, reset != 0);
   if (e == cudaSuccess) e = dev::read_oob_adjoint(&j, reset != 0);
   if (e != cudaSuccess) return fail(nullptr, SGNB_ERR_CUDA, cudaGetErrorString(e));
-  *count = (long long)(a + b + m + j);
+  *count = (long long)(a + b + l + k + j);
   return SGNB_OK;
 #else
   (void)device; (void)reset;
@@ -1635,7 +1668,7 @@ int sgnb_batch_autotune(sgnb_batch* b, const double* dt0, int reps, double* ms_o
   sgnb_rk_opts_init(&o);
   // One attempt's three stage launches per repetition. Without the controller the
   // ping-pong index never flips, so the state the instances hold is left as it was:
-  // the launches only write k2, k3, the other state buffer and the error partials.
+  // the launches only write the stage buffers, the other state buffer and the partials.
   if (int rc = batch_init_ctrls(b, dt0, 1, o)) return rc;
   if (int rc = batch_prepare(b)) return rc;
   int sms = 148;
@@ -1655,7 +1688,7 @@ int sgnb_batch_autotune(sgnb_batch* b, const double* dt0, int reps, double* ms_o
         cudaError_t e = cudaSuccess;
         for (int r = 0; r < count && e == cudaSuccess; ++r) {
           e = batch_launch(b, 1, sh, blocks, 0, 0.5);
-          if (e == cudaSuccess) e = batch_launch(b, 1, sh, blocks, 1, 0.75);
+          if (e == cudaSuccess) e = batch_launch(b, 3, sh, blocks, 1, 0.75);
           if (e == cudaSuccess) e = batch_launch(b, 2, sh, blocks, 0, 0.0);
         }
         return e;

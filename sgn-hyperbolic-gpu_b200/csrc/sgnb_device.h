@@ -6,6 +6,17 @@
 
 namespace sgnb {
 
+// The GLL differentiation matrix and the g_DG correction derivatives split into their even
+// and odd halves (D changes sign when its rows and columns are reversed, gRp is minus the
+// reversed gLp): with e_k = F_k + F_{4-k} - 2 F_2 and o_k = F_k - F_{4-k},
+//   (D F)_m = E_m + O_m, (D F)_{4-m} = O_m - E_m,
+//   E_m = A[2m] e_0 + A[2m+1] e_1 + b[m] (jl + jr)      (m = 0, 1)
+//   O_m = B[2m] o_0 + B[2m+1] o_1 + a[m] (jl - jr)      (m = 0, 1, 2)
+// including the lifts jl gLp + jr gRp of the face jumps.
+struct LineTables {
+  double A[4], B[6], a[3], b[2];
+};
+
 // Everything the fused right-hand-side kernel needs besides the state: mesh size,
 // boundary kinds, the physical constants in the exact forms the reference multiplies
 // them in (src/physics/sgn_flux2d.h:89-161), the FR tables, and the bathymetry statics.
@@ -54,6 +65,11 @@ struct RhsConsts {
   // the differentiation and correction tables rounded to FP32 (the mixed mode's FP32
   // contractions)
   float Df[25], gLpf[5], gRpf[5];
+  LineTables eo;  // the fast mode's split tables; sym: the tables have the symmetry it needs
+  int sym;
+  // rows that bulk copies can take (every row starts and ends at a multiple of 16 bytes): 0
+  // none, 1 those of FP64 buffers (Nx even), 2 also those of FP32 ones (Nx a multiple of 4)
+  int bulk;
 };
 
 // Device-resident state of the adaptive integrator: the scalar loop variables of
@@ -177,16 +193,9 @@ struct TileMaps {
   int ok, inOk;
 };
 
-// The mixed-precision mode's counterparts (intermediate stage): the FP32 stage buffers as
-// [field][element row][Nx * 25] with a [1][4][200] box (one field of one tile per copy),
-// the nodal depth as for the FP64 kernels.
-struct TileMapsM {
-  CUtensorMap K1[2], K2, K3, H;
-  int ok;
-};
-
 // Buffers of one fused launch.
 struct StageArgs {
+  using K = double;   // storage type of the stage derivatives
   const double* in;   // MODE_RHS input state
   double* out;        // MODE_RHS / MODE_STAGE output derivative
   double* U[2];       // state ping-pong pair
@@ -194,16 +203,17 @@ struct StageArgs {
   double* K2;
   double* K3;
   int kin_k2;         // MODE_STAGE: add k2 (1) or k1 = K1[cur] (0) to u
-  double coef;        // MODE_STAGE: 0.5 or 0.75
+  double coef;        // MODE_STAGE, MODE_CAND: 0.5 or 0.75
   const CtrlState* ctrl;
   double* partials;   // MODE_FSAL: 3 doubles per CTA (sum r^2, max |r|, NaN count)
 };
 
 // Buffers of one mixed-precision launch: FP64 state, FP32 stage derivatives.
 struct StageArgsM {
+  using K = float;
   const double* in;   // MODE_RHS input state
-  double* outd;       // MODE_RHS output derivative (FP64)
-  float* out;         // MODE_STAGE output derivative
+  double* outd;       // MODE_RHS output derivative (FP64), or NULL: out
+  float* out;         // MODE_STAGE (and MODE_RHS without outd) output derivative
   double* U[2];
   float* K1[2];
   float* K2;
@@ -219,9 +229,11 @@ struct StageArgsM {
 struct FrTablesDev {
   double D[25], gLp[5], gRp[5];
   float Df[25], gLpf[5], gRpf[5];  // FP32 roundings (mixed mode)
+  LineTables eo;                   // the split tables (fast mode)
 };
 
 struct BatchArgs {
+  using Args = StageArgs;
   FrTablesDev tables;   // shared by every instance (P = 4 GLL)
   const RhsConsts* consts;
   const StageArgs* args;
@@ -274,6 +286,7 @@ struct GatherArgs {
 
 // Work list of a batched mixed-precision launch (8x4 tiles), as BatchArgs.
 struct BatchArgsM {
+  using Args = StageArgsM;
   FrTablesDev tables;
   const RhsConsts* consts;
   const StageArgsM* args;
@@ -285,14 +298,11 @@ struct BatchArgsM {
 };
 
 namespace dev {
-// Batched mixed-precision launch: `blocks` persistent CTAs, or one CTA per tile (0).
-cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s);
-cudaError_t prepare_mixed_batch();
-
-// Out-of-range access counts of the checked build (exact and fast translation units).
+// Out-of-range access counts of the checked build, per translation unit.
 cudaError_t read_oob_exact(unsigned long long* out, bool reset);
 cudaError_t read_oob_fast(unsigned long long* out, bool reset);
-cudaError_t read_oob_mixed(unsigned long long* out, bool reset);
+cudaError_t read_oob_line(unsigned long long* out, bool reset);
+cudaError_t read_oob_batch(unsigned long long* out, bool reset);
 cudaError_t read_oob_adjoint(unsigned long long* out, bool reset);
 
 // The fast mode's reciprocal (fn 0) and square root (fn 1) elementwise, for tests.
@@ -311,7 +321,7 @@ cudaError_t launch_controller_slabs(CtrlState* c, const SlabPartials& L, long lo
 
 // Slab edges: the stage inputs of the first and last element columns' edge nodes
 // (a = 0 / a = 4), [field][row][node], for the neighbours' ghosts. mode 0: rhs of in;
-// 1: intermediate stage (kin_k2, coef of A); 2: end-point candidate.
+// 1: intermediate stage (kin_k2, coef of A); 2: the candidate that the third stage left.
 cudaError_t launch_pack_ghosts(int mode, const RhsConsts& C, const StageArgs& A, double* sendL,
                                double* sendR, cudaStream_t s);
 
@@ -331,18 +341,19 @@ cudaError_t launch_gauges_back(double* lam, const long long* nodes, int ng, cons
 // by the tensor-memory accelerator).
 cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A,
                                cudaStream_t s, const TileMaps* M = nullptr);
-cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A,
-                              cudaStream_t s, const TileMaps* M = nullptr);
+cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
+cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
+cudaError_t prepare_line();
 cudaError_t prepare_fused_exact();
 cudaError_t prepare_fused_fast();
-cudaError_t launch_fused_mixed(int mode, const RhsConsts& C, const StageArgsM& A,
-                               cudaStream_t s, const TileMapsM* M = nullptr);
-cudaError_t prepare_fused_mixed();
+cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgsM& A, cudaStream_t s);
 int fused_grid_blocks(int Nx, int Ny);
 // Batched launch (FP64 fast): tile shape shape_id (0: 8x4, 1: 16x2, 2: 4x8); `blocks`
 // persistent CTAs looping over the work list, or one CTA per tile when blocks == 0.
 cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchArgs& B,
                                cudaStream_t s);
+// The mixed mode's (8x4 tiles).
+cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s);
 cudaError_t prepare_fused_batch();
 int batch_tile_tx(int shape_id);
 cudaError_t launch_controller_batch(CtrlState* ctrls, const double* const* partials,

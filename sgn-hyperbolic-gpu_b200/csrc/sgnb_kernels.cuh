@@ -56,7 +56,11 @@ static_assert(TE * NPP == NIT * NTHR, "own nodes split evenly over the threads")
 enum : int {
   MODE_RHS = 0,    // dU = R(U)
   MODE_STAGE = 1,  // k_out = R(u + coef*dt*k_in)
-  MODE_FSAL = 2    // uNew = u + dt(2/9 k1 + 1/3 k2 + 4/9 k3); k4 = R(uNew); error partials
+  MODE_FSAL = 2,   // k4 = R(uNew) of the candidate the third stage left; error partials
+  // third stage of a BS3(2) attempt: k3 = R(u + 3/4 dt k2) is used up in the launch that forms
+  // it; the candidate uNew = u + dt (2/9 k1 + 1/3 k2 + 4/9 k3) goes to the spare state buffer
+  // and the part 7/24 k1 + 1/4 k2 + 1/3 k3 of the embedded solution to the K3 buffer
+  MODE_CAND = 3
 };
 
 // A tile of TX x TY = 32 elements (TX in 4, 8, 16) and its shared-memory layout.
@@ -115,12 +119,9 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // Read-only views of the stage inputs of one launch.
 struct StageIn {
-  const double* __restrict__ in;
+  const double* __restrict__ in;  // MODE_RHS, MODE_FSAL
   const double* __restrict__ u;
-  const double* __restrict__ k;   // MODE_STAGE: the derivative added to u
-  const double* __restrict__ k1;
-  const double* __restrict__ k2;
-  const double* __restrict__ k3;
+  const double* __restrict__ k;   // MODE_STAGE, MODE_CAND: the derivative added to u
   double acoef, dt;
 };
 
@@ -137,15 +138,45 @@ __device__ __forceinline__ double fsal_finish(double u, double part, double k3, 
   return __dadd_rn(u, __dmul_rn(dt, __dadd_rn(part, __dmul_rn(4.0 / 9.0, k3))));
 }
 
-// Stage input of one value: plain, u + (coef dt) k, or the BS3 candidate.
+// The k1, k2, k3 part of the embedded solution's sum (rk.cpp:118-121), which adds 1/8 k4 to it.
+__device__ __forceinline__ double emb_part(double k1, double k2, double k3) {
+  return 7.0 / 24.0 * k1 + 0.25 * k2 + 1.0 / 3.0 * k3;
+}
+
+// Stage input of one value: plain (the end-point stage reads the candidate) or u + (coef dt) k.
 template <int MODE>
 __device__ __forceinline__ double stage_value(const StageIn& I, long long idx) {
-  if constexpr (MODE == MODE_RHS) {
-    return I.in[idx];
-  } else if constexpr (MODE == MODE_STAGE) {
-    return stage_axpy(I.u[idx], I.acoef, I.k[idx]);
-  } else {
-    return fsal_finish(I.u[idx], fsal_part(I.k1[idx], I.k2[idx]), I.k3[idx], I.dt);
+  if constexpr (MODE == MODE_RHS || MODE == MODE_FSAL) return I.in[idx];
+  else return stage_axpy(I.u[idx], I.acoef, I.k[idx]);
+}
+
+// Error partials of one CTA: fixed shuffle tree within each warp, then the warps in order.
+__device__ __forceinline__ void reduce_error(double esum, double emax, int enan, double (*red)[3],
+                                             double* partials, long long blk) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    esum += __shfl_down_sync(0xffffffffu, esum, off);
+    const double om = __shfl_down_sync(0xffffffffu, emax, off);
+    emax = emax < om ? om : emax;
+    enan |= __shfl_down_sync(0xffffffffu, enan, off);
+  }
+  if (lane == 0) {
+    red[warp][0] = esum;
+    red[warp][1] = emax;
+    red[warp][2] = (double)enan;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0, m = 0.0, n = 0.0;
+    for (int w = 0; w < NWARP; ++w) {
+      s += red[w][0];
+      m = m < red[w][1] ? red[w][1] : m;
+      n += red[w][2];
+    }
+    partials[3 * blk + 0] = s;
+    partials[3 * blk + 1] = m;
+    partials[3 * blk + 2] = n;
   }
 }
 
@@ -449,7 +480,6 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
 
   // ---- controller state (stage modes only) ---------------------------------
   int cur = 0;
-  double atol = 0.0, rtol = 0.0;
   StageIn I;
   I.in = A.in;
   I.dt = 0.0;
@@ -459,14 +489,11 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     cur = A.ctrl->cur;
     I.dt = A.ctrl->dt;
     I.acoef = A.coef * I.dt;  // 0.5 * dt or 0.75 * dt as in rk.cpp:100-103
-    atol = A.ctrl->atol;
-    rtol = A.ctrl->rtol;
   }
   I.u = A.U[cur];
   I.k = A.kin_k2 ? A.K2 : A.K1[cur];
-  I.k1 = A.K1[cur];
-  I.k2 = A.K2;
-  I.k3 = A.K3;
+  if constexpr (MODE == MODE_FSAL) I.in = A.U[cur ^ 1];
+  constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND;
 
   // the thread index read through an opaque move: in the persistent batched kernel this
   // keeps the compiler from hoisting the per-thread item and halo descriptors out of the
@@ -523,31 +550,30 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
   item_map();
 
   // ---- load phase --------------------------------------------------------------
-  // TMA: one thread issues the tile's copies (rhs: the input; stage: u and k; end point: k1
-  // and k2; each [5][4][200] doubles; and the [4][200] nodal depths) on an mbarrier that
-  // aliases the (not yet used) reduction slots.
+  // TMA: one thread issues the tile's copies (rhs and end point: the input; stages: u and k;
+  // each [5][4][200] doubles; and the [4][200] nodal depths) on an mbarrier that aliases the
+  // (not yet used) reduction slots.
   const unsigned mbar = smem_addr(&S.red[0][0]);
   if constexpr (TMA) {
     if (tid == 0) mbar_init(mbar);
     __syncthreads();
     if (tid == 0) {
       const int x = ex0 * NPP;  // 16-byte aligned: 1600 bytes per tile column
-      constexpr int narr = MODE == MODE_RHS ? 1 : 2;
+      constexpr int narr = AXPY ? 2 : 1;
       mbar_expect_tx(mbar, (unsigned)((narr * NV + 1) * TE * NPP * sizeof(double)));
-      const CUtensorMap* mu = MODE == MODE_RHS ? &M->In : (MODE == MODE_STAGE ? &M->U[cur] : &M->K1[cur]);
+      const CUtensorMap* mu = MODE == MODE_RHS ? &M->In : &M->U[AXPY ? cur : cur ^ 1];
       tma_load_3d(smem_addr(&S.U[0][0][0]), mu, x, ey0, 0, mbar);
-      if constexpr (MODE != MODE_RHS) {
-        const CUtensorMap* mg = MODE == MODE_STAGE ? (A.kin_k2 ? &M->K2 : &M->K1[cur]) : &M->K2;
+      if constexpr (AXPY) {
+        const CUtensorMap* mg = A.kin_k2 ? &M->K2 : &M->K1[cur];
         tma_load_3d(smem_addr(&S.G[0][0][0]), mg, x, ey0, 0, mbar);
       }
       tma_load_2d(smem_addr(&S.H[0][0]), &M->H, x, ey0, mbar);
     }
   }
   {
-    // Otherwise the statics, and the state of the rhs and stage modes, arrive by
-    // per-thread asynchronous copies straight into shared memory: a tile's loads are all in
-    // flight at once without holding registers. The stage mode stages k in the (still
-    // unused) G area and forms u + (c dt) k in shared memory once the copies have landed.
+    // Otherwise the statics and the state arrive by per-thread asynchronous copies straight
+    // into shared memory: a tile's loads are all in flight at once without holding
+    // registers. The stage modes keep k in the (still unused) G area and forms u + (c dt) k in shared memory once the copies have landed.
     if constexpr (!TMA) {
 #pragma unroll
       for (int u = 0; u < NIT; ++u)
@@ -557,26 +583,16 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     }
     if constexpr (TMA) {
       // the tile copies above
-    } else if constexpr (MODE == MODE_RHS || MODE == MODE_STAGE) {
-      const double* __restrict__ src = MODE == MODE_RHS ? I.in : I.u;
+    } else {
+      const double* __restrict__ src = AXPY ? I.u : I.in;
 #pragma unroll
       for (int v = 0; v < NV; ++v)
 #pragma unroll
         for (int u = 0; u < NIT; ++u)
           if (okk[u] && SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) {
             cp_async8(&(&S.U[v][0][0])[sof[u]], (src + (long long)v * Nd) + gof[u]);
-            if constexpr (MODE == MODE_STAGE)
+            if constexpr (AXPY)
               cp_async8(&(&S.G[v][0][0])[sof[u]], (I.k + (long long)v * Nd) + gof[u]);
-          }
-    } else {
-      // end-point stage, round 1: k1 and k2 into the U and G areas
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int u = 0; u < NIT; ++u)
-          if (okk[u] && SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) {
-            cp_async8(&(&S.U[v][0][0])[sof[u]], (I.k1 + (long long)v * Nd) + gof[u]);
-            cp_async8(&(&S.G[v][0][0])[sof[u]], (I.k2 + (long long)v * Nd) + gof[u]);
           }
     }
     // halo items: descriptors, then loads
@@ -704,7 +720,7 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
           }
       }
     }
-    if constexpr (MODE == MODE_STAGE) {
+    if constexpr (AXPY) {
       // u + (c dt) k for this thread's own items (rk.cpp:100-103), in shared memory
 #pragma unroll
       for (int v = 0; v < NV; ++v)
@@ -714,41 +730,6 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
             double& y = (&S.U[v][0][0])[sof[u]];
             y = stage_axpy(y, I.acoef, (&S.G[v][0][0])[sof[u]]);
           }
-    } else if constexpr (MODE == MODE_FSAL) {
-      // round 2: 2/9 k1 + 1/3 k2 in place, k3 into the G area while u comes through
-      // registers, then uNew = u + dt ((2/9 k1 + 1/3 k2) + 4/9 k3) (rk.cpp:106-108),
-      // written to shared memory and out as the candidate state
-      // every u load of the tile is issued first, so that they are in flight together
-      // with the k3 copies (one memory round trip for the round, not one per field)
-      double ux[NV][NIT];
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int u = 0; u < NIT; ++u)
-          if (okk[u] && SGNB_INB(gof[u], Nd)) ux[v][u] = (I.u + (long long)v * Nd)[gof[u]];
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int u = 0; u < NIT; ++u)
-          if (okk[u]) {
-            double& y = (&S.U[v][0][0])[sof[u]];
-            y = fsal_part(y, (&S.G[v][0][0])[sof[u]]);
-            if (SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP))
-              cp_async8(&(&S.G[v][0][0])[sof[u]], (I.k3 + (long long)v * Nd) + gof[u]);
-          }
-      double* __restrict__ unew = A.U[cur ^ 1];  // stored evict-first (see the copy-out)
-      cp_async_wait_all();
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-#pragma unroll
-        for (int u = 0; u < NIT; ++u)
-          if (okk[u]) {
-            double& y = (&S.U[v][0][0])[sof[u]];
-            const double un = fsal_finish(ux[v][u], y, (&S.G[v][0][0])[sof[u]], I.dt);
-            y = un;
-            if (SGNB_INB(gof[u], Nd)) __stcs(&(unew + (long long)v * Nd)[gof[u]], un);
-          }
-      }
     }
   }
   __syncthreads();
@@ -895,96 +876,85 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
   }
   __syncthreads();
 
-  // ---- copy-out (and the embedded error of the FSAL stage) ------------------
+  // ---- copy-out (the candidate of the third stage; the end point's embedded error) ----
   double esum = 0.0, emax = 0.0;
   int enan = 0;
   item_map();
   {
-    // reload the controller values and stage pointers instead of keeping them live
-    // through the passes
-    if constexpr (MODE == MODE_FSAL) {
-      const CtrlReload rc = ctrl_reload(A.ctrl);
-      cur = rc.cur;
-      I.dt = rc.dt;
-      atol = rc.atol;
-      rtol = rc.rtol;
-      I.u = A.U[cur];
-      I.k1 = A.K1[cur];
-      I.k2 = A.K2;
-      I.k3 = A.K3;
-    }
-    // L2 use: every result (dU, k2, k3, uNew, k4) is next read by another launch, after
-    // gigabytes of other traffic, so it is stored with the streaming (evict-first) hint;
-    // the end-point stage's second reads of u, k1, k2, k3 below are their last use in the
-    // launch and are loaded the same way. The lines the launch still reads (its inputs,
-    // which the epilogue and the neighbour tiles' halos read again) keep L2 to themselves:
-    // 5.01 -> 4.73 ms for the end-point stage at 2048 x 1024.
-    double* __restrict__ outp;
-    if constexpr (MODE == MODE_RHS || MODE == MODE_STAGE) outp = A.out;
-    else outp = A.K1[cur ^ 1];
-    if constexpr (MODE != MODE_FSAL) {
+    // L2 use: every result (dU, k2, uNew, k4 and the embedded part) is next read by another
+    // launch, after gigabytes of other traffic, so it is stored with the streaming
+    // (evict-first) hint; the second reads of the launch's inputs below are their last use
+    // in it and are loaded the same way. The lines the launch still reads (inputs that the
+    // neighbour tiles' halos read again) keep L2 to themselves.
+    if constexpr (MODE == MODE_RHS || MODE == MODE_STAGE) {
+      double* __restrict__ outp = A.out;
 #pragma unroll 1
       for (int v = 0; v < NV; ++v)
 #pragma unroll
         for (int u = 0; u < NIT; ++u)
           if (okk[u] && SGNB_INB(gof[u], Nd)) __stcs(&(outp + (long long)v * Nd)[gof[u]], (&S.G[v][0][0])[sof[u]]);
     } else {
-      // One field at a time, with the next field's four arrays prefetched while the
-      // current field's error is formed: hoisting every field's loads at once would
-      // overflow the register budget.
-      double uu[NIT], c1[NIT], c2[NIT], c3[NIT];
-      double nu[NIT], n1[NIT], n2[NIT], n3[NIT];
-#pragma unroll
-      for (int u = 0; u < NIT; ++u)
-        if (okk[u]) {
-          const int g = gof[u];
-          if (SGNB_INB(g, Nd)) { uu[u] = __ldcs(&I.u[g]); c1[u] = __ldcs(&I.k1[g]); c2[u] = __ldcs(&I.k2[g]); c3[u] = __ldcs(&I.k3[g]); }
-        }
+      // the controller values and stage pointers again, instead of keeping them live through
+      // the passes; one field at a time, with all of its loads in flight
+      const CtrlReload rc = ctrl_reload(A.ctrl);
+      const double dt = rc.dt;
+      const double* __restrict__ u0 = A.U[rc.cur];
+      const double* __restrict__ k1 = A.K1[rc.cur];
+      const double* __restrict__ k2 = A.K2;
+      const double* __restrict__ part = A.K3;
+      double* __restrict__ un_out = A.U[rc.cur ^ 1];
+      double* __restrict__ part_out = A.K3;
+      double* __restrict__ k4_out = A.K1[rc.cur ^ 1];
 #pragma unroll 1
       for (int v = 0; v < NV; ++v) {
-        if (v + 1 < NV) {
-#pragma unroll
-          for (int u = 0; u < NIT; ++u)
-            if (okk[u]) {
-              const long long o = (long long)(v + 1) * Nd;  // per-field base, 32-bit item offset
-              const int g = gof[u];
-              if (SGNB_INB(o + g, NV * Nd)) { nu[u] = __ldcs(&(I.u + o)[g]); n1[u] = __ldcs(&(I.k1 + o)[g]); n2[u] = __ldcs(&(I.k2 + o)[g]); n3[u] = __ldcs(&(I.k3 + o)[g]); }
-            }
-        }
+        const long long o = (long long)v * Nd;  // per-field base, 32-bit item offset
+        double c0[NIT], c1[NIT], c2[NIT];
 #pragma unroll
         for (int u = 0; u < NIT; ++u)
-          if (okk[u]) {
-            const double k4 = (&S.G[v][0][0])[sof[u]];
-            if (SGNB_INB(gof[u], Nd)) __stcs(&(outp + (long long)v * Nd)[gof[u]], k4);
-            // scaled embedded error, src/solver/rk.cpp:118-128; the candidate uNew is
-            // still in the tile (the passes only read S.U)
-            const double dt = I.dt;
-            const double un = (&S.U[v][0][0])[sof[u]];
-            const double uEmb = uu[u] + dt * (7.0 / 24.0 * c1[u] + 0.25 * c2[u] + 1.0 / 3.0 * c3[u] +
-                                              0.125 * k4);
-            const double e = un - uEmb;
-            const double au = fabs(uu[u]), an = fabs(un);
-            const double sc = atol + rtol * (au < an ? an : au);
-            double rr;
-            if constexpr (EXACT) {
-              rr = e / sc;
+          if (okk[u] && SGNB_INB(o + gof[u], NV * Nd)) {
+            const int g = gof[u];
+            c0[u] = __ldcs(&(u0 + o)[g]);
+            if constexpr (MODE == MODE_CAND) {
+              c1[u] = __ldcs(&(k1 + o)[g]);
+              c2[u] = __ldcs(&(k2 + o)[g]);
             } else {
-              // the fast mode's reciprocal (a few ulp) where sc is a normal number
-              rr = sc >= 2.2250738585072014e-308 ? e * fast_rcp(sc) : e / sc;
+              c1[u] = __ldcs(&(part + o)[g]);
             }
-            esum += rr * rr;
-            const double ar = fabs(rr);
-            emax = emax < ar ? ar : emax;
-            enan |= (rr != rr);
           }
 #pragma unroll
-        for (int u = 0; u < NIT; ++u) {
-          uu[u] = nu[u]; c1[u] = n1[u]; c2[u] = n2[u]; c3[u] = n3[u];
-        }
+        for (int u = 0; u < NIT; ++u)
+          if (okk[u] && SGNB_INB(o + gof[u], NV * Nd)) {
+            const int g = gof[u];
+            const double kk = (&S.G[v][0][0])[sof[u]];
+            if constexpr (MODE == MODE_CAND) {
+              __stcs(&(un_out + o)[g], fsal_finish(c0[u], fsal_part(c1[u], c2[u]), kk, dt));
+              __stcs(&(part_out + o)[g], emb_part(c1[u], c2[u], kk));
+            } else {
+              __stcs(&(k4_out + o)[g], kk);
+              // scaled embedded error, src/solver/rk.cpp:118-128; the candidate uNew is still
+              // in the tile (the passes only read S.U)
+              const double un = (&S.U[v][0][0])[sof[u]];
+              const double uEmb = c0[u] + dt * (c1[u] + 0.125 * kk);
+              const double e = un - uEmb;
+              const double au = fabs(c0[u]), an = fabs(un);
+              const double sc = rc.atol + rc.rtol * (au < an ? an : au);
+              double rr;
+              if constexpr (EXACT) {
+                rr = e / sc;
+              } else {
+                // the fast mode's reciprocal (a few ulp) where sc is a normal number
+                rr = sc >= 2.2250738585072014e-308 ? e * fast_rcp(sc) : e / sc;
+              }
+              esum += rr * rr;
+              const double ar = fabs(rr);
+              emax = emax < ar ? ar : emax;
+              enan |= (rr != rr);
+            }
+          }
       }
     }
   }
-  if constexpr (GHOST && MODE == MODE_STAGE) {
+  if constexpr (GHOST && AXPY) {
     // Fused edge exchange: the slab-edge tiles form the next stage's input at their edge
     // nodes (a = 0 of the first column, a = 4 of the last) from this launch's result and
     // store it straight into the neighbours' ghost arrays, [field][row][node], while the
@@ -1012,39 +982,13 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
         const double kout = S.G[v][TX * iy + ixe][node];
         const long long ge = (long long)v * Ny * NP + (long long)(ey0 + iy) * NP + t;
         if (!SGNB_INB(g, NV * Nd) || !SGNB_INB(ge, (long long)NV * Ny * NP)) continue;
-        const double val = A.kin_k2 == 0 ? stage_axpy(u0[g], 0.75 * dt, kout)
-                                          : fsal_finish(u0[g], fsal_part(k1[g], k2[g]), kout, dt);
+        const double val = MODE == MODE_STAGE ? stage_axpy(u0[g], 0.75 * dt, kout)
+                                              : fsal_finish(u0[g], fsal_part(k1[g], k2[g]), kout, dt);
         (side == 0 ? C.edgeL : C.edgeR)[ge] = val;
       }
     }
   }
-  if constexpr (MODE == MODE_FSAL) {
-    // deterministic block reduction: fixed shuffle tree, then warps in order
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      esum += __shfl_down_sync(0xffffffffu, esum, off);
-      const double om = __shfl_down_sync(0xffffffffu, emax, off);
-      emax = emax < om ? om : emax;
-      enan |= __shfl_down_sync(0xffffffffu, enan, off);
-    }
-    if (lane == 0) {
-      S.red[warp][0] = esum;
-      S.red[warp][1] = emax;
-      S.red[warp][2] = (double)enan;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double s = 0.0, m = 0.0, n = 0.0;
-      for (int w = 0; w < NWARP; ++w) {
-        s += S.red[w][0];
-        m = m < S.red[w][1] ? S.red[w][1] : m;
-        n += S.red[w][2];
-      }
-      A.partials[3 * blk + 0] = s;
-      A.partials[3 * blk + 1] = m;
-      A.partials[3 * blk + 2] = n;
-    }
-  }
+  if constexpr (MODE == MODE_FSAL) reduce_error(esum, emax, enan, S.red, A.partials, blk);
 }
 
 
@@ -1097,9 +1041,7 @@ __global__ void __launch_bounds__(256) k_traces(const RhsConsts C, const StageAr
   }
   I.u = A.U[cur];
   I.k = A.kin_k2 ? A.K2 : A.K1[cur];
-  I.k1 = A.K1[cur];
-  I.k2 = A.K2;
-  I.k3 = A.K3;
+  if constexpr (MODE == MODE_FSAL) I.in = A.U[cur ^ 1];
   const int dir = (int)(q / (ne * NP));
   const long long r = q - dir * ne * NP;
   const long long e = r / NP;
@@ -1115,57 +1057,6 @@ __global__ void __launch_bounds__(256) k_traces(const RhsConsts C, const StageAr
     const long long hi = ((long long)((fl + 1) * NV + v) * ne + e) * NP + t;
     if (SGNB_INB(lo, 100 * ne)) C.tr[lo] = face_trace(C.lL, line, 1);
     if (SGNB_INB(hi, 100 * ne)) C.tr[hi] = face_trace(C.lR, line, 1);
-  }
-}
-
-// Batched form: one launch per stage walks the tiles of many independent instances
-// (the work list tile_inst / tile_start), each with its own constants, buffers and
-// controller. The instance's constants and buffer pointers are copied into shared
-// memory once per tile. PERSIST: a fixed grid of CTAs loops over the work list;
-// otherwise one CTA per tile (no loop: the compiler then keeps nothing live from one tile
-// to the next, which the loop costs in spilled registers).
-template <int MODE, bool EXACT, int TX_, int TY_>
-__device__ __forceinline__ void batch_tile(const BatchArgs& B, long long t,
-                                           typename Tile<TX_, TY_, EXACT>::Smem& S, RhsConsts& Cs,
-                                           StageArgs& As) {
-  const int inst = B.tile_inst[t];
-  const long long lt = t - B.tile_start[inst];
-  __syncthreads();  // the previous tile is done with Cs / As
-  {
-    // both blocks' loads in flight before the first store (one round trip per tile)
-    block_copy2<(int)(sizeof(RhsConsts) / 4), (int)(sizeof(StageArgs) / 4), NTHR>(
-        reinterpret_cast<unsigned*>(&Cs), reinterpret_cast<const unsigned*>(B.consts + inst),
-        reinterpret_cast<unsigned*>(&As), reinterpret_cast<const unsigned*>(B.args + inst));
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    As.kin_k2 = B.kin_k2;
-    As.coef = B.coef;
-    if (MODE == MODE_STAGE) As.out = B.kin_k2 ? As.K3 : As.K2;
-  }
-  __syncthreads();
-  const int ntx = (Cs.Nx + TX_ - 1) / TX_;
-  // volatile views: per-instance values are re-read from shared memory at each use
-  // rather than held in registers through the passes
-  fused_tile<MODE, EXACT, TX_, TY_>(static_cast<const volatile RhsConsts&>(Cs), B.tables,
-                                    static_cast<const volatile StageArgs&>(As),
-                                    (int)(lt % ntx), (int)(lt / ntx), lt, S);
-}
-
-template <int MODE, bool EXACT, int TX_, int TY_, bool PERSIST>
-__global__ void __launch_bounds__(NTHR, 2) k_fused_batch(const BatchArgs B) {
-  // FR tables come from the kernel parameters (constant bank): the same for every
-  // instance (P = 4 GLL)
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  using T = Tile<TX_, TY_, EXACT>;
-  typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_raw);
-  __shared__ RhsConsts Cs;
-  __shared__ StageArgs As;
-  if constexpr (PERSIST) {
-    for (long long t = blockIdx.x; t < B.ntiles; t += gridDim.x)
-      batch_tile<MODE, EXACT, TX_, TY_>(B, t, S, Cs, As);
-  } else {
-    if ((long long)blockIdx.x < B.ntiles) batch_tile<MODE, EXACT, TX_, TY_>(B, blockIdx.x, S, Cs, As);
   }
 }
 

@@ -1,0 +1,143 @@
+// sgnb_kernels_batch.cu -- batched kernels of the fast and mixed modes on GLL points: one
+// launch per stage over the tiles of many independent instances. Built with -fmad=true.
+#include "sgnb_kernels_line.cuh"
+
+namespace sgnb {
+namespace dev {
+
+// Batched form: one launch per stage walks the tiles of many independent instances
+// (the work list tile_inst / tile_start), each with its own constants, buffers and
+// controller. The instance's constants and buffer pointers are copied into shared
+// memory once per tile. PERSIST: a fixed grid of CTAs loops over the work list;
+// otherwise one CTA per tile (no loop: the compiler then keeps nothing live from one tile
+// to the next, which the loop costs in spilled registers).
+template <int MODE, int TX_, int TY_, class BA>
+__device__ __forceinline__ void batch_tile(const BA& B, long long t,
+                                           typename LineTile<TX_, TY_>::Smem& S, RhsConsts& Cs,
+                                           typename BA::Args& As) {
+  using Args = typename BA::Args;
+  const int inst = B.tile_inst[t];
+  const long long lt = t - B.tile_start[inst];
+  __syncthreads();  // the previous tile is done with Cs / As
+  {
+    // both blocks' loads in flight before the first store (one round trip per tile)
+    block_copy2<(int)(sizeof(RhsConsts) / 4), (int)(sizeof(Args) / 4), NTHR>(
+        reinterpret_cast<unsigned*>(&Cs), reinterpret_cast<const unsigned*>(B.consts + inst),
+        reinterpret_cast<unsigned*>(&As), reinterpret_cast<const unsigned*>(B.args + inst));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    As.kin_k2 = B.kin_k2;
+    As.coef = B.coef;
+    if (MODE == MODE_STAGE) As.out = As.K2;
+  }
+  __syncthreads();
+  const int ntx = (Cs.Nx + TX_ - 1) / TX_;
+  // volatile views: per-instance values are re-read from shared memory at each use
+  // rather than held in registers through the passes
+  line_tile<MODE, TX_, TY_, false, false, typename Args::K>(
+      static_cast<const volatile RhsConsts&>(Cs), B.tables.eo, static_cast<const volatile Args&>(As),
+      (int)(lt % ntx), (int)(lt / ntx), lt, Cs.bulk >= (sizeof(typename Args::K) == 4 ? 2 : 1), S);
+}
+
+template <int MODE, int TX_, int TY_, bool PERSIST, class BA>
+__global__ void __launch_bounds__(NTHR, PERSIST || TX_ == 16 ? 2 : 3) k_line_batch(const BA B) {
+  // FR tables come from the kernel parameters (constant bank): the same for every
+  // instance (P = 4 GLL)
+  extern __shared__ __align__(128) unsigned char smem_batch[];
+  using T = LineTile<TX_, TY_>;
+  typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_batch);
+  __shared__ RhsConsts Cs;
+  __shared__ typename BA::Args As;
+  if constexpr (PERSIST) {
+    for (long long t = blockIdx.x; t < B.ntiles; t += gridDim.x)
+      batch_tile<MODE, TX_, TY_>(B, t, S, Cs, As);
+  } else {
+    if ((long long)blockIdx.x < B.ntiles) batch_tile<MODE, TX_, TY_>(B, blockIdx.x, S, Cs, As);
+  }
+}
+
+template <int MODE, int TXs, int TYs, class BA>
+static cudaError_t launch_b(int blocks, const BA& B, cudaStream_t s) {
+  const size_t smem = sizeof(typename LineTile<TXs, TYs>::Smem);
+  if (blocks > 0) {
+    k_line_batch<MODE, TXs, TYs, true, BA><<<blocks, NTHR, smem, s>>>(B);
+  } else {
+    if (B.ntiles < 1 || B.ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;
+    k_line_batch<MODE, TXs, TYs, false, BA><<<(unsigned)B.ntiles, NTHR, smem, s>>>(B);
+  }
+  return cudaGetLastError();
+}
+
+template <int TXs, int TYs, class BA>
+static cudaError_t launch_shape(int mode, int blocks, const BA& B, cudaStream_t s) {
+  switch (mode) {
+    case MODE_RHS: return launch_b<MODE_RHS, TXs, TYs>(blocks, B, s);
+    case MODE_STAGE: return launch_b<MODE_STAGE, TXs, TYs>(blocks, B, s);
+    case MODE_FSAL: return launch_b<MODE_FSAL, TXs, TYs>(blocks, B, s);
+    case MODE_CAND: return launch_b<MODE_CAND, TXs, TYs>(blocks, B, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchArgs& B,
+                               cudaStream_t s) {
+  switch (shape_id) {
+    case 0: return launch_shape<8, 4>(mode, blocks, B, s);
+    case 1: return launch_shape<16, 2>(mode, blocks, B, s);
+    case 2: return launch_shape<4, 8>(mode, blocks, B, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s) {
+  return launch_shape<8, 4>(mode, blocks, B, s);
+}
+
+int batch_tile_tx(int shape_id) { return shape_id == 1 ? 16 : (shape_id == 2 ? 4 : 8); }
+
+template <int MODE, int TXs, int TYs, class BA>
+static cudaError_t prepare_mode() {
+  const int bytes = (int)sizeof(typename LineTile<TXs, TYs>::Smem);
+  cudaError_t e = cudaFuncSetAttribute(k_line_batch<MODE, TXs, TYs, true, BA>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_line_batch<MODE, TXs, TYs, false, BA>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+template <int TXs, int TYs, class BA>
+static cudaError_t prepare_shape() {
+  cudaError_t e = prepare_mode<MODE_RHS, TXs, TYs, BA>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE, TXs, TYs, BA>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL, TXs, TYs, BA>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_CAND, TXs, TYs, BA>();
+  return e;
+}
+
+cudaError_t prepare_fused_batch() {
+  cudaError_t e = prepare_shape<8, 4, BatchArgs>();
+  if (e == cudaSuccess) e = prepare_shape<16, 2, BatchArgs>();
+  if (e == cudaSuccess) e = prepare_shape<4, 8, BatchArgs>();
+  if (e == cudaSuccess) e = prepare_shape<8, 4, BatchArgsM>();
+  return e;
+}
+
+// The checked build's out-of-range count of this translation unit's kernels (reset: then
+// zero it); cudaErrorNotSupported in the normal build.
+cudaError_t read_oob_batch(unsigned long long* out, bool reset) {
+#ifdef SGNB_CHECKED
+  cudaError_t e = cudaMemcpyFromSymbol(out, g_sgnb_oob, sizeof(*out));
+  if (e == cudaSuccess && reset) {
+    const unsigned long long z = 0;
+    e = cudaMemcpyToSymbol(g_sgnb_oob, &z, sizeof(z));
+  }
+  return e;
+#else
+  *out = 0;
+  (void)reset;
+  return cudaErrorNotSupported;
+#endif
+}
+}  // namespace dev
+}  // namespace sgnb

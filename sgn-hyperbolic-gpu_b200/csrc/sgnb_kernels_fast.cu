@@ -1,16 +1,31 @@
-// sgnb_kernels_fast.cu -- fused kernels in the fast arithmetic mode.
-// Built with -fmad=true: FMA contraction, reciprocals of h and of the Jacobians.
-// Agrees with the reference to round-off (relative 1e-13 per field is the test bound).
+// sgnb_kernels_fast.cu -- the fast arithmetic mode's dispatch, its Gauss-point kernels and the
+// slab packs. Built with -fmad=true: FMA contraction, reciprocals of h and of the Jacobians.
+// Agrees with the reference to round-off (relative 1e-13 per field is the test bound). The
+// kernels on GLL points are in sgnb_kernels_line.cu.
 #define SGNB_EXACT false
 #include "sgnb_kernels_inst.cuh"
 
 namespace sgnb {
 namespace dev {
-cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s,
-                              const TileMaps* M) {
-  return launch_any(mode, C, A, s, M);
+cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
+  // FR tables without the reflection symmetry of the GLL ones (given by the caller): the exact
+  // mode's kernels, which take any tables
+  if (!C.gauss && !C.sym) return launch_fused_exact(mode, C, A, s, nullptr);
+  if (!C.gauss) return launch_line(mode, C, A, s);
+  switch (mode) {
+    case MODE_RHS: return launch_gauss<MODE_RHS>(C, A, s);
+    case MODE_STAGE: return launch_gauss<MODE_STAGE>(C, A, s);
+    case MODE_FSAL: return launch_gauss<MODE_FSAL>(C, A, s);
+    case MODE_CAND: return launch_gauss<MODE_CAND>(C, A, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
-cudaError_t prepare_fused_fast() { return prepare_all(); }
+cudaError_t prepare_fused_fast() {
+  cudaError_t e = prepare_variant<false, false, true>();
+  if (e == cudaSuccess) e = prepare_variant<true, false, true>();
+  if (e == cudaSuccess) e = prepare_line();
+  return e;
+}
 
 // The checked build's out-of-range count of this translation unit's kernels (reset: then
 // zero it); cudaErrorNotSupported in the normal build.
@@ -68,7 +83,7 @@ __global__ void k_pack_ghosts(int mode, const RhsConsts C, const StageArgs A, do
       const double* k = A.kin_k2 ? A.K2 : A.K1[cur];
       val = stage_axpy(A.U[cur][g], A.coef * dt, k[g]);
     } else {
-      val = fsal_finish(A.U[cur][g], fsal_part(A.K1[cur][g], A.K2[g]), A.K3[g], dt);
+      val = A.U[cur ^ 1][g];
     }
   }
   (side == 0 ? sendL : sendR)[r] = val;
@@ -83,63 +98,5 @@ cudaError_t launch_pack_ghosts(int mode, const RhsConsts& C, const StageArgs& A,
   return cudaGetLastError();
 }
 
-template <int MODE, int TXs, int TYs>
-static cudaError_t launch_b(int blocks, const BatchArgs& B, cudaStream_t s) {
-  const size_t smem = sizeof(typename Tile<TXs, TYs, false>::Smem);
-  if (blocks > 0) {
-    k_fused_batch<MODE, false, TXs, TYs, true><<<blocks, NTHR, smem, s>>>(B);
-  } else {
-    if (B.ntiles < 1 || B.ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    k_fused_batch<MODE, false, TXs, TYs, false><<<(unsigned)B.ntiles, NTHR, smem, s>>>(B);
-  }
-  return cudaGetLastError();
-}
-
-template <int TXs, int TYs>
-static cudaError_t launch_shape(int mode, int blocks, const BatchArgs& B, cudaStream_t s) {
-  switch (mode) {
-    case MODE_RHS: return launch_b<MODE_RHS, TXs, TYs>(blocks, B, s);
-    case MODE_STAGE: return launch_b<MODE_STAGE, TXs, TYs>(blocks, B, s);
-    case MODE_FSAL: return launch_b<MODE_FSAL, TXs, TYs>(blocks, B, s);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchArgs& B,
-                               cudaStream_t s) {
-  switch (shape_id) {
-    case 0: return launch_shape<8, 4>(mode, blocks, B, s);
-    case 1: return launch_shape<16, 2>(mode, blocks, B, s);
-    case 2: return launch_shape<4, 8>(mode, blocks, B, s);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-int batch_tile_tx(int shape_id) { return shape_id == 1 ? 16 : (shape_id == 2 ? 4 : 8); }
-
-template <int MODE, int TXs, int TYs>
-static cudaError_t prepare_mode() {
-  const int bytes = (int)sizeof(typename Tile<TXs, TYs, false>::Smem);
-  cudaError_t e = cudaFuncSetAttribute(k_fused_batch<MODE, false, TXs, TYs, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_fused_batch<MODE, false, TXs, TYs, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
-template <int TXs, int TYs>
-static cudaError_t prepare_shape() {
-  cudaError_t e = prepare_mode<MODE_RHS, TXs, TYs>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE, TXs, TYs>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL, TXs, TYs>();
-  return e;
-}
-
-cudaError_t prepare_fused_batch() {
-  cudaError_t e = prepare_shape<8, 4>();
-  if (e == cudaSuccess) e = prepare_shape<16, 2>();
-  if (e == cudaSuccess) e = prepare_shape<4, 8>();
-  return e;
-}
 }  // namespace dev
 }  // namespace sgnb

@@ -1,0 +1,93 @@
+// sgnb_kernels_line.cu -- single-instance and slab kernels of the fast arithmetic mode on GLL
+// points, and the mixed mode's. Built with -fmad=true.
+#include "sgnb_kernels_line.cuh"
+
+namespace sgnb {
+namespace dev {
+
+// bulk row copies need aligned buffers besides aligned rows (C.bulk): the right-hand side's
+// input and output are the caller's
+template <class Args>
+static int bulk_rows(const RhsConsts& C, const Args& A, const void* outd) {
+  auto ok = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+  return C.bulk >= (sizeof(typename Args::K) == 4 ? 2 : 1) && ok(A.in) && ok(A.out) && ok(outd) &&
+         ok(A.U[0]) && ok(A.U[1]) && ok(A.K1[0]) && ok(A.K1[1]) && ok(A.K2) && ok(A.K3) && ok(C.Hnod);
+}
+
+template <int MODE, bool FRIC, bool GHOST, class Args>
+static cudaError_t launch_variant(const RhsConsts& C, const Args& A, int bulk, cudaStream_t s) {
+  const dim3 grid((C.Nx + 7) / 8, (C.Ny + 3) / 4);
+  k_line<MODE, FRIC, GHOST, Args><<<grid, NTHR, sizeof(LineTile<8, 4>::Smem), s>>>(C, A, bulk);
+  return cudaGetLastError();
+}
+
+template <int MODE>
+static cudaError_t launch_mode(const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
+  const int bulk = bulk_rows(C, A, nullptr);
+  const bool ghost = C.ghostL != nullptr || C.ghostR != nullptr;
+  if (C.manning)
+    return ghost ? launch_variant<MODE, true, true>(C, A, bulk, s) : launch_variant<MODE, true, false>(C, A, bulk, s);
+  return ghost ? launch_variant<MODE, false, true>(C, A, bulk, s) : launch_variant<MODE, false, false>(C, A, bulk, s);
+}
+template <int MODE>
+static cudaError_t launch_mode(const RhsConsts& C, const StageArgsM& A, cudaStream_t s) {
+  const int bulk = bulk_rows(C, A, A.outd);
+  return C.manning ? launch_variant<MODE, true, false>(C, A, bulk, s) : launch_variant<MODE, false, false>(C, A, bulk, s);
+}
+
+template <class Args>
+static cudaError_t launch_any(int mode, const RhsConsts& C, const Args& A, cudaStream_t s) {
+  switch (mode) {
+    case MODE_RHS: return launch_mode<MODE_RHS>(C, A, s);
+    case MODE_STAGE: return launch_mode<MODE_STAGE>(C, A, s);
+    case MODE_FSAL: return launch_mode<MODE_FSAL>(C, A, s);
+    case MODE_CAND: return launch_mode<MODE_CAND>(C, A, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
+  return launch_any(mode, C, A, s);
+}
+cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgsM& A, cudaStream_t s) {
+  return launch_any(mode, C, A, s);
+}
+
+template <int MODE>
+static cudaError_t prepare_mode() {
+  const int bytes = (int)sizeof(LineTile<8, 4>::Smem);
+  const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_line<MODE, false, false, StageArgs>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, false, StageArgs>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, false, true, StageArgs>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, true, StageArgs>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, false, false, StageArgsM>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, false, StageArgsM>, at, bytes);
+  return e;
+}
+
+cudaError_t prepare_line() {
+  cudaError_t e = prepare_mode<MODE_RHS>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_CAND>();
+  return e;
+}
+
+// The checked build's out-of-range count of this translation unit's kernels (reset: then
+// zero it); cudaErrorNotSupported in the normal build.
+cudaError_t read_oob_line(unsigned long long* out, bool reset) {
+#ifdef SGNB_CHECKED
+  cudaError_t e = cudaMemcpyFromSymbol(out, g_sgnb_oob, sizeof(*out));
+  if (e == cudaSuccess && reset) {
+    const unsigned long long z = 0;
+    e = cudaMemcpyToSymbol(g_sgnb_oob, &z, sizeof(z));
+  }
+  return e;
+#else
+  *out = 0;
+  (void)reset;
+  return cudaErrorNotSupported;
+#endif
+}
+}  // namespace dev
+}  // namespace sgnb
