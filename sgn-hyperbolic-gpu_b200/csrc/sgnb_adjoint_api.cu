@@ -28,7 +28,6 @@ struct sgnb_adj {
   int K = 0, ng = 0, nseg = 0;
   std::vector<double> dts;
   std::vector<long long> gnodes;
-  std::vector<double> means;  // of the last forward
   bool haveForward = false;
   double* block = nullptr;    // every device buffer below lives in this allocation
   double* dts_dev = nullptr;
@@ -120,29 +119,14 @@ cudaError_t download_stats(const sgnb_ctx* c, const GatherArgs& G, Bathymetry& b
   return cudaSuccess;
 }
 
-// Replaces the context's depth statics.
-cudaError_t upload_statics(sgnb_ctx* c, const Bathymetry& b) {
-  auto put = [&](const std::vector<double>& v, const double* dst) {
-    return cudaMemcpyAsync(const_cast<double*>(dst), v.data(), v.size() * sizeof(double),
-                           cudaMemcpyHostToDevice, c->stream);
-  };
-  cudaError_t e = put(b.Hnod, c->C.Hnod);
-  if (e == cudaSuccess) e = put(b.Hx, c->C.Hx);
-  if (e == cudaSuccess) e = put(b.Hy, c->C.Hy);
-  if (e == cudaSuccess) e = put(b.HfX, c->C.HfX);
-  if (e == cudaSuccess) e = put(b.HfY, c->C.HfY);
-  if (e == cudaSuccess) e = put(b.HfXEnd, c->C.HfXEnd);
-  if (e == cudaSuccess) e = put(b.HfYEnd, c->C.HfYEnd);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  return e;
-}
-
-std::vector<double> cell_params(const sgnb_ctx* c, const double* means) {
-  const long long nm = (long long)c->desc.Nx * c->desc.Ny;
-  std::vector<double> p(4 + nm);
-  p[0] = c->desc.Nx; p[1] = c->desc.Ny; p[2] = c->desc.Lx; p[3] = c->desc.Ly;
-  std::memcpy(p.data() + 4, means, nm * sizeof(double));
-  return p;
+CellGrid grid_of(const sgnb_ctx* c) {
+  CellGrid g{};
+  g.Nx = c->desc.Nx; g.Ny = c->desc.Ny;
+  g.Lx = c->desc.Lx; g.Ly = c->desc.Ly;
+  g.hx = c->mesh.hx; g.hy = c->mesh.hy;
+  for (int k = 0; k < 5; ++k) g.nodes[k] = c->tab.nodes[k];
+  for (int k = 0; k < 25; ++k) g.D[k] = c->tab.D[k];
+  return g;
 }
 
 // One BS3(2) step u -> out at step index n (dt read from the device list).
@@ -245,16 +229,15 @@ int sgnb_adj_forward(sgnb_adj* a, const double* means, const double* eta0, doubl
   SGNB_ACU(c, cudaSetDevice(c->device));
   cudaStream_t s = c->stream;
   const long long Nd = c->Nd, S = c->ntot;
-  // statics from the element means (host set-up, as at context creation)
-  a->means.assign(means, means + (long long)c->desc.Nx * c->desc.Ny);
-  const std::vector<double> p = cell_params(c, means);
-  Bathymetry b;
-  bathymetry(c->mesh, c->tab, 5, p.data(), b);
-  SGNB_ACU(c, upload_statics(c, b));
-  // u0 = (H + eta0, 0, 0, 0, 0)
-  std::vector<double> u0(S, 0.0);
-  for (long long i = 0; i < Nd; ++i) u0[i] = b.Hnod[i] + eta0[i];
-  SGNB_ACU(c, cudaMemcpyAsync(a->u[0], u0.data(), S * sizeof(double), cudaMemcpyHostToDevice, s));
+  // statics from the element means and u0 = (H + eta0, 0, 0, 0, 0), in scratch that the run
+  // does not use yet
+  const long long nm = (long long)c->desc.Nx * c->desc.Ny;
+  SGNB_ACU(c, cudaMemcpyAsync(a->y2b, means, nm * sizeof(double), cudaMemcpyHostToDevice, s));
+  SGNB_ACU(c, cudaMemcpyAsync(a->y3b, eta0, Nd * sizeof(double), cudaMemcpyHostToDevice, s));
+  auto rw = [](const double* q) { return const_cast<double*>(q); };
+  SGNB_ACU(c, dev::launch_cells_statics(grid_of(c), a->y2b, a->y3b, rw(c->C.Hnod), rw(c->C.Hx), rw(c->C.Hy),
+                                        rw(c->C.HfX), rw(c->C.HfY), rw(c->C.HfXEnd), rw(c->C.HfYEnd),
+                                        a->u[0], s));
   int cur = 0;
   for (long long n = 0; n < a->N; ++n) {
     if (n % a->K == 0)
@@ -340,19 +323,15 @@ int sgnb_adj_vjp(sgnb_adj* a, const double* eta_bar, double* grad_means, double*
     }
   }
   // lam = dL/du0; h0 = H + eta0
-  std::vector<double> lh(Nd);
-  SGNB_ACU(c, cudaMemcpyAsync(lh.data(), lam, Nd * sizeof(double), cudaMemcpyDeviceToHost, s));
-  SGNB_ACU(c, cudaStreamSynchronize(s));
-  if (grad_eta0) std::memcpy(grad_eta0, lh.data(), Nd * sizeof(double));
+  if (grad_eta0)
+    SGNB_ACU(c, cudaMemcpyAsync(grad_eta0, lam, Nd * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (grad_means) {
-    Bathymetry bar;
-    SGNB_ACU(c, download_stats(c, a->G, bar));
-    for (long long i = 0; i < Nd; ++i) bar.Hnod[i] += lh[i];
-    for (long long n = 0; n < a->N; ++n)
-      for (int g = 0; g < ng; ++g) bar.Hnod[a->gnodes[g]] -= eta_bar[n * ng + g];  // eta = h - H
-    const std::vector<double> p = cell_params(c, a->means.data());
-    cells_transpose(c->mesh, c->tab, p.data(), bar, grad_means);
+    const long long nm = (long long)c->desc.Nx * c->desc.Ny;
+    SGNB_ACU(c, dev::launch_cells_back(grid_of(c), a->G, lam, a->gnodes_dev, ng, a->N, a->etab_dev, a->y3b,
+                                       a->y2b, s));
+    SGNB_ACU(c, cudaMemcpyAsync(grad_means, a->y2b, nm * sizeof(double), cudaMemcpyDeviceToHost, s));
   }
+  SGNB_ACU(c, cudaStreamSynchronize(s));
   return SGNB_OK;
 }
 

@@ -297,6 +297,14 @@ struct BatchArgsM {
   double coef;
 };
 
+// The mesh and tables of the depth interpolant of element means (adjoint), Nx x Ny cells that
+// are the mesh's elements.
+struct CellGrid {
+  int Nx, Ny;
+  double Lx, Ly, hx, hy;
+  double nodes[5], D[25];
+};
+
 namespace dev {
 // Out-of-range access counts of the checked build, per translation unit.
 cudaError_t read_oob_exact(unsigned long long* out, bool reset);
@@ -324,6 +332,16 @@ cudaError_t launch_controller_slabs(CtrlState* c, const SlabPartials& L, long lo
 // 1: intermediate stage (kin_k2, coef of A); 2: the candidate that the third stage left.
 cudaError_t launch_pack_ghosts(int mode, const RhsConsts& C, const StageArgs& A, double* sendL,
                                double* sendR, cudaStream_t s);
+
+// Depth statics of the means (the bits of the host set-up) and the state (H + eta0, 0, 0, 0, 0).
+cudaError_t launch_cells_statics(const CellGrid& g, const double* means, const double* eta0, double* Hnod,
+                                 double* Hx, double* Hy, double* HfX, double* HfY, double* HfXEnd,
+                                 double* HfYEnd, double* u0, cudaStream_t s);
+// Their transpose: from the statics' cotangents G, the initial depth's lam (Nd) and the gauge
+// records' etab [nsteps][ng] to the gradient of the means. Hb: scratch (Nd).
+cudaError_t launch_cells_back(const CellGrid& g, const GatherArgs& G, const double* lam,
+                              const long long* gauges, int ng, long long nsteps, const double* etab,
+                              double* Hb, double* grad, cudaStream_t s);
 
 // Adjoint kernels (FP64, fast arithmetic).
 cudaError_t launch_vjp_rhs(const RhsConsts& C, const FrTablesDev& T, const VjpArgs& A,

@@ -40,9 +40,5 @@ void bathymetry(const Mesh& m, const FrTables& t, int kind, const double* p, Bat
 // depth tile instead of reading them.
 void depth_gradients(const Mesh& m, const FrTables& t, const double* Hnod, double* Hx,
                      double* Hy);
-// Transpose of bathymetry() for kind 5 (cell means p = {Mx, My, Lx, Ly, means...}):
-// cotangents of every static (bar) -> cotangent of the Mx * My means.
-void cells_transpose(const Mesh& m, const FrTables& t, const double* p, const Bathymetry& bar,
-                     double* means_bar);
 
 }  // namespace sgnb
