@@ -15,18 +15,86 @@ constexpr int kCtrlThreads = 256;
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }  // std::max
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }  // std::min
 
+// The decision of one attempt. errPow = errNorm^-alpha; prevPow = errPrev^beta with the error of
+// the last accepted attempt, this one included.
+__device__ __forceinline__ void decide(CtrlState* c, double errNorm, double errMax, bool bad,
+                                       double errPow, double prevPow) {
+  if (c->log && c->attempts < c->logCap) {
+    double* row = c->log + 4 * c->attempts;
+    row[0] = c->t;
+    row[1] = c->dt;
+    row[2] = errNorm;
+    row[3] = (c->frozen || errNorm <= 1.0) ? 1.0 : 0.0;
+  }
+  c->attempts += 1;
+  c->rhsEvals += 3;
+  c->errLast = errNorm;
+  if (c->frozen) {  // replay of a given dt sequence: every step is taken
+    c->t += c->dt;
+    c->cur ^= 1;
+    c->accepted += 1;
+    c->tReached = c->t;
+    c->dtLast = c->dt;
+    c->maxNormLast = errMax;
+    if (bad) { c->done = 3; return; }
+    if (c->accepted >= c->nList) { c->done = 1; return; }
+    c->dt = c->dtList[c->accepted];
+    return;
+  }
+  bool stop = false;
+  if (errNorm <= 1.0) {
+    c->t += c->dt;
+    c->cur ^= 1;  // uNew becomes u and k4 becomes k1 (FSAL)
+    c->accepted += 1;
+    c->tReached = c->t;
+    c->dtLast = c->dt;
+    c->maxNormLast = errMax;
+    c->errPrev = errNorm;
+    stop = c->maxAccepted > 0 && c->accepted >= c->maxAccepted;
+  } else {
+    c->rejected += 1;
+  }
+  if (bad) { c->done = 3; return; }  // the reference would loop forever here
+  double fac = c->safety * errPow * prevPow;
+  fac = (fac < c->facMin) ? c->facMin : ((c->facMax < fac) ? c->facMax : fac);
+  double dtNext = c->dt * fac;
+  dtNext = dmin(dtNext, c->dtMax);
+  if (dtNext < c->dtMin) {
+    c->done = 2;
+    c->dtLast = dtNext;
+    return;
+  }
+  c->dt = dtNext;
+  if (stop) { c->done = 1; return; }  // fixed number of accepted steps reached
+  const double tEnd = c->tEnd;
+  if (!(c->t < tEnd - 1e-15 * dmax(1.0, fabs(tEnd)))) { c->done = 1; return; }
+  if (c->t + c->dt > tEnd) c->dt = tEnd - c->t;
+}
+
 // One adaptive attempt has just written its per-CTA error partials. Reduce them in a
 // fixed order (so reruns are bit-reproducible), then apply the reference controller:
 // accept if the RMS scaled error <= 1 (rk.cpp:129-142), PI update clamped to
 // [facMin, facMax] (:148-152), dtMin abort (:155-160), and the loop test and the
 // end-time clip of the next attempt (:95-97).
-// row(b): the three partials (sum r^2, max |r|, NaN count) of error block b.
+// row(b): the three partials (sum r^2, max |r|, NaN count) of error block b. Returns, on thread
+// 0, whether the run goes on (and this launch of the device-side loop may go on with it).
+//
+// Bound by latency: one block, and what follows the reduction is a serial chain. So the state
+// is read at the start, with the partials, and written once at the end (it lives in shared
+// memory in between: field by field from global memory the chain had a dozen L2 round trips),
+// and the two powers of the step-size factor run on two warps.
 template <class Row>
-__device__ __forceinline__ void controller_core(CtrlState* c, const Row& row, long long nblk,
+__device__ __forceinline__ bool controller_core(CtrlState* cg, const Row& row, long long nblk,
                                                 long long n) {
   __shared__ double ss[kCtrlThreads], sm[kCtrlThreads], sn[kCtrlThreads];
-  if (c->done) return;
+  __shared__ __align__(8) CtrlState state;
+  __shared__ double prevPow;
+  constexpr int W = sizeof(CtrlState) / 8;
+  static_assert(sizeof(CtrlState) % 8 == 0 && W <= kCtrlThreads, "copied by one word per thread");
+  if (cg->done) return false;
   const int t = threadIdx.x;
+  CtrlState* const c = &state;
+  if (t < W) reinterpret_cast<long long*>(c)[t] = reinterpret_cast<const long long*>(cg)[t];
   double s = 0.0, m = 0.0, nn = 0.0;
   // rows b = t, t + T, t + 2T, ... in this order; eight rows' loads are issued before
   // they are summed, so the walk takes one memory latency per eight rows
@@ -66,66 +134,22 @@ __device__ __forceinline__ void controller_core(CtrlState* c, const Row& row, lo
     }
     __syncthreads();
   }
-  if (t != 0) return;
   const double errL2 = sqrt(ss[0] / (double)n);
-  const double errMax = sm[0];
   const double errNorm = dmax(errL2, 1e-300);
-  const bool bad = (sn[0] > 0.0) || (errNorm != errNorm);
-  if (c->log && c->attempts < c->logCap) {
-    double* row = c->log + 4 * c->attempts;
-    row[0] = c->t;
-    row[1] = c->dt;
-    row[2] = errNorm;
-    row[3] = (c->frozen || errNorm <= 1.0) ? 1.0 : 0.0;
-  }
-  c->attempts += 1;
-  c->rhsEvals += 3;
-  c->errLast = errNorm;
-  if (c->frozen) {  // replay of a given dt sequence: every step is taken
-    c->t += c->dt;
-    c->cur ^= 1;
-    c->accepted += 1;
-    c->tReached = c->t;
-    c->dtLast = c->dt;
-    c->maxNormLast = errMax;
-    if (bad) { c->done = 3; return; }
-    if (c->accepted >= c->nList) { c->done = 1; return; }
-    c->dt = c->dtList[c->accepted];
-    return;
-  }
-  bool stop = false;
-  if (errNorm <= 1.0) {
-    c->t += c->dt;
-    c->cur ^= 1;  // uNew becomes u and k4 becomes k1 (FSAL)
-    c->accepted += 1;
-    c->tReached = c->t;
-    c->dtLast = c->dt;
-    c->maxNormLast = errMax;
-    c->errPrev = errNorm;
-    stop = c->maxAccepted > 0 && c->accepted >= c->maxAccepted;
-  } else {
-    c->rejected += 1;
-  }
-  if (bad) { c->done = 3; return; }  // the reference would loop forever here
-  double fac = c->safety * pow(errNorm, -c->alpha) * pow(c->errPrev, c->beta);
-  fac = (fac < c->facMin) ? c->facMin : ((c->facMax < fac) ? c->facMax : fac);
-  double dtNext = c->dt * fac;
-  dtNext = dmin(dtNext, c->dtMax);
-  if (dtNext < c->dtMin) {
-    c->done = 2;
-    c->dtLast = dtNext;
-    return;
-  }
-  c->dt = dtNext;
-  if (stop) { c->done = 1; return; }  // fixed number of accepted steps reached
-  const double tEnd = c->tEnd;
-  if (!(c->t < tEnd - 1e-15 * dmax(1.0, fabs(tEnd)))) { c->done = 1; return; }
-  if (c->t + c->dt > tEnd) c->dt = tEnd - c->t;
+  const bool ok = errNorm <= 1.0;
+  if (t == 32 && !c->frozen) prevPow = pow(ok ? errNorm : c->errPrev, c->beta);
+  double errPow = 0.0;
+  if (t == 0 && !c->frozen) errPow = pow(errNorm, -c->alpha);
+  __syncthreads();
+  if (t == 0) decide(c, errNorm, sm[0], (sn[0] > 0.0) || (errNorm != errNorm), errPow, prevPow);
+  __syncthreads();
+  if (t < W) reinterpret_cast<long long*>(cg)[t] = reinterpret_cast<const long long*>(c)[t];
+  return c->done == 0 && c->attempts < c->attemptCap;
 }
 
-__device__ __forceinline__ void controller_block(CtrlState* c, const double* partials, int nblk,
+__device__ __forceinline__ bool controller_block(CtrlState* c, const double* partials, int nblk,
                                                  long long n) {
-  controller_core(c, [&](long long b) { return partials + 3 * b; }, nblk, n);
+  return controller_core(c, [&](long long b) { return partials + 3 * b; }, nblk, n);
 }
 
 __global__ void __launch_bounds__(kCtrlThreads) k_controller(CtrlState* c, const double* partials,
@@ -138,19 +162,17 @@ __global__ void __launch_bounds__(kCtrlThreads) k_controller(CtrlState* c, const
 __global__ void __launch_bounds__(kCtrlThreads) k_controller_loop(CtrlState* c, const double* partials,
                                                                   int nblk, long long n,
                                                                   cudaGraphConditionalHandle loop) {
-  controller_block(c, partials, nblk, n);
-  if (threadIdx.x == 0)
-    cudaGraphSetConditional(loop, (c->done == 0 && c->attempts < c->attemptCap) ? 1u : 0u);
+  const bool running = controller_block(c, partials, nblk, n);
+  if (threadIdx.x == 0) cudaGraphSetConditional(loop, running ? 1u : 0u);
 }
 
 __global__ void __launch_bounds__(kCtrlThreads) k_controller_batch_loop(
     CtrlState* ctrls, const double* const* partials, const int* nblk, const long long* n,
     int* counters, cudaGraphConditionalHandle loop) {
   const int i = blockIdx.x;
-  CtrlState* c = ctrls + i;
-  controller_block(c, partials[i], nblk[i], n[i]);
+  const bool goes_on = controller_block(ctrls + i, partials[i], nblk[i], n[i]);
   if (threadIdx.x != 0) return;
-  if (c->done == 0 && c->attempts < c->attemptCap) atomicAdd(&counters[0], 1);
+  if (goes_on) atomicAdd(&counters[0], 1);
   __threadfence();
   if (atomicAdd(&counters[1], 1) == (int)gridDim.x - 1) {  // the last block of this attempt
     __threadfence();
