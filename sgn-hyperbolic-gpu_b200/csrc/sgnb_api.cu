@@ -42,7 +42,8 @@ int cuda_fail(sgnb_ctx* c, cudaError_t e, const char* what) {
   } while (0)
 
 // One fused launch: mode 0 rhs (in -> out), 1 second stage (u + dt/2 k1 -> K2), 2 end-point
-// stage, 3 third stage with the candidate. Dispatches on the arithmetic mode of the context.
+// stage, 3 third stage with the candidate (the mixed mode: k3 -> K3, and the end-point stage
+// forms the candidate). Dispatches on the arithmetic mode of the context.
 struct Launch {
   int mode = 0;
   const double* in = nullptr;  // mode 0
@@ -54,7 +55,7 @@ static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
                              CUtensorMapDataType type, size_t elem, cuuint32_t nz);
 
 cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
-  if (c->k32) {
+  if (c->mixed) {
     StageArgsM A{};
     A.U[0] = c->U[0]; A.U[1] = c->U[1];
     A.K1[0] = (float*)c->K1[0]; A.K1[1] = (float*)c->K1[1];
@@ -66,8 +67,8 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
     A.kin_k2 = L.stage == 3;
     A.coef = L.stage == 3 ? 0.75 : 0.5;
     if (L.mode == 0) A.out = L.out ? nullptr : A.K1[c->cur];  // no FP64 output: the FSAL head
-    else A.out = A.K2;
-    return dev::launch_line(L.mode, c->C, A, s);
+    else A.out = L.stage == 3 ? A.K3 : A.K2;
+    return dev::launch_fused_mixed(L.mode == 3 ? 1 : L.mode, c->C, A, s, c->mapsM.ok ? &c->mapsM : nullptr);
   }
   StageArgs A{};
   A.U[0] = c->U[0]; A.U[1] = c->U[1];
@@ -79,7 +80,7 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
   A.kin_k2 = L.stage == 3;
   A.coef = L.stage == 3 ? 0.75 : 0.5;
   A.out = L.mode == 0 ? L.out : A.K2;
-  if (c->precision != SGNB_FP64_EXACT) return dev::launch_fused_fast(L.mode, c->C, A, s);
+  if (c->precision == SGNB_FP64_FAST) return dev::launch_fused_fast(L.mode, c->C, A, s);
   // tile copies by the tensor-memory accelerator: A names the context's buffers; the
   // right-hand side's input gets its own map, encoded for this launch
   const TileMaps* M = nullptr;
@@ -226,8 +227,9 @@ static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
 static void build_tile_maps(sgnb_ctx* c) {
   c->maps.ok = 0;
   c->maps.inOk = 0;
+  c->mapsM.ok = 0;
   c->encode_tiled = nullptr;
-  if (c->precision != SGNB_FP64_EXACT) return;  // the other modes' kernels copy rows
+  if (c->precision == SGNB_FP64_FAST) return;  // its kernels copy rows
   if (c->desc.Nx % 8 != 0 || c->desc.Ny % 4 != 0) return;
   const char* sw = std::getenv("SGNB_TMA");
   if (sw && sw[0] == '0') return;
@@ -252,7 +254,15 @@ static void build_tile_maps(sgnb_ctx* c) {
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
            CUDA_SUCCESS;
   };
-  const auto F64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+  const auto F64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64, F32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  if (c->mixed) {
+    const bool okm = encode_state_map(c, &c->mapsM.K1[0], c->K1[0], F32, 4, 1) &&
+                     encode_state_map(c, &c->mapsM.K1[1], c->K1[1], F32, 4, 1) &&
+                     encode_state_map(c, &c->mapsM.K2, c->K2, F32, 4, 1) &&
+                     encode_state_map(c, &c->mapsM.K3, c->K3, F32, 4, 1) && mapH(&c->mapsM.H);
+    c->mapsM.ok = okm ? 1 : 0;
+    return;
+  }
   const bool ok = encode_state_map(c, &c->maps.U[0], c->U[0], F64, 8, 5) &&
                   encode_state_map(c, &c->maps.U[1], c->U[1], F64, 8, 5) &&
                   encode_state_map(c, &c->maps.K1[0], c->K1[0], F64, 8, 5) &&
@@ -321,8 +331,7 @@ void fill_consts(sgnb_ctx* c) {
     if (m < 2) C.eo.b[m] = 0.5 * (gl[m] - gl[4 - m]);
   }
   const char* sw = std::getenv("SGNB_TMA");
-  C.bulk = (sw && sw[0] == '0') ? 0 : (d.Nx % 4 == 0 ? 2 : (d.Nx % 2 == 0 ? 1 : 0));
-  c->k32 = c->mixed && C.sym;
+  C.bulk = d.Nx % 2 == 0 && !(sw && sw[0] == '0');
 }
 
 // The device-side loop: a CUDA graph whose one node is a WHILE conditional node; its body
@@ -388,7 +397,7 @@ int run_loop(sgnb_ctx* c) {
   const long long per_rhs = c->tab.gauss ? 2 : 1, per_attempt = 3 * per_rhs + 1;
   const long long attempts0 = h.attempts;
   // FSAL head: k1 = R(u) into K1[cur] (FP32 in the mixed mode)
-  SGNB_CU(c, launch(c, rhs_launch(c->U[c->cur], c->k32 ? nullptr : (double*)c->K1[c->cur]),
+  SGNB_CU(c, launch(c, rhs_launch(c->U[c->cur], c->mixed ? nullptr : (double*)c->K1[c->cur]),
                     c->stream));
   long long host_attempts = 0;  // attempts launched by the host loop (finished runs' exit at entry)
   for (;;) {
@@ -532,7 +541,9 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   if ((rc = set_device(c))) { g_create_error = c->err; delete c; return rc; }
   e = dev::prepare_fused_exact();
   if (e == cudaSuccess) e = dev::prepare_fused_fast();
+  if (e == cudaSuccess) e = dev::prepare_fused_mixed();
   if (e == cudaSuccess) e = dev::prepare_fused_batch();
+  if (e == cudaSuccess) e = dev::prepare_mixed_batch();
   if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
 
   // statics: Hnod, Hx, Hy (Nd each), HfX, HfY (5 ne each), HfXEnd (5 Ny), HfYEnd (5 Nx)
@@ -587,7 +598,7 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   const size_t sbytes = (size_t)c->ntot * sizeof(double);
   // stage derivatives are FP32 in the mixed mode; K2 and K3 are allocated as one block so
   // that together they always hold an FP64 state (scratch for sgnb_rhs_host)
-  const size_t kbytes = (size_t)c->ntot * (c->k32 ? sizeof(float) : sizeof(double));
+  const size_t kbytes = (size_t)c->ntot * (c->mixed ? sizeof(float) : sizeof(double));
   for (double** bp : {&c->U[0], &c->U[1]}) {
     e = cudaMalloc(bp, sbytes);
     if (e != cudaSuccess) { cuda_fail(c, e, "cudaMalloc(state)"); g_create_error = c->err; return bail(SGNB_ERR_NOMEM); }
@@ -601,7 +612,9 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   c->K3 = (char*)c->K2 + kbytes;
   build_tile_maps(c);
   e = cudaMemset(c->U[0], 0, sbytes);
-  c->nblk = dev::fused_grid_blocks(d->Nx, d->Ny);
+  // error partials: one row per tile of the kernels that this context runs
+  c->nblk = d->precision == SGNB_FP64_FAST && c->C.sym && !c->tab.gauss
+                ? dev::line_grid_blocks(d->Nx, d->Ny) : dev::fused_grid_blocks(d->Nx, d->Ny);
   c->ndiag = 592;
   if (e == cudaSuccess) e = cudaMalloc(&c->partials, 3 * (size_t)c->nblk * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&c->diag, (size_t)c->ndiag * sizeof(double));
@@ -679,7 +692,7 @@ int sgnb_rhs_host(sgnb_ctx* c, const double* U, double* dU) {
   // is not allowed, so the input goes to U[cur ^ 1] and the output to the FP64 view of the
   // stage buffers (K2, K3 together hold one FP64 state in every precision mode)
   double* in = c->U[c->cur ^ 1];
-  double* out = c->k32 ? (double*)c->K2 : (double*)c->K3;
+  double* out = c->mixed ? (double*)c->K2 : (double*)c->K3;
   SGNB_CU(c, cudaMemcpyAsync(in, U, c->ntot * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   if (int rc = sgnb_rhs_device(c, in, out, c->stream)) return rc;
   SGNB_CU(c, cudaMemcpyAsync(dU, out, c->ntot * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -937,7 +950,8 @@ struct sgnb_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
   std::vector<sgnb_ctx*> ctx;          // per-instance buffers and statics
-  RhsConsts* dconsts = nullptr;        // [n]
+  LineConsts* dconsts = nullptr;       // [n]
+  RhsConsts* dconstsM = nullptr;       // [n], mixed batches
   bool mixed = false;                  // every instance SGNB_MIXED (else SGNB_FP64_FAST)
   StageArgs* dargs = nullptr;          // [n]
   StageArgs* hargs = nullptr;          // pinned host mirror
@@ -983,13 +997,7 @@ cudaError_t batch_launch(sgnb_batch* b, int mode, int shape, int blocks, int kin
 
 BatchArgs batch_args(sgnb_batch* b, int shape, int kin_k2, double coef) {
   BatchArgs B{};
-  const RhsConsts& C0 = b->ctx[0]->C;
-  for (int k = 0; k < 25; ++k) { B.tables.D[k] = C0.D[k]; B.tables.Df[k] = C0.Df[k]; }
-  for (int k = 0; k < 5; ++k) {
-    B.tables.gLp[k] = C0.gLp[k]; B.tables.gRp[k] = C0.gRp[k];
-    B.tables.gLpf[k] = C0.gLpf[k]; B.tables.gRpf[k] = C0.gRpf[k];
-  }
-  B.tables.eo = C0.eo;
+  B.tables = b->ctx[0]->C.eo;
   B.consts = b->dconsts;
   B.args = b->dargs;
   B.tile_inst = b->dtile_inst[shape];
@@ -998,6 +1006,24 @@ BatchArgs batch_args(sgnb_batch* b, int shape, int kin_k2, double coef) {
   B.kin_k2 = kin_k2;
   B.coef = coef;
   return B;
+}
+
+BatchArgsM batch_args_mixed(sgnb_batch* b, int kin_k2, double coef) {
+  BatchArgsM M{};
+  const RhsConsts& C0 = b->ctx[0]->C;
+  for (int k = 0; k < 25; ++k) { M.tables.D[k] = C0.D[k]; M.tables.Df[k] = C0.Df[k]; }
+  for (int k = 0; k < 5; ++k) {
+    M.tables.gLp[k] = C0.gLp[k]; M.tables.gRp[k] = C0.gRp[k];
+    M.tables.gLpf[k] = C0.gLpf[k]; M.tables.gRpf[k] = C0.gRpf[k];
+  }
+  M.consts = b->dconstsM;
+  M.args = b->dargsM;
+  M.tile_inst = b->dtile_inst[0];
+  M.tile_start = b->dtile_start[0];
+  M.ntiles = b->ntiles[0];
+  M.kin_k2 = kin_k2;
+  M.coef = coef;
+  return M;
 }
 
 // The batch's device-side loop: a WHILE conditional node whose body is one attempt of
@@ -1052,19 +1078,10 @@ bool all_done(const sgnb_batch* b) {
 // Stage arguments of every instance and the controllers (already initialised in
 // b->hctrl) to the device.
 cudaError_t batch_launch(sgnb_batch* b, int mode, int shape, int blocks, int kin_k2, double coef) {
-  if (!b->mixed) return dev::launch_fused_batch(mode, shape, blocks, batch_args(b, shape, kin_k2, coef), b->stream);
-  if (shape != 0) return cudaErrorInvalidValue;  // mixed batches use 8x4 tiles
-  const BatchArgs B = batch_args(b, 0, kin_k2, coef);
-  BatchArgsM M{};
-  M.tables = B.tables;
-  M.consts = B.consts;
-  M.args = b->dargsM;
-  M.tile_inst = B.tile_inst;
-  M.tile_start = B.tile_start;
-  M.ntiles = B.ntiles;
-  M.kin_k2 = kin_k2;
-  M.coef = coef;
-  return dev::launch_mixed_batch(mode, blocks, M, b->stream);
+  if (!b->mixed)
+    return dev::launch_fused_batch(mode, shape, blocks, batch_args(b, shape, kin_k2, coef), b->stream);
+  if (shape != 0) return cudaErrorInvalidValue;  // mixed batches use one tile shape
+  return dev::launch_mixed_batch(mode == 3 ? 1 : mode, blocks, batch_args_mixed(b, kin_k2, coef), b->stream);
 }
 
 int batch_prepare(sgnb_batch* b) {
@@ -1107,7 +1124,9 @@ int batch_prepare(sgnb_batch* b) {
 // graph launch up to 4096 attempts (a bound on one launch; the host then relaunches).
 int batch_run(sgnb_batch* b) {
   constexpr long long kAttemptsPerLaunch = 4096;
-  if (!b->ctx[0]->C.sym) {
+  bool sym = true;
+  for (const sgnb_ctx* c : b->ctx) sym = sym && c->C.sym;
+  if (!b->mixed && !sym) {
     // caller-given FR tables without the reflection symmetry that the batched kernels need:
     // one instance after the other, each through its own loop
     for (int i = 0; i < b->n; ++i) {
@@ -1151,14 +1170,15 @@ int sgnb_checked_oob(int device, long long* count, int reset) {
   *count = 0;
 #ifdef SGNB_CHECKED
   cudaError_t e = cudaSetDevice(device);
-  unsigned long long a = 0, b = 0, l = 0, k = 0, j = 0;
+  unsigned long long a = 0, b = 0, l = 0, k = 0, m = 0, j = 0;
   if (e == cudaSuccess) e = dev::read_oob_exact(&a, reset != 0);
   if (e == cudaSuccess) e = dev::read_oob_fast(&b, reset != 0);
   if (e == cudaSuccess) e = dev::read_oob_line(&l, reset != 0);
   if (e == cudaSuccess) e = dev::read_oob_batch(&k, reset != 0);
+  if (e == cudaSuccess) e = dev::read_oob_mixed(&m, reset != 0);
   if (e == cudaSuccess) e = dev::read_oob_adjoint(&j, reset != 0);
   if (e != cudaSuccess) return fail(nullptr, SGNB_ERR_CUDA, cudaGetErrorString(e));
-  *count = (long long)(a + b + l + k + j);
+  *count = (long long)(a + b + l + k + m + j);
   return SGNB_OK;
 #else
   (void)device; (void)reset;
@@ -1500,7 +1520,8 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
   };
   cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evRead, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc(&b->dconsts, n * sizeof(RhsConsts));
+  if (e == cudaSuccess) e = cudaMalloc(&b->dconsts, n * sizeof(LineConsts));
+  if (e == cudaSuccess) e = cudaMalloc(&b->dconstsM, n * sizeof(RhsConsts));
   if (e == cudaSuccess) e = cudaMalloc(&b->dargs, n * sizeof(StageArgs));
   if (e == cudaSuccess) e = cudaMallocHost(&b->hargs, n * sizeof(StageArgs));
   if (e == cudaSuccess) e = cudaMalloc(&b->dargsM, n * sizeof(StageArgsM));
@@ -1512,20 +1533,23 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
   if (e == cudaSuccess) e = cudaMalloc(&b->dpart, n * sizeof(double*));
   if (e == cudaSuccess) e = cudaMalloc(&b->dntot, n * sizeof(long long));
   if (e != cudaSuccess) return bail(e, "batch buffers");
-  std::vector<RhsConsts> hc(n);
+  std::vector<LineConsts> hc(n);
+  std::vector<RhsConsts> hcM(n);
   std::vector<long long> ht(n);
   for (int i = 0; i < n; ++i) {
-    hc[i] = b->ctx[i]->C;
+    hc[i] = line_consts(b->ctx[i]->C);
+    hcM[i] = b->ctx[i]->C;
     ht[i] = b->ctx[i]->ntot;
   }
-  e = cudaMemcpy(b->dconsts, hc.data(), n * sizeof(RhsConsts), cudaMemcpyHostToDevice);
+  e = cudaMemcpy(b->dconsts, hc.data(), n * sizeof(LineConsts), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(b->dconstsM, hcM.data(), n * sizeof(RhsConsts), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->dntot, ht.data(), n * sizeof(long long), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return bail(e, "batch upload");
   std::vector<long long> maxTiles(n, 0);
-  // work lists per tile shape: instance-major tiles (8x4 tiles also fix the per-instance
-  // partial count, which the controllers reduce; other shapes have more or fewer tiles)
+  // work lists per tile shape: instance-major tiles (their number is also the instance's
+  // partial count, which the controllers reduce)
   for (int sh = 0; sh < 3; ++sh) {
-    const int tx = dev::batch_tile_tx(sh), ty = 32 / tx;
+    const int tx = b->mixed ? 8 : dev::batch_tile_tx(sh), ty = b->mixed ? 4 : dev::batch_tile_ty(sh);
     std::vector<int> inst;
     std::vector<long long> start(n + 1, 0);
     std::vector<int> nb(n);
@@ -1568,7 +1592,7 @@ int sgnb_batch_destroy(sgnb_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->chunk) cudaGraphExecDestroy(b->chunk);
   if (b->evRead) cudaEventDestroy(b->evRead);
-  cudaFree(b->dconsts); cudaFree(b->dargs); cudaFree(b->dctrl); cudaFree(b->dpart);
+  cudaFree(b->dconsts); cudaFree(b->dconstsM); cudaFree(b->dargs); cudaFree(b->dctrl); cudaFree(b->dpart);
   cudaFree(b->dcount);
   cudaFree(b->dntot); cudaFree(b->dpartbuf);
   if (b->hargs) cudaFreeHost(b->hargs);
@@ -1598,7 +1622,7 @@ sgnb_ctx* sgnb_batch_instance(sgnb_batch* b, int i) {
 
 int sgnb_batch_set_config(sgnb_batch* b, int shape, int blocks) {
   if (!b || shape < 0 || shape > 2 || blocks < 0) return bfail(b, SGNB_ERR_INVALID, "shape 0..2, blocks >= 0");
-  if (b->mixed && shape != 0) return bfail(b, SGNB_ERR_UNSUPPORTED, "mixed batches use 8x4 tiles");
+  if (b->mixed && shape != 0) return bfail(b, SGNB_ERR_UNSUPPORTED, "mixed batches use tile shape 0");
   b->shape = shape;
   b->blocks = blocks;
   return SGNB_OK;

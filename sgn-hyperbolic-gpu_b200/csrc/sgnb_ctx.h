@@ -21,16 +21,16 @@ struct sgnb_ctx {
   long long Nd = 0, ntot = 0;
   sgnb::RhsConsts C{};
   sgnb::TileMaps maps{};  // tensor maps of U, K1, K2, K3, Hnod (exact mode, whole tiles)
+  sgnb::TileMapsM mapsM{};  // the mixed mode's (FP32 K1, K2, K3; Hnod)
   void* encode_tiled = nullptr;  // the driver's tensor-map encoder (set with the maps)
   double* Hbuf = nullptr;  // one allocation holding all statics
   double* trbuf = nullptr;  // Gauss points: face traces, 4 faces x 5 fields x 5 ne
   double* U[2] = {nullptr, nullptr};
-  // stage derivatives: FP64, or FP32 (k32: the mixed mode, on FR tables its kernels take)
+  // stage derivatives: FP64 (exact / fast) or FP32 (mixed precision)
   void* K1[2] = {nullptr, nullptr};
   void* K2 = nullptr;
   void* K3 = nullptr;
   bool mixed = false;
-  bool k32 = false;
   double* partials = nullptr;
   int nblk = 0;
   double* diag = nullptr;  // diagnostic partials

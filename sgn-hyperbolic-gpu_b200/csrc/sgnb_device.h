@@ -65,12 +65,32 @@ struct RhsConsts {
   // the differentiation and correction tables rounded to FP32 (the mixed mode's FP32
   // contractions)
   float Df[25], gLpf[5], gRpf[5];
-  LineTables eo;  // the fast mode's split tables; sym: the tables have the symmetry it needs
+  LineTables eo;  // the line kernels' split tables; sym: the tables have the symmetry they need
   int sym;
-  // rows that bulk copies can take (every row starts and ends at a multiple of 16 bytes): 0
-  // none, 1 those of FP64 buffers (Nx even), 2 also those of FP32 ones (Nx a multiple of 4)
-  int bulk;
+  int bulk;       // bulk row copies: the rows of FP64 buffers start and end at multiples of 16
+                  // bytes (Nx even)
 };
+
+// What the line kernels (fast mode) take of RhsConsts.
+struct LineConsts {
+  int Nx, Ny, bcx, bcy;
+  long long Nd;
+  double g, halfg, gamma, c2, n2g, iJx, iJy;
+  const double* Hnod;
+  const double *ghostL, *ghostR;
+  double *edgeL, *edgeR;
+  int bulk, pad_;
+};
+inline LineConsts line_consts(const RhsConsts& C) {
+  LineConsts L{};
+  L.Nx = C.Nx; L.Ny = C.Ny; L.bcx = C.bcx; L.bcy = C.bcy; L.Nd = C.Nd;
+  L.g = C.g; L.halfg = C.halfg; L.gamma = C.gamma; L.c2 = C.c2; L.n2g = C.n2g;
+  L.iJx = C.iJx; L.iJy = C.iJy;
+  L.Hnod = C.Hnod;
+  L.ghostL = C.ghostL; L.ghostR = C.ghostR; L.edgeL = C.edgeL; L.edgeR = C.edgeR;
+  L.bulk = C.bulk;
+  return L;
+}
 
 // Device-resident state of the adaptive integrator: the scalar loop variables of
 // src/solver/rk.cpp:67-164 plus the index of the buffer pair that holds u and k1.
@@ -193,9 +213,16 @@ struct TileMaps {
   int ok, inOk;
 };
 
+// The mixed-precision mode's counterparts (intermediate stage): the FP32 stage buffers as
+// [field][element row][Nx * 25] with a [1][4][200] box (one field of one tile per copy),
+// the nodal depth as for the FP64 kernels.
+struct TileMapsM {
+  CUtensorMap K1[2], K2, K3, H;
+  int ok;
+};
+
 // Buffers of one fused launch.
 struct StageArgs {
-  using K = double;   // storage type of the stage derivatives
   const double* in;   // MODE_RHS input state
   double* out;        // MODE_RHS / MODE_STAGE output derivative
   double* U[2];       // state ping-pong pair
@@ -210,10 +237,9 @@ struct StageArgs {
 
 // Buffers of one mixed-precision launch: FP64 state, FP32 stage derivatives.
 struct StageArgsM {
-  using K = float;
   const double* in;   // MODE_RHS input state
-  double* outd;       // MODE_RHS output derivative (FP64), or NULL: out
-  float* out;         // MODE_STAGE (and MODE_RHS without outd) output derivative
+  double* outd;       // MODE_RHS output derivative (FP64)
+  float* out;         // MODE_STAGE output derivative
   double* U[2];
   float* K1[2];
   float* K2;
@@ -224,18 +250,17 @@ struct StageArgsM {
   double* partials;
 };
 
-// Work list of a batched launch: tile t belongs to instance tile_inst[t] and is that
-// instance's local tile t - tile_start[inst]; per-instance constants and buffers.
+// Differentiation and correction tables (adjoint, mixed batch).
 struct FrTablesDev {
   double D[25], gLp[5], gRp[5];
   float Df[25], gLpf[5], gRpf[5];  // FP32 roundings (mixed mode)
-  LineTables eo;                   // the split tables (fast mode)
 };
 
+// Work list of a batched launch: tile t belongs to instance tile_inst[t] and is that
+// instance's local tile t - tile_start[inst]; per-instance constants and buffers.
 struct BatchArgs {
-  using Args = StageArgs;
-  FrTablesDev tables;   // shared by every instance (P = 4 GLL)
-  const RhsConsts* consts;
+  LineTables tables;    // shared by every instance (P = 4 GLL)
+  const LineConsts* consts;
   const StageArgs* args;
   const int* tile_inst;
   const long long* tile_start;
@@ -286,7 +311,6 @@ struct GatherArgs {
 
 // Work list of a batched mixed-precision launch (8x4 tiles), as BatchArgs.
 struct BatchArgsM {
-  using Args = StageArgsM;
   FrTablesDev tables;
   const RhsConsts* consts;
   const StageArgsM* args;
@@ -306,11 +330,16 @@ struct CellGrid {
 };
 
 namespace dev {
+// Batched mixed-precision launch: `blocks` persistent CTAs, or one CTA per tile (0).
+cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s);
+cudaError_t prepare_mixed_batch();
+
 // Out-of-range access counts of the checked build, per translation unit.
 cudaError_t read_oob_exact(unsigned long long* out, bool reset);
 cudaError_t read_oob_fast(unsigned long long* out, bool reset);
 cudaError_t read_oob_line(unsigned long long* out, bool reset);
 cudaError_t read_oob_batch(unsigned long long* out, bool reset);
+cudaError_t read_oob_mixed(unsigned long long* out, bool reset);
 cudaError_t read_oob_adjoint(unsigned long long* out, bool reset);
 
 // The fast mode's reciprocal (fn 0) and square root (fn 1) elementwise, for tests.
@@ -364,16 +393,18 @@ cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaSt
 cudaError_t prepare_line();
 cudaError_t prepare_fused_exact();
 cudaError_t prepare_fused_fast();
-cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgsM& A, cudaStream_t s);
+cudaError_t launch_fused_mixed(int mode, const RhsConsts& C, const StageArgsM& A,
+                               cudaStream_t s, const TileMapsM* M = nullptr);
+cudaError_t prepare_fused_mixed();
 int fused_grid_blocks(int Nx, int Ny);
-// Batched launch (FP64 fast): tile shape shape_id (0: 8x4, 1: 16x2, 2: 4x8); `blocks`
-// persistent CTAs looping over the work list, or one CTA per tile when blocks == 0.
+// Batched launch (fast mode): tile shape shape_id (0: 6x4 elements, 1: 12x2, 2: 24x1);
+// `blocks` persistent CTAs looping over the work list, or one CTA per tile when blocks == 0.
 cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchArgs& B,
                                cudaStream_t s);
-// The mixed mode's (8x4 tiles).
-cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s);
 cudaError_t prepare_fused_batch();
 int batch_tile_tx(int shape_id);
+int batch_tile_ty(int shape_id);
+int line_grid_blocks(int Nx, int Ny);
 cudaError_t launch_controller_batch(CtrlState* ctrls, const double* const* partials,
                                     const int* nblk, const long long* n, int ninst,
                                     cudaStream_t s);

@@ -151,6 +151,7 @@ __device__ __forceinline__ double stage_value(const StageIn& I, long long idx) {
 }
 
 // Error partials of one CTA: fixed shuffle tree within each warp, then the warps in order.
+template <int NW = NWARP>
 __device__ __forceinline__ void reduce_error(double esum, double emax, int enan, double (*red)[3],
                                              double* partials, long long blk) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -169,7 +170,7 @@ __device__ __forceinline__ void reduce_error(double esum, double emax, int enan,
   __syncthreads();
   if (threadIdx.x == 0) {
     double s = 0.0, m = 0.0, n = 0.0;
-    for (int w = 0; w < NWARP; ++w) {
+    for (int w = 0; w < NW; ++w) {
       s += red[w][0];
       m = m < red[w][1] ? red[w][1] : m;
       n += red[w][2];

@@ -1,4 +1,4 @@
-// sgnb_kernels_batch.cu -- batched kernels of the fast and mixed modes on GLL points: one
+// sgnb_kernels_batch.cu -- batched kernels of the fast mode on GLL points: one
 // launch per stage over the tiles of many independent instances. Built with -fmad=true.
 #include "sgnb_kernels_line.cuh"
 
@@ -11,17 +11,16 @@ namespace dev {
 // memory once per tile. PERSIST: a fixed grid of CTAs loops over the work list;
 // otherwise one CTA per tile (no loop: the compiler then keeps nothing live from one tile
 // to the next, which the loop costs in spilled registers).
-template <int MODE, int TX_, int TY_, class BA>
-__device__ __forceinline__ void batch_tile(const BA& B, long long t,
-                                           typename LineTile<TX_, TY_>::Smem& S, RhsConsts& Cs,
-                                           typename BA::Args& As) {
-  using Args = typename BA::Args;
+template <int MODE, int WX>
+__device__ __forceinline__ void batch_tile(const BatchArgs& B, long long t,
+                                           typename LineTile<WX>::Smem& S, LineConsts& Cs,
+                                           StageArgs& As) {
   const int inst = B.tile_inst[t];
   const long long lt = t - B.tile_start[inst];
   __syncthreads();  // the previous tile is done with Cs / As
   {
     // both blocks' loads in flight before the first store (one round trip per tile)
-    block_copy2<(int)(sizeof(RhsConsts) / 4), (int)(sizeof(Args) / 4), NTHR>(
+    block_copy2<(int)(sizeof(LineConsts) / 4), (int)(sizeof(StageArgs) / 4), LTHR>(
         reinterpret_cast<unsigned*>(&Cs), reinterpret_cast<const unsigned*>(B.consts + inst),
         reinterpret_cast<unsigned*>(&As), reinterpret_cast<const unsigned*>(B.args + inst));
   }
@@ -32,50 +31,55 @@ __device__ __forceinline__ void batch_tile(const BA& B, long long t,
     if (MODE == MODE_STAGE) As.out = As.K2;
   }
   __syncthreads();
-  const int ntx = (Cs.Nx + TX_ - 1) / TX_;
+  const int ntx = (Cs.Nx + LineTile<WX>::TX - 1) / LineTile<WX>::TX;
   // volatile views: per-instance values are re-read from shared memory at each use
   // rather than held in registers through the passes
-  line_tile<MODE, TX_, TY_, false, false, typename Args::K>(
-      static_cast<const volatile RhsConsts&>(Cs), B.tables.eo, static_cast<const volatile Args&>(As),
-      (int)(lt % ntx), (int)(lt / ntx), lt, Cs.bulk >= (sizeof(typename Args::K) == 4 ? 2 : 1), S);
+  line_tile<MODE, WX, false, false>(
+      static_cast<const volatile LineConsts&>(Cs), B.tables, static_cast<const volatile StageArgs&>(As),
+      (int)(lt % ntx), (int)(lt / ntx), lt, Cs.bulk != 0, S);
 }
 
-template <int MODE, int TX_, int TY_, bool PERSIST, class BA>
-__global__ void __launch_bounds__(NTHR, PERSIST || TX_ == 16 ? 2 : 3) k_line_batch(const BA B) {
+template <int MODE, int WX, bool PERSIST>
+__global__ void __launch_bounds__(LTHR, (PERSIST ? 3 : kLineCtas<MODE, WX>)) k_line_batch(const BatchArgs B) {
   // FR tables come from the kernel parameters (constant bank): the same for every
   // instance (P = 4 GLL)
   extern __shared__ __align__(128) unsigned char smem_batch[];
-  using T = LineTile<TX_, TY_>;
+  using T = LineTile<WX>;
   typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_batch);
-  __shared__ RhsConsts Cs;
-  __shared__ typename BA::Args As;
+  __shared__ LineConsts Cs;
+  __shared__ StageArgs As;
+  if (kStash<MODE> && threadIdx.x < 32) stash_alloc(&S.stash);
   if constexpr (PERSIST) {
     for (long long t = blockIdx.x; t < B.ntiles; t += gridDim.x)
-      batch_tile<MODE, TX_, TY_>(B, t, S, Cs, As);
+      batch_tile<MODE, WX>(B, t, S, Cs, As);
   } else {
-    if ((long long)blockIdx.x < B.ntiles) batch_tile<MODE, TX_, TY_>(B, blockIdx.x, S, Cs, As);
+    if ((long long)blockIdx.x < B.ntiles) batch_tile<MODE, WX>(B, blockIdx.x, S, Cs, As);
+  }
+  if constexpr (kStash<MODE>) {
+    __syncthreads();
+    if (threadIdx.x < 32) stash_free(S.stash);
   }
 }
 
-template <int MODE, int TXs, int TYs, class BA>
-static cudaError_t launch_b(int blocks, const BA& B, cudaStream_t s) {
-  const size_t smem = sizeof(typename LineTile<TXs, TYs>::Smem);
+template <int MODE, int WX>
+static cudaError_t launch_b(int blocks, const BatchArgs& B, cudaStream_t s) {
+  const size_t smem = sizeof(typename LineTile<WX>::Smem);
   if (blocks > 0) {
-    k_line_batch<MODE, TXs, TYs, true, BA><<<blocks, NTHR, smem, s>>>(B);
+    k_line_batch<MODE, WX, true><<<blocks, LTHR, smem, s>>>(B);
   } else {
     if (B.ntiles < 1 || B.ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    k_line_batch<MODE, TXs, TYs, false, BA><<<(unsigned)B.ntiles, NTHR, smem, s>>>(B);
+    k_line_batch<MODE, WX, false><<<(unsigned)B.ntiles, LTHR, smem, s>>>(B);
   }
   return cudaGetLastError();
 }
 
-template <int TXs, int TYs, class BA>
-static cudaError_t launch_shape(int mode, int blocks, const BA& B, cudaStream_t s) {
+template <int WX>
+static cudaError_t launch_shape(int mode, int blocks, const BatchArgs& B, cudaStream_t s) {
   switch (mode) {
-    case MODE_RHS: return launch_b<MODE_RHS, TXs, TYs>(blocks, B, s);
-    case MODE_STAGE: return launch_b<MODE_STAGE, TXs, TYs>(blocks, B, s);
-    case MODE_FSAL: return launch_b<MODE_FSAL, TXs, TYs>(blocks, B, s);
-    case MODE_CAND: return launch_b<MODE_CAND, TXs, TYs>(blocks, B, s);
+    case MODE_RHS: return launch_b<MODE_RHS, WX>(blocks, B, s);
+    case MODE_STAGE: return launch_b<MODE_STAGE, WX>(blocks, B, s);
+    case MODE_FSAL: return launch_b<MODE_FSAL, WX>(blocks, B, s);
+    case MODE_CAND: return launch_b<MODE_CAND, WX>(blocks, B, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -83,43 +87,39 @@ static cudaError_t launch_shape(int mode, int blocks, const BA& B, cudaStream_t 
 cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchArgs& B,
                                cudaStream_t s) {
   switch (shape_id) {
-    case 0: return launch_shape<8, 4>(mode, blocks, B, s);
-    case 1: return launch_shape<16, 2>(mode, blocks, B, s);
-    case 2: return launch_shape<4, 8>(mode, blocks, B, s);
+    case 0: return launch_shape<1>(mode, blocks, B, s);
+    case 1: return launch_shape<2>(mode, blocks, B, s);
+    case 2: return launch_shape<4>(mode, blocks, B, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
-cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s) {
-  return launch_shape<8, 4>(mode, blocks, B, s);
-}
+int batch_tile_tx(int shape_id) { return LROW * (shape_id == 1 ? 2 : (shape_id == 2 ? 4 : 1)); }
+int batch_tile_ty(int shape_id) { return shape_id == 1 ? 2 : (shape_id == 2 ? 1 : 4); }
 
-int batch_tile_tx(int shape_id) { return shape_id == 1 ? 16 : (shape_id == 2 ? 4 : 8); }
-
-template <int MODE, int TXs, int TYs, class BA>
+template <int MODE, int WX>
 static cudaError_t prepare_mode() {
-  const int bytes = (int)sizeof(typename LineTile<TXs, TYs>::Smem);
-  cudaError_t e = cudaFuncSetAttribute(k_line_batch<MODE, TXs, TYs, true, BA>,
+  const int bytes = (int)sizeof(typename LineTile<WX>::Smem);
+  cudaError_t e = cudaFuncSetAttribute(k_line_batch<MODE, WX, true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_line_batch<MODE, TXs, TYs, false, BA>,
+  return cudaFuncSetAttribute(k_line_batch<MODE, WX, false>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-template <int TXs, int TYs, class BA>
+template <int WX>
 static cudaError_t prepare_shape() {
-  cudaError_t e = prepare_mode<MODE_RHS, TXs, TYs, BA>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE, TXs, TYs, BA>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL, TXs, TYs, BA>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_CAND, TXs, TYs, BA>();
+  cudaError_t e = prepare_mode<MODE_RHS, WX>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE, WX>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL, WX>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_CAND, WX>();
   return e;
 }
 
 cudaError_t prepare_fused_batch() {
-  cudaError_t e = prepare_shape<8, 4, BatchArgs>();
-  if (e == cudaSuccess) e = prepare_shape<16, 2, BatchArgs>();
-  if (e == cudaSuccess) e = prepare_shape<4, 8, BatchArgs>();
-  if (e == cudaSuccess) e = prepare_shape<8, 4, BatchArgsM>();
+  cudaError_t e = prepare_shape<1>();
+  if (e == cudaSuccess) e = prepare_shape<2>();
+  if (e == cudaSuccess) e = prepare_shape<4>();
   return e;
 }
 

@@ -1,5 +1,5 @@
 // sgnb_kernels_line.cu -- single-instance and slab kernels of the fast arithmetic mode on GLL
-// points, and the mixed mode's. Built with -fmad=true.
+// points. Built with -fmad=true.
 #include "sgnb_kernels_line.cuh"
 
 namespace sgnb {
@@ -7,36 +7,31 @@ namespace dev {
 
 // bulk row copies need aligned buffers besides aligned rows (C.bulk): the right-hand side's
 // input and output are the caller's
-template <class Args>
-static int bulk_rows(const RhsConsts& C, const Args& A, const void* outd) {
+static int bulk_rows(const RhsConsts& C, const StageArgs& A) {
   auto ok = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-  return C.bulk >= (sizeof(typename Args::K) == 4 ? 2 : 1) && ok(A.in) && ok(A.out) && ok(outd) &&
-         ok(A.U[0]) && ok(A.U[1]) && ok(A.K1[0]) && ok(A.K1[1]) && ok(A.K2) && ok(A.K3) && ok(C.Hnod);
+  return C.bulk && ok(A.in) && ok(A.out) && ok(A.U[0]) && ok(A.U[1]) && ok(A.K1[0]) && ok(A.K1[1]) &&
+         ok(A.K2) && ok(A.K3) && ok(C.Hnod);
 }
 
-template <int MODE, bool FRIC, bool GHOST, class Args>
-static cudaError_t launch_variant(const RhsConsts& C, const Args& A, int bulk, cudaStream_t s) {
-  const dim3 grid((C.Nx + 7) / 8, (C.Ny + 3) / 4);
-  k_line<MODE, FRIC, GHOST, Args><<<grid, NTHR, sizeof(LineTile<8, 4>::Smem), s>>>(C, A, bulk);
+template <int MODE, bool FRIC, bool GHOST>
+static cudaError_t launch_variant(const RhsConsts& C, const StageArgs& A, int bulk, cudaStream_t s) {
+  using L = LineTile<1>;
+  const dim3 grid((C.Nx + L::TX - 1) / L::TX, (C.Ny + L::TY - 1) / L::TY);
+  LineConsts LC = line_consts(C);
+  LC.bulk = bulk;
+  k_line<MODE, FRIC, GHOST><<<grid, LTHR, sizeof(typename L::Smem), s>>>(LC, C.eo, A);
   return cudaGetLastError();
 }
 
 template <int MODE>
 static cudaError_t launch_mode(const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
-  const int bulk = bulk_rows(C, A, nullptr);
+  const int bulk = bulk_rows(C, A);
   const bool ghost = C.ghostL != nullptr || C.ghostR != nullptr;
   if (C.manning)
     return ghost ? launch_variant<MODE, true, true>(C, A, bulk, s) : launch_variant<MODE, true, false>(C, A, bulk, s);
   return ghost ? launch_variant<MODE, false, true>(C, A, bulk, s) : launch_variant<MODE, false, false>(C, A, bulk, s);
 }
-template <int MODE>
-static cudaError_t launch_mode(const RhsConsts& C, const StageArgsM& A, cudaStream_t s) {
-  const int bulk = bulk_rows(C, A, A.outd);
-  return C.manning ? launch_variant<MODE, true, false>(C, A, bulk, s) : launch_variant<MODE, false, false>(C, A, bulk, s);
-}
-
-template <class Args>
-static cudaError_t launch_any(int mode, const RhsConsts& C, const Args& A, cudaStream_t s) {
+cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
   switch (mode) {
     case MODE_RHS: return launch_mode<MODE_RHS>(C, A, s);
     case MODE_STAGE: return launch_mode<MODE_STAGE>(C, A, s);
@@ -45,23 +40,19 @@ static cudaError_t launch_any(int mode, const RhsConsts& C, const Args& A, cudaS
     default: return cudaErrorInvalidValue;
   }
 }
-cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
-  return launch_any(mode, C, A, s);
-}
-cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgsM& A, cudaStream_t s) {
-  return launch_any(mode, C, A, s);
+int line_grid_blocks(int Nx, int Ny) {
+  using L = LineTile<1>;
+  return ((Nx + L::TX - 1) / L::TX) * ((Ny + L::TY - 1) / L::TY);
 }
 
 template <int MODE>
 static cudaError_t prepare_mode() {
-  const int bytes = (int)sizeof(LineTile<8, 4>::Smem);
+  const int bytes = (int)sizeof(typename LineTile<1>::Smem);
   const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(k_line<MODE, false, false, StageArgs>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, false, StageArgs>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, false, true, StageArgs>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, true, StageArgs>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, false, false, StageArgsM>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, false, StageArgsM>, at, bytes);
+  cudaError_t e = cudaFuncSetAttribute(k_line<MODE, false, false>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, false>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, false, true>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, true>, at, bytes);
   return e;
 }
 

@@ -1,10 +1,16 @@
 // sgnb_kernels_line.cuh -- the fast arithmetic mode's fused right-hand-side and stage
-// kernels on Gauss-Lobatto points (single instances, slabs and batches). The mixed mode runs
-// the same kernels with its stage derivatives k1, k2, k4 and the embedded part stored in FP32.
+// kernels on Gauss-Lobatto points (single instances, slabs and batches).
 //
-// Same tile and thread layout as sgnb_kernels.cuh (a CTA of 5 warps owns 32 elements; lane
-// i of every warp is tile element i, warp j its j-th line of solution points), with the
-// arithmetic arranged for the fast mode:
+// Work decomposition. A warp owns a row of six elements and holds one line of solution points per
+// lane (30 of 32 lanes): lane (e, j) is line j of element e, first along y (column pass), then
+// along x (row pass). All five lines of an element are in one warp, so between the passes a warp
+// synchronises with itself only; a CTA of four warps stacks four such rows (or 2 x 2, or 4 x 1)
+// and synchronises once, when its tile has landed and every warp has formed its stage inputs.
+// With the lanes over 32 elements and one warp per line instead (as the exact mode's kernels),
+// two of the eight cycles a warp took per instruction were waits at the barriers between the
+// passes.
+//
+// The arithmetic is arranged for the fast mode:
 //   * every flux component is the normal velocity times a state component, F = u_n U_v (plus
 //     the hydrostatic term and c^2 h u_n where they belong), so a line keeps u_n and reads one
 //     field at a time from shared memory;
@@ -16,9 +22,15 @@
 //     lifts splits into an even and an odd half (27 operations instead of 35);
 //   * each pass adds its own direction's sources, so no pass differentiates the depth along
 //     the other direction, and h_n and H_n of the hp equation share one derivative.
-// What bounds it: the FP64 pipe and HBM are both within 1.5x of each other at the target
-// (about 190 FP64 instructions and 90 to 130 bytes per node), so what matters is enough warps to
-// overlap them: 128 registers and 75 KB of shared memory per CTA, three CTAs per SM.
+// What bounds it. At 1024 x 512 elements a right-hand side takes 0.227 ms (5.1 TB/s, 79 % of a
+// plain copy's rate), the second, third and end-point stage 0.320, 0.508 and 0.476 ms (5.2, 5.4
+// and 4.6 TB/s); the kernels before these took 0.408, 0.497, 0.497 and 0.981 ms (the end point
+// then read four inputs twice). What is left is latency: HBM, FP64 issue (59 % busy in the
+// right-hand side) and shared memory (66 %) are all within 1.5x of their limits. The
+// right-hand side and the end point run four CTAs of 128 registers per SM (at three 0.247 and
+// 0.503 ms); the stages that add k run three (at four 0.358 and 0.556 ms: their halos read two
+// arrays, whose sectors only stay in L1 if shared memory leaves it more than 24 KB). Tiles of
+// 2 x 2 or 4 x 1 warps are slower (second stage 0.334 and 0.349 ms).
 #pragma once
 
 #include "sgnb_kernels.cuh"
@@ -26,26 +38,49 @@
 namespace sgnb {
 namespace dev {
 
-// Shared memory of one tile. Field v of the tile's nodes and of the nodes across its edges lie
-// in one block, so a line's neighbour is reached with the line's own field stride:
-//   U[v][i * 25 + a + 5 b]        node (a, b) of tile element i
-//   U[v][800 + 5 * slot + t]      halo slots as in Tile (left, right, bottom, top)
-template <int TX_, int TY_>
+constexpr int LROW = 6;             // elements of a warp's row
+constexpr int LWARPS = 4;           // warps of a CTA
+constexpr int LTHR = 32 * LWARPS;
+
+// A tile of WX x WY warps, and its shared memory. Field v of the tile's nodes and of the nodes
+// across its edges lie in one block, so a line's neighbour is reached with the line's own field
+// stride:
+//   U[v][i * 25 + a + 5 b]        node (a, b) of tile element i = ix + TX iy
+//   U[v][TN + 5 * slot + t]       slots left [TY], right [TY], bottom [TX], top [TX]
+template <int WX_>
 struct LineTile {
-  static constexpr int TX = TX_, TY = TY_;
-  static_assert(TX * TY == TE && TX % 2 == 0, "one tile element per lane, rows of whole pairs");
+  static constexpr int WX = WX_, WY = LWARPS / WX_;
+  static constexpr int TX = LROW * WX, TY = WY;
+  static_assert(WX * WY == LWARPS, "four warps");
   static constexpr int NHALO = 2 * TY + 2 * TX;
-  static constexpr int TN = TE * NPP;             // nodes per tile
+  static constexpr int TN = TX * TY * NPP;        // nodes per tile
   static constexpr int US = TN + NHALO * NP;      // field stride of U
-  static constexpr int RUN = TX * NPP;            // doubles per tile row
   struct Smem {
     double U[NV][US];
     double H[TN];
     double G[NV][TN];        // stage derivative on load; column-pass results; then dU
-    double red[NWARP][3];
-    unsigned long long mbar;
+    double red[LWARPS][3];   // (with the barriers: room for the reads of idle lanes past G)
+    unsigned long long mbar[LWARPS];
+    unsigned stash;          // base of the CTA's tensor memory
+    unsigned pad_;
   };
 };
+// CTAs per SM that a kernel is compiled for: see the note on what bounds these kernels.
+template <int MODE, int WX>
+constexpr int kLineCtas = sizeof(typename LineTile<WX>::Smem) <= 57000 && (MODE == MODE_RHS || MODE == MODE_FSAL) ? 4 : 3;
+constexpr int LRUN = LROW * NPP;    // nodes of a warp's row per field
+// Pairs of neighbouring nodes for element-wise work on a row: lane l < 25 takes pairs l, l + 25,
+// l + 50 of every field (constant strides: no index arithmetic per pair; 32 lanes over all 375
+// pairs of a row spent 20 integer instructions on each).
+constexpr int LPL = 25, LPF = 3;
+static_assert(2 * LPL * LPF == LRUN, "pairs of a row");
+
+// Line of a lane in the column pass, 8 e + a. A half-warp's 16 accesses of 8 bytes should hit 16
+// different bank pairs: elements lie 25 doubles apart, so line (e, a) starts in pair (9 e + a) mod 16.
+// The first 16 lanes cover every pair once, the last 14 collide twice.
+__constant__ unsigned char kColumnLane[32] = {
+    0, 1, 2, 3, 4, 8, 9, 10, 11, 12, 19, 20, 27, 28, 35, 36,
+    16, 17, 18, 24, 25, 26, 32, 33, 34, 40, 41, 42, 43, 44, 0, 0};
 
 // Row copies between global and shared memory by the bulk copy engine. Sizes are multiples
 // of 16 bytes and both addresses 16-byte aligned (rows of an even number of elements).
@@ -77,30 +112,67 @@ __device__ __forceinline__ void bulk_store_wait() {
 template <class P>
 __device__ __forceinline__ auto pick(const P& p, int c) { return c ? p[1] : p[0]; }
 
-// Per-thread asynchronous copy of one value of 4 or 8 bytes.
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(smem_addr(smem)), "l"(gmem), "n"(BYTES) : "memory");
+// Tensor memory as a stash. The epilogues of the third and the end-point stage need values that
+// the passes have no room for (128 registers, and shared memory that sets the CTAs per SM):
+// u and k2 as they were before the stage input replaced them, or u and the embedded part, which
+// are best requested at the start, together with the tile. A lane keeps 2 x 30 doubles of its own
+// in 120 columns of its lane of tensor memory; four CTAs of 128 columns fill an SM's 512.
+// (Read from L2 a second time, one batch of pairs after the other, the two epilogues waited for
+// memory in 4.1 and 2.6 of the 10 and 8 cycles a warp took per instruction.)
+constexpr unsigned kStashCols = 128;
+template <int MODE>
+constexpr bool kStash = MODE == MODE_CAND || MODE == MODE_FSAL;
+__device__ __forceinline__ void stash_alloc(unsigned* smem) {  // one warp
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(smem)),
+               "r"(kStashCols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
 }
-template <class T> struct Pair;
-template <> struct Pair<double> { using type = double2; };
-template <> struct Pair<float> { using type = float2; };
+__device__ __forceinline__ void stash_free(unsigned base) {  // the same warp
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(base), "r"(kStashCols));
+}
+// Three pairs of this lane (one field) to 12 columns at addr; the whole warp together.
+__device__ __forceinline__ void stash_put(unsigned addr, const double2 (&x)[LPF]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%2, %3, %4, %5, %6, %7, %8, %9};\n"
+      "tcgen05.st.sync.aligned.32x32b.x4.b32 [%1], {%10, %11, %12, %13};\n" ::"r"(addr),
+      "r"(addr + 8),
+      "r"(__double2loint(x[0].x)), "r"(__double2hiint(x[0].x)), "r"(__double2loint(x[0].y)),
+        "r"(__double2hiint(x[0].y)), "r"(__double2loint(x[1].x)), "r"(__double2hiint(x[1].x)),
+        "r"(__double2loint(x[1].y)), "r"(__double2hiint(x[1].y)), "r"(__double2loint(x[2].x)),
+        "r"(__double2hiint(x[2].x)), "r"(__double2loint(x[2].y)), "r"(__double2hiint(x[2].y))
+      : "memory");
+}
+__device__ __forceinline__ void stash_put_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+// The reads and the wait for them in one statement: nothing may touch the registers in between.
+__device__ __forceinline__ void stash_get(unsigned addr, double2 (&x)[LPF]) {
+  int r[4 * LPF];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%12];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8, %9, %10, %11}, [%13];\n"
+      "tcgen05.wait::ld.sync.aligned;\n"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]),
+        "=&r"(r[7]), "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11])
+      : "r"(addr), "r"(addr + 8)
+      : "memory");
+#pragma unroll
+  for (int m = 0; m < LPF; ++m)
+    x[m] = make_double2(__hiloint2double(r[4 * m + 1], r[4 * m]), __hiloint2double(r[4 * m + 3], r[4 * m + 2]));
+}
+
 // Two neighbouring values, in one access where rows start aligned (vec); the second one only if
-// two. The same values reach the same thread either way, so both ways give the same sums.
+// two. The same values reach the same lane either way, so both ways give the same sums.
 // Streaming (evict-first) accesses: no other CTA reads these lines soon.
-template <class T>
-__device__ __forceinline__ typename Pair<T>::type load_pair(const T* p, bool vec, bool two) {
-  using T2 = typename Pair<T>::type;
-  if (vec) return __ldcs((const T2*)p);
-  T2 r;
+__device__ __forceinline__ double2 load_pair(const double* p, bool vec, bool two) {
+  if (vec) return __ldcs((const double2*)p);
+  double2 r;
   r.x = __ldcs(p);
-  r.y = two ? __ldcs(p + 1) : T(0);
+  r.y = two ? __ldcs(p + 1) : 0.0;
   return r;
 }
-template <class T>
-__device__ __forceinline__ void store_pair(T* p, typename Pair<T>::type x, bool vec, bool two) {
+__device__ __forceinline__ void store_pair(double* p, double2 x, bool vec, bool two) {
   if (vec) {
-    __stcs((typename Pair<T>::type*)p, x);
+    __stcs((double2*)p, x);
   } else {
     __stcs(p, x.x);
     if (two) __stcs(p + 1, x.y);
@@ -167,8 +239,9 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
   const double ihL = fast_rcp(hL), ihR = fast_rcp(hR);
   const double unL = hnL * ihL, unR = hnR * ihR;
   auto speed = [&](double hh, double pp, double uu) {
+    // sqrt(max(a, 0)), with 1e-150 for 0: far below the last bit of c
     const double a = fma(g, hh, pp) + c2;
-    return fabs(uu) + fast_sqrt(a > 0.0 ? a : 0.0);
+    return fabs(uu) + fast_sqrt_normal(a > 1e-300 ? a : 1e-300);
   };
   const double lamL = 0.5 * fmax(speed(hL, hpL * ihL, unL), speed(h[0], hp[0] * ih[0], un[0]));
   const double lamR = 0.5 * fmax(speed(h[4], hp[4] * ih[4], un[4]), speed(hR, hpR * ihR, unR));
@@ -252,17 +325,16 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
   for (int k = 0; k < NP; ++k) emit(0, k, iJ * d[k]);
 }
 
-// One tile. bulk: rows are copied by the bulk copy engine (Nx even, so every row starts
-// 16-byte aligned in every buffer); otherwise by per-thread 8-byte copies.
-template <int MODE, int TX_, int TY_, bool FRIC, bool GHOST, class K, class TC, class TE_, class TA>
+// One tile. The CTA holds its stash (S.stash, written before or visible after the first barrier
+// here) in the modes that use one. bulk: rows start 16-byte aligned in every buffer (Nx even) and come and go by the bulk
+// copy engine; otherwise value by value.
+template <int MODE, int WX, bool FRIC, bool GHOST, class TC, class TE_, class TA>
 __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A, int bx, int by,
                                           long long blk, const bool bulk,
-                                          typename LineTile<TX_, TY_>::Smem& S) {
-  using L = LineTile<TX_, TY_>;
-  constexpr int TX = L::TX, TY = L::TY, NHALO = L::NHALO, TN = L::TN, US = L::US, RUN = L::RUN;
+                                          typename LineTile<WX>::Smem& S) {
+  using L = LineTile<WX>;
+  constexpr int TX = L::TX, TY = L::TY, NHALO = L::NHALO, TN = L::TN, US = L::US;
   constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND;
-  using KT = K;                                  // storage type of the stage derivatives
-  constexpr bool K32 = sizeof(KT) == 4;
 
   // ---- controller state -----------------------------------------------------------
   int cur = 0;
@@ -274,15 +346,17 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     acoef = A.coef * dt;
   }
   const double* __restrict__ src = MODE == MODE_RHS ? A.in : (MODE == MODE_FSAL ? pick(A.U, cur ^ 1) : pick(A.U, cur));
-  const KT* __restrict__ kin = AXPY ? (A.kin_k2 ? A.K2 : pick(A.K1, cur)) : nullptr;
+  const double* __restrict__ kin = AXPY ? (A.kin_k2 ? A.K2 : pick(A.K1, cur)) : nullptr;
 
   int tid;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
-  const int j = tid >> 5, i = tid & 31;  // line index of this warp, tile element of this lane
+  const int w = tid >> 5, lane = tid & 31;
+  const int wx = WX == 1 ? 0 : w % WX, iy = WX == 1 ? w : w / WX;  // this warp's row of the tile
   const int Nx = C.Nx, Ny = C.Ny;
   const long long Nd = C.Nd;
   const int ex0 = bx * TX, ey0 = by * TY;
   const int TXv = min(TX, Nx - ex0), TYv = min(TY, Ny - ey0);
+  const int RXv = iy < TYv ? max(0, min(LROW, TXv - wx * LROW)) : 0;  // elements of the row in the mesh
   bool ghostL = false, ghostR = false;
   if constexpr (GHOST) {
     ghostL = C.ghostL != nullptr && ex0 == 0;
@@ -290,60 +364,74 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   }
   const bool wallL = C.bcx && ex0 == 0 && !ghostL, wallR = C.bcx && ex0 + TXv == Nx && !ghostR;
   const bool wallB = C.bcy && ey0 == 0, wallT = C.bcy && ey0 + TYv == Ny;
-  const int row0 = (ex0 + Nx * ey0) * NPP;  // the tile's first node within a field (Nd < 2^31)
+  const int row0 = (ex0 + wx * LROW + Nx * (ey0 + iy)) * NPP;  // the row's first node in a field (Nd < 2^31)
+  const int s0 = (wx * LROW + TX * iy) * NPP;                  // and in the tile
+  const int rowv = RXv * NPP;                                  // its nodes in the mesh
 
-  // ---- own nodes ------------------------------------------------------------------
-  const unsigned mbar = smem_addr(&S.mbar);
-  KT* const ks = reinterpret_cast<KT*>(&S.G[0][0]);  // the stage derivative, until the passes
+  // ---- the row's own nodes ------------------------------------------------------------
+  const unsigned mbar = smem_addr(&S.mbar[w]);
+  double* const ks = &S.G[0][0];  // the stage derivative, until the passes
+  // pair m of a field: nodes kp + 2 LPL m and the next one, where in[m] (and two[m])
+  const int kp = 2 * lane;
+  bool in[LPF], two[LPF];
+#pragma unroll
+  for (int m = 0; m < LPF; ++m) {
+    in[m] = lane < LPL && kp + 2 * LPL * m < rowv;
+    two[m] = kp + 2 * LPL * m + 1 < rowv;
+  }
   if (bulk) {
-    const unsigned bytes = (unsigned)TXv * NPP * sizeof(double), kbytes = (unsigned)TXv * NPP * sizeof(KT);
-    if (tid == 0) {
+    constexpr int NROW = NV + 1 + (AXPY ? NV : 0);
+    const unsigned bytes = (unsigned)rowv * sizeof(double);
+    if (lane == 0) {
       mbar_init(mbar);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      mbar_expect_tx(mbar, TYv * ((NV + 1) * bytes + (AXPY ? NV * kbytes : 0)));
+      mbar_expect_tx(mbar, NROW * bytes);
     }
-    __syncthreads();
-    // one row copy per thread, spread over the warps (a warp issues its lanes' copies one by
-    // one); the rows that the epilogue reads start their way to L2 as well
-    constexpr int NARR = AXPY ? 2 : 1;
-    for (int q = i * NWARP + j; q < (NARR * NV + 1) * TY; q += NTHR) {
-      const int iy = q % TY, f = q / TY;
-      if (iy >= TYv) continue;
-      int g = row0 + Nx * NPP * iy;
-      if (!SGNB_INB(g, Nd - TXv * NPP + 1)) g = 0;
-      if (f == 0) bulk_load(smem_addr(&S.H[iy * RUN]), C.Hnod + g, bytes, mbar);
-      else if (f <= NV) bulk_load(smem_addr(&S.U[f - 1][iy * RUN]), src + (f - 1) * Nd + g, bytes, mbar);
-      else bulk_load(smem_addr(ks + (f - 1 - NV) * TN + iy * RUN), kin + (f - 1 - NV) * Nd + g, kbytes, mbar);
+    __syncwarp();
+    if (lane < NROW && RXv > 0) {
+      int g = row0;
+      if (!SGNB_INB(g, Nd - rowv + 1)) g = 0;
+      if (lane < NV) bulk_load(smem_addr(&S.U[lane][s0]), src + lane * Nd + g, bytes, mbar);
+      else if (lane == NV) bulk_load(smem_addr(&S.H[s0]), C.Hnod + g, bytes, mbar);
+      else bulk_load(smem_addr(ks + (lane - NV - 1) * TN + s0), kin + (lane - NV - 1) * Nd + g, bytes, mbar);
     }
+    // what the epilogue reads starts its way to L2
     if constexpr (MODE == MODE_CAND || MODE == MODE_FSAL) {
-      for (int q = i * NWARP + j; q < (MODE == MODE_CAND ? 1 : 2) * NV * TY; q += NTHR) {
-        const int iy = q % TY, f = q / TY, v = f % NV;
-        const int g = row0 + Nx * NPP * iy;
-        if (iy >= TYv || !SGNB_INB(g, Nd - TXv * NPP + 1)) continue;
-        if (MODE == MODE_CAND) bulk_prefetch(pick(A.K1, cur) + v * Nd + g, kbytes);
-        else if (f < NV) bulk_prefetch(pick(A.U, cur) + v * Nd + g, bytes);
-        else bulk_prefetch(A.K3 + v * Nd + g, kbytes);
-      }
+      const int f = lane - 16;  // lanes that copy no row
+      if (f >= 0 && f < NV && RXv > 0 && SGNB_INB(row0, Nd - rowv + 1))
+        bulk_prefetch((MODE == MODE_CAND ? pick(A.K1, cur) : A.K3) + f * Nd + row0, bytes);
     }
   } else {
 #pragma unroll
-    for (int m = 0; m < NIT; ++m) {
-      const int q = tid + NTHR * m, iy = q / RUN, k = q - iy * RUN;
-      if (iy < TYv && k < TXv * NPP) {
-        const int g = row0 + Nx * NPP * iy + k;
-        if (!SGNB_INB(g, Nd)) continue;
-        cp_async<8>(&S.H[q], C.Hnod + g);
+    for (int m = 0; m < (LRUN + 31) / 32; ++m) {
+      const int k = lane + 32 * m, g = row0 + k;
+      if (k < rowv && SGNB_INB(g, Nd)) {
+        cp_async8(&S.H[s0 + k], C.Hnod + g);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-          cp_async<8>(&S.U[v][q], src + v * Nd + g);
-          if constexpr (AXPY) cp_async<sizeof(KT)>(ks + v * TN + q, kin + v * Nd + g);
+          cp_async8(&S.U[v][s0 + k], src + v * Nd + g);
+          if constexpr (AXPY) cp_async8(ks + v * TN + s0 + k, kin + v * Nd + g);
         }
       }
     }
   }
+  // end point: u is requested along with the tile
+  static_assert(2 * 4 * LPF * NV <= (int)kStashCols, "two arrays in the stash");
+  constexpr int NE = MODE == MODE_FSAL ? NV : 1;
+  double2 eu[NE][LPF];
+  if constexpr (MODE == MODE_FSAL) {
+    const double* __restrict__ u0 = pick(A.U, cur) + row0 + kp;
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+      for (int m = 0; m < LPF; ++m) {
+        eu[v][m] = make_double2(0.0, 0.0);
+        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) eu[v][m] = load_pair(u0 + v * Nd + 2 * LPL * m, bulk, two[m]);
+      }
+  }
   // ---- nodes across the tile's edges: one (slot, transverse node) per thread, five fields ---
 #pragma unroll
-  for (int q = tid; q < NHALO * NP; q += NTHR) {
+  for (int q = tid; q < NHALO * NP; q += LTHR) {
     const int slot = q / NP, t = q - NP * slot;
     const double* gh = nullptr;
     bool ok;
@@ -376,7 +464,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
 #pragma unroll
           for (int v = 0; v < NV; ++v) val[v] = src[v * Nd + g];
           if constexpr (AXPY) {
-            KT kv[NV];
+            double kv[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) kv[v] = kin[v * Nd + g];
 #pragma unroll
@@ -388,189 +476,165 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       for (int v = 0; v < NV; ++v) S.U[v][TN + q] = val[v];
     }
   }
+
+  // ---- this warp's row has landed; stage input u + (c dt) k in place; then the whole tile ---
+  const int ce = kColumnLane[lane] >> 3, cj = kColumnLane[lane] & 7;  // column pass: element, line
+  const bool cvalid = lane < LROW * NP && ce < RXv;
+  double* const uc = &S.U[0][s0 + ce * NPP + cj];
   if (!bulk) cp_async_wait_all();
-  __syncthreads();  // halo, per-thread copies and the barrier's initialisation
-  bool landed = true;
   if (bulk) {
-    landed = false;
+    bool landed = RXv == 0;
     for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
-  }
-
-  const int ix = i % TX, iy = i / TX;
-  const bool valid = ix < TXv && iy < TYv;
-
-  // ---- column pass: y-line a = j ---------------------------------------------------
-  {
-    double* const u = &S.U[0][i * NPP + j];
-    if constexpr (AXPY) {
-      // the stage input u + (c dt) k, in place: this warp alone touches the lines a = j here
-      if (valid) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-          for (int b = 0; b < NP; ++b)
-            u[v * US + b * NP] = stage_axpy(u[v * US + b * NP], acoef, ks[v * TN + i * NPP + j + b * NP]);
-      }
-      // FP32 derivatives lie elsewhere than the results that overwrite them: every warp has
-      // read its own
-      if constexpr (K32) __syncthreads(); else __syncwarp();
-    }
     // the copies did not complete: NaN, so that the launch's results are non-finite and the
     // controller ends the run with that error
-    if (!landed) u[0] = __longlong_as_double(0x7ff8000000000000LL);
-    if (valid) {
-      const bool mlo = iy == 0 && wallB, mhi = iy + 1 >= TYv && wallT;
-      const double* const lo = mlo ? u : (iy > 0 ? u - TX * NPP + NP * (NP - 1) : &S.U[0][TN + (2 * TY + ix) * NP + j]);
-      const double* const hi = mhi ? u + NP * (NP - 1)
-                                   : (iy + 1 < TYv ? u + TX * NPP : &S.U[0][TN + (2 * TY + TX + ix) * NP + j]);
-      double* const gp = &S.G[0][i * NPP + j];
-      line_terms<1, US, false>(C, T, u, &S.H[i * NPP + j], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
-                               [&](int v, int k, double r) { gp[v * TN + k * NP] = r; });
+    if (!landed) uc[0] = __longlong_as_double(0x7ff8000000000000LL);
+  }
+  if constexpr (MODE == MODE_CAND) __syncthreads();  // the stash's address
+  else if constexpr (AXPY) __syncwarp();             // the lanes' own copies
+  if constexpr (AXPY) {
+    // in the linear order of the row (no bank conflicts, 16 bytes per access), the next field's
+    // reads ahead of this one's writes
+    double2 x[2][LPF], y[2][LPF];
+    auto read = [&](int v) {
+#pragma unroll
+      for (int m = 0; m < LPF; ++m) {
+        x[v & 1][m] = y[v & 1][m] = make_double2(0.0, 0.0);
+        if (in[m]) {
+          x[v & 1][m] = *(const double2*)&S.U[v][s0 + kp + 2 * LPL * m];
+          y[v & 1][m] = *(const double2*)&ks[v * TN + s0 + kp + 2 * LPL * m];
+        }
+      }
+    };
+    read(0);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      if (v + 1 < NV) read(v + 1);
+      const double2(&xv)[LPF] = x[v & 1];
+      const double2(&yv)[LPF] = y[v & 1];
+#pragma unroll
+      for (int m = 0; m < LPF; ++m)
+        if (in[m])
+          *(double2*)&S.U[v][s0 + kp + 2 * LPL * m] =
+              make_double2(stage_axpy(xv[m].x, acoef, yv[m].x), stage_axpy(xv[m].y, acoef, yv[m].y));
+      if constexpr (MODE == MODE_CAND) {
+        __syncwarp();
+        const unsigned st = S.stash + ((unsigned)w << 21) + 4 * LPF * v;
+        stash_put(st, xv);
+        stash_put(st + 4 * LPF * NV, yv);
+      }
     }
   }
   __syncthreads();
-  // ---- row pass: x-line b = j, completes dU -------------------------------------------
-  if (valid) {
-    const double* const u = &S.U[0][i * NPP + NP * j];
-    const bool mlo = ix == 0 && wallL, mhi = ix + 1 >= TXv && wallR;
-    const double* const lo = mlo ? u : (ix > 0 ? u - NPP + (NP - 1) : &S.U[0][TN + iy * NP + j]);
-    const double* const hi = mhi ? u + (NP - 1) : (ix + 1 < TXv ? u + NPP : &S.U[0][TN + (TY + iy) * NP + j]);
-    double* const gp = &S.G[0][i * NPP + NP * j];
-    line_terms<0, US, FRIC>(C, T, u, &S.H[i * NPP + NP * j], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
-                            [&](int v, int k, double r) { gp[v * TN + k] = -r - gp[v * TN + k]; });
+  if constexpr (MODE == MODE_FSAL) {
+    const unsigned st = S.stash + ((unsigned)w << 21);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) stash_put(st + 4 * LPF * v, eu[v]);
   }
-  // the results leave as they lie in shared memory (FP64 rows by bulk copies), or rounded to
-  // the storage type of the stage derivatives
-  double* out64 = nullptr;
-  KT* outk = nullptr;
-  if constexpr (MODE == MODE_RHS) {
-    if constexpr (K32) { out64 = A.outd; outk = A.out; }  // the head of a run has no outd
-    else out64 = A.out;
-  } else if constexpr (MODE == MODE_STAGE || MODE == MODE_FSAL) {
-    KT* o = MODE == MODE_FSAL ? pick(A.K1, cur ^ 1) : A.out;
-    if constexpr (K32) outk = o; else out64 = o;
+
+  // ---- column pass: y-lines ----------------------------------------------------------
+  if (cvalid) {
+    const bool mlo = iy == 0 && wallB, mhi = iy + 1 >= TYv && wallT;
+    const int ix = wx * LROW + ce;
+    const double* const lo = mlo ? uc : (iy > 0 ? uc - TX * NPP + NP * (NP - 1) : &S.U[0][TN + (2 * TY + ix) * NP + cj]);
+    const double* const hi = mhi ? uc + NP * (NP - 1)
+                                 : (iy + 1 < TYv ? uc + TX * NPP : &S.U[0][TN + (2 * TY + TX + ix) * NP + cj]);
+    const int o = s0 + ce * NPP + cj;
+    double* const gp = &S.G[0][o];
+    line_terms<1, US, false>(C, T, uc, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
+                             [&](int v, int k, double r) { gp[v * TN + k * NP] = r; });
   }
-  const bool bulk_out = bulk && MODE != MODE_CAND && (!K32 || out64 != nullptr);
+  __syncwarp();
+  // ---- row pass: x-lines, completes dU --------------------------------------------------
+  {
+    const int e = lane / NP, j = lane - NP * e, ix = wx * LROW + e;
+    if (lane < LROW * NP && e < RXv) {
+      const int o = s0 + NP * lane;
+      const double* const u = &S.U[0][o];
+      const bool mlo = ix == 0 && wallL, mhi = ix + 1 >= TXv && wallR;
+      const double* const lo = mlo ? u : (ix > 0 ? u - NPP + (NP - 1) : &S.U[0][TN + iy * NP + j]);
+      const double* const hi = mhi ? u + (NP - 1) : (ix + 1 < TXv ? u + NPP : &S.U[0][TN + (TY + iy) * NP + j]);
+      double* const gp = &S.G[0][o];
+      line_terms<0, US, FRIC>(C, T, u, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
+                              [&](int v, int k, double r) { gp[v * TN + k] = -r - gp[v * TN + k]; });
+    }
+  }
+  const bool bulk_out = bulk && MODE != MODE_CAND;
   if (bulk_out) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  __syncthreads();
+  __syncwarp();
 
   // ---- results ---------------------------------------------------------------------
   if constexpr (MODE != MODE_CAND) {
+    double* __restrict__ outp = MODE == MODE_FSAL ? pick(A.K1, cur ^ 1) : A.out;
     if (bulk_out) {
-      if (j == 0) {
-        const unsigned bytes = (unsigned)TXv * NPP * sizeof(double);
-        for (int q = i; q < NV * TY; q += 32) {
-          const int r = q % TY, v = q / TY;
-          const int g = row0 + Nx * NPP * r;
-          if (r < TYv && SGNB_INB(g, Nd - TXv * NPP + 1))
-            bulk_store(out64 + v * Nd + g, smem_addr(&S.G[v][r * RUN]), bytes);
-        }
-      }
-    } else if (K32 && bulk) {
-      if constexpr (K32) {
-#pragma unroll
-        for (int m = 0; m < (TN / 2 + NTHR - 1) / NTHR; ++m) {
-          const int q = 2 * (tid + NTHR * m), r = q / RUN, k = q - r * RUN;
-          const int g = row0 + Nx * NPP * r + k;
-          if (r < TYv && k < TXv * NPP && SGNB_INB(g, Nd - 1)) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-              const double2 x = *(const double2*)&S.G[v][q];
-              __stcs((float2*)(outk + v * Nd + g), make_float2((float)x.x, (float)x.y));
-            }
-          }
-        }
-      }
+      if (lane < NV && RXv > 0 && SGNB_INB(row0, Nd - rowv + 1))
+        bulk_store(outp + lane * Nd + row0, smem_addr(&S.G[lane][s0]), (unsigned)rowv * sizeof(double));
     } else {
 #pragma unroll
-      for (int m = 0; m < NIT; ++m) {
-        const int q = tid + NTHR * m, r = q / RUN, k = q - r * RUN;
-        const int g = row0 + Nx * NPP * r + k;
-        if (r < TYv && k < TXv * NPP && SGNB_INB(g, Nd)) {
+      for (int v = 0; v < NV; ++v)
 #pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            if (!K32 || out64 != nullptr) __stcs(&out64[v * Nd + g], S.G[v][q]);
-            else __stcs(&outk[v * Nd + g], (KT)S.G[v][q]);
-          }
-        }
-      }
-    }
-  }
-  // pairs of neighbouring nodes of this thread in one field of the tile, at 2 (tid + NTHR m):
-  // their offset in the field (-1: outside the mesh)
-  constexpr int NPR = (TN / 2 + NTHR - 1) / NTHR;
-  int gof[NPR];
-  bool two[NPR];
-  if constexpr (MODE == MODE_CAND || MODE == MODE_FSAL) {
-#pragma unroll
-    for (int m = 0; m < NPR; ++m) {
-      const int q = 2 * (tid + NTHR * m), r = q / RUN, k = q - r * RUN;
-      gof[m] = r < TYv && k < TXv * NPP ? row0 + Nx * NPP * r + k : -1;
-      two[m] = k + 1 < TXv * NPP;
+        for (int m = 0; m < LPF; ++m)
+          if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd))
+            store_pair(outp + v * Nd + row0 + kp + 2 * LPL * m, *(const double2*)&S.G[v][s0 + kp + 2 * LPL * m],
+                       false, two[m]);
     }
   }
   if constexpr (MODE == MODE_CAND) {
     // k3 is used up here: the candidate uNew = u + dt (2/9 k1 + 1/3 k2 + 4/9 k3) and the part
     // 7/24 k1 + 1/4 k2 + 1/3 k3 of the embedded solution leave instead (rk.cpp:106-121)
-    const double* __restrict__ u0 = pick(A.U, cur);
-    const KT* __restrict__ k1 = pick(A.K1, cur);
-    const KT* __restrict__ k2 = A.K2;
-    double* __restrict__ un = pick(A.U, cur ^ 1);
-    KT* __restrict__ pe = A.K3;
-    using KT2 = typename Pair<KT>::type;
-    double2 a[NPR], na[NPR];
-    KT2 b[NPR], c[NPR], nb[NPR], nc[NPR];
-    auto load = [&](int v, double2 (&x)[NPR], KT2 (&y)[NPR], KT2 (&z)[NPR]) {
-      const long long o = v * Nd;
+    const double* __restrict__ k1 = pick(A.K1, cur) + row0 + kp;
+    double* __restrict__ un = pick(A.U, cur ^ 1) + row0 + kp;
+    double* __restrict__ pe = A.K3 + row0 + kp;
+    // a rolled loop over the fields (unrolled, warps waited for instructions), the next field's
+    // k1 in flight
+    double2 b[LPF], nb[LPF];
+    auto load = [&](int v, double2 (&x)[LPF]) {
 #pragma unroll
-      for (int m = 0; m < NPR; ++m)
-        if (gof[m] >= 0 && SGNB_INB(o + gof[m], NV * Nd)) {
-          x[m] = load_pair(u0 + o + gof[m], bulk, two[m]);
-          y[m] = load_pair(k1 + o + gof[m], bulk, two[m]);
-          z[m] = load_pair(k2 + o + gof[m], bulk, two[m]);
-        }
+      for (int m = 0; m < LPF; ++m)
+        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) x[m] = load_pair(k1 + v * Nd + 2 * LPL * m, bulk, two[m]);
     };
-    load(0, a, b, c);
+    load(0, nb);
+    stash_put_wait();
+    const unsigned st = S.stash + ((unsigned)w << 21);
 #pragma unroll 1
     for (int v = 0; v < NV; ++v) {
-      if (v + 1 < NV) load(v + 1, na, nb, nc);  // the next field's, in flight
-      const long long o = v * Nd;
 #pragma unroll
-      for (int m = 0; m < NPR; ++m)
-        if (gof[m] >= 0 && SGNB_INB(o + gof[m], NV * Nd)) {
-          const double2 k3 = *(const double2*)&S.G[v][2 * (tid + NTHR * m)];
-          double2 x;
-          KT2 p;
-          x.x = fsal_finish(a[m].x, fsal_part(b[m].x, c[m].x), k3.x, dt);
-          x.y = fsal_finish(a[m].y, fsal_part(b[m].y, c[m].y), k3.y, dt);
-          p.x = (KT)emb_part(b[m].x, c[m].x, k3.x);
-          p.y = (KT)emb_part(b[m].y, c[m].y, k3.y);
-          store_pair(un + o + gof[m], x, bulk, two[m]);
-          store_pair(pe + o + gof[m], p, bulk, two[m]);
+      for (int m = 0; m < LPF; ++m) b[m] = nb[m];
+      if (v + 1 < NV) load(v + 1, nb);
+      double2 a[LPF], c[LPF];
+      __syncwarp();
+      stash_get(st + 4 * LPF * v, a);
+      stash_get(st + 4 * LPF * (NV + v), c);
+#pragma unroll
+      for (int m = 0; m < LPF; ++m) {
+        const double2 k3 = *(const double2*)&S.G[v][s0 + kp + 2 * LPL * m];  // (within shared memory)
+        double2 x, p;
+        x.x = fsal_finish(a[m].x, fsal_part(b[m].x, c[m].x), k3.x, dt);
+        x.y = fsal_finish(a[m].y, fsal_part(b[m].y, c[m].y), k3.y, dt);
+        p.x = emb_part(b[m].x, c[m].x, k3.x);
+        p.y = emb_part(b[m].y, c[m].y, k3.y);
+        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) {
+          store_pair(un + v * Nd + 2 * LPL * m, x, bulk, two[m]);
+          store_pair(pe + v * Nd + 2 * LPL * m, p, bulk, two[m]);
         }
-#pragma unroll
-      for (int m = 0; m < NPR; ++m) { a[m] = na[m]; b[m] = nb[m]; c[m] = nc[m]; }
+      }
     }
   }
   if constexpr (GHOST && AXPY) {
-    // Fused edge exchange (as in fused_tile): the next stage's input at the slab's edge
-    // nodes, straight into the neighbours' ghost arrays
-    const bool outLo = C.edgeL != nullptr && ex0 == 0, outHi = C.edgeR != nullptr && ex0 + TXv == Nx;
-    if (outLo || outHi) {
+    // Fused edge exchange (as in fused_tile): the next stage's input at the slab's edge nodes of
+    // this row, straight into the neighbours' ghost arrays
+    const bool outLo = C.edgeL != nullptr && ex0 == 0 && wx == 0;
+    const bool outHi = C.edgeR != nullptr && ex0 + wx * LROW + RXv == Nx;
+    if (RXv > 0 && (outLo || outHi)) {
       const double* __restrict__ u0 = pick(A.U, cur);
-      const KT* __restrict__ k1 = pick(A.K1, cur);
-      const KT* __restrict__ k2 = A.K2;
-      const int per = NV * TYv * NP;
-      for (int q = tid; q < 2 * per; q += NTHR) {
-        const int side = q / per;
+      const double* __restrict__ k1 = pick(A.K1, cur);
+      const double* __restrict__ k2 = A.K2;
+      for (int q = lane; q < 2 * NV * NP; q += 32) {
+        const int side = q / (NV * NP), r = q - side * NV * NP, t = r % NP, v = r / NP;
         if (side == 0 ? !outLo : !outHi) continue;
-        const int r = q - side * per;
-        const int t = r % NP, ry = (r / NP) % TYv, v = r / (NP * TYv);
-        const int ixe = side == 0 ? 0 : TXv - 1;
-        const int node = (side == 0 ? 0 : NP - 1) + NP * t;
-        const long long g = (long long)v * Nd + ((long long)(ex0 + ixe) + (long long)Nx * (ey0 + ry)) * NPP + node;
-        const double kout = S.G[v][(TX * ry + ixe) * NPP + node];
-        const long long ge = (long long)v * Ny * NP + (long long)(ey0 + ry) * NP + t;
+        const int at = side == 0 ? NP * t : (RXv - 1) * NPP + NP - 1 + NP * t;
+        const long long g = (long long)v * Nd + row0 + at;
+        const double kout = S.G[v][s0 + at];
+        const long long ge = (long long)v * Ny * NP + (long long)(ey0 + iy) * NP + t;
         if (!SGNB_INB(g, NV * Nd) || !SGNB_INB(ge, (long long)NV * Ny * NP)) continue;
         (side == 0 ? C.edgeL : C.edgeR)[ge] =
             MODE == MODE_STAGE ? stage_axpy(u0[g], 0.75 * dt, kout)
@@ -579,70 +643,77 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     }
   }
   if constexpr (MODE == MODE_FSAL) {
-    // scaled embedded error (rk.cpp:118-128) of the tile
+    // scaled embedded error (rk.cpp:118-128) of the row, then of the tile
     const CtrlReload rc = ctrl_reload(A.ctrl);
-    const double* __restrict__ u0 = pick(A.U, rc.cur);
-    const KT* __restrict__ pe = A.K3;
-    using KT2 = typename Pair<KT>::type;
     double esum = 0.0, emax = 0.0;
-    // sc >= atol: where that is a normal number, so is sc, and the reciprocal of a few ulp serves
-    const bool normal = rc.atol >= 2.2250738585072014e-308;
-    auto err = [&](double u, double p, double un, double k4) {
-      const double e = un - fma(rc.dt, fma(0.125, k4, p), u);
-      const double au = fabs(u), an = fabs(un);
-      const double sc = fma(rc.rtol, au < an ? an : au, rc.atol);
-      const double rr = normal ? e * fast_rcp(sc) : e / sc;
-      esum = fma(rr, rr, esum);  // a NaN stays in the sum
-      const double ar = fabs(rr);
-      emax = emax < ar ? ar : emax;
-    };
-    double2 a[NPR], na[NPR];
-    KT2 p[NPR], np[NPR];
-    auto load = [&](int v, double2 (&x)[NPR], KT2 (&y)[NPR]) {
-      const long long o = v * Nd;
+    const double* __restrict__ pe = A.K3 + row0 + kp;
+    double2 p[LPF], np[LPF];
+    auto load = [&](int v, double2 (&x)[LPF]) {
 #pragma unroll
-      for (int m = 0; m < NPR; ++m)
-        if (gof[m] >= 0 && SGNB_INB(o + gof[m], NV * Nd)) {
-          x[m] = load_pair(u0 + o + gof[m], bulk, two[m]);
-          y[m] = load_pair(pe + o + gof[m], bulk, two[m]);
-        }
+      for (int m = 0; m < LPF; ++m)
+        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) x[m] = load_pair(pe + v * Nd + 2 * LPL * m, bulk, two[m]);
     };
-    load(0, a, p);
+    load(0, np);
+    stash_put_wait();
+    const unsigned st = S.stash + ((unsigned)w << 21);
+    // every lane computes every value, and those outside the mesh are dropped by selection (their
+    // operands are whatever shared memory holds): branches would keep the values from overlapping
+    auto errors = [&](auto divide) {
+      auto err = [&](double u, double q, double un, double k4, bool there) {
+        const double e = un - fma(rc.dt, fma(0.125, k4, q), u);
+        const double au = fabs(u), an = fabs(un);
+        double rr = divide(e, fma(rc.rtol, au < an ? an : au, rc.atol));
+        rr = there ? rr : 0.0;
+        esum = fma(rr, rr, esum);  // a NaN stays in the sum
+        const double ar = fabs(rr);
+        emax = emax < ar ? ar : emax;
+      };
 #pragma unroll 1
-    for (int v = 0; v < NV; ++v) {
-      if (v + 1 < NV) load(v + 1, na, np);  // the next field's, in flight
+      for (int v = 0; v < NV; ++v) {
 #pragma unroll
-      for (int m = 0; m < NPR; ++m)
-        if (gof[m] >= 0) {
-          const int q = 2 * (tid + NTHR * m);
-          const double2 un = *(const double2*)&S.U[v][q], k4 = *(const double2*)&S.G[v][q];
-          err(a[m].x, p[m].x, un.x, k4.x);
-          if (two[m]) err(a[m].y, p[m].y, un.y, k4.y);
+        for (int m = 0; m < LPF; ++m) p[m] = np[m];
+        if (v + 1 < NV) load(v + 1, np);
+        double2 a[LPF];
+        __syncwarp();
+        stash_get(st + 4 * LPF * v, a);
+#pragma unroll
+        for (int m = 0; m < LPF; ++m) {
+          const double2 un = *(const double2*)&S.U[v][s0 + kp + 2 * LPL * m];
+          const double2 k4 = *(const double2*)&S.G[v][s0 + kp + 2 * LPL * m];
+          err(a[m].x, p[m].x, un.x, k4.x, in[m]);
+          err(a[m].y, p[m].y, un.y, k4.y, in[m] && two[m]);
         }
-#pragma unroll
-      for (int m = 0; m < NPR; ++m) { a[m] = na[m]; p[m] = np[m]; }
-    }
-    const int enan = esum != esum;
-    reduce_error(esum, emax, enan, S.red, A.partials, blk);
+      }
+    };
+    // the scale is at least atol: where that is a normal number, so is the scale, and the
+    // reciprocal of a few ulp serves
+    if (rc.atol >= 2.2250738585072014e-308) errors([](double e, double sc) { return e * fast_rcp(sc); });
+    else errors([](double e, double sc) { return e / sc; });
+    reduce_error<LWARPS>(esum, emax, esum != esum, S.red, A.partials, blk);
   }
-  if (bulk_out && j == 0) bulk_store_wait();  // shared memory is read out
+  if (bulk_out && lane < NV) bulk_store_wait();  // shared memory is read out
   if (bulk) {
     // a persistent CTA's next tile: its copies write what this one read and wrote, and its
-    // first thread initialises the barrier again
+    // warps initialise their barriers again
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
-    if (tid == 0) mbar_inval(mbar);
+    __syncwarp();
+    if (lane == 0) mbar_inval(mbar);
   }
 }
 
-// FRIC: Manning friction compiled in. GHOST: slab edges compiled in. Args: StageArgs (FP64
-// stage derivatives) or StageArgsM (FP32).
-template <int MODE, bool FRIC, bool GHOST, class Args>
-__global__ void __launch_bounds__(NTHR, 3) k_line(const RhsConsts C, const Args A, const int bulk) {
+// FRIC: Manning friction compiled in. GHOST: slab edges compiled in.
+template <int MODE, bool FRIC, bool GHOST>
+__global__ void __launch_bounds__(LTHR, (kLineCtas<MODE, 1>))
+    k_line(const LineConsts C, const LineTables T, const StageArgs A) {
   extern __shared__ __align__(128) unsigned char smem_line[];
-  auto& S = *reinterpret_cast<typename LineTile<8, 4>::Smem*>(smem_line);
-  line_tile<MODE, 8, 4, FRIC, GHOST, typename Args::K>(C, C.eo, A, blockIdx.x, blockIdx.y,
-                                                       (long long)blockIdx.y * gridDim.x + blockIdx.x, bulk != 0, S);
+  auto& S = *reinterpret_cast<typename LineTile<1>::Smem*>(smem_line);
+  if (kStash<MODE> && threadIdx.x < 32) stash_alloc(&S.stash);
+  line_tile<MODE, 1, FRIC, GHOST>(C, T, A, blockIdx.x, blockIdx.y,
+                                  (long long)blockIdx.y * gridDim.x + blockIdx.x, C.bulk != 0, S);
+  if constexpr (kStash<MODE>) {
+    __syncthreads();
+    if (threadIdx.x < 32) stash_free(S.stash);
+  }
 }
 
 }  // namespace dev
