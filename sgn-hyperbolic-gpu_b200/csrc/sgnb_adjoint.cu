@@ -17,24 +17,20 @@
 //   * the cotangent of the neighbour's trace node across each face (a per-face buffer the
 //     gather kernel adds to the neighbour's node) or, at a wall, folded back through the
 //     mirror ghost onto the own trace;
-//   * the cotangents of the depth statics: nodal H (fluxes and sources), the nodal dH/dx,
-//     dH/dy (sources, x pass) and the face depths, per face side.
+//   * the cotangents of the depth statics: nodal H (fluxes and sources) and the nodal dH/dx,
+//     dH/dy (sources, x pass); that of the face depths is zero (they cancel in F* - F(own)).
 // The gather kernel (one thread per node) sums the two directions and the neighbours'
 // face contributions in a fixed order, so the result is deterministic without atomics,
 // and folds in the RK-stage combination. Built with -fmad=true like the fast forward.
 #include "sgnb_checked.cuh"
 #include "sgnb_device.h"
+#include "sgnb_fastmath.cuh"
 
 namespace sgnb {
 namespace dev {
 namespace {
 
 constexpr int NP = 5, NPP = 25, NV = 5;
-
-struct LineIn {
-  double U[NP][NV];  // stage input y at the line's nodes
-  double H[NP];
-};
 
 __device__ __forceinline__ double stage_in(const VjpArgs& A, long long idx) {
   // y = u or u + (c dt) k, with the forward's rounding (stage_axpy of the fused kernels)
@@ -43,314 +39,339 @@ __device__ __forceinline__ double stage_in(const VjpArgs& A, long long idx) {
 
 __device__ __forceinline__ double sgn0(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? -1.0 : 0.0); }
 
-// Cotangent of the primitive variables (u, v, w, p) = (hu, hv, hw, hp) / h at a point,
-// added to the conserved cotangent Ub.
-__device__ __forceinline__ void prim_back(const double* U, double ub, double vb, double wb,
-                                          double pb, double* Ub) {
-  const double ih = 1.0 / U[0];
-  const double u = U[1] * ih, v = U[2] * ih, w = U[3] * ih, p = U[4] * ih;
-  Ub[1] += ub * ih;
-  Ub[2] += vb * ih;
-  Ub[3] += wb * ih;
-  Ub[4] += pb * ih;
-  Ub[0] -= (ub * u + vb * v + wb * w + pb * p) * ih;
-}
-
-// Reverse of the directional flux F = flux_DIR(U, H): adds to Ub, returns dH.
+// One line: reverse of its contribution to R (see the file comment). With the forward in the
+// form F_v = u_n U_v (plus g/2 (h^2 - H^2) + hp in the normal discharge and c^2 h u_n in hp), the
+// cotangent of a field's flux at a node goes to U_v and to u_n, and the fields can be taken one
+// after the other: a field's cotangent and state are loaded when its turn comes, and what stays
+// live is h, h u_n, hp, 1/h, u_n and their accumulators. (With every field's state, cotangent and
+// result live at once the kernels took 254 registers, 8 warps per SM.) The Rusanov flux minus the
+// own face flux does not depend on the face depth, so its cotangent is zero.
 template <int DIR>
-__device__ __forceinline__ double flux_back(const RhsConsts& C, const double* U, double H,
-                                            const double* Fb, double* Ub) {
-  constexpr int nd = 1 + DIR, td = 2 - DIR;
-  const double ih = 1.0 / U[0];
-  const double hn = U[nd];
-  const double n = hn * ih, t = U[td] * ih, w = U[3] * ih, p = U[4] * ih;
-  // F0 = hn, F[nd] = hn n + g/2 (h^2 - H^2) + hp, F[td] = hn t, F3 = hn w, F4 = hn (p + c^2)
-  const double hnb = Fb[0] + Fb[nd] * n + Fb[td] * t + Fb[3] * w + Fb[4] * (p + C.c2);
-  const double nb = Fb[nd] * hn, tb = Fb[td] * hn, wb = Fb[3] * hn, pb = Fb[4] * hn;
-  Ub[0] += Fb[nd] * C.g * U[0];
-  Ub[4] += Fb[nd];
-  Ub[nd] += hnb;
-  double q[4] = {0.0, 0.0, wb, pb};
-  q[nd - 1] = nb;
-  q[td - 1] = tb;
-  prim_back(U, q[0], q[1], q[2], q[3], Ub);
-  return -Fb[nd] * C.g * H;
-}
-
-// Wave speed ws = |u_n| + sqrt(max(g h + p + c^2, 0)) (sgn_flux2d.h:73-86).
-template <int DIR>
-__device__ __forceinline__ double wave_speed(const RhsConsts& C, const double* U) {
-  const double ih = 1.0 / U[0];
-  const double arg = C.g * U[0] + U[4] * ih + C.c2;
-  return fabs(U[1 + DIR] * ih) + sqrt(arg > 0.0 ? arg : 0.0);
-}
-
-template <int DIR>
-__device__ __forceinline__ void wave_speed_back(const RhsConsts& C, const double* U,
-                                                double lb, double* Ub) {
-  const double ih = 1.0 / U[0];
-  const double un = U[1 + DIR] * ih;
-  const double arg = C.g * U[0] + U[4] * ih + C.c2;
-  const double unb = sgn0(un) * lb;  // |x|' = sign(x), 0 at 0 (the central difference)
-  double ab = 0.0;
-  if (arg > 0.0) ab = 0.5 * lb / sqrt(arg);
-  Ub[0] += C.g * ab;
-  double q[4] = {0.0, 0.0, 0.0, ab};
-  q[DIR] = unb;
-  prim_back(U, q[0], q[1], q[2], q[3], Ub);
-}
-
-// One line: reverse of its contribution to R (see the file comment).
-template <int DIR>
-__global__ void __launch_bounds__(128) k_vjp_lines(const RhsConsts C, const FrTablesDev T,
-                                                   const VjpArgs A) {
-  const long long ne = (long long)C.Nx * C.Ny;
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= ne * NP) return;
+__device__ __forceinline__ void vjp_line(const RhsConsts& C, const FrTablesDev& T, const VjpArgs& A,
+                                         long long idx) {
   const long long e = idx / NP;
   const int j = (int)(idx - e * NP);
   const int ex = (int)(e % C.Nx), ey = (int)(e / C.Nx);
   const long long Nd = C.Nd;
-  constexpr int nd = 1 + DIR;
-  auto node = [&](int m) -> long long {
-    return e * NPP + (DIR == 0 ? m + NP * j : j + NP * m);
+  constexpr int N = 1 + DIR, TG = 2 - DIR;  // normal and tangential discharge
+  constexpr int SN = DIR == 0 ? 1 : NP;
+  const long long g0 = e * NPP + (DIR == 0 ? NP * j : j);  // the line's first node
+  const double iJ = DIR == 0 ? C.iJx : C.iJy, c2 = C.c2, gr = C.g;
+  [[maybe_unused]] const bool line_ok = SGNB_INB(g0, Nd) && SGNB_INB(g0 + 4 * SN, Nd);
+#ifdef SGNB_CHECKED
+  if (!line_ok) return;
+#endif
+  auto state = [&](int v, long long g) { return stage_in(A, v * Nd + g); };
+  auto cot = [&](int v, int m) {
+    const long long g = v * Nd + g0 + SN * m;
+    double r = A.alpha * A.ra[g];
+    if (A.rb) r += A.beta * A.rb[g];
+    return r;
   };
-  const double iJ = DIR == 0 ? C.iJx : C.iJy;
-
-  // ---- forward quantities of the line ---------------------------------------------
-  LineIn L;
-  double Rb[NP][NV];
-#pragma unroll
-  for (int m = 0; m < NP; ++m) {
-    const long long g = node(m);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const bool ok = SGNB_INB(v * Nd + g, NV * Nd);
-      L.U[m][v] = ok ? stage_in(A, v * Nd + g) : 0.0;
-      double r = ok ? A.alpha * A.ra[v * Nd + g] : 0.0;
-      if (A.rb && ok) r += A.beta * A.rb[v * Nd + g];
-      Rb[m][v] = r;
-    }
-    L.H[m] = SGNB_INB(g, Nd) ? C.Hnod[g] : 0.0;
-  }
-  bool wallLo, wallHi;
-  long long nLo, nHi;  // neighbour trace nodes
-  double HfLo, HfHi;
+  // neighbour trace nodes
+  const bool wallLo = DIR == 0 ? (C.bcx && ex == 0) : (C.bcy && ey == 0);
+  const bool wallHi = DIR == 0 ? (C.bcx && ex == C.Nx - 1) : (C.bcy && ey == C.Ny - 1);
+  long long nLo, nHi;
   if (DIR == 0) {
-    wallLo = C.bcx && ex == 0;
-    wallHi = C.bcx && ex == C.Nx - 1;
-    const long long eL = (long long)((ex - 1 + C.Nx) % C.Nx) + (long long)C.Nx * ey;
-    const long long eR = (long long)((ex + 1) % C.Nx) + (long long)C.Nx * ey;
-    nLo = eL * NPP + (NP - 1) + NP * j;
-    nHi = eR * NPP + NP * j;
-    HfLo = SGNB_INB(e * NP + j, ne * NP) ? C.HfX[e * NP + j] : 0.0;
-    HfHi = SGNB_INB(wallHi ? (long long)ey * NP + j : eR * NP + j, wallHi ? (long long)C.Ny * NP : ne * NP)
-               ? (wallHi ? C.HfXEnd[(long long)ey * NP + j] : C.HfX[eR * NP + j]) : 0.0;
+    nLo = ((ex == 0 ? C.Nx - 1 : ex - 1) + (long long)C.Nx * ey) * NPP + (NP - 1) + NP * j;
+    nHi = ((ex == C.Nx - 1 ? 0 : ex + 1) + (long long)C.Nx * ey) * NPP + NP * j;
   } else {
-    wallLo = C.bcy && ey == 0;
-    wallHi = C.bcy && ey == C.Ny - 1;
-    const long long eB = (long long)ex + (long long)C.Nx * ((ey - 1 + C.Ny) % C.Ny);
-    const long long eT = (long long)ex + (long long)C.Nx * ((ey + 1) % C.Ny);
-    nLo = eB * NPP + j + NP * (NP - 1);
-    nHi = eT * NPP + j;
-    HfLo = SGNB_INB(e * NP + j, ne * NP) ? C.HfY[e * NP + j] : 0.0;
-    HfHi = SGNB_INB(wallHi ? (long long)ex * NP + j : eT * NP + j, wallHi ? (long long)C.Nx * NP : ne * NP)
-               ? (wallHi ? C.HfYEnd[(long long)ex * NP + j] : C.HfY[eT * NP + j]) : 0.0;
+    nLo = (ex + (long long)C.Nx * (ey == 0 ? C.Ny - 1 : ey - 1)) * NPP + j + NP * (NP - 1);
+    nHi = (ex + (long long)C.Nx * (ey == C.Ny - 1 ? 0 : ey + 1)) * NPP + j;
   }
-  double sLo[NV], sHi[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    sLo[v] = wallLo ? (v == nd ? -L.U[0][v] : L.U[0][v])
-                    : (SGNB_INB(v * Nd + nLo, NV * Nd) ? stage_in(A, v * Nd + nLo) : 0.0);
-    sHi[v] = wallHi ? (v == nd ? -L.U[NP - 1][v] : L.U[NP - 1][v])
-                    : (SGNB_INB(v * Nd + nHi, NV * Nd) ? stage_in(A, v * Nd + nHi) : 0.0);
-  }
-  const double* tLo = L.U[0];
-  const double* tHi = L.U[NP - 1];
-  const double jhLo = 0.5 * (sLo[0] + tLo[0]) - tLo[0];
-  const double jhHi = 0.5 * (tHi[0] + sHi[0]) - tHi[0];
+  if (wallLo) nLo = g0;
+  if (wallHi) nHi = g0 + 4 * SN;
+#ifdef SGNB_CHECKED
+  if (!SGNB_INB(nLo, Nd) || !SGNB_INB(nHi, Nd)) return;
+#endif
+  const double sgnLo = wallLo ? -1.0 : 1.0, sgnHi = wallHi ? -1.0 : 1.0;
 
-  double Ub[NP][NV];
-  double Hb[NP];
+  // ---- forward quantities ---------------------------------------------------------------
+  double h[NP], hn[NP], hp[NP], ih[NP], un[NP];
 #pragma unroll
-  for (int m = 0; m < NP; ++m) {
-    Hb[m] = 0.0;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) Ub[m][v] = 0.0;
+  for (int k = 0; k < NP; ++k) {
+    const long long g = g0 + SN * k;
+    h[k] = state(0, g);
+    hn[k] = state(N, g);
+    hp[k] = state(4, g);
+    ih[k] = fast_rcp(h[k]);
+    un[k] = hn[k] * ih[k];
   }
-  double sLb[NV], sHb[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) { sLb[v] = 0.0; sHb[v] = 0.0; }
-  double HfLb = 0.0, HfHb = 0.0;
+  const double hL = state(0, nLo), hnL = sgnLo * state(N, nLo), hpL = state(4, nLo);
+  const double hR = state(0, nHi), hnR = sgnHi * state(N, nHi), hpR = state(4, nHi);
+  const double ihL = fast_rcp(hL), ihR = fast_rcp(hR), unL = hnL * ihL, unR = hnR * ihR;
+  // root of the wave speed (0 where its argument is not positive: its derivative is dropped then)
+  auto root = [&](double hh, double pp) {
+    const double a = fma(gr, hh, pp) + c2;
+    return a > 0.0 ? fast_sqrt(a) : 0.0;
+  };
+  const double cLs = root(hL, hpL * ihL), cLt = root(h[0], hp[0] * ih[0]);
+  const double cRs = root(hR, hpR * ihR), cRt = root(h[4], hp[4] * ih[4]);
+  const double wLs = fabs(unL) + cLs, wLt = fabs(un[0]) + cLt, wRs = fabs(unR) + cRs, wRt = fabs(un[4]) + cRt;
+  const bool sideL = wLs >= wLt, sideR = !(wRt >= wRs);  // the neighbour's speed is the larger one
+  const double lamL = 0.5 * fmax(wLs, wLt), lamR = 0.5 * fmax(wRs, wRt);
 
-  // ---- non-conservative term B_m = -c^2 u_n dh_m, R[hp] -= B_m -----------------------
-  {
-    double dhb[NP];
+  // accumulators: own nodes, and the neighbours' traces (left L, right R)
+  double hb[NP], hnb[NP], hpb[NP], unb[NP], Hb[NP];
+  double hLb = 0.0, hnLb = 0.0, hpLb = 0.0, unLb = 0.0, lamLb = 0.0;
+  double hRb = 0.0, hnRb = 0.0, hpRb = 0.0, unRb = 0.0, lamRb = 0.0;
+
+  double R[NP], Fb[NP], jL, jR;
+  // cotangents of field v's fluxes (nodes; low and high jump) from its cotangent R
+  auto flux_cot = [&](int v) {
+    jL = 0.0;
+    jR = 0.0;
 #pragma unroll
     for (int m = 0; m < NP; ++m) {
-      double s = jhLo * T.gLp[m] + jhHi * T.gRp[m];
-#pragma unroll
-      for (int k = 0; k < NP; ++k) s += T.D[m * NP + k] * L.U[k][0];
-      const double dh = s * iJ;
-      const double Bb = -Rb[m][4];
-      const double un = L.U[m][nd] / L.U[m][0];
-      dhb[m] = C.mc2 * un * Bb;
-      double q[4] = {0.0, 0.0, 0.0, 0.0};
-      q[DIR] = C.mc2 * dh * Bb;
-      prim_back(L.U[m], q[0], q[1], q[2], q[3], Ub[m]);
+      R[m] = cot(v, m);
+      jL = fma(T.gLp[m], R[m], jL);
+      jR = fma(T.gRp[m], R[m], jR);
     }
-    double jhLb = 0.0, jhHb = 0.0;
+    jL *= -iJ;
+    jR *= -iJ;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      double s = 0.0;
+#pragma unroll
+      for (int m = 0; m < NP; ++m) s = fma(T.D[m * NP + k], R[m], s);
+      Fb[k] = -iJ * s;
+    }
+  };
+  // the own face fluxes leave with -1/2 of the jump; the wave speed's cotangent
+  auto own_faces = [&]() {
+    Fb[0] = fma(-0.5, jL, Fb[0]);
+    Fb[4] = fma(-0.5, jR, Fb[4]);
+  };
+  auto lam_cot = [&](double sL, double tL, double sR, double tR) {
+    lamLb = fma(0.5 * jL, sL - tL, lamLb);
+    lamRb = fma(-0.5 * jR, sR - tR, lamRb);
+  };
+
+  // ---- hp: flux u_n hp + c^2 h u_n; R[hp] += c^2 u_n dh ------------------------------------
+  flux_cot(4);
+  {
+    double gh[NP];
+    const double jhL = 0.5 * (hL - h[0]), jhR = 0.5 * (hR - h[4]);
+    double bL = 0.0, bR = 0.0;
 #pragma unroll
     for (int m = 0; m < NP; ++m) {
-      jhLb += T.gLp[m] * dhb[m];
-      jhHb += T.gRp[m] * dhb[m];
+      double s = fma(jhL, T.gLp[m], jhR * T.gRp[m]);
+#pragma unroll
+      for (int k = 0; k < NP; ++k) s = fma(T.D[m * NP + k], h[k], s);
+      const double r = c2 * iJ * R[m];
+      unb[m] = s * r;
+      gh[m] = un[m] * r;
+      bL = fma(T.gLp[m], gh[m], bL);
+      bR = fma(T.gRp[m], gh[m], bR);
     }
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
       double s = 0.0;
 #pragma unroll
-      for (int m = 0; m < NP; ++m) s += T.D[m * NP + k] * dhb[m];
-      Ub[k][0] += s * iJ;
+      for (int m = 0; m < NP; ++m) s = fma(T.D[m * NP + k], gh[m], s);
+      hb[k] = s;
     }
-    jhLb *= iJ;
-    jhHb *= iJ;
-    sLb[0] += 0.5 * jhLb;
-    Ub[0][0] -= 0.5 * jhLb;
-    sHb[0] += 0.5 * jhHb;
-    Ub[NP - 1][0] -= 0.5 * jhHb;
+    hLb = 0.5 * bL;
+    hb[0] -= 0.5 * bL;
+    hRb = 0.5 * bR;
+    hb[4] -= 0.5 * bR;
+  }
+  own_faces();
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    hpb[k] = un[k] * Fb[k];
+    unb[k] = fma(hp[k], Fb[k], unb[k]);
+    hnb[k] = c2 * Fb[k];
+  }
+  hpLb = fma(0.5 * jL, unL, lamL * jL);
+  unLb = 0.5 * jL * hpL;
+  hnLb = 0.5 * c2 * jL;
+  hpb[0] -= lamL * jL;
+  hpRb = fma(0.5 * jR, unR, -lamR * jR);
+  unRb = 0.5 * jR * hpR;
+  hnRb = 0.5 * c2 * jR;
+  hpb[4] += lamR * jR;
+  lam_cot(hpL, hp[0], hpR, hp[4]);
+
+  // ---- mass: h u_n -----------------------------------------------------------------------
+  flux_cot(0);
+  own_faces();
+#pragma unroll
+  for (int k = 0; k < NP; ++k) hnb[k] += Fb[k];
+  hnLb = fma(0.5, jL, hnLb);
+  hnRb = fma(0.5, jR, hnRb);
+  hLb = fma(lamL, jL, hLb);
+  hb[0] -= lamL * jL;
+  hRb = fma(-lamR, jR, hRb);
+  hb[4] += lamR * jR;
+  lam_cot(hL, h[0], hR, h[4]);
+
+  // ---- normal discharge: u_n (h u_n) + g/2 (h^2 - H^2) + hp ---------------------------------
+  flux_cot(N);
+#pragma unroll
+  for (int k = 0; k < NP; ++k) Hb[k] = -gr * C.Hnod[g0 + SN * k] * Fb[k];
+  own_faces();
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    unb[k] = fma(hn[k], Fb[k], unb[k]);
+    hnb[k] = fma(un[k], Fb[k], hnb[k]);
+    hb[k] = fma(gr * h[k], Fb[k], hb[k]);
+    hpb[k] += Fb[k];
+  }
+  unLb = fma(0.5 * jL, hnL, unLb);
+  hnLb = fma(0.5 * jL, unL, fma(lamL, jL, hnLb));
+  hLb = fma(0.5 * jL, gr * hL, hLb);
+  hpLb = fma(0.5, jL, hpLb);
+  hnb[0] -= lamL * jL;
+  unRb = fma(0.5 * jR, hnR, unRb);
+  hnRb = fma(0.5 * jR, unR, fma(-lamR, jR, hnRb));
+  hRb = fma(0.5 * jR, gr * hR, hRb);
+  hpRb = fma(0.5, jR, hpRb);
+  hnb[4] += lamR * jR;
+  lam_cot(hnL, hn[0], hnR, hn[4]);
+  // sources (x pass only; pointwise, sgn_flux2d.h:122-134): (g (h - H) + gamma p) dH/dx and the
+  // u dH/dx part of -2 c^2 (w + u dH/dx + v dH/dy)
+  if constexpr (DIR == 0) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      const long long g = g0 + SN * k;
+      const double Hx = C.Hx[g], r4 = C.m2c2 * cot(4, k), p = hp[k] * ih[k];
+      const double bath = fma(gr, h[k] - C.Hnod[g], C.gamma * p), s = Hx * R[k];
+      hb[k] = fma(gr, s, hb[k]);
+      Hb[k] = fma(-gr, s, Hb[k]);
+      hpb[k] = fma(C.gamma * s, ih[k], hpb[k]);
+      hb[k] = fma(-C.gamma * s * p, ih[k], hb[k]);
+      unb[k] = fma(Hx, r4, unb[k]);
+      A.Hxb[g] = fma(bath, R[k], un[k] * r4);
+    }
   }
 
-  // ---- flux divergence: dF_m = (D F + jLo gL' + jHi gR') / J, R -= dF ----------------
-  double jLb[NV], jHb[NV];
+  double* const oL = A.Sn[DIR][0] + idx * NV;
+  double* const oR = A.Sn[DIR][1] + idx * NV;
+  // ---- hw and the tangential discharge: u_n U_v ---------------------------------------------
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    double a = 0.0, b = 0.0;
+  for (int q = 0; q < 2; ++q) {
+    const int v = q == 0 ? 3 : TG;
+    double w[NP], wb[NP];
 #pragma unroll
-    for (int m = 0; m < NP; ++m) {
-      a -= T.gLp[m] * Rb[m][v];
-      b -= T.gRp[m] * Rb[m][v];
+    for (int k = 0; k < NP; ++k) w[k] = state(v, g0 + SN * k);
+    const double wL = state(v, nLo), wR = state(v, nHi);
+    flux_cot(v);
+    own_faces();
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      wb[k] = un[k] * Fb[k];
+      unb[k] = fma(w[k], Fb[k], unb[k]);
     }
-    jLb[v] = a * iJ;
-    jHb[v] = b * iJ;
+    wb[0] -= lamL * jL;
+    wb[4] += lamR * jR;
+    const double wLb = fma(0.5 * jL, unL, lamL * jL), wRb = fma(0.5 * jR, unR, -lamR * jR);
+    unLb = fma(0.5 * jL, wL, unLb);
+    unRb = fma(0.5 * jR, wR, unRb);
+    lam_cot(wL, w[0], wR, w[4]);
+    if constexpr (DIR == 0) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const long long g = g0 + SN * k;
+        const double r4 = C.m2c2 * cot(4, k), p = hp[k] * ih[k], x = w[k] * ih[k];
+        if (q == 0) {
+          // gamma p in hw, w in hp
+          wb[k] = fma(r4, ih[k], wb[k]);
+          const double pb = C.gamma * R[k];
+          hpb[k] = fma(pb, ih[k], hpb[k]);
+          hb[k] = fma(-ih[k], fma(r4, x, pb * p), hb[k]);
+        } else {
+          // (g (h - H) + gamma p) dH/dy, v dH/dy in hp, friction
+          const double Hy = C.Hy[g], s = Hy * R[k];
+          const double bath = fma(gr, h[k] - C.Hnod[g], C.gamma * p);
+          A.Hyb[g] = fma(bath, R[k], x * r4);
+          double vb = Hy * r4;
+          hb[k] = fma(gr, s, hb[k]);
+          Hb[k] = fma(-gr, s, Hb[k]);
+          if (C.manning) {
+            // (-cf u, -cf v), cf = n^2 g |vel| h^(-1/3)
+            const double r1 = cot(1, k), vm = sqrt(un[k] * un[k] + x * x);
+            const double kc = C.n2g / cbrt(h[k]), cf = kc * vm, ruv = r1 * un[k] + R[k] * x;
+            unb[k] -= r1 * cf;
+            vb -= R[k] * cf;
+            if (vm > 0.0) {
+              unb[k] -= kc * ruv * un[k] / vm;
+              vb -= kc * ruv * x / vm;
+            }
+            hb[k] += ruv * cf / (3.0 * h[k]);  // d/dh of h^(-1/3)
+          }
+          const double pb = C.gamma * s;
+          hpb[k] = fma(pb, ih[k], hpb[k]);
+          wb[k] = fma(vb, ih[k], wb[k]);
+          hb[k] = fma(-ih[k], fma(vb, x, pb * p), hb[k]);
+        }
+      }
+    }
+    // mirror ghosts fold back onto the own trace
+    if (wallLo) wb[0] += wLb; else oL[v] = wLb;
+    if (wallHi) wb[4] += wRb; else oR[v] = wRb;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) A.Ub[DIR][v * Nd + g0 + SN * k] = wb[k];
+  }
+
+  // ---- wave speed |u_n| + sqrt(g h + p + c^2) of the side that has the larger one; |x|' is
+  // sign(x), 0 at 0 (as the central difference) ------------------------------------------------
+  auto speed_back = [&](double lb, double cc, double hp_, double ih_, double un_, double& hb_, double& hpb_,
+                        double& unb_) {
+    unb_ = fma(sgn0(un_), lb, unb_);
+    const double ab = cc > 0.0 ? 0.5 * lb * fast_rcp(cc) : 0.0;
+    hpb_ = fma(ab, ih_, hpb_);
+    hb_ = fma(ab, fma(-hp_ * ih_, ih_, gr), hb_);
+  };
+  if (sideL) speed_back(lamLb, cLs, hpL, ihL, unL, hLb, hpLb, unLb);
+  else speed_back(lamLb, cLt, hp[0], ih[0], un[0], hb[0], hpb[0], unb[0]);
+  if (sideR) speed_back(lamRb, cRs, hpR, ihR, unR, hRb, hpRb, unRb);
+  else speed_back(lamRb, cRt, hp[4], ih[4], un[4], hb[4], hpb[4], unb[4]);
+
+  // ---- u_n = h u_n / h; results -----------------------------------------------------------
+  hnLb = fma(unLb, ihL, hnLb);
+  hLb = fma(-unLb * unL, ihL, hLb);
+  hnRb = fma(unRb, ihR, hnRb);
+  hRb = fma(-unRb * unR, ihR, hRb);
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    hnb[k] = fma(unb[k], ih[k], hnb[k]);
+    hb[k] = fma(-unb[k] * un[k], ih[k], hb[k]);
+  }
+  if (wallLo) {
+    hb[0] += hLb;
+    hnb[0] -= hnLb;
+    hpb[0] += hpLb;
+  } else {
+    oL[0] = hLb;
+    oL[N] = hnLb;
+    oL[4] = hpLb;
+  }
+  if (wallHi) {
+    hb[4] += hRb;
+    hnb[4] -= hnRb;
+    hpb[4] += hpRb;
+  } else {
+    oR[0] = hRb;
+    oR[N] = hnRb;
+    oR[4] = hpRb;
   }
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
-    double Fb[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      double s = 0.0;
-#pragma unroll
-      for (int m = 0; m < NP; ++m) s -= T.D[m * NP + k] * Rb[m][v];
-      Fb[v] = s * iJ;
-    }
-    Hb[k] += flux_back<DIR>(C, L.U[k], L.H[k], Fb, Ub[k]);
+    const long long g = g0 + SN * k;
+    A.Ub[DIR][g] = hb[k];
+    A.Ub[DIR][N * Nd + g] = hnb[k];
+    A.Ub[DIR][4 * Nd + g] = hpb[k];
+    A.Hb[DIR][g] = Hb[k];
   }
+}
 
-  // ---- faces: j = F* - F(t), Rusanov F* (low face: neighbour on the left) ------------
-  {
-    // low face: j = 1/2 Fn - 1/2 Fd - 1/2 lam (t - s)
-    const double wsS = wave_speed<DIR>(C, sLo), wsT = wave_speed<DIR>(C, tLo);
-    const double lam = fmax(wsS, wsT);
-    double Fnb[NV], Fdb[NV], lb = 0.0;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      Fnb[v] = 0.5 * jLb[v];
-      Fdb[v] = -0.5 * jLb[v];
-      lb -= 0.5 * jLb[v] * (tLo[v] - sLo[v]);
-      Ub[0][v] -= 0.5 * lam * jLb[v];
-      sLb[v] += 0.5 * lam * jLb[v];
-    }
-    HfLb += flux_back<DIR>(C, tLo, HfLo, Fdb, Ub[0]);
-    HfLb += flux_back<DIR>(C, sLo, HfLo, Fnb, sLb);
-    if (wsS >= wsT) wave_speed_back<DIR>(C, sLo, lb, sLb);
-    else wave_speed_back<DIR>(C, tLo, lb, Ub[0]);
-  }
-  {
-    // high face: j = 1/2 Fn - 1/2 Fd - 1/2 lam (s - t)
-    const double wsT = wave_speed<DIR>(C, tHi), wsS = wave_speed<DIR>(C, sHi);
-    const double lam = fmax(wsT, wsS);
-    double Fnb[NV], Fdb[NV], lb = 0.0;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      Fnb[v] = 0.5 * jHb[v];
-      Fdb[v] = -0.5 * jHb[v];
-      lb -= 0.5 * jHb[v] * (sHi[v] - tHi[v]);
-      sHb[v] -= 0.5 * lam * jHb[v];
-      Ub[NP - 1][v] += 0.5 * lam * jHb[v];
-    }
-    HfHb += flux_back<DIR>(C, tHi, HfHi, Fdb, Ub[NP - 1]);
-    HfHb += flux_back<DIR>(C, sHi, HfHi, Fnb, sHb);
-    if (wsT >= wsS) wave_speed_back<DIR>(C, tHi, lb, Ub[NP - 1]);
-    else wave_speed_back<DIR>(C, sHi, lb, sHb);
-  }
-
-  // ---- sources (x pass only; pointwise, sgn_flux2d.h:122-134) --------------------------
-  if (DIR == 0) {
-#pragma unroll
-    for (int m = 0; m < NP; ++m) {
-      const long long g = node(m);
-      const double* U = L.U[m];
-      if (!SGNB_INB(g, Nd)) continue;
-      const double Hx = C.Hx[g], Hy = C.Hy[g];
-      const double ih = 1.0 / U[0];
-      const double u = U[1] * ih, v = U[2] * ih, p = U[4] * ih;
-      const double r1 = Rb[m][1], r2 = Rb[m][2], r3 = Rb[m][3], r4 = Rb[m][4];
-      const double bath = C.g * (U[0] - L.H[m]) + C.gamma * p;
-      const double sHr = Hx * r1 + Hy * r2;
-      Ub[m][0] += C.g * sHr;
-      Hb[m] -= C.g * sHr;
-      A.Hxb[g] = bath * r1 + C.m2c2 * u * r4;
-      A.Hyb[g] = bath * r2 + C.m2c2 * v * r4;
-      double ub = C.m2c2 * Hx * r4, vb = C.m2c2 * Hy * r4;
-      if (C.manning) {
-        // friction (-cf u, -cf v), cf = n^2 g |vel| h^(-1/3)
-        const double vm = sqrt(u * u + v * v);
-        const double kc = C.n2g / cbrt(U[0]);
-        const double cf = kc * vm;
-        const double ruv = r1 * u + r2 * v;
-        ub -= r1 * cf;
-        vb -= r2 * cf;
-        if (vm > 0.0) {
-          ub -= kc * ruv * u / vm;
-          vb -= kc * ruv * v / vm;
-        }
-        Ub[m][0] += ruv * cf / (3.0 * U[0]);  // d/dh of h^(-1/3)
-      }
-      prim_back(U, ub, vb, C.m2c2 * r4, C.gamma * sHr + C.gamma * r3, Ub[m]);
-    }
-  }
-
-  // ---- mirror ghosts fold back onto the own trace ------------------------------------
-  if (wallLo) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) Ub[0][v] += v == nd ? -sLb[v] : sLb[v];
-  } else {
-    double* o = A.Sn[DIR][0] + idx * NV;
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      if (SGNB_INB(idx * NV + v, ne * NP * NV)) o[v] = sLb[v];
-  }
-  if (wallHi) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) Ub[NP - 1][v] += v == nd ? -sHb[v] : sHb[v];
-  } else {
-    double* o = A.Sn[DIR][1] + idx * NV;
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      if (SGNB_INB(idx * NV + v, ne * NP * NV)) o[v] = sHb[v];
-  }
-  if (SGNB_INB(idx, ne * NP)) {
-    A.Hf[DIR][0][idx] = HfLb;
-    A.Hf[DIR][1][idx] = HfHb;
-  }
-#pragma unroll
-  for (int m = 0; m < NP; ++m) {
-    const long long g = node(m);
-    if (!SGNB_INB(g, Nd)) continue;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) A.Ub[DIR][v * Nd + g] = Ub[m][v];
-    A.Hb[DIR][g] = Hb[m];
-  }
+// Both directions' lines in one launch (blockIdx.y: direction).
+__global__ void __launch_bounds__(128, 3) k_vjp_lines(const RhsConsts C, const FrTablesDev T, const VjpArgs A) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (long long)C.Nx * C.Ny * NP) return;
+  if (blockIdx.y == 0) vjp_line<0>(C, T, A, idx);
+  else vjp_line<1>(C, T, A, idx);
 }
 
 // One thread per node: the node's cotangent from both directions and from the
@@ -387,23 +408,6 @@ __global__ void __launch_bounds__(256) k_vjp_gather(const RhsConsts C, const Vjp
   G.Hacc[gnode] += A.Hb[0][gnode] + A.Hb[1][gnode];
   G.Hxacc[gnode] += A.Hxb[gnode];
   G.Hyacc[gnode] += A.Hyb[gnode];
-  [[maybe_unused]] const long long nf = (long long)C.Nx * C.Ny * NP;
-  if (a == 0 && SGNB_INB(e * NP + b, nf) && SGNB_INB(eL * NP + b, nf)) {
-    double s = A.Hf[0][0][e * NP + b];
-    if (!wL) s += A.Hf[0][1][eL * NP + b];
-    G.HfXacc[e * NP + b] += s;
-  }
-  if (a == NP - 1 && wR && SGNB_INB((long long)ey * NP + b, (long long)C.Ny * NP) &&
-      SGNB_INB(e * NP + b, nf))
-    G.HfXEndacc[(long long)ey * NP + b] += A.Hf[0][1][e * NP + b];
-  if (b == 0 && SGNB_INB(e * NP + a, nf) && SGNB_INB(eB * NP + a, nf)) {
-    double s = A.Hf[1][0][e * NP + a];
-    if (!wB) s += A.Hf[1][1][eB * NP + a];
-    G.HfYacc[e * NP + a] += s;
-  }
-  if (b == NP - 1 && wT && SGNB_INB((long long)ex * NP + a, (long long)C.Nx * NP) &&
-      SGNB_INB(e * NP + a, nf))
-    G.HfYEndacc[(long long)ex * NP + a] += A.Hf[1][1][e * NP + a];
 }
 
 // u_new = u + dt ((2/9 k1 + 1/3 k2) + 4/9 k3) with the end-point stage's rounding
@@ -458,8 +462,7 @@ cudaError_t launch_vjp_rhs(const RhsConsts& C, const FrTablesDev& T, const VjpAr
                            const GatherArgs& G, cudaStream_t s) {
   const long long lines = (long long)C.Nx * C.Ny * NP;
   const unsigned nb = (unsigned)((lines + 127) / 128);
-  k_vjp_lines<0><<<nb, 128, 0, s>>>(C, T, A);
-  k_vjp_lines<1><<<nb, 128, 0, s>>>(C, T, A);
+  k_vjp_lines<<<dim3(nb, 2), 128, 0, s>>>(C, T, A);
   const unsigned ng = (unsigned)((C.Nd + 255) / 256);
   k_vjp_gather<<<ng, 256, 0, s>>>(C, A, G);
   return cudaGetLastError();

@@ -77,7 +77,7 @@ cudaError_t fused(const sgnb_ctx* c, int mode, const StageArgs& A, cudaStream_t 
 
 // Scratch of one right-hand-side VJP, carved from `p` (advanced past it).
 size_t vjp_scratch_doubles(long long Nd, long long ne) {
-  return 2 * 5 * (size_t)Nd + 2 * (size_t)Nd + 2 * (size_t)Nd + 4 * 25 * (size_t)ne + 4 * 5 * (size_t)ne;
+  return 2 * 5 * (size_t)Nd + 2 * (size_t)Nd + 2 * (size_t)Nd + 4 * 25 * (size_t)ne;
 }
 void carve_vjp(VjpArgs& V, double*& p, long long Nd, long long ne) {
   for (int d = 0; d < 2; ++d) { V.Ub[d] = p; p += 5 * Nd; }
@@ -86,8 +86,6 @@ void carve_vjp(VjpArgs& V, double*& p, long long Nd, long long ne) {
   V.Hyb = p; p += Nd;
   for (int d = 0; d < 2; ++d)
     for (int f = 0; f < 2; ++f) { V.Sn[d][f] = p; p += 25 * ne; }
-  for (int d = 0; d < 2; ++d)
-    for (int f = 0; f < 2; ++f) { V.Hf[d][f] = p; p += 5 * ne; }
 }
 size_t stat_doubles(const sgnb_ctx* c) {
   const long long ne = (long long)c->desc.Nx * c->desc.Ny;

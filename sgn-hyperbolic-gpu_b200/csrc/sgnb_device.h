@@ -277,7 +277,6 @@ struct BatchArgs {
 //   Hxb,Hyb [Nd]     cotangents of dH/dx, dH/dy (x lines: sources)
 //   Sn[d][f][5 ne 5] cotangent of the neighbour's trace node across face f (0 low,
 //                    1 high) of line (e, j), field-minor
-//   Hf[d][f][5 ne]   cotangent of the face depth of face f of line (e, j)
 struct VjpArgs {
   const double* u;
   const double* k;
@@ -290,7 +289,6 @@ struct VjpArgs {
   double* Hxb;
   double* Hyb;
   double* Sn[2][2];
-  double* Hf[2][2];
 };
 
 // Outputs of the gather: ybar (optional) = the node cotangent of R's input;
