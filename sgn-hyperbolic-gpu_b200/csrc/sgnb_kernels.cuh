@@ -794,6 +794,7 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
   }
   __syncthreads();
 
+  let_next_start();
   // ---- row pass: x-line b = j, then assembly ---------------------------------
   // dU of node (a, j) replaces that node's column-pass results in S.G; only this
   // thread touches those slots in this phase.
@@ -1004,6 +1005,7 @@ __global__ void __launch_bounds__(NTHR, EXACT ? 2 : SGNB_FAST_MIN_CTAS) k_fused(
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using T = Tile<8, 4, EXACT>;
   typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_raw);
+  wait_for_previous();
   fused_tile<MODE, EXACT, 8, 4, RhsConsts, RhsConsts, StageArgs, FRIC, GHOST, GAUSS, FULL>(C, C, A, blockIdx.x, blockIdx.y,
                                 (long long)blockIdx.y * gridDim.x + blockIdx.x, S);
 }
@@ -1016,6 +1018,7 @@ __global__ void __launch_bounds__(NTHR, EXACT ? 2 : SGNB_FAST_MIN_CTAS)
   extern __shared__ __align__(128) unsigned char smem_tiles[];  // the copies' destinations
   using T = Tile<8, 4, EXACT>;
   typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_tiles);
+  wait_for_previous();
   fused_tile<MODE, EXACT, 8, 4, RhsConsts, RhsConsts, StageArgs, false, GHOST, false, true, true>(
       C, C, A, blockIdx.x, blockIdx.y, (long long)blockIdx.y * gridDim.x + blockIdx.x, S, &M);
 }
@@ -1026,6 +1029,7 @@ __global__ void __launch_bounds__(NTHR, EXACT ? 2 : SGNB_FAST_MIN_CTAS)
 // explicitly rounded, so both arithmetic modes (EXACT) form the same bits.
 template <int MODE, bool EXACT>
 __global__ void __launch_bounds__(256) k_traces(const RhsConsts C, const StageArgs A) {
+  wait_for_previous();
   const long long ne = (long long)C.Nx * C.Ny;
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= 2 * ne * NP) return;

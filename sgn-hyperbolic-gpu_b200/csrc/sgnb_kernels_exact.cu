@@ -12,29 +12,30 @@ static cudaError_t launch_mode(const RhsConsts& C, const StageArgs& A, cudaStrea
   if (C.gauss) return launch_gauss<MODE>(C, A, s);
   const dim3 grid((C.Nx + 7) / 8, (C.Ny + 3) / 4);
   const size_t smem = sizeof(Tile<8, 4, SGNB_EXACT>::Smem);
+  cudaError_t e;
   const bool ghost = C.ghostL != nullptr || C.ghostR != nullptr;
   if (C.manning) {
-    if (ghost) k_fused<MODE, SGNB_EXACT, true, true><<<grid, NTHR, smem, s>>>(C, A);
-    else k_fused<MODE, SGNB_EXACT, true, false><<<grid, NTHR, smem, s>>>(C, A);
+    if (ghost) e = launch_dependent(k_fused<MODE, SGNB_EXACT, true, true>, grid, dim3(NTHR), smem, s, C, A);
+    else e = launch_dependent(k_fused<MODE, SGNB_EXACT, true, false>, grid, dim3(NTHR), smem, s, C, A);
   } else {
     const bool full = C.Nx % 8 == 0 && C.Ny % 4 == 0;  // every tile full
     // the own-node tiles by the tensor-memory accelerator where the context's tensor maps
     // describe the buffers (and, for the rhs mode, a map of its input)
     const bool tma = full && M != nullptr && M->ok && (MODE != MODE_RHS || M->inOk);
     if (ghost) {
-      if (tma) k_fused_tma<MODE, SGNB_EXACT, true><<<grid, NTHR, smem, s>>>(C, A, *M);
-      else if (full) k_fused<MODE, SGNB_EXACT, false, true, false, true><<<grid, NTHR, smem, s>>>(C, A);
-      else k_fused<MODE, SGNB_EXACT, false, true><<<grid, NTHR, smem, s>>>(C, A);
+      if (tma) e = launch_dependent(k_fused_tma<MODE, SGNB_EXACT, true>, grid, dim3(NTHR), smem, s, C, A, *M);
+      else if (full) e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, true, false, true>, grid, dim3(NTHR), smem, s, C, A);
+      else e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, true>, grid, dim3(NTHR), smem, s, C, A);
     } else if (full) {
       if (tma)
-        k_fused_tma<MODE, SGNB_EXACT><<<grid, NTHR, smem, s>>>(C, A, *M);
+        e = launch_dependent(k_fused_tma<MODE, SGNB_EXACT>, grid, dim3(NTHR), smem, s, C, A, *M);
       else
-        k_fused<MODE, SGNB_EXACT, false, false, false, true><<<grid, NTHR, smem, s>>>(C, A);
+        e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, false, false, true>, grid, dim3(NTHR), smem, s, C, A);
     } else {
-      k_fused<MODE, SGNB_EXACT, false, false><<<grid, NTHR, smem, s>>>(C, A);
+      e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, false>, grid, dim3(NTHR), smem, s, C, A);
     }
   }
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s,

@@ -14,10 +14,11 @@ static cudaError_t launch_gauss(const RhsConsts& C, const StageArgs& A, cudaStre
   const dim3 grid((C.Nx + 7) / 8, (C.Ny + 3) / 4);
   const size_t smem = sizeof(Tile<8, 4, SGNB_EXACT>::Smem);
   const long long n = 2LL * C.Nx * C.Ny * NP;
-  k_traces<MODE, SGNB_EXACT><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(C, A);
-  if (C.manning) k_fused<MODE, SGNB_EXACT, true, false, true><<<grid, NTHR, smem, s>>>(C, A);
-  else k_fused<MODE, SGNB_EXACT, false, false, true><<<grid, NTHR, smem, s>>>(C, A);
-  return cudaGetLastError();
+  cudaError_t e = launch_dependent(k_traces<MODE, SGNB_EXACT>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, C, A);
+  if (e != cudaSuccess) return e;
+  if (C.manning) e = launch_dependent(k_fused<MODE, SGNB_EXACT, true, false, true>, grid, dim3(NTHR), smem, s, C, A);
+  else e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, false, true>, grid, dim3(NTHR), smem, s, C, A);
+  return e;
 }
 
 template <class K>

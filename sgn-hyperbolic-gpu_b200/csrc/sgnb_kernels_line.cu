@@ -19,8 +19,7 @@ static cudaError_t launch_variant(const RhsConsts& C, const StageArgs& A, int bu
   const dim3 grid((C.Nx + L::TX - 1) / L::TX, (C.Ny + L::TY - 1) / L::TY);
   LineConsts LC = line_consts(C);
   LC.bulk = bulk;
-  k_line<MODE, FRIC, GHOST><<<grid, LTHR, sizeof(typename L::Smem), s>>>(LC, C.eo, A);
-  return cudaGetLastError();
+  return launch_dependent(k_line<MODE, FRIC, GHOST>, grid, dim3(LTHR), sizeof(typename L::Smem), s, LC, C.eo, A);
 }
 
 template <int MODE>

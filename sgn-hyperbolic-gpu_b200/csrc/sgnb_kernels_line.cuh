@@ -544,6 +544,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
                              [&](int v, int k, double r) { gp[v * TN + k * NP] = r; });
   }
   __syncwarp();
+  let_next_start();
   // ---- row pass: x-lines, completes dU --------------------------------------------------
   {
     const int e = lane / NP, j = lane - NP * e, ix = wx * LROW + e;
@@ -708,6 +709,7 @@ __global__ void __launch_bounds__(LTHR, (kLineCtas<MODE, 1>))
   extern __shared__ __align__(128) unsigned char smem_line[];
   auto& S = *reinterpret_cast<typename LineTile<1>::Smem*>(smem_line);
   if (kStash<MODE> && threadIdx.x < 32) stash_alloc(&S.stash);
+  wait_for_previous();
   line_tile<MODE, 1, FRIC, GHOST>(C, T, A, blockIdx.x, blockIdx.y,
                                   (long long)blockIdx.y * gridDim.x + blockIdx.x, C.bulk != 0, S);
   if constexpr (kStash<MODE>) {

@@ -91,6 +91,7 @@ __device__ __forceinline__ bool controller_core(CtrlState* cg, const Row& row, l
   __shared__ double prevPow;
   constexpr int W = sizeof(CtrlState) / 8;
   static_assert(sizeof(CtrlState) % 8 == 0 && W <= kCtrlThreads, "copied by one word per thread");
+  wait_for_previous();
   if (cg->done) return false;
   const int t = threadIdx.x;
   CtrlState* const c = &state;
@@ -252,35 +253,30 @@ __global__ void __launch_bounds__(256) k_diag(int what, const RhsConsts C, const
 
 cudaError_t launch_controller(CtrlState* c, const double* partials, int nblk, long long n,
                               cudaStream_t s) {
-  k_controller<<<1, kCtrlThreads, 0, s>>>(c, partials, nblk, n);
-  return cudaGetLastError();
+  return launch_dependent(k_controller, dim3(1), dim3(kCtrlThreads), 0, s, c, partials, nblk, n);
 }
 
 cudaError_t launch_controller_loop(CtrlState* c, const double* partials, int nblk, long long n,
                                    cudaGraphConditionalHandle loop, cudaStream_t s) {
-  k_controller_loop<<<1, kCtrlThreads, 0, s>>>(c, partials, nblk, n, loop);
-  return cudaGetLastError();
+  return launch_dependent(k_controller_loop, dim3(1), dim3(kCtrlThreads), 0, s, c, partials, nblk, n, loop);
 }
 
 cudaError_t launch_controller_batch_loop(CtrlState* ctrls, const double* const* partials,
                                          const int* nblk, const long long* n, int ninst,
                                          int* counters, cudaGraphConditionalHandle loop,
                                          cudaStream_t s) {
-  k_controller_batch_loop<<<ninst, kCtrlThreads, 0, s>>>(ctrls, partials, nblk, n, counters, loop);
-  return cudaGetLastError();
+  return launch_dependent(k_controller_batch_loop, dim3(ninst), dim3(kCtrlThreads), 0, s, ctrls, partials, nblk, n, counters, loop);
 }
 
 cudaError_t launch_controller_slabs(CtrlState* c, const SlabPartials& L, long long n,
                                     cudaStream_t s) {
-  k_controller_slabs<<<1, kCtrlThreads, 0, s>>>(c, L, n);
-  return cudaGetLastError();
+  return launch_dependent(k_controller_slabs, dim3(1), dim3(kCtrlThreads), 0, s, c, L, n);
 }
 
 cudaError_t launch_controller_batch(CtrlState* ctrls, const double* const* partials,
                                     const int* nblk, const long long* n, int ninst,
                                     cudaStream_t s) {
-  k_controller_batch<<<ninst, kCtrlThreads, 0, s>>>(ctrls, partials, nblk, n);
-  return cudaGetLastError();
+  return launch_dependent(k_controller_batch, dim3(ninst), dim3(kCtrlThreads), 0, s, ctrls, partials, nblk, n);
 }
 
 // ---- rk4Step (src/solver/rk.cpp:23-38) -------------------------------------------------
