@@ -51,9 +51,6 @@ struct Launch {
   int stage = 2;               // 2 (adds k1) or 3 (adds k2)
 };
 
-static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
-                             CUtensorMapDataType type, size_t elem, cuuint32_t nz);
-
 cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
   if (c->mixed) {
     StageArgsM A{};
@@ -81,22 +78,7 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
   A.coef = L.stage == 3 ? 0.75 : 0.5;
   A.out = L.mode == 0 ? L.out : A.K2;
   if (c->precision == SGNB_FP64_FAST) return dev::launch_fused_fast(L.mode, c->C, A, s);
-  // tile copies by the tensor-memory accelerator: A names the context's buffers; the
-  // right-hand side's input gets its own map, encoded for this launch
-  const TileMaps* M = nullptr;
-  TileMaps Mr;
-  if (c->maps.ok) {
-    if (L.mode != 0) {
-      M = &c->maps;
-    } else if (L.in != nullptr) {
-      Mr = c->maps;
-      if (encode_state_map(c, &Mr.In, L.in, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, 5)) {
-        Mr.inOk = 1;
-        M = &Mr;
-      }
-    }
-  }
-  return dev::launch_fused_exact(L.mode, c->C, A, s, M);
+  return dev::launch_fused_exact(L.mode, c->C, A, s);
 }
 
 Launch rhs_launch(const double* in, double* out) {
@@ -225,11 +207,9 @@ static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
 // compiler chooses on its own, so they agree to round-off (tests/test_tma_gpu.py finds
 // the same bits for the whole-mesh kernels).
 static void build_tile_maps(sgnb_ctx* c) {
-  c->maps.ok = 0;
-  c->maps.inOk = 0;
   c->mapsM.ok = 0;
   c->encode_tiled = nullptr;
-  if (c->precision == SGNB_FP64_FAST) return;  // its kernels copy rows
+  if (!c->mixed) return;  // the FP64 modes' kernels copy rows
   if (c->desc.Nx % 8 != 0 || c->desc.Ny % 4 != 0) return;
   const char* sw = std::getenv("SGNB_TMA");
   if (sw && sw[0] == '0') return;
@@ -254,22 +234,12 @@ static void build_tile_maps(sgnb_ctx* c) {
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
            CUDA_SUCCESS;
   };
-  const auto F64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64, F32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  if (c->mixed) {
-    const bool okm = encode_state_map(c, &c->mapsM.K1[0], c->K1[0], F32, 4, 1) &&
-                     encode_state_map(c, &c->mapsM.K1[1], c->K1[1], F32, 4, 1) &&
-                     encode_state_map(c, &c->mapsM.K2, c->K2, F32, 4, 1) &&
-                     encode_state_map(c, &c->mapsM.K3, c->K3, F32, 4, 1) && mapH(&c->mapsM.H);
-    c->mapsM.ok = okm ? 1 : 0;
-    return;
-  }
-  const bool ok = encode_state_map(c, &c->maps.U[0], c->U[0], F64, 8, 5) &&
-                  encode_state_map(c, &c->maps.U[1], c->U[1], F64, 8, 5) &&
-                  encode_state_map(c, &c->maps.K1[0], c->K1[0], F64, 8, 5) &&
-                  encode_state_map(c, &c->maps.K1[1], c->K1[1], F64, 8, 5) &&
-                  encode_state_map(c, &c->maps.K2, c->K2, F64, 8, 5) &&
-                  encode_state_map(c, &c->maps.K3, c->K3, F64, 8, 5) && mapH(&c->maps.H);
-  c->maps.ok = ok ? 1 : 0;
+  const auto F32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  const bool ok = encode_state_map(c, &c->mapsM.K1[0], c->K1[0], F32, 4, 1) &&
+                  encode_state_map(c, &c->mapsM.K1[1], c->K1[1], F32, 4, 1) &&
+                  encode_state_map(c, &c->mapsM.K2, c->K2, F32, 4, 1) &&
+                  encode_state_map(c, &c->mapsM.K3, c->K3, F32, 4, 1) && mapH(&c->mapsM.H);
+  c->mapsM.ok = ok ? 1 : 0;
 }
 
 void fill_consts(sgnb_ctx* c) {
@@ -613,7 +583,7 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   build_tile_maps(c);
   e = cudaMemset(c->U[0], 0, sbytes);
   // error partials: one row per tile of the kernels that this context runs
-  c->nblk = d->precision == SGNB_FP64_FAST && c->C.sym && !c->tab.gauss
+  c->nblk = !c->mixed && !c->tab.gauss
                 ? dev::line_grid_blocks(d->Nx, d->Ny) : dev::fused_grid_blocks(d->Nx, d->Ny);
   c->ndiag = 592;
   if (e == cudaSuccess) e = cudaMalloc(&c->partials, 3 * (size_t)c->nblk * sizeof(double));

@@ -20,7 +20,6 @@ struct sgnb_ctx {
   sgnb::FrTables tab;
   long long Nd = 0, ntot = 0;
   sgnb::RhsConsts C{};
-  sgnb::TileMaps maps{};  // tensor maps of U, K1, K2, K3, Hnod (exact mode, whole tiles)
   sgnb::TileMapsM mapsM{};  // the mixed mode's (FP32 K1, K2, K3; Hnod)
   void* encode_tiled = nullptr;  // the driver's tensor-map encoder (set with the maps)
   double* Hbuf = nullptr;  // one allocation holding all statics

@@ -234,17 +234,6 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map
 constexpr int kTmaTries = 1 << 20;
 #endif
 
-// Tensor maps of a context's FP64 buffers for the fused kernels' tile loads on meshes that
-// are a whole number of 8x4 tiles: each state-sized buffer as [field][element row]
-// [Nx * 25 nodes] with an [5][4][200] box (one tile's 5 x 32 x 25 doubles, in the shared
-// layout), the nodal depth as [element row][Nx * 25] with a [4][200] box. ok = 0: none.
-// In: the right-hand-side mode's input (any 16-byte-aligned device state, encoded per
-// launch); inOk = 0: none.
-struct TileMaps {
-  CUtensorMap U[2], K1[2], K2, K3, H, In;
-  int ok, inOk;
-};
-
 // The mixed-precision mode's counterparts (intermediate stage): the FP32 stage buffers as
 // [field][element row][Nx * 25] with a [1][4][200] box (one field of one tile per copy),
 // the nodal depth as for the FP64 kernels.
@@ -266,6 +255,14 @@ struct StageArgs {
   const CtrlState* ctrl;
   double* partials;   // MODE_FSAL: 3 doubles per CTA (sum r^2, max |r|, NaN count)
 };
+
+// Whether the rows of every buffer of a launch can move by bulk copies: aligned rows (C.bulk) in
+// aligned buffers (the right-hand side's input and output are the caller's).
+inline bool bulk_rows(const RhsConsts& C, const StageArgs& A) {
+  auto ok = [](const void* p) { return ((unsigned long long)p & 15) == 0; };
+  return C.bulk && ok(A.in) && ok(A.out) && ok(A.U[0]) && ok(A.U[1]) && ok(A.K1[0]) && ok(A.K1[1]) &&
+         ok(A.K2) && ok(A.K3) && ok(C.Hnod);
+}
 
 // Buffers of one mixed-precision launch: FP64 state, FP32 stage derivatives.
 struct StageArgsM {
@@ -414,10 +411,7 @@ cudaError_t launch_gauges_back(double* lam, const long long* nodes, int ng, cons
                                cudaStream_t s);
 
 // Launchers (one translation unit per arithmetic mode).
-// M: tensor maps of the buffers A names (the context's own), or nullptr (no tile loads
-// by the tensor-memory accelerator).
-cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A,
-                               cudaStream_t s, const TileMaps* M = nullptr);
+cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t prepare_line();

@@ -100,12 +100,6 @@ struct Tile {
   }
 };
 
-// Resident CTAs per SM the fast-mode single-instance kernels are compiled for (the
-// register budget per thread follows: 2 -> 168 registers, 3 -> 128).
-#ifndef SGNB_FAST_MIN_CTAS
-#define SGNB_FAST_MIN_CTAS 2
-#endif
-
 // Asynchronous global -> shared copy of one double (cp.async, no register staging), and
 // the wait for all of this thread's outstanding copies.
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
@@ -450,31 +444,45 @@ __device__ __forceinline__ double depth_grad(const TC& C, const TB& Tb, const do
   }
 }
 
-// Mirror ghost across a wall normal to DIR: the normal discharge changes sign.
-template <int DIR>
-__device__ __forceinline__ void mirror(const double* own, double* ghost) {
-#pragma unroll
-  for (int v = 0; v < NV; ++v) ghost[v] = own[v];
-  ghost[DIR == 0 ? 1 : 2] = -own[DIR == 0 ? 1 : 2];
+// dU of field v at node (a, b) of an element with nodal depths He, from the x derivative d of its
+// flux, the y pass's result g, the depth derivative dhx and the y non-conservative product by
+// (exact mode; the fast mode has it in g): dU = -dF - dG - Bx - By + S (sgn2d.cpp:285-287) with
+// the source of sgn_flux2d.h:122-142; Bx, By vanish except in hp.
+template <bool EXACT, bool FRIC, class TC, class TB>
+__device__ __forceinline__ double assemble(const TC& C, const TB& Tb, double h, double H, const double* He,
+                                           int a, int b, int v, double d, double g, double dhx, double by,
+                                           const Prim<EXACT>& q) {
+  if (v == 0) return EXACT ? (-d - g) + 0.0 : -(d + g);
+  if (v == 3) {
+    const double S3 = C.gamma * q.p;
+    return EXACT ? (-d - g) + S3 : S3 - (d + g);
+  }
+  if (v == 1 || v == 2) {
+    const double bath = C.g * (h - H) + C.gamma * q.p;
+    double Sv = bath * (v == 1 ? depth_grad<EXACT, 0>(C, Tb, He, a, b) : depth_grad<EXACT, 1>(C, Tb, He, a, b));
+    if constexpr (FRIC) {
+      // Manning friction along the velocity, n^2 g |vel| vel / h^(1/3) (sgn_flux2d.h:135-142)
+      const double vmag = sqrt(q.u * q.u + q.v * q.v);
+      const double cf = C.n2g * vmag / cbrt(h);
+      Sv = Sv - cf * (v == 1 ? q.u : q.v);
+    }
+    return EXACT ? (-d - g) + Sv : Sv - (d + g);
+  }
+  const double Hxl = depth_grad<EXACT, 0>(C, Tb, He, a, b);
+  const double Hyl = depth_grad<EXACT, 1>(C, Tb, He, a, b);
+  const double S4 = C.m2c2 * (q.w + q.u * Hxl + q.v * Hyl);
+  const double Bx = C.mc2 * q.u * dhx;  // ncpX (sgn_flux2d.h:150-155)
+  if constexpr (EXACT) return (((-d - g) - Bx) - by) + S4;
+  else return S4 - (d + g) - Bx;  // g holds dG + By
 }
 
-
-// One tile of the fused right-hand side / stage kernel: tile (bx, by) of the mesh whose
-// constants are C, error partial slot blk. Shared by the single-instance kernel and the
-// batched kernel. Returns early (uniformly over the CTA) when the instance's run is done.
-// FULL: the mesh is a whole number of tiles, so every tile is full and the per-item range
-// checks and their branches are compiled out (8 % off the end-point stage at 2048 x 1024).
-// TMA: the own-node tiles (state or stage derivatives, nodal depth) arrive by
-// tensor-memory-accelerator copies described by M (full tiles of the single-instance
-// kernel only).
-template <int MODE, bool EXACT, int TX_, int TY_, class TC, class TB, class TA, bool FRIC = false,
-          bool GHOST = false, bool GAUSS = false, bool FULL = false, bool TMA = false>
-__device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& A,
+// One tile of the fused right-hand side / stage kernel on Gauss-Legendre points: tile (bx, by) of
+// the mesh whose constants are C, error partial slot blk. Returns early (uniformly over the CTA)
+// when the run is done.
+template <int MODE, bool EXACT, int TX_, int TY_, bool FRIC>
+__device__ __forceinline__ void fused_tile(const RhsConsts& C, const RhsConsts& Tb, const StageArgs& A,
                                            int bx, int by, long long blk,
-                                           typename Tile<TX_, TY_, EXACT>::Smem& S,
-                                           const TileMaps* M = nullptr) {
-  static_assert(!TMA || (FULL && !GAUSS && TX_ == 8 && TY_ == 4),
-                "tile loads by the tensor-memory accelerator: full 8x4 tiles");
+                                           typename Tile<TX_, TY_, EXACT>::Smem& S) {
   using T = Tile<TX_, TY_, EXACT>;
   constexpr int TX = T::TX, TY = T::TY, NHALO = T::NHALO, RUN = T::RUN;
   constexpr int NHIT = T::NHIT, NFACE = T::NFACE, NFIT = T::NFIT;
@@ -496,54 +504,32 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
   if constexpr (MODE == MODE_FSAL) I.in = A.U[cur ^ 1];
   constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND;
 
-  // the thread index read through an opaque move: in the persistent batched kernel this
-  // keeps the compiler from hoisting the per-thread item and halo descriptors out of the
-  // tile loop (they would stay live, in registers, across every tile's passes)
-  int tid;
-  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+  const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int Nx = C.Nx, Ny = C.Ny;
   const long long Nd = C.Nd;
   const int ex0 = bx * TX, ey0 = by * TY;
-  const int TXv = FULL ? TX : min(TX, Nx - ex0), TYv = FULL ? TY : min(TY, Ny - ey0);
+  const int TXv = min(TX, Nx - ex0), TYv = min(TY, Ny - ey0);
   // the element columns and rows across the tile's edges, wrapped periodically (a compare
   // instead of an integer remainder by the mesh size)
   const int exL = ex0 == 0 ? Nx - 1 : ex0 - 1, exR = ex0 + TXv == Nx ? 0 : ex0 + TXv;
   const int eyB = ey0 == 0 ? Ny - 1 : ey0 - 1, eyT = ey0 + TYv == Ny ? 0 : ey0 + TYv;
-  // slab edges: the trace nodes across come from the neighbours' ghost arrays
-  bool ghostL = false, ghostR = false;
-  if constexpr (GHOST) {
-    ghostL = C.ghostL != nullptr && ex0 == 0;
-    ghostR = C.ghostR != nullptr && ex0 + TXv == Nx;
-  }
-  const bool wallL = C.bcx && ex0 == 0 && !ghostL, wallR = C.bcx && ex0 + TXv == Nx && !ghostR;
+  const bool wallL = C.bcx && ex0 == 0, wallR = C.bcx && ex0 + TXv == Nx;
   const bool wallB = C.bcy && ey0 == 0, wallT = C.bcy && ey0 + TYv == Ny;
 
   // ---- own-node item map: NIT items per thread, shared by every array -------
   // item u of a thread is double k of tile row iy: global (e_row*25 + k), shared
-  // iy*RUN + k (the [TE][NPP] layout of one field). The stage modes on full tiles keep a
-  // thread's items in one tile row, NTHR / TY doubles apart (one base address and
-  // immediate offsets: the end-point stage 1.3 % faster); the rhs-only mode and partial
-  // tiles (the batched kernels) take q = tid + NTHR*u in tile-row order (1 % and 0.3 %
-  // faster there). Recomputed after the passes rather than kept live through them.
+  // iy*RUN + k (the [TE][NPP] layout of one field). Recomputed after the passes rather than kept
+  // live through them.
   int gof[NIT];  // node offset within one field (Nd <= 2^31 by the mesh-size limit)
   int sof[NIT];
   bool okk[NIT];
   auto item_map = [&]() {
 #pragma unroll
     for (int u = 0; u < NIT; ++u) {
-      constexpr int PER_ROW = NTHR / TY;
-      static_assert(NTHR % TY == 0 && RUN == NIT * PER_ROW, "items split evenly over the rows");
-      int iy, k;
-      if constexpr (MODE != MODE_RHS && FULL) {
-        iy = tid / PER_ROW;
-        k = tid - iy * PER_ROW + PER_ROW * u;
-      } else {
-        const int q = tid + NTHR * u;
-        iy = q / RUN;
-        k = q - iy * RUN;
-      }
-      okk[u] = FULL || (iy < TYv && k < TXv * NPP);
+      const int q = tid + NTHR * u;
+      const int iy = q / RUN, k = q - iy * RUN;
+      okk[u] = iy < TYv && k < TXv * NPP;
       gof[u] = (int)(((long long)ex0 + (long long)Nx * (ey0 + iy)) * NPP + k);
       sof[u] = iy * RUN + k;
     }
@@ -551,55 +537,28 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
   item_map();
 
   // ---- load phase --------------------------------------------------------------
-  // TMA: one thread issues the tile's copies (rhs and end point: the input; stages: u and k;
-  // each [5][4][200] doubles; and the [4][200] nodal depths) on an mbarrier that aliases the
-  // (not yet used) reduction slots.
-  const unsigned mbar = smem_addr(&S.red[0][0]);
-  if constexpr (TMA) {
-    if (tid == 0) mbar_init(mbar);
-    __syncthreads();
-    if (tid == 0) {
-      const int x = ex0 * NPP;  // 16-byte aligned: 1600 bytes per tile column
-      constexpr int narr = AXPY ? 2 : 1;
-      mbar_expect_tx(mbar, (unsigned)((narr * NV + 1) * TE * NPP * sizeof(double)));
-      const CUtensorMap* mu = MODE == MODE_RHS ? &M->In : &M->U[AXPY ? cur : cur ^ 1];
-      tma_load_3d(smem_addr(&S.U[0][0][0]), mu, x, ey0, 0, mbar);
-      if constexpr (AXPY) {
-        const CUtensorMap* mg = A.kin_k2 ? &M->K2 : &M->K1[cur];
-        tma_load_3d(smem_addr(&S.G[0][0][0]), mg, x, ey0, 0, mbar);
-      }
-      tma_load_2d(smem_addr(&S.H[0][0]), &M->H, x, ey0, mbar);
-    }
-  }
   {
-    // Otherwise the statics and the state arrive by per-thread asynchronous copies straight
+    // The statics and the state arrive by per-thread asynchronous copies straight
     // into shared memory: a tile's loads are all in flight at once without holding
     // registers. The stage modes keep k in the (still unused) G area and forms u + (c dt) k in shared memory once the copies have landed.
-    if constexpr (!TMA) {
+#pragma unroll
+    for (int u = 0; u < NIT; ++u)
+      if (okk[u]) {
+        if (SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) cp_async8(&(&S.H[0][0])[sof[u]], C.Hnod + gof[u]);
+      }
+    const double* __restrict__ src = AXPY ? I.u : I.in;
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
 #pragma unroll
       for (int u = 0; u < NIT; ++u)
-        if (okk[u]) {
-          if (SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) cp_async8(&(&S.H[0][0])[sof[u]], C.Hnod + gof[u]);
+        if (okk[u] && SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) {
+          cp_async8(&(&S.U[v][0][0])[sof[u]], (src + (long long)v * Nd) + gof[u]);
+          if constexpr (AXPY)
+            cp_async8(&(&S.G[v][0][0])[sof[u]], (I.k + (long long)v * Nd) + gof[u]);
         }
-    }
-    if constexpr (TMA) {
-      // the tile copies above
-    } else {
-      const double* __restrict__ src = AXPY ? I.u : I.in;
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int u = 0; u < NIT; ++u)
-          if (okk[u] && SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) {
-            cp_async8(&(&S.U[v][0][0])[sof[u]], (src + (long long)v * Nd) + gof[u]);
-            if constexpr (AXPY)
-              cp_async8(&(&S.G[v][0][0])[sof[u]], (I.k + (long long)v * Nd) + gof[u]);
-          }
-    }
     // halo items: descriptors, then loads
     double hv[NHIT];
     int hq[NHIT];
-    int hs[NHIT];  // source: 0 the state, 1 the left ghost, 2 the right ghost
     long long hg[NHIT];
 #pragma unroll
     for (int u = 0; u < NHIT; ++u) {
@@ -608,49 +567,29 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
       const int slot = r % NHALO, v = r / NHALO;
       bool ok = q < NV * NHALO * NP;
       long long e = 0;
-      int node = 0;
-      hs[u] = 0;
       if (slot < TY) {
-        if (GHOST && ghostL) hs[u] = 1;
         ok = ok && slot < TYv && !wallL;
         e = (long long)(exL) + (long long)Nx * (ey0 + slot);
-        node = (NP - 1) + NP * t;
       } else if (slot < 2 * TY) {
-        if (GHOST && ghostR) hs[u] = 2;
         ok = ok && slot - TY < TYv && !wallR;
         e = (long long)(exR) + (long long)Nx * (ey0 + slot - TY);
-        node = NP * t;
       } else if (slot < 2 * TY + TX) {
         ok = ok && slot - 2 * TY < TXv && !wallB;
         e = (long long)(ex0 + slot - 2 * TY) + (long long)Nx * (eyB);
-        node = t + NP * (NP - 1);
       } else {
         ok = ok && slot - 2 * TY - TX < TXv && !wallT;
         e = (long long)(ex0 + slot - 2 * TY - TX) + (long long)Nx * (eyT);
-        node = t;
       }
       hq[u] = ok ? q : -1;
-      hg[u] = (GHOST && hs[u]) ? (long long)v * Ny * NP + (long long)(ey0 + (slot < TY ? slot : slot - TY)) * NP + t
-                               : (long long)v * Nd + e * NPP + node;
-      if constexpr (GAUSS) {
-        // the neighbour's trace on the shared face: the left neighbour's right face (1),
-        // the right neighbour's left face (0), the bottom one's top face (3), the top
-        // one's bottom face (2)
-        const int f = slot < TY ? 1 : (slot < 2 * TY ? 0 : (slot < 2 * TY + TX ? 3 : 2));
-        hg[u] = ((long long)(f * NV + v) * (Nd / NPP) + e) * NP + t;
-      }
+      // the neighbour's trace on the shared face: the left neighbour's right face (1), the
+      // right neighbour's left face (0), the bottom one's top face (3), the top one's bottom
+      // face (2)
+      const int f = slot < TY ? 1 : (slot < 2 * TY ? 0 : (slot < 2 * TY + TX ? 3 : 2));
+      hg[u] = ((long long)(f * NV + v) * (Nd / NPP) + e) * NP + t;
     }
 #pragma unroll
     for (int u = 0; u < NHIT; ++u)
-      if (hq[u] >= 0) {
-        if constexpr (GAUSS)
-          hv[u] = SGNB_INB(hg[u], 4 * Nd) ? C.tr[hg[u]] : 0.0;
-        else if constexpr (GHOST)
-          hv[u] = hs[u] == 0 ? (SGNB_INB(hg[u], NV * Nd) ? stage_value<MODE>(I, hg[u]) : 0.0)
-                             : (SGNB_INB(hg[u], (long long)NV * Ny * NP) ? (hs[u] == 1 ? C.ghostL : C.ghostR)[hg[u]] : 0.0);
-        else
-          hv[u] = SGNB_INB(hg[u], NV * Nd) ? stage_value<MODE>(I, hg[u]) : 0.0;
-      }
+      if (hq[u] >= 0) hv[u] = SGNB_INB(hg[u], 4 * Nd) ? C.tr[hg[u]] : 0.0;
     // face depths
     double fv[NFIT];
     int fq[NFIT];
@@ -675,10 +614,10 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
 #ifdef SGNB_CHECKED
             const long long fe = (long long)ey * NP + t;
             const long long fx = ((long long)(exR) + (long long)Nx * ey) * NP + t;
-            fv[u] = (wallR || ghostR) ? (SGNB_INB(fe, (long long)Ny * NP) ? C.HfXEnd[fe] : 0.0)
+            fv[u] = wallR ? (SGNB_INB(fe, (long long)Ny * NP) ? C.HfXEnd[fe] : 0.0)
                                       : (SGNB_INB(fx, Nd / NP) ? C.HfX[fx] : 0.0);
 #else
-            fv[u] = (wallR || ghostR) ? C.HfXEnd[(long long)ey * NP + t]
+            fv[u] = wallR ? C.HfXEnd[(long long)ey * NP + t]
                           : C.HfX[((long long)(exR) + (long long)Nx * ey) * NP + t];
 #endif
             fq[u] = q;
@@ -705,22 +644,6 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     for (int u = 0; u < NFIT; ++u)
       if (fq[u] >= 0 && SGNB_INB(fq[u], NFACE)) S.Hf[fq[u]] = fv[u];
     cp_async_wait_all();
-    if constexpr (TMA) {
-      bool landed = false;
-      for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
-      if (!landed) {
-        // the copies did not complete: this thread's items become NaN, so the launch's
-        // results are non-finite and the controller ends the run with that error
-        const double nan = __longlong_as_double(0x7ff8000000000000LL);
-#pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-          for (int u = 0; u < NIT; ++u) {
-            (&S.U[v][0][0])[sof[u]] = nan;
-            (&S.G[v][0][0])[sof[u]] = nan;
-          }
-      }
-    }
     if constexpr (AXPY) {
       // u + (c dt) k for this thread's own items (rk.cpp:100-103), in shared memory
 #pragma unroll
@@ -734,13 +657,10 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     }
   }
   __syncthreads();
-  if constexpr (TMA) {
-    if (tid == 0) mbar_inval(mbar);  // its slots serve the error reduction later
-  }
 
   const int i = lane;  // tile element of this lane
   const int ix = i % TX, iy = i / TX;
-  const bool valid = FULL || (ix < TXv && iy < TYv);
+  const bool valid = ix < TXv && iy < TYv;
   const int j = warp;  // GLL line index of this warp
 
   // ---- column pass: y-line a = j ---------------------------------------------
@@ -756,11 +676,8 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     if (iy > 0) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        if constexpr (GAUSS) nLo[v] = face_trace(Tb.lR, &S.U[v][i - TX][j], NP);
-        else nLo[v] = S.U[v][i - TX][j + NP * (NP - 1)];
+        nLo[v] = face_trace(Tb.lR, &S.U[v][i - TX][j], NP);
       }
-    } else if (wallB) {
-      if constexpr (!GAUSS) mirror<1>(Un[0], nLo);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v) nLo[v] = T::halo_at(S, v, 2 * TY + ix, j);
@@ -768,11 +685,8 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     if (iy + 1 < TYv) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        if constexpr (GAUSS) nHi[v] = face_trace(Tb.lL, &S.U[v][i + TX][j], NP);
-        else nHi[v] = S.U[v][i + TX][j];
+        nHi[v] = face_trace(Tb.lL, &S.U[v][i + TX][j], NP);
       }
-    } else if (wallT) {
-      if constexpr (!GAUSS) mirror<1>(Un[NP - 1], nHi);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v) nHi[v] = T::halo_at(S, v, 2 * TY + TX + ix, j);
@@ -780,7 +694,7 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     const double HfLo = T::hf_y(S, i, j);
     const double HfHi = (iy + 1 < TYv) ? T::hf_y(S, i + TX, j) : T::hf_yt(S, ix, j);
     double by[NP];  // ncpY, -c^2 v h_y (sgn_flux2d.h:156-161)
-    line_pass<EXACT, 1, GAUSS>(
+    line_pass<EXACT, 1, true>(
         C, Tb, Un, Hn, nLo, nHi, HfLo, HfHi,
         [&](int b, double dh, const Prim<EXACT>& q) {
           if constexpr (EXACT) S.G[NV][i][j + NP * b] = C.mc2 * q.v * dh;
@@ -810,11 +724,8 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     if (ix > 0) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        if constexpr (GAUSS) nLo[v] = face_trace(Tb.lR, &S.U[v][i - 1][NP * j], 1);
-        else nLo[v] = S.U[v][i - 1][(NP - 1) + NP * j];
+        nLo[v] = face_trace(Tb.lR, &S.U[v][i - 1][NP * j], 1);
       }
-    } else if (wallL) {
-      if constexpr (!GAUSS) mirror<0>(Un[0], nLo);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v) nLo[v] = T::halo_at(S, v, iy, j);
@@ -822,11 +733,8 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     if (ix + 1 < TXv) {
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
-        if constexpr (GAUSS) nHi[v] = face_trace(Tb.lL, &S.U[v][i + 1][NP * j], 1);
-        else nHi[v] = S.U[v][i + 1][NP * j];
+        nHi[v] = face_trace(Tb.lL, &S.U[v][i + 1][NP * j], 1);
       }
-    } else if (wallR) {
-      if constexpr (!GAUSS) mirror<0>(Un[NP - 1], nHi);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v) nHi[v] = T::halo_at(S, v, TY + iy, j);
@@ -834,44 +742,13 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
     const double HfLo = T::hf_x(S, i, j);
     const double HfHi = (ix + 1 < TXv) ? T::hf_x(S, i + 1, j) : T::hf_xr(S, iy, j);
     double dhx[NP];
-    line_pass<EXACT, 0, GAUSS>(
+    line_pass<EXACT, 0, true>(
         C, Tb, Un, Hn, nLo, nHi, HfLo, HfHi,
         [&](int a, double dh, const Prim<EXACT>&) { dhx[a] = dh; },
         [&](int a, int v, double d, const Prim<EXACT>& q) {
           const int loc = a + NP * j;
-          const double g = S.G[v][i][loc];
-          double res;
-          // dU = -dF - dG - Bx - By + S (sgn2d.cpp:285-287) with the source of
-          // sgn_flux2d.h:122-134 (Manning off); Bx, By vanish except in hp
-          if (v == 0) {
-            res = EXACT ? (-d - g) + 0.0 : -(d + g);
-          } else if (v == 3) {
-            const double S3 = C.gamma * q.p;
-            res = EXACT ? (-d - g) + S3 : S3 - (d + g);
-          } else if (v == 1 || v == 2) {
-            const double bath = C.g * (Un[a][0] - Hn[a]) + C.gamma * q.p;
-            double Sv = bath * (v == 1 ? depth_grad<EXACT, 0>(C, Tb, S.H[i], a, j)
-                                       : depth_grad<EXACT, 1>(C, Tb, S.H[i], a, j));
-            if constexpr (FRIC) {
-              // Manning friction along the velocity, n^2 g |vel| vel / h^(1/3)
-              // (sgn_flux2d.h:135-142)
-              const double vmag = sqrt(q.u * q.u + q.v * q.v);
-              const double cf = C.n2g * vmag / cbrt(Un[a][0]);
-              Sv = Sv - cf * (v == 1 ? q.u : q.v);
-            }
-            res = EXACT ? (-d - g) + Sv : Sv - (d + g);
-          } else {
-            const double Hxl = depth_grad<EXACT, 0>(C, Tb, S.H[i], a, j);
-            const double Hyl = depth_grad<EXACT, 1>(C, Tb, S.H[i], a, j);
-            const double S4 = C.m2c2 * (q.w + q.u * Hxl + q.v * Hyl);
-            const double Bx = C.mc2 * q.u * dhx[a];  // ncpX (sgn_flux2d.h:150-155)
-            if constexpr (EXACT) {
-              const double By = S.G[NV][i][loc];
-              res = (((-d - g) - Bx) - By) + S4;
-            } else {
-              res = S4 - (d + g) - Bx;  // g holds dG + By
-            }
-          }
+          const double res = assemble<EXACT, FRIC>(C, Tb, Un[a][0], Hn[a], S.H[i], a, j, v, d, S.G[v][i][loc], dhx[a],
+                                                   EXACT ? S.G[EXACT ? NV : 0][i][loc] : 0.0, q);
           S.G[v][i][loc] = res;
         },
         ix == 0 && wallL, ix + 1 >= TXv && wallR);
@@ -956,71 +833,20 @@ __device__ __forceinline__ void fused_tile(const TC& C, const TB& Tb, const TA& 
       }
     }
   }
-  if constexpr (GHOST && AXPY) {
-    // Fused edge exchange: the slab-edge tiles form the next stage's input at their edge
-    // nodes (a = 0 of the first column, a = 4 of the last) from this launch's result and
-    // store it straight into the neighbours' ghost arrays, [field][row][node], while the
-    // other tiles still compute. After stage 2 (k1 added) that is u + 3/4 dt k2, the next
-    // launch's own stage input; after stage 3 the end-point candidate. Both with the
-    // explicitly rounded combinations of the stage inputs, so the neighbour sees the bits
-    // this slab's own next launch forms.
-    const bool outLo = C.edgeL != nullptr && ex0 == 0, outHi = C.edgeR != nullptr && ex0 + TXv == Nx;
-    if (outLo || outHi) {
-      const CtrlReload rc = ctrl_reload(A.ctrl);
-      const int cr = rc.cur;
-      const double dt = rc.dt;
-      const double* __restrict__ u0 = A.U[cr];
-      const double* __restrict__ k1 = A.K1[cr];
-      const double* __restrict__ k2 = A.K2;
-      const int per = NV * TYv * NP;
-      for (int q = tid; q < 2 * per; q += NTHR) {
-        const int side = q / per;
-        if (side == 0 ? !outLo : !outHi) continue;
-        const int r = q - side * per;
-        const int t = r % NP, iy = (r / NP) % TYv, v = r / (NP * TYv);
-        const int ixe = side == 0 ? 0 : TXv - 1;
-        const int node = (side == 0 ? 0 : NP - 1) + NP * t;
-        const long long g = (long long)v * Nd + ((long long)(ex0 + ixe) + (long long)Nx * (ey0 + iy)) * NPP + node;
-        const double kout = S.G[v][TX * iy + ixe][node];
-        const long long ge = (long long)v * Ny * NP + (long long)(ey0 + iy) * NP + t;
-        if (!SGNB_INB(g, NV * Nd) || !SGNB_INB(ge, (long long)NV * Ny * NP)) continue;
-        const double val = MODE == MODE_STAGE ? stage_axpy(u0[g], 0.75 * dt, kout)
-                                              : fsal_finish(u0[g], fsal_part(k1[g], k2[g]), kout, dt);
-        (side == 0 ? C.edgeL : C.edgeR)[ge] = val;
-      }
-    }
-  }
   if constexpr (MODE == MODE_FSAL) reduce_error(esum, emax, enan, S.red, A.partials, blk);
 }
 
 
-// FRIC: Manning friction compiled in (instantiated only for contexts that use it, so the
-// frictionless kernels carry none of its code).
-// GHOST: slab edges compiled in (only contexts with ghost arrays launch these variants).
-// GAUSS: Gauss-Legendre points (after k_traces of the same stage).
-// FULL: Nx a multiple of 8 and Ny of 4 (every tile full).
-template <int MODE, bool EXACT, bool FRIC = false, bool GHOST = false, bool GAUSS = false,
-          bool FULL = false>
-__global__ void __launch_bounds__(NTHR, EXACT ? 2 : SGNB_FAST_MIN_CTAS) k_fused(const RhsConsts C, const StageArgs A) {
+// Gauss-Legendre points, after k_traces of the same stage (the GLL kernels are in
+// sgnb_kernels_line.cuh). FRIC: Manning friction compiled in.
+template <int MODE, bool EXACT, bool FRIC>
+__global__ void __launch_bounds__(NTHR, 2) k_fused(const RhsConsts C, const StageArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using T = Tile<8, 4, EXACT>;
   typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_raw);
   wait_for_previous();
-  fused_tile<MODE, EXACT, 8, 4, RhsConsts, RhsConsts, StageArgs, FRIC, GHOST, GAUSS, FULL>(C, C, A, blockIdx.x, blockIdx.y,
-                                (long long)blockIdx.y * gridDim.x + blockIdx.x, S);
-}
-
-// A mesh of whole tiles, with the own-node tiles loaded by the tensor-memory accelerator
-// from the buffers that M describes. GHOST: slab edges compiled in (x-slab contexts).
-template <int MODE, bool EXACT, bool GHOST = false>
-__global__ void __launch_bounds__(NTHR, EXACT ? 2 : SGNB_FAST_MIN_CTAS)
-    k_fused_tma(const RhsConsts C, const StageArgs A, const __grid_constant__ TileMaps M) {
-  extern __shared__ __align__(128) unsigned char smem_tiles[];  // the copies' destinations
-  using T = Tile<8, 4, EXACT>;
-  typename T::Smem& S = *reinterpret_cast<typename T::Smem*>(smem_tiles);
-  wait_for_previous();
-  fused_tile<MODE, EXACT, 8, 4, RhsConsts, RhsConsts, StageArgs, false, GHOST, false, true, true>(
-      C, C, A, blockIdx.x, blockIdx.y, (long long)blockIdx.y * gridDim.x + blockIdx.x, S, &M);
+  fused_tile<MODE, EXACT, 8, 4, FRIC>(C, C, A, blockIdx.x, blockIdx.y,
+                                      (long long)blockIdx.y * gridDim.x + blockIdx.x, S);
 }
 
 // Face traces of every element for Gauss-Legendre points (sgn2d.cpp:141-177), of the

@@ -1,75 +1,55 @@
-// sgnb_kernels_exact.cu -- fused kernels in the exact arithmetic mode.
+// sgnb_kernels_exact.cu -- kernels in the exact arithmetic mode.
 // Built with -fmad=false: every product and sum rounds separately, in the operation
 // order of the reference CPU solver, so the results are bit-identical to it.
 #define SGNB_EXACT true
 #include "sgnb_kernels_inst.cuh"
+#include "sgnb_kernels_line.cuh"
 
 namespace sgnb {
 namespace dev {
-template <int MODE>
-static cudaError_t launch_mode(const RhsConsts& C, const StageArgs& A, cudaStream_t s,
-                               const TileMaps* M) {
-  if (C.gauss) return launch_gauss<MODE>(C, A, s);
-  const dim3 grid((C.Nx + 7) / 8, (C.Ny + 3) / 4);
-  const size_t smem = sizeof(Tile<8, 4, SGNB_EXACT>::Smem);
-  cudaError_t e;
-  const bool ghost = C.ghostL != nullptr || C.ghostR != nullptr;
-  if (C.manning) {
-    if (ghost) e = launch_dependent(k_fused<MODE, SGNB_EXACT, true, true>, grid, dim3(NTHR), smem, s, C, A);
-    else e = launch_dependent(k_fused<MODE, SGNB_EXACT, true, false>, grid, dim3(NTHR), smem, s, C, A);
-  } else {
-    const bool full = C.Nx % 8 == 0 && C.Ny % 4 == 0;  // every tile full
-    // the own-node tiles by the tensor-memory accelerator where the context's tensor maps
-    // describe the buffers (and, for the rhs mode, a map of its input)
-    const bool tma = full && M != nullptr && M->ok && (MODE != MODE_RHS || M->inOk);
-    if (ghost) {
-      if (tma) e = launch_dependent(k_fused_tma<MODE, SGNB_EXACT, true>, grid, dim3(NTHR), smem, s, C, A, *M);
-      else if (full) e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, true, false, true>, grid, dim3(NTHR), smem, s, C, A);
-      else e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, true>, grid, dim3(NTHR), smem, s, C, A);
-    } else if (full) {
-      if (tma)
-        e = launch_dependent(k_fused_tma<MODE, SGNB_EXACT>, grid, dim3(NTHR), smem, s, C, A, *M);
-      else
-        e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, false, false, true>, grid, dim3(NTHR), smem, s, C, A);
-    } else {
-      e = launch_dependent(k_fused<MODE, SGNB_EXACT, false, false>, grid, dim3(NTHR), smem, s, C, A);
-    }
-  }
-  return e;
+template <int MODE, bool FRIC, bool GHOST>
+static cudaError_t launch_variant(const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
+  using L = LineTile<1, true>;
+  const dim3 grid((C.Nx + L::TX - 1) / L::TX, (C.Ny + L::TY - 1) / L::TY);
+  return launch_dependent(k_line_exact<MODE, FRIC, GHOST>, grid, dim3(LTHR), sizeof(typename L::Smem), s, C, A,
+                          (int)bulk_rows(C, A));
 }
 
-cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s,
-                              const TileMaps* M) {
+template <int MODE>
+static cudaError_t launch_mode(const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
+  if (C.gauss) return launch_gauss<MODE>(C, A, s);
+  const bool ghost = C.ghostL != nullptr || C.ghostR != nullptr;
+  if (C.manning) return ghost ? launch_variant<MODE, true, true>(C, A, s) : launch_variant<MODE, true, false>(C, A, s);
+  return ghost ? launch_variant<MODE, false, true>(C, A, s) : launch_variant<MODE, false, false>(C, A, s);
+}
+
+cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
   switch (mode) {
-    case MODE_RHS: return launch_mode<MODE_RHS>(C, A, s, M);
-    case MODE_STAGE: return launch_mode<MODE_STAGE>(C, A, s, M);
-    case MODE_FSAL: return launch_mode<MODE_FSAL>(C, A, s, M);
-    case MODE_CAND: return launch_mode<MODE_CAND>(C, A, s, M);
+    case MODE_RHS: return launch_mode<MODE_RHS>(C, A, s);
+    case MODE_STAGE: return launch_mode<MODE_STAGE>(C, A, s);
+    case MODE_FSAL: return launch_mode<MODE_FSAL>(C, A, s);
+    case MODE_CAND: return launch_mode<MODE_CAND>(C, A, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
-template <bool GHOST>
-static cudaError_t prepare_tma() {
-  const size_t bytes = sizeof(Tile<8, 4, true>::Smem);
-  cudaError_t e = raise_smem(k_fused_tma<MODE_RHS, true, GHOST>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_fused_tma<MODE_STAGE, true, GHOST>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_fused_tma<MODE_CAND, true, GHOST>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_fused_tma<MODE_FSAL, true, GHOST>, bytes);
+template <int MODE>
+static cudaError_t prepare_mode() {
+  const size_t bytes = sizeof(LineTile<1, true>::Smem);
+  cudaError_t e = raise_smem(k_line_exact<MODE, false, false>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE, true, false>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE, false, true>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE, true, true>, bytes);
   return e;
 }
 
 cudaError_t prepare_fused_exact() {
-  cudaError_t e = prepare_variant<false, false>();
-  if (e == cudaSuccess) e = prepare_variant<true, false>();
-  if (e == cudaSuccess) e = prepare_variant<false, true>();
-  if (e == cudaSuccess) e = prepare_variant<true, true>();
-  if (e == cudaSuccess) e = prepare_variant<false, false, true>();
-  if (e == cudaSuccess) e = prepare_variant<true, false, true>();
-  if (e == cudaSuccess) e = prepare_variant<false, false, false, true>();
-  if (e == cudaSuccess) e = prepare_variant<false, true, false, true>();
-  if (e == cudaSuccess) e = prepare_tma<false>();
-  if (e == cudaSuccess) e = prepare_tma<true>();
+  cudaError_t e = prepare_variant<false>();
+  if (e == cudaSuccess) e = prepare_variant<true>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_RHS>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_CAND>();
+  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL>();
   return e;
 }
 int fused_grid_blocks(int Nx, int Ny) { return ((Nx + 7) / 8) * ((Ny + 3) / 4); }

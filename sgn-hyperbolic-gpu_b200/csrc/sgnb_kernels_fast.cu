@@ -10,7 +10,7 @@ namespace dev {
 cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
   // FR tables without the reflection symmetry of the GLL ones (given by the caller): the exact
   // mode's kernels, which take any tables
-  if (!C.gauss && !C.sym) return launch_fused_exact(mode, C, A, s, nullptr);
+  if (!C.gauss && !C.sym) return launch_fused_exact(mode, C, A, s);
   if (!C.gauss) return launch_line(mode, C, A, s);
   switch (mode) {
     case MODE_RHS: return launch_gauss<MODE_RHS>(C, A, s);
@@ -21,8 +21,8 @@ cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, 
   }
 }
 cudaError_t prepare_fused_fast() {
-  cudaError_t e = prepare_variant<false, false, true>();
-  if (e == cudaSuccess) e = prepare_variant<true, false, true>();
+  cudaError_t e = prepare_variant<false>();
+  if (e == cudaSuccess) e = prepare_variant<true>();
   if (e == cudaSuccess) e = prepare_line();
   return e;
 }

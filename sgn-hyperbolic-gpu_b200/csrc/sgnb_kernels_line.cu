@@ -5,14 +5,6 @@
 namespace sgnb {
 namespace dev {
 
-// bulk row copies need aligned buffers besides aligned rows (C.bulk): the right-hand side's
-// input and output are the caller's
-static int bulk_rows(const RhsConsts& C, const StageArgs& A) {
-  auto ok = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-  return C.bulk && ok(A.in) && ok(A.out) && ok(A.U[0]) && ok(A.U[1]) && ok(A.K1[0]) && ok(A.K1[1]) &&
-         ok(A.K2) && ok(A.K3) && ok(C.Hnod);
-}
-
 template <int MODE, bool FRIC, bool GHOST>
 static cudaError_t launch_variant(const RhsConsts& C, const StageArgs& A, int bulk, cudaStream_t s) {
   using L = LineTile<1>;

@@ -47,7 +47,7 @@ constexpr int LTHR = 32 * LWARPS;
 // stride:
 //   U[v][i * 25 + a + 5 b]        node (a, b) of tile element i = ix + TX iy
 //   U[v][TN + 5 * slot + t]       slots left [TY], right [TY], bottom [TX], top [TX]
-template <int WX_>
+template <int WX_, bool EXACT_ = false>
 struct LineTile {
   static constexpr int WX = WX_, WY = LWARPS / WX_;
   static constexpr int TX = LROW * WX, TY = WY;
@@ -58,7 +58,9 @@ struct LineTile {
   struct Smem {
     double U[NV][US];
     double H[TN];
-    double G[NV][TN];        // stage derivative on load; column-pass results; then dU
+    // stage derivative on load; column-pass results (the exact mode: the non-conservative product
+    // of hp on its own); then dU
+    double G[NV + (EXACT_ ? 1 : 0)][TN];
     double red[LWARPS][3];   // (with the barriers: room for the reads of idle lanes past G)
     unsigned long long mbar[LWARPS];
     unsigned stash;          // base of the CTA's tensor memory
@@ -328,11 +330,11 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
 // One tile. The CTA holds its stash (S.stash, written before or visible after the first barrier
 // here) in the modes that use one. bulk: rows start 16-byte aligned in every buffer (Nx even) and come and go by the bulk
 // copy engine; otherwise value by value.
-template <int MODE, int WX, bool FRIC, bool GHOST, class TC, class TE_, class TA>
+template <int MODE, int WX, bool FRIC, bool GHOST, bool EXACT = false, class TC, class TE_, class TA>
 __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A, int bx, int by,
                                           long long blk, const bool bulk,
-                                          typename LineTile<WX>::Smem& S) {
-  using L = LineTile<WX>;
+                                          typename LineTile<WX, EXACT>::Smem& S) {
+  using L = LineTile<WX, EXACT>;
   constexpr int TX = L::TX, TY = L::TY, NHALO = L::NHALO, TN = L::TN, US = L::US;
   constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND;
 
@@ -477,8 +479,32 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     }
   }
 
-  // ---- this warp's row has landed; stage input u + (c dt) k in place; then the whole tile ---
+  // exact mode: the depths of the faces at both ends of this lane's two lines
   const int ce = kColumnLane[lane] >> 3, cj = kColumnLane[lane] & 7;  // column pass: element, line
+  double fy0 = 0.0, fy1 = 0.0, fx0 = 0.0, fx1 = 0.0;
+  if constexpr (EXACT) {
+    const int ey = ey0 + iy;
+    if (lane < LROW * NP && ce < RXv) {
+      const int ex = ex0 + wx * LROW + ce;
+      const bool end = C.bcy && ey + 1 == Ny;
+      const long long f0 = ((long long)ex + (long long)Nx * ey) * NP + cj;
+      const long long f1 = end ? (long long)ex * NP + cj
+                               : ((long long)ex + (long long)Nx * (ey + 1 == Ny ? 0 : ey + 1)) * NP + cj;
+      if (SGNB_INB(f0, Nd / NP)) fy0 = C.HfY[f0];
+      if (SGNB_INB(f1, end ? (long long)Nx * NP : Nd / NP)) fy1 = (end ? C.HfYEnd : C.HfY)[f1];
+    }
+    if (lane < LROW * NP && lane / NP < RXv) {
+      const int ex = ex0 + wx * LROW + lane / NP, t = lane % NP;
+      const bool end = ex + 1 == Nx && (C.bcx || ghostR);
+      const long long f0 = ((long long)ex + (long long)Nx * ey) * NP + t;
+      const long long f1 = end ? (long long)ey * NP + t
+                               : ((long long)(ex + 1 == Nx ? 0 : ex + 1) + (long long)Nx * ey) * NP + t;
+      if (SGNB_INB(f0, Nd / NP)) fx0 = C.HfX[f0];
+      if (SGNB_INB(f1, end ? (long long)Ny * NP : Nd / NP)) fx1 = (end ? C.HfXEnd : C.HfX)[f1];
+    }
+  }
+
+  // ---- this warp's row has landed; stage input u + (c dt) k in place; then the whole tile ---
   const bool cvalid = lane < LROW * NP && ce < RXv;
   double* const uc = &S.U[0][s0 + ce * NPP + cj];
   if (!bulk) cp_async_wait_all();
@@ -540,8 +566,29 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
                                  : (iy + 1 < TYv ? uc + TX * NPP : &S.U[0][TN + (2 * TY + TX + ix) * NP + cj]);
     const int o = s0 + ce * NPP + cj;
     double* const gp = &S.G[0][o];
-    line_terms<1, US, false>(C, T, uc, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
-                             [&](int v, int k, double r) { gp[v * TN + k * NP] = r; });
+    if constexpr (EXACT) {
+      double Un[NP][NV], Hn[NP], nLo[NV], nHi[NV];
+#pragma unroll
+      for (int b = 0; b < NP; ++b) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) Un[b][v] = uc[v * US + b * NP];
+        Hn[b] = S.H[o + b * NP];
+      }
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        nLo[v] = lo[v * US];
+        nHi[v] = hi[v * US];
+      }
+      if (mlo) nLo[2] = -nLo[2];
+      if (mhi) nHi[2] = -nHi[2];
+      line_pass<true, 1>(
+          C, T, Un, Hn, nLo, nHi, fy0, fy1,
+          [&](int b, double dh, const Prim<true>& q) { gp[NV * TN + b * NP] = C.mc2 * q.v * dh; },
+          [&](int b, int v, double d, const Prim<true>&) { gp[v * TN + b * NP] = d; });
+    } else {
+      line_terms<1, US, false>(C, T, uc, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
+                               [&](int v, int k, double r) { gp[v * TN + k * NP] = r; });
+    }
   }
   __syncwarp();
   let_next_start();
@@ -555,8 +602,32 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       const double* const lo = mlo ? u : (ix > 0 ? u - NPP + (NP - 1) : &S.U[0][TN + iy * NP + j]);
       const double* const hi = mhi ? u + (NP - 1) : (ix + 1 < TXv ? u + NPP : &S.U[0][TN + (TY + iy) * NP + j]);
       double* const gp = &S.G[0][o];
-      line_terms<0, US, FRIC>(C, T, u, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
-                              [&](int v, int k, double r) { gp[v * TN + k] = -r - gp[v * TN + k]; });
+      if constexpr (EXACT) {
+        double Un[NP][NV], Hn[NP], nLo[NV], nHi[NV], dhx[NP];
+        const double* const He = &S.H[s0 + e * NPP];
+#pragma unroll
+        for (int a = 0; a < NP; ++a) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) Un[a][v] = u[v * US + a];
+          Hn[a] = S.H[o + a];
+        }
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          nLo[v] = lo[v * US];
+          nHi[v] = hi[v * US];
+        }
+        if (mlo) nLo[1] = -nLo[1];
+        if (mhi) nHi[1] = -nHi[1];
+        line_pass<true, 0>(
+            C, T, Un, Hn, nLo, nHi, fx0, fx1, [&](int a, double dh, const Prim<true>&) { dhx[a] = dh; },
+            [&](int a, int v, double d, const Prim<true>& q) {
+              gp[v * TN + a] = assemble<true, FRIC>(C, T, Un[a][0], Hn[a], He, a, j, v, d, gp[v * TN + a], dhx[a],
+                                                    gp[NV * TN + a], q);
+            });
+      } else {
+        line_terms<0, US, FRIC>(C, T, u, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
+                                [&](int v, int k, double r) { gp[v * TN + k] = -r - gp[v * TN + k]; });
+      }
     }
   }
   const bool bulk_out = bulk && MODE != MODE_CAND;
@@ -661,11 +732,12 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     // operands are whatever shared memory holds): branches would keep the values from overlapping
     auto errors = [&](auto divide) {
       auto err = [&](double u, double q, double un, double k4, bool there) {
-        const double e = un - fma(rc.dt, fma(0.125, k4, q), u);
-        const double au = fabs(u), an = fabs(un);
-        double rr = divide(e, fma(rc.rtol, au < an ? an : au, rc.atol));
+        const double au = fabs(u), an = fabs(un), am = au < an ? an : au;
+        double rr;
+        if constexpr (EXACT) rr = (un - (u + rc.dt * (q + 0.125 * k4))) / (rc.atol + rc.rtol * am);
+        else rr = divide(un - fma(rc.dt, fma(0.125, k4, q), u), fma(rc.rtol, am, rc.atol));
         rr = there ? rr : 0.0;
-        esum = fma(rr, rr, esum);  // a NaN stays in the sum
+        esum = EXACT ? esum + rr * rr : fma(rr, rr, esum);  // a NaN stays in the sum
         const double ar = fabs(rr);
         emax = emax < ar ? ar : emax;
       };
@@ -688,7 +760,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     };
     // the scale is at least atol: where that is a normal number, so is the scale, and the
     // reciprocal of a few ulp serves
-    if (rc.atol >= 2.2250738585072014e-308) errors([](double e, double sc) { return e * fast_rcp(sc); });
+    if (!EXACT && rc.atol >= 2.2250738585072014e-308) errors([](double e, double sc) { return e * fast_rcp(sc); });
     else errors([](double e, double sc) { return e / sc; });
     reduce_error<LWARPS>(esum, emax, esum != esum, S.red, A.partials, blk);
   }
@@ -712,6 +784,22 @@ __global__ void __launch_bounds__(LTHR, (kLineCtas<MODE, 1>))
   wait_for_previous();
   line_tile<MODE, 1, FRIC, GHOST>(C, T, A, blockIdx.x, blockIdx.y,
                                   (long long)blockIdx.y * gridDim.x + blockIdx.x, C.bulk != 0, S);
+  if constexpr (kStash<MODE>) {
+    __syncthreads();
+    if (threadIdx.x < 32) stash_free(S.stash);
+  }
+}
+
+// The exact mode's: the reference's operation order and IEEE divisions in the same tiles. Three
+// CTAs per SM (62 KB with the sixth field of column results).
+template <int MODE, bool FRIC, bool GHOST>
+__global__ void __launch_bounds__(LTHR, 3) k_line_exact(const RhsConsts C, const StageArgs A, const int bulk) {
+  extern __shared__ __align__(128) unsigned char smem_line_exact[];
+  auto& S = *reinterpret_cast<typename LineTile<1, true>::Smem*>(smem_line_exact);
+  if (kStash<MODE> && threadIdx.x < 32) stash_alloc(&S.stash);
+  wait_for_previous();
+  line_tile<MODE, 1, FRIC, GHOST, true>(C, C, A, blockIdx.x, blockIdx.y,
+                                        (long long)blockIdx.y * gridDim.x + blockIdx.x, bulk != 0, S);
   if constexpr (kStash<MODE>) {
     __syncthreads();
     if (threadIdx.x < 32) stash_free(S.stash);
