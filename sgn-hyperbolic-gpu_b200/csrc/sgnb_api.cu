@@ -42,8 +42,7 @@ int cuda_fail(sgnb_ctx* c, cudaError_t e, const char* what) {
   } while (0)
 
 // One fused launch: mode 0 rhs (in -> out), 1 second stage (u + dt/2 k1 -> K2), 2 end-point
-// stage, 3 third stage with the candidate (the mixed mode: k3 -> K3, and the end-point stage
-// forms the candidate). Dispatches on the arithmetic mode of the context.
+// stage, 3 third stage with the candidate. Dispatches on the arithmetic mode of the context.
 struct Launch {
   int mode = 0;
   const double* in = nullptr;  // mode 0
@@ -65,7 +64,7 @@ cudaError_t launch(sgnb_ctx* c, const Launch& L, cudaStream_t s) {
     A.coef = L.stage == 3 ? 0.75 : 0.5;
     if (L.mode == 0) A.out = L.out ? nullptr : A.K1[c->cur];  // no FP64 output: the FSAL head
     else A.out = L.stage == 3 ? A.K3 : A.K2;
-    return dev::launch_fused_mixed(L.mode == 3 ? 1 : L.mode, c->C, A, s, c->mapsM.ok ? &c->mapsM : nullptr);
+    return dev::launch_fused_mixed(L.mode, c->C, A, s, c->mapsM.ok ? &c->mapsM : nullptr);
   }
   StageArgs A{};
   A.U[0] = c->U[0]; A.U[1] = c->U[1];
@@ -198,14 +197,12 @@ static bool encode_state_map(const sgnb_ctx* c, CUtensorMap* m, const void* p,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps of the context's buffers for the fused kernels' tile loads (meshes that are
-// a whole number of 8x4 tiles). The encoder comes from the driver through the runtime, so
-// the library links no driver library; without it (or on any encoding error), or with
-// SGNB_TMA=0 in the environment at creation, the kernels keep their per-thread
-// asynchronous copies. Only the data movement differs: the exact mode gives the same bits;
-// in the fast mode the TMA kernels are separate instantiations whose FMA contractions the
-// compiler chooses on its own, so they agree to round-off (tests/test_tma_gpu.py finds
-// the same bits for the whole-mesh kernels).
+// Tensor maps of a mixed-precision context's buffers for its intermediate stage's tile loads
+// (meshes that are a whole number of 8x4 tiles; the FP64 kernels copy rows and need no maps).
+// The encoder comes from the driver through the runtime, so the library links no driver
+// library; without it (or on any encoding error), or with SGNB_TMA=0 in the environment at
+// creation, the kernel keeps its per-thread asynchronous copies. Only the data movement
+// differs.
 static void build_tile_maps(sgnb_ctx* c) {
   c->mapsM.ok = 0;
   c->encode_tiled = nullptr;
@@ -1051,7 +1048,7 @@ cudaError_t batch_launch(sgnb_batch* b, int mode, int shape, int blocks, int kin
   if (!b->mixed)
     return dev::launch_fused_batch(mode, shape, blocks, batch_args(b, shape, kin_k2, coef), b->stream);
   if (shape != 0) return cudaErrorInvalidValue;  // mixed batches use one tile shape
-  return dev::launch_mixed_batch(mode == 3 ? 1 : mode, blocks, batch_args_mixed(b, kin_k2, coef), b->stream);
+  return dev::launch_mixed_batch(mode, blocks, batch_args_mixed(b, kin_k2, coef), b->stream);
 }
 
 int batch_prepare(sgnb_batch* b) {

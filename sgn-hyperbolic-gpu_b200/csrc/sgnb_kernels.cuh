@@ -1,5 +1,7 @@
-// sgnb_kernels.cuh -- fused sm_100a kernels for the 2D hyperbolic-SGN FR right-hand side
-// and the Bogacki-Shampine 3(2) stage loop.
+// sgnb_kernels.cuh -- the model, the FR line operators and the stage combinations of the 2D
+// hyperbolic-SGN FR right-hand side and the Bogacki-Shampine 3(2) stage loop, shared by the
+// FP64 kernels, and the fused kernels on Gauss-Legendre points (on Gauss-Lobatto points:
+// sgnb_kernels_line.cuh).
 //
 // One launch evaluates the whole right-hand side R(U) of a tile of elements: the five
 // phases of the reference CPU solver (face traces, nodal fluxes with per-direction GLL
@@ -9,11 +11,11 @@
 // traffic is the state in, the bathymetry statics in and dU out.
 //
 // The same kernel body also serves the three Runge-Kutta stages of one BS3(2) attempt
-// (src/solver/rk.cpp:95-131): the stage input u + a dt k, or the third-order candidate
-// uNew, is formed while the tile is loaded, and the end-point stage additionally
-// writes uNew and reduces the scaled embedded error of its tile.
+// (src/solver/rk.cpp:95-131): the stage input u + a dt k is formed while the tile is loaded,
+// the third stage writes the third-order candidate uNew, and the end-point stage reduces the
+// scaled embedded error of its tile.
 //
-// Work decomposition. A CTA owns a tile of TX x TY elements (element-contiguous rows of
+// Work decomposition on Gauss-Legendre points. A CTA owns a tile of TX x TY elements (element-contiguous rows of
 // the reference's variable-major layout U[v*Nd + e*25 + a + 5b], e = ex + Nx*ey) and
 // runs 5 warps. Lane i of every warp is tile element i; warp j is the element's
 // j-th GLL line:

@@ -1,14 +1,14 @@
-// sgnb_kernels_line.cuh -- the fast arithmetic mode's fused right-hand-side and stage
-// kernels on Gauss-Lobatto points (single instances, slabs and batches).
+// sgnb_kernels_line.cuh -- the FP64 modes' fused right-hand-side and stage kernels on
+// Gauss-Lobatto points (single instances, slabs; in the fast mode also batches).
 //
 // Work decomposition. A warp owns a row of six elements and holds one line of solution points per
 // lane (30 of 32 lanes): lane (e, j) is line j of element e, first along y (column pass), then
 // along x (row pass). All five lines of an element are in one warp, so between the passes a warp
 // synchronises with itself only; a CTA of four warps stacks four such rows (or 2 x 2, or 4 x 1)
 // and synchronises once, when its tile has landed and every warp has formed its stage inputs.
-// With the lanes over 32 elements and one warp per line instead (as the exact mode's kernels),
-// two of the eight cycles a warp took per instruction were waits at the barriers between the
-// passes.
+// With the lanes over 32 elements and one warp per line instead (as the Gauss-point kernels of
+// sgnb_kernels.cuh), two of the eight cycles a warp took per instruction were waits at the
+// barriers between the passes.
 //
 // The arithmetic is arranged for the fast mode:
 //   * every flux component is the normal velocity times a state component, F = u_n U_v (plus

@@ -13,9 +13,8 @@ static cudaError_t launch_m(const RhsConsts& C, const StageArgsM& A, cudaStream_
     mix::k_mixed<MODE, true><<<grid, mix::NTHR, sizeof(mix::Smem), s>>>(C, A);
   } else if (C.Nx % mix::TX == 0 && C.Ny % mix::TY == 0) {  // every tile full
     bool tma = false;
-    // the intermediate stage's tiles by the tensor-memory accelerator (the end-point stage
-    // was 1.4 % slower so: its per-thread copies land in five scattered areas)
-    if constexpr (MODE == mix::MODE_STAGE) {
+    // the tiles of the stages that add k by the tensor-memory accelerator
+    if constexpr (MODE == mix::MODE_STAGE || MODE == mix::MODE_CAND) {
       if (M != nullptr && M->ok) {
         mix::k_mixed_tma<MODE><<<grid, mix::NTHR, sizeof(mix::Smem), s>>>(C, A, *M);
         tma = true;
@@ -51,6 +50,7 @@ cudaError_t launch_fused_mixed(int mode, const RhsConsts& C, const StageArgsM& A
     case 0: return launch_m<mix::MODE_RHS>(C, A, s, M);
     case 1: return launch_m<mix::MODE_STAGE>(C, A, s, M);
     case 2: return launch_m<mix::MODE_FSAL>(C, A, s, M);
+    case 3: return launch_m<mix::MODE_CAND>(C, A, s, M);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -65,6 +65,9 @@ static cudaError_t prepare_mixed_fric() {
   if ((e = cudaFuncSetAttribute(mix::k_mixed<mix::MODE_STAGE, FRIC, FULL>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
     return e;
+  if ((e = cudaFuncSetAttribute(mix::k_mixed<mix::MODE_CAND, FRIC, FULL>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
+    return e;
   return cudaFuncSetAttribute(mix::k_mixed<mix::MODE_FSAL, FRIC, FULL>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
@@ -74,6 +77,9 @@ cudaError_t prepare_fused_mixed() {
   if (e == cudaSuccess) e = prepare_mixed_fric<false, true>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(mix::k_mixed_tma<mix::MODE_STAGE>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(mix::Smem));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(mix::k_mixed_tma<mix::MODE_CAND>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(mix::Smem));
   return e == cudaSuccess ? prepare_mixed_fric<true>() : e;
 }
@@ -94,6 +100,7 @@ cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaSt
     case 0: return launch_mb<mix::MODE_RHS>(blocks, B, s);
     case 1: return launch_mb<mix::MODE_STAGE>(blocks, B, s);
     case 2: return launch_mb<mix::MODE_FSAL>(blocks, B, s);
+    case 3: return launch_mb<mix::MODE_CAND>(blocks, B, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -111,6 +118,7 @@ static cudaError_t prepare_mb() {
 cudaError_t prepare_mixed_batch() {
   cudaError_t e = prepare_mb<mix::MODE_RHS>();
   if (e == cudaSuccess) e = prepare_mb<mix::MODE_STAGE>();
+  if (e == cudaSuccess) e = prepare_mb<mix::MODE_CAND>();
   if (e == cudaSuccess) e = prepare_mb<mix::MODE_FSAL>();
   return e;
 }

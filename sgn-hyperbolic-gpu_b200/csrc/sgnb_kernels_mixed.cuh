@@ -29,6 +29,13 @@
 //
 // Layout and work decomposition are those of sgnb_kernels.cuh (8 x 4 element tiles, 5 warps,
 // lane = element, warp = GLL line); shared memory is 56.3 KB, so 3 CTAs fit per SM.
+//
+// What bounds it: instruction latency and the conversions between the two precisions (XU pipe). At
+// 1024 x 512 elements, ms per launch: right-hand side 0.393, second stage 0.425, third stage with
+// the candidate 0.577, end point 0.606; with the candidate formed by the end point, from four arrays
+// at every own and halo node, 0.425 and 0.789. Storing the k1..k3 part of the embedded solution
+// instead of k3 took 0.62 and 0.58. The third stage prefetches its epilogue's k1 to L2 (0.592
+// without); the same for all that the end point's epilogue reads cost it 0.03 ms.
 #pragma once
 
 #include <cstdint>
@@ -51,7 +58,15 @@ constexpr int NHIT = (NV * NHALO * NP + NTHR - 1) / NTHR;
 constexpr int NFACE = (2 * TE + TY + TX) * NP;
 constexpr int NFIT = (NFACE + NTHR - 1) / NTHR;
 
-enum : int { MODE_RHS = 0, MODE_STAGE = 1, MODE_FSAL = 2 };
+enum : int {
+  MODE_RHS = 0,    // dU = R(U)
+  MODE_STAGE = 1,  // second stage: k2 = R(u + dt/2 k1)
+  MODE_FSAL = 2,   // k4 = R(uNew) of the candidate the third stage left; error partials
+  // third stage: k3 = R(u + 3/4 dt k2), and the candidate uNew to the spare state buffer. The end
+  // point then loads one array with its halo, where it formed the candidate from four at every
+  // own and halo node
+  MODE_CAND = 3
+};
 
 struct Smem {
   double h[TE][NPP];          // full depth (FP64)
@@ -82,9 +97,6 @@ struct StageInM {
   const double* __restrict__ in;
   const double* __restrict__ u;
   const float* __restrict__ k;
-  const float* __restrict__ k1;
-  const float* __restrict__ k2;
-  const float* __restrict__ k3;
   double acoef, dt;
 };
 
@@ -102,13 +114,8 @@ __device__ __forceinline__ double fsal_m(double u, float k1, float k2, float k3,
 
 template <int MODE>
 __device__ __forceinline__ double stage_value(const StageInM& I, long long idx) {
-  if constexpr (MODE == MODE_RHS) {
-    return I.in[idx];
-  } else if constexpr (MODE == MODE_STAGE) {
-    return stage_m(I.u[idx], I.acoef, I.k[idx]);
-  } else {
-    return fsal_m(I.u[idx], I.k1[idx], I.k2[idx], I.k3[idx], I.dt);
-  }
+  if constexpr (MODE == MODE_RHS || MODE == MODE_FSAL) return I.in[idx];
+  else return stage_m(I.u[idx], I.acoef, I.k[idx]);
 }
 
 // Nodal still-depth gradient at node (a, b) of an element from its nodal depths He (FP64):
@@ -285,7 +292,7 @@ __device__ __forceinline__ void line_mixed(const TC& C, const TB& Tb, const doub
 // One tile (bx, by) of the mixed-precision right-hand side / stage kernel, error partial
 // slot blk. Shared by the single-instance kernel and the batched kernel. FULL: the mesh is
 // a whole number of tiles (the per-item range checks are compiled out).
-// TMA: the intermediate stage's nodal depths and FP32 stage derivatives arrive by
+// TMA: the nodal depths and the FP32 stage derivative of the stages that add one arrive by
 // tensor-memory-accelerator copies described by M (full tiles of the single-instance
 // kernel only).
 template <int MODE, class TC, class TB, class TA, bool FRIC = false, bool FULL = false,
@@ -293,7 +300,8 @@ template <int MODE, class TC, class TB, class TA, bool FRIC = false, bool FULL =
 __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& A, int bx, int by,
                                            long long blk, Smem& S,
                                            const TileMapsM* M = nullptr) {
-  static_assert(!TMA || (FULL && MODE == MODE_STAGE), "tile copies: full tiles, intermediate stage");
+  constexpr bool kAddsK = MODE == MODE_STAGE || MODE == MODE_CAND;
+  static_assert(!TMA || (FULL && kAddsK), "tile copies: full tiles, stages that add k");
 
   int cur = 0;
   double atol = 0.0, rtol = 0.0;
@@ -311,9 +319,7 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
   }
   I.u = A.U[cur];
   I.k = A.kin_k2 ? A.K2 : A.K1[cur];
-  I.k1 = A.K1[cur];
-  I.k2 = A.K2;
-  I.k3 = A.K3;
+  if constexpr (MODE == MODE_FSAL) I.in = A.U[cur ^ 1];
 
   int tid;  // opaque: keeps per-thread descriptors out of the batched kernel's tile loop
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
@@ -502,8 +508,7 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
         }
       }
     }
-    double* __restrict__ unew = A.U[cur ^ 1];
-    if constexpr (MODE == MODE_STAGE && !TMA) {
+    if constexpr (kAddsK && !TMA) {
       // k (FP32) by asynchronous copies into the still unused G area
 #pragma unroll
       for (int v = 0; v < NV; ++v)
@@ -515,46 +520,40 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
                          "l"((I.k + (long long)v * Nd) + gof[u]) : "memory");
           }
     }
-    // end-point stage: k1 and k2 by asynchronous copies into the (still unused) G, q and d
-    // areas, ten FP32 fields: those of fields 0, 1, 2 in G (never written while the
-    // candidate is formed), of field 3 in q (hw and hp, written by the same thread at the
-    // same index after their read), of field 4 in d viewed as floats (written, as doubles
-    // at other indices, only after a barrier that follows every read)
-    auto k12_slot = [&](int w, int v) -> float* {  // w: 0 = k1, 1 = k2
-      if (v < 3) return &S.G[2 * v + w][0][0];
-      if (v == 3) return &S.q[w][0][0];
-      return reinterpret_cast<float*>(&S.d[0][0][0]) + w * TE * NPP;
-    };
     if constexpr (MODE == MODE_FSAL) {
+      // h, hu, hv straight into place
 #pragma unroll
-      for (int w = 0; w < 2; ++w)
+      for (int v = 0; v < 3; ++v)
 #pragma unroll
-        for (int v = 0; v < NV; ++v)
-#pragma unroll
-          for (int u = 0; u < NIT; ++u)
-            if (okk[u] && SGNB_INB(gof[u], Nd)) {
-              const unsigned sa = (unsigned)__cvta_generic_to_shared(k12_slot(w, v) + sof[u]);
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa),
-                           "l"(((w == 0 ? I.k1 : I.k2) + (long long)v * Nd) + gof[u]) : "memory");
-            }
+        for (int u = 0; u < NIT; ++u)
+          if (okk[u] && SGNB_INB(gof[u], Nd))
+            cp_async8(&(v == 0 ? &S.h[0][0] : &S.d[v - 1][0][0])[sof[u]], (I.in + (long long)v * Nd) + gof[u]);
+    }
+    // k1, which the epilogue will read, on its way to L2 while the tile is computed
+    if constexpr (MODE == MODE_CAND) {
+      constexpr int LK = (RUN * 4 + 127) / 128;  // lines of a row
+#pragma unroll 1
+      for (int q = tid; q < NV * TY * LK; q += NTHR) {
+        const int n = 32 * (q % LK), iy = (q / LK) % TY, v = q / (LK * TY);
+        const long long g = (long long)v * Nd + ((long long)ex0 + (long long)Nx * (ey0 + iy)) * NPP + n;
+        if (iy < TYv && n < TXv * NPP && SGNB_INB(g, NV * Nd))
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(A.K1[cur] + g));
+      }
     }
     // end-point stage: the halo loads go first, in flight together with the tile's own
     // (the other modes are faster issuing them after the combination)
     if constexpr (MODE == MODE_FSAL) halo_load();
-    // every u load (and, at the end point, every k3 load) of the tile in flight before the
+    // every u load of the tile (the end point: hw and hp of the candidate) in flight before the
     // first combination
     double ux[NV][NIT];
-    float k3x[NV][NIT];
     if constexpr (MODE != MODE_RHS) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v)
+      for (int v = MODE == MODE_FSAL ? 3 : 0; v < NV; ++v)
 #pragma unroll
         for (int u = 0; u < NIT; ++u)
-          if (okk[u] && SGNB_INB(gof[u], Nd)) {
-            ux[v][u] = (I.u + (long long)v * Nd)[gof[u]];
-            if constexpr (MODE == MODE_FSAL) k3x[v][u] = (I.k3 + (long long)v * Nd)[gof[u]];
-          }
-      cp_async_wait_all();  // k (k1, k2) and the statics have landed
+          if (okk[u] && SGNB_INB(gof[u], Nd))
+            ux[v][u] = ((MODE == MODE_FSAL ? I.in : I.u) + (long long)v * Nd)[gof[u]];
+      cp_async_wait_all();  // k (the end point's h, hu, hv) and the statics have landed
       if constexpr (TMA) {
         bool landed = false;
         for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
@@ -569,21 +568,16 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
         }
       }
     }
-    // fields in the order 3, 4, 0, 1, 2: the end-point stage's field-4 derivatives sit in
-    // the d area, which fields 1 and 2 overwrite after the barrier
 #pragma unroll
-    for (int o = 0; o < NV; ++o) {
-      const int v = (o + 3) % NV;
-      if (MODE == MODE_FSAL && v == 1) __syncthreads();
+    for (int v = MODE == MODE_FSAL ? 3 : 0; v < NV; ++v) {
       double x[NIT];
 #pragma unroll
       for (int u = 0; u < NIT; ++u)
         if (okk[u]) {
-          if constexpr (MODE == MODE_STAGE)
+          if constexpr (kAddsK)
             x[u] = stage_m(ux[v][u], I.acoef, (&S.G[v][0][0])[sof[u]]);
           else if constexpr (MODE == MODE_FSAL)
-            x[u] = fsal_m(ux[v][u], k12_slot(0, v)[sof[u]], k12_slot(1, v)[sof[u]], k3x[v][u],
-                          I.dt);
+            x[u] = ux[v][u];
           else
             x[u] = SGNB_INB(gof[u], Nd) ? stage_value<MODE>(I, (long long)v * Nd + gof[u]) : 0.0;
         }
@@ -593,8 +587,6 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
           if (v == 0) (&S.h[0][0])[sof[u]] = x[u];
           else if (v < 3) (&S.d[v - 1][0][0])[sof[u]] = x[u];
           else (&S.q[v - 3][0][0])[sof[u]] = (float)x[u];
-          if constexpr (MODE == MODE_FSAL)
-            if (SGNB_INB(gof[u], Nd)) __stcs(&(unew + (long long)v * Nd)[gof[u]], x[u]);
         }
     }
     if constexpr (MODE != MODE_FSAL) halo_load();
@@ -757,8 +749,8 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
   __syncthreads();
 
   // ---- copy-out and the FP64 embedded error of the end-point stage ---------------
-  // Results are stored, and the end-point stage's last reads of u, k1, k2, k3 loaded,
-  // with the streaming (evict-first) hint, as in the FP64 kernels.
+  // Results are stored, and the end-point stage's reads of u, k1, k2, k3 loaded, with the
+  // streaming (evict-first) hint, as in the FP64 kernels.
   double esum = 0.0, emax = 0.0;
   int enan = 0;
   item_map();
@@ -779,6 +771,44 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
 #pragma unroll
       for (int u = 0; u < NIT; ++u)
         if (okk[u] && SGNB_INB(gof[u], Nd)) __stcs(&(A.out + (long long)v * Nd)[gof[u]], (&S.G[v][0][0])[sof[u]]);
+  } else if constexpr (MODE == MODE_CAND) {
+    // k3 and the candidate; the next field's u, k1, k2 load while this one's is formed
+    const CtrlReload rc = ctrl_reload(A.ctrl);
+    cur = rc.cur;
+    const double dt = rc.dt;
+    const double* __restrict__ u0 = A.U[cur];
+    const float* __restrict__ k1p = A.K1[cur];
+    const float* __restrict__ k2p = A.K2;
+    double* __restrict__ unew = A.U[cur ^ 1];
+    double uu[NIT], nu[NIT];
+    float c1[NIT], c2[NIT], n1[NIT], n2[NIT];
+#pragma unroll
+    for (int u = 0; u < NIT; ++u)
+      if (okk[u]) {
+        const int g = gof[u];
+        if (SGNB_INB(g, Nd)) { uu[u] = u0[g]; c1[u] = k1p[g]; c2[u] = k2p[g]; }
+      }
+#pragma unroll 1
+    for (int v = 0; v < NV; ++v) {
+      if (v + 1 < NV) {
+#pragma unroll
+        for (int u = 0; u < NIT; ++u)
+          if (okk[u]) {
+            const long long o = (long long)(v + 1) * Nd;
+            const int g = gof[u];
+            if (SGNB_INB(o + g, NV * Nd)) { nu[u] = (u0 + o)[g]; n1[u] = (k1p + o)[g]; n2[u] = (k2p + o)[g]; }
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < NIT; ++u)
+        if (okk[u] && SGNB_INB(gof[u], Nd)) {
+          const float k3 = (&S.G[v][0][0])[sof[u]];
+          __stcs(&(A.out + (long long)v * Nd)[gof[u]], k3);
+          __stcs(&(unew + (long long)v * Nd)[gof[u]], fsal_m(uu[u], c1[u], c2[u], k3, dt));
+        }
+#pragma unroll
+      for (int u = 0; u < NIT; ++u) { uu[u] = nu[u]; c1[u] = n1[u]; c2[u] = n2[u]; }
+    }
   } else {
     const CtrlReload rc = ctrl_reload(A.ctrl);
     cur = rc.cur;
@@ -874,7 +904,7 @@ __global__ void __launch_bounds__(NTHR, SGNB_MIXED_MIN_CTAS) k_mixed(const RhsCo
       C, C, A, blockIdx.x, blockIdx.y, (long long)blockIdx.y * gridDim.x + blockIdx.x, S);
 }
 
-// Intermediate stage on a mesh of whole tiles, with the nodal depths and the stage
+// A stage that adds k on a mesh of whole tiles, with the nodal depths and the stage
 // derivative loaded by the tensor-memory accelerator from the context's buffers that M
 // describes.
 template <int MODE>
@@ -905,7 +935,8 @@ __device__ __forceinline__ void mixed_batch_tile(const BatchArgsM& B, long long 
   if (threadIdx.x == 0) {
     As.kin_k2 = B.kin_k2;
     As.coef = B.coef;
-    if (MODE == MODE_STAGE) As.out = B.kin_k2 ? As.K3 : As.K2;
+    if (MODE == MODE_STAGE) As.out = As.K2;
+    if (MODE == MODE_CAND) As.out = As.K3;
   }
   __syncthreads();
   const int ntx = (Cs.Nx + TX - 1) / TX;
