@@ -506,12 +506,6 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   c->ntot = 5 * c->Nd;
   auto bail = [&](int code) { sgnb_destroy(c); return code; };
   if ((rc = set_device(c))) { g_create_error = c->err; delete c; return rc; }
-  e = dev::prepare_fused_exact();
-  if (e == cudaSuccess) e = dev::prepare_fused_fast();
-  if (e == cudaSuccess) e = dev::prepare_fused_mixed();
-  if (e == cudaSuccess) e = dev::prepare_fused_batch();
-  if (e == cudaSuccess) e = dev::prepare_mixed_batch();
-  if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
 
   // statics: Hnod, Hx, Hy (Nd each), HfX, HfY (5 ne each), HfXEnd (5 Ny), HfYEnd (5 Nx)
   Bathymetry b;
@@ -561,6 +555,10 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
     if (e != cudaSuccess) { cuda_fail(c, e, "cudaMalloc(traces)"); g_create_error = c->err; return bail(SGNB_ERR_NOMEM); }
   }
   fill_consts(c);
+  // only the kernels that this context launches: raising a kernel's shared memory loads its code
+  e = c->mixed ? dev::prepare_fused_mixed()
+               : (c->precision == SGNB_FP64_FAST ? dev::prepare_fused_fast(c->C) : dev::prepare_fused_exact(c->C));
+  if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
 
   const size_t sbytes = (size_t)c->ntot * sizeof(double);
   // stage derivatives are FP32 in the mixed mode; K2 and K3 are allocated as one block so
@@ -1485,7 +1483,9 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
     sgnb_batch_destroy(b);
     return bfail(nullptr, e == cudaErrorMemoryAllocation ? SGNB_ERR_NOMEM : SGNB_ERR_CUDA, m);
   };
-  cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  cudaError_t e = b->mixed ? dev::prepare_mixed_batch() : dev::prepare_fused_batch();
+  if (e != cudaSuccess) return bail(e, "kernel attributes");
+  e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evRead, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&b->dconsts, n * sizeof(LineConsts));
   if (e == cudaSuccess) e = cudaMalloc(&b->dconstsM, n * sizeof(RhsConsts));

@@ -415,8 +415,8 @@ cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A,
 cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t prepare_line();
-cudaError_t prepare_fused_exact();
-cudaError_t prepare_fused_fast();
+cudaError_t prepare_fused_exact(const RhsConsts& C);
+cudaError_t prepare_fused_fast(const RhsConsts& C);
 cudaError_t launch_fused_mixed(int mode, const RhsConsts& C, const StageArgsM& A,
                                cudaStream_t s, const TileMapsM* M = nullptr);
 cudaError_t prepare_fused_mixed();

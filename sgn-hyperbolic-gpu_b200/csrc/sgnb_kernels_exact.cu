@@ -43,10 +43,12 @@ static cudaError_t prepare_mode() {
   return e;
 }
 
-cudaError_t prepare_fused_exact() {
-  cudaError_t e = prepare_variant<false>();
-  if (e == cudaSuccess) e = prepare_variant<true>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_RHS>();
+cudaError_t prepare_fused_exact(const RhsConsts& C) {
+  if (C.gauss) {
+    const cudaError_t g = prepare_variant<false>();
+    return g == cudaSuccess ? prepare_variant<true>() : g;
+  }
+  cudaError_t e = prepare_mode<MODE_RHS>();
   if (e == cudaSuccess) e = prepare_mode<MODE_STAGE>();
   if (e == cudaSuccess) e = prepare_mode<MODE_CAND>();
   if (e == cudaSuccess) e = prepare_mode<MODE_FSAL>();

@@ -20,11 +20,10 @@ cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, 
     default: return cudaErrorInvalidValue;
   }
 }
-cudaError_t prepare_fused_fast() {
-  cudaError_t e = prepare_variant<false>();
-  if (e == cudaSuccess) e = prepare_variant<true>();
-  if (e == cudaSuccess) e = prepare_line();
-  return e;
+cudaError_t prepare_fused_fast(const RhsConsts& C) {
+  if (!C.gauss) return C.sym ? prepare_line() : prepare_fused_exact(C);
+  const cudaError_t e = prepare_variant<false>();
+  return e == cudaSuccess ? prepare_variant<true>() : e;
 }
 
 // The checked build's out-of-range count of this translation unit's kernels (reset: then
