@@ -52,21 +52,25 @@ sys.path.insert(0, os.path.join(ROOT, "sgn-hyperbolic-gpu_b200"))
 
 METRIC = "DOF-updates/s per RK stage"
 UNIT = "DOF-updates/s"
-# Algorithmic HBM bytes per DOF (8 B doubles) of the fused kernels: U in and dU out (16),
-# the nodal depth H (8 / 5 fields = 1.6) and the face depths (2 x 5 per element / 125 DOF
-# x 8 = 0.64). The nodal depth gradients dH/dx, dH/dy (3.2 B/DOF more if read) are formed
-# from the depth tile in shared memory, so they are not part of the kernels' traffic.
-STATIC_B = 1.6 + 0.64
+# Algorithmic HBM bytes per DOF (8 B doubles) of the FP64 kernels: state-sized arrays in and
+# out and the nodal depth H (8 / 5 fields = 1.6). The nodal depth gradients are formed from the
+# depth tile, and the fast mode reads no face depths (they cancel; the exact mode's 0.64 more
+# are not counted).
+STATIC_B = 1.6
 BYTES_PER_DOF = {
-    "rhs": 16.0 + STATIC_B,                  # 18.24
-    "stage": 8 + 8 + STATIC_B + 8,           # u, k in; k_out out: 26.24
-    "fsal": 4 * 8 + STATIC_B + 2 * 8,        # u, k1..k3 in; uNew, k4 out: 50.24
+    "rhs": 16.0 + STATIC_B,                  # 17.6
+    "stage": 3 * 8 + STATIC_B,               # stage 2: u, k1 in; k2 out: 25.6
+    "cand": 5 * 8 + STATIC_B,                # stage 3: u, k1, k2 in; uNew, embedded part out: 41.6
+    "fsal": 4 * 8 + STATIC_B,                # end point: uNew, u, part in; k4 out: 33.6
 }
-# Mixed precision: FP64 state, FP32 stage derivatives (4 B), FP64 statics.
+# Mixed precision: FP64 state, FP32 stage derivatives (4 B), FP64 statics with the face depths
+# (0.64).
+STATIC_M = 1.6 + 0.64
 BYTES_PER_DOF_MIXED = {
-    "rhs": 16.0 + STATIC_B,                  # FP64 in and out (rhs callers): 18.24
-    "stage": 8 + 4 + STATIC_B + 4,           # u (8), k (4) in; k_out (4): 18.24
-    "fsal": 8 + 3 * 4 + STATIC_B + 8 + 4,    # u, k1..k3 in; uNew (8), k4 (4) out: 34.24
+    "rhs": 16.0 + STATIC_M,                  # FP64 in and out (rhs callers): 18.24
+    "stage": 8 + 4 + STATIC_M + 4,           # u (8), k (4) in; k_out (4): 18.24
+    "cand": 8 + 2 * 4 + STATIC_M + 4 + 8,    # u, k1, k2 in; k3 (4), uNew (8) out: 30.24
+    "fsal": 2 * 8 + 3 * 4 + STATIC_M + 4,    # uNew, u, k1..k3 in; k4 (4) out: 34.24
 }
 
 
@@ -228,7 +232,7 @@ def run_ours(args):
     # ---- roofline of the fused stage kernels, timed alone on the same stream -------
     dt_probe = st.dtLast if st.dtLast > 0 else dt0
     per = {}
-    for stage, key in ((2, "stage"), (4, "fsal")):
+    for stage, key in ((2, "stage"), (3, "cand"), (4, "fsal")):
         solver.launch_stage(stage, dt_probe, 2)
         torch.cuda.synchronize()
         reps = 10
@@ -239,26 +243,25 @@ def run_ours(args):
         a1.record(stream)
         torch.cuda.synchronize()
         per[key] = a0.elapsed_time(a1) / 1e3 / reps
-    dominant = "fsal" if per["fsal"] >= 2 * per["stage"] else "stage"
+    dominant = max(per, key=per.get)
     peak, peak_kind = measured_peak_hbm()
     bpd = BYTES_PER_DOF_MIXED if args.precision == "mixed" else BYTES_PER_DOF
     achieved = bpd[dominant] * dof / per[dominant] / 1e9
     tpd = traffic_per_dof()
-    traffic = tpd.get(dominant) if args.precision != "mixed" else None
-    roofline = {"bound": "hbm", "kernel": f"k_fused_tma ({dominant} mode; k_fused on meshes of partial tiles)",
+    traffic = tpd.get({"fsal": "endpoint"}.get(dominant, dominant)) if args.precision != "mixed" else None
+    roofline = {"bound": "hbm", "kernel": f"{'k_mixed' if args.precision == 'mixed' else 'k_line'} ({dominant} mode)",
                 "achieved": round(achieved, 1), "peak": peak, "peak_kind": peak_kind,
                 "unit": "GB/s", "frac": round(achieved / peak, 4),
                 "traffic": (round(traffic * dof) if traffic else None),
                 "algorithmic_bytes": round(bpd[dominant] * dof),
                 "launch_ms": {k: round(v * 1e3, 4) for k, v in per.items()}}
-    # both stage kernels, with their shares of an attempt (two intermediate stages and one
-    # end point): the two are close to even, so the dominant one can change between runs
-    attempt = 2 * per["stage"] + per["fsal"]
+    # the three stage kernels, with their shares of an attempt
+    attempt = sum(per.values())
     roofline["kernels"] = {
         k: {"achieved": round(bpd[k] * dof / per[k] / 1e9, 1),
             "frac": round(bpd[k] * dof / per[k] / 1e9 / peak, 4),
-            "share_of_attempt": round((2 if k == "stage" else 1) * per[k] / attempt, 4)}
-        for k in ("stage", "fsal")}
+            "share_of_attempt": round(per[k] / attempt, 4)}
+        for k in per}
 
     # ---- e2e through the public API with host buffers ----------------------------
     torch.cuda.synchronize()

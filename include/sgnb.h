@@ -170,10 +170,12 @@ int sgnb_rk4_steps(sgnb_ctx* ctx, double t0, const double* dts, long long n);
 int sgnb_attempt_log(sgnb_ctx* ctx, double* out, long long cap, long long* n);
 
 /* Profiling hook, no reference counterpart: launches `count` copies of one fused stage
- * kernel of a BS3(2) attempt (stage 2: k2 = R(u + dt/2 k1); 3: k3 = R(u + 3dt/4 k2);
- * 4: the end-point stage with uNew, k4 and the error partials) on the uploaded state with
- * step dt, on `stream` (NULL = context stream), asynchronously. It overwrites only the
- * stage buffers, so the uploaded state is unchanged; run an integration first so that
+ * kernel of a BS3(2) attempt (stage 2: k2 = R(u + dt/2 k1); 3: k3 = R(u + 3dt/4 k2), which
+ * the FP64 modes leave on chip: the kernel writes the candidate uNew into the spare state
+ * buffer and k1, k2, k3's part of the embedded error; 4: the end-point stage with k4 and the
+ * error partials, of the candidate stage 3 left) on the uploaded state with step dt, on
+ * `stream` (NULL = context stream), asynchronously. It overwrites only the stage buffers and
+ * the spare state, so the uploaded state is unchanged; run an integration first so that
  * k1 is defined. */
 int sgnb_launch_stage(sgnb_ctx* ctx, int stage, double dt, int count, void* stream);
 
@@ -247,7 +249,8 @@ int sgnb_checked_oob(int device, long long* count, int reset);
  *   sgnb_slab_pack    this slab's edge nodes for the neighbours: stage 0 = the input
  *                     `in` of a right-hand side (NULL: the current state), 2 / 3 = the
  *                     intermediate stages of the running attempt, 4 = its end-point
- *                     candidate; sendL / sendR are [5][Ny][5] device arrays
+ *                     candidate (which its stage 3 has written: pack 4 comes after
+ *                     stage 3's launch); sendL / sendR are [5][Ny][5] device arrays
  *   sgnb_slab_begin   the controller from t0 with dt0 until tEnd (HUGE_VAL: none) or
  *                     nsteps accepted steps (0: none), whichever comes first (dts != NULL:
  *                     nsteps frozen step sizes, the bs3Step replay)
@@ -312,8 +315,8 @@ int sgnb_write_vtk(sgnb_ctx* ctx, const char* path);
  * instance with its own adaptive controller; the attempts run as a device-side loop (a
  * CUDA graph whose WHILE conditional node repeats one attempt of every still-running
  * instance until all are done). All
- * instances of a batch run in one arithmetic mode: SGNB_FP64_FAST (tile shapes 8x4, 16x2,
- * 4x8) or SGNB_MIXED (8x4 tiles). Instance i is an ordinary context
+ * instances of a batch run in one arithmetic mode: SGNB_FP64_FAST (tile shapes 6x4, 12x2,
+ * 24x1) or SGNB_MIXED (8x4 tiles). Instance i is an ordinary context
  * (sgnb_batch_instance) for upload / download / diagnostics between runs. */
 typedef struct sgnb_batch sgnb_batch;
 int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out);
@@ -326,9 +329,10 @@ sgnb_ctx* sgnb_batch_instance(sgnb_batch* b, int i);
 /* nsteps accepted steps for every instance, starting from dt0[i]; stats[n]. */
 int sgnb_batch_integrate_steps(sgnb_batch* b, const double* dt0, long long nsteps,
                                const sgnb_rk_opts* opts, sgnb_rk_stats* stats);
-/* Launch configuration: tile shape (0: 8x4, 1: 16x2, 2: 4x8 elements) and the grid:
- * blocks == 0 launches one CTA per tile of the work list, blocks > 0 that many persistent
- * CTAs looping over it (default: 8x4, one CTA per tile; sgnb_batch_autotune picks one). */
+/* Launch configuration: tile shape (0: 6x4, 1: 12x2, 2: 24x1 elements; in a
+ * mixed batch 8x4, shape 0 only) and the grid: blocks == 0 launches one CTA per tile of the
+ * work list, blocks > 0 that many persistent CTAs looping over it (default: shape 0, one CTA
+ * per tile; sgnb_batch_autotune picks one). */
 int sgnb_batch_set_config(sgnb_batch* b, int shape, int blocks);
 int sgnb_batch_get_config(const sgnb_batch* b, int* shape, int* blocks);
 /* Autotuner: times one adaptive attempt (three stage launches, reps times) for every tile

@@ -644,7 +644,7 @@ class SGNBatch:
 
     def autotune(self, dt0, reps=3):
         """Times every (tile shape, grid) pair; keeps the fastest. Returns ms per attempt,
-        [3 shapes (8x4, 16x2, 4x8), 5 grids (one CTA per tile, 1..4 persistent CTAs per
+        [3 shapes (6x4, 12x2, 24x1; mixed: 8x4), 5 grids (one CTA per tile, 1..4 persistent CTAs per
         SM)]."""
         d = np.ascontiguousarray(np.broadcast_to(np.asarray(dt0, dtype=np.float64), (self.n,)))
         ms = np.zeros(15)

@@ -30,10 +30,10 @@ from . import workloads as W
 
 METRIC = "DOF-updates/s per RK stage"
 UNIT = "DOF-updates/s"
-# algorithmic bytes per DOF of one fused BS3(2) attempt (two intermediate stages and the
-# end-point stage; nodal depth gradients formed on chip): FP64 and mixed precision
-STAGE_LOOP_BYTES = 2 * 26.24 + 50.24
-MIXED_LOOP_BYTES = 2 * 18.24 + 34.24
+# algorithmic bytes per DOF of one fused BS3(2) attempt (two intermediate stages, the
+# second with the candidate, and the end-point stage; nodal depth gradients formed on chip): FP64 and mixed precision
+STAGE_LOOP_BYTES = 25.6 + 41.6 + 33.6
+MIXED_LOOP_BYTES = 18.24 + 30.24 + 34.24
 
 
 def _rel_per_field(a, b):
@@ -114,13 +114,14 @@ def run_sweep(args, clock_sampler, peak):
                                "alpha U[1.5,6], shoal crest U[0.3,0.9], Gaussian hump), "
                                "walls, per-instance adaptive BS3(2), K accepted steps each",
                    "instances": n, "dof_total": int(dofs.sum()),
-                   "tile_shape": ["8x4", "16x2", "4x8"][shape],
+                   "tile_shape": "8x4" if mixed else ["6x4", "12x2", "24x1"][shape],
                    "grid": "one CTA per tile" if blocks == 0 else f"{blocks} persistent CTAs",
                    "rejected": int(sum(s.rejected for s in st)),
                    "l2": f"inputs larger than L2 ({8 * dofs.sum() / 1e9:.1f} GB per state)"},
         "sequential_single_instance": {"value": seq_value, "unit": UNIT, "time_s": t_seq},
         "speedup_vs_sequential": value / seq_value,
-        "autotune_ms_per_attempt": {"shapes": ["8x4", "16x2", "4x8 (-1: not used)"],
+        "autotune_ms_per_attempt": {"shapes": (["8x4"] + 2 * ["not used (-1)"]) if mixed else
+                                    ["6x4", "12x2", "24x1"],
                                     "grids": ["per tile", "1/SM", "2/SM", "3/SM", "4/SM"],
                                     "ms": np.round(tune, 3).tolist()},
         "roofline": {"bound": "hbm", "kernel": "batched stage kernels, one attempt",

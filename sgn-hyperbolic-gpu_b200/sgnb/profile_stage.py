@@ -14,7 +14,7 @@ launch needs. Prints the CUDA-event time per launch.
 runs the batched stage kernels instead: the first N instances of configuration 4's sweep
 (one autotune pass, `count` attempts per tile shape and grid form, each attempt the three
 stage launches, all launched directly rather than inside the device-side loop's graph).
-The first end-point launch is the 8x4-tile, one-CTA-per-tile form. Prints the
+The first end-point launch is the first tile shape, one CTA per tile. Prints the
 autotuner's time per attempt for each form.
 """
 from __future__ import annotations
@@ -42,7 +42,7 @@ def profile_batch(a, prec):
         tune = b.autotune(dt0, reps=a.count)
         dof = sum(125 * kw["Nx"] * kw["Ny"] for kw in inst)
         print(f"batch of {len(inst)} instances ({dof:,} DOF), {a.precision}: ms per attempt "
-              f"[8x4, 16x2, 4x8] x [per tile, 1..4 per SM] = {np.round(tune, 4).tolist()}")
+              f"[6x4, 12x2, 24x1] x [per tile, 1..4 per SM] = {np.round(tune, 4).tolist()}")
 
 
 def main():

@@ -53,7 +53,8 @@ def neighbours(rank: int, size: int, periodic: bool) -> tuple[int | None, int | 
 
 
 def tile_count(Nx: int, Ny: int) -> int:
-    """Tiles (8 x 4 elements) of one slab's fused grid = its error partial blocks."""
+    """Tiles of 8 x 4 elements of a mesh (how many error partials a slab has depends on its
+    kernels' tiles: sgnb_slab_partials says)."""
     return ((Nx + 7) // 8) * ((Ny + 3) // 4)
 
 
