@@ -19,7 +19,7 @@
 //     same one): no face depths are read;
 //   * the GLL differentiation matrix changes sign under reflection of its rows and columns and
 //     the two correction functions mirror each other, so a 5-point derivative with both
-//     lifts splits into an even and an odd half (27 operations instead of 35);
+//     lifts splits into an even and an odd half (29 operations instead of 35);
 //   * each pass adds its own direction's sources, so no pass differentiates the depth along
 //     the other direction, and h_n and H_n of the hp equation share one derivative.
 // What bounds it. At 1024 x 512 elements a right-hand side takes 0.227 ms (5.1 TB/s, 79 % of a
@@ -182,12 +182,15 @@ __device__ __forceinline__ void store_pair(double* p, double2 x, bool vec, bool 
 }
 
 // Derivative of the five values F along a line plus the lifts of the face jumps jl, jr, all
-// before the division by J.
+// before the division by J. The rows of D sum to zero, so it acts on the differences to the centre
+// value, which are exact or nearly so where F varies little along the line; F_0 + F_4 first and
+// 2 F_2 off it would round at the size of F itself (two operations less; a right-hand side of 128 x
+// 64 elements was then up to 1.35 times as far from the true value in a field).
 template <class TE_>
 __device__ __forceinline__ void line_derivative(const TE_& T, const double (&F)[NP], double jl,
                                                 double jr, double (&d)[NP]) {
   const double o0 = F[0] - F[4], o1 = F[1] - F[3];
-  const double e0 = fma(-2.0, F[2], F[0] + F[4]), e1 = fma(-2.0, F[2], F[1] + F[3]);
+  const double e0 = (F[0] - F[2]) + (F[4] - F[2]), e1 = (F[1] - F[2]) + (F[3] - F[2]);
   const double js = jl + jr, jd = jl - jr;
   const double E0 = fma(T.A[0], e0, fma(T.A[1], e1, T.b[0] * js));
   const double E1 = fma(T.A[2], e0, fma(T.A[3], e1, T.b[1] * js));
@@ -203,7 +206,7 @@ __device__ __forceinline__ void line_derivative(const TE_& T, const double (&F)[
 template <class TE_>
 __device__ __forceinline__ void line_derivative(const TE_& T, const double (&F)[NP], double (&d)[NP]) {
   const double o0 = F[0] - F[4], o1 = F[1] - F[3];
-  const double e0 = fma(-2.0, F[2], F[0] + F[4]), e1 = fma(-2.0, F[2], F[1] + F[3]);
+  const double e0 = (F[0] - F[2]) + (F[4] - F[2]), e1 = (F[1] - F[2]) + (F[3] - F[2]);
   const double E0 = fma(T.A[0], e0, T.A[1] * e1), E1 = fma(T.A[2], e0, T.A[3] * e1);
   const double O0 = fma(T.B[0], o0, T.B[1] * o1), O1 = fma(T.B[2], o0, T.B[3] * o1);
   d[2] = fma(T.B[4], o0, T.B[5] * o1);
@@ -219,7 +222,10 @@ __device__ __forceinline__ void line_derivative(const TE_& T, const double (&F)[
 // the line's own end node). Calls emit(v, k, r) with r = the line's share of -dU at node k: the
 // divergence of flux v, the non-conservative product and minus the direction's sources; the
 // sources without a direction (gamma p, -2 c^2 w) go with y, friction with x.
-template <int DIR, int US, bool FRIC, class TC, class TE_, class Emit>
+// LATE: the faces' discharge differences are formed where they are used instead of once. The end
+// point, whose other state leaves the passes fewer registers, spills without (1024 x 512 elements:
+// 0.495 ms instead of 0.517); the right-hand side is 2.4 % slower with it.
+template <int DIR, int US, bool FRIC, bool LATE, class TC, class TE_, class Emit>
 __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const double* u,
                                            const double* hl, const double* lo, const double* hi,
                                            double slo, double shi, Emit&& emit) {
@@ -247,19 +253,26 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
   };
   const double lamL = 0.5 * fmax(speed(hL, hpL * ihL, unL), speed(h[0], hp[0] * ih[0], un[0]));
   const double lamR = 0.5 * fmax(speed(h[4], hp[4] * ih[4], un[4]), speed(hR, hpR * ihR, unR));
-  const double dnL = hnL - hn[0], dnR = hnR - hn[4];
+  double dL = 0.0, dR = 0.0;
+  if constexpr (!LATE) {
+    dL = hnL - hn[0];
+    dR = hnR - hn[4];
+  }
+  auto dnL = [&] { return LATE ? hnL - hn[0] : dL; };
+  auto dnR = [&] { return LATE ? hnR - hn[4] : dR; };
   double F[NP], d[NP];
-  // hp: flux u_n hp + c^2 h u_n; the non-conservative product -c^2 u_n h_n and the source
-  // -2 c^2 u_n H_n together are -c^2 u_n (h - 2 H)_n
+  // hp: flux h u_n (p + c^2); the non-conservative product -c^2 u_n h_n and the source
+  // -2 c^2 u_n H_n together are -c^2 u_n (h - 2 H)_n, h and H each as differences to the centre
+  // (h - 2 H itself would round at the size of H)
   {
     double dh[NP];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) F[k] = fma(-2.0, hl[k * SN], h[k]);
+    for (int k = 0; k < NP; ++k) F[k] = k == 2 ? 0.0 : fma(-2.0, hl[k * SN] - hl[2 * SN], h[k] - h[2]);
     line_derivative(T, F, 0.5 * (hL - h[0]), 0.5 * (hR - h[4]), dh);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) F[k] = fma(un[k], hp[k], c2 * hn[k]);
-    const double jl = fma(0.5, fma(unL, hpL, fma(c2, dnL, -un[0] * hp[0])), lamL * (hpL - hp[0]));
-    const double jr = fma(0.5, fma(unR, hpR, fma(c2, dnR, -un[4] * hp[4])), lamR * (hp[4] - hpR));
+    for (int k = 0; k < NP; ++k) F[k] = hn[k] * fma(hp[k], ih[k], c2);
+    const double jl = fma(0.5, fma(hnL, fma(hpL, ihL, c2), -F[0]), lamL * (hpL - hp[0]));
+    const double jr = fma(0.5, fma(hnR, fma(hpR, ihR, c2), -F[4]), lamR * (hp[4] - hpR));
     line_derivative(T, F, jl, jr, d);
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
@@ -288,7 +301,7 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
       F[k] = fma(hn[k], un[k], hydro(C, h[k], Hn[k]) + hp[k]);
     const double fl = fma(unL, hnL, fma(0.5 * g * (hL - h[0]), hL + h[0], (hpL - hp[0]) - un[0] * hn[0]));
     const double fr = fma(unR, hnR, fma(0.5 * g * (hR - h[4]), hR + h[4], (hpR - hp[4]) - un[4] * hn[4]));
-    line_derivative(T, F, fma(0.5, fl, lamL * dnL), fma(0.5, fr, -lamR * dnR), d);
+    line_derivative(T, F, fma(0.5, fl, lamL * dnL()), fma(0.5, fr, -lamR * dnR()), d);
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
       const double bath = fma(g, h[k] - Hn[k], C.gamma * (hp[k] * ih[k]));
@@ -322,7 +335,7 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
     }
   }
   // mass: h u_n
-  line_derivative(T, hn, fma(0.5, dnL, lamL * (hL - h[0])), fma(0.5, dnR, lamR * (h[4] - hR)), d);
+  line_derivative(T, hn, fma(0.5, dnL(), lamL * (hL - h[0])), fma(0.5, dnR(), lamR * (h[4] - hR)), d);
 #pragma unroll
   for (int k = 0; k < NP; ++k) emit(0, k, iJ * d[k]);
 }
@@ -586,7 +599,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
           [&](int b, double dh, const Prim<true>& q) { gp[NV * TN + b * NP] = C.mc2 * q.v * dh; },
           [&](int b, int v, double d, const Prim<true>&) { gp[v * TN + b * NP] = d; });
     } else {
-      line_terms<1, US, false>(C, T, uc, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
+      line_terms<1, US, false, MODE == MODE_FSAL>(C, T, uc, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
                                [&](int v, int k, double r) { gp[v * TN + k * NP] = r; });
     }
   }
@@ -625,7 +638,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
                                                     gp[NV * TN + a], q);
             });
       } else {
-        line_terms<0, US, FRIC>(C, T, u, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
+        line_terms<0, US, FRIC, MODE == MODE_FSAL>(C, T, u, &S.H[o], lo, hi, mlo ? -1.0 : 1.0, mhi ? -1.0 : 1.0,
                                 [&](int v, int k, double r) { gp[v * TN + k] = -r - gp[v * TN + k]; });
       }
     }
