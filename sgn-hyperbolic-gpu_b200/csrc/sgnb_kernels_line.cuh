@@ -771,10 +771,12 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
         }
       }
     };
-    // the scale is at least atol: where that is a normal number, so is the scale, and the
-    // reciprocal of a few ulp serves
-    if (!EXACT && rc.atol >= 2.2250738585072014e-308) errors([](double e, double sc) { return e * fast_rcp(sc); });
-    else errors([](double e, double sc) { return e / sc; });
+    // the fast mode's reciprocal where the scale is a normal number: everywhere if atol is one, else
+    // value by value (a purely relative tolerance; a division by every scale instead took 20 steps
+    // of 512 x 256 elements from 7.59 to 7.91 ms, this takes 7.83)
+    constexpr double kNormal = 2.2250738585072014e-308;
+    if (EXACT || rc.atol >= kNormal) errors([](double e, double sc) { return e * fast_rcp(sc); });  // (exact: divides)
+    else errors([](double e, double sc) { return sc >= kNormal ? e * fast_rcp(sc) : e / sc; });
     reduce_error<LWARPS>(esum, emax, esum != esum, S.red, A.partials, blk);
   }
   if (bulk_out && lane < NV) bulk_store_wait();  // shared memory is read out
