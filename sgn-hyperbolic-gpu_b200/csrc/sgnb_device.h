@@ -118,7 +118,9 @@ struct CtrlState {
 // kernel before it in its stream still runs, once all of that one's CTAs have called
 // let_next_start or left; it touches no global memory before wait_for_previous, which returns
 // when the kernel before it has completed with its writes visible (every kernel launched this
-// way calls it, in all threads). Launch latency and the kernel's own set-up then overlap the
+// way calls it first, in all threads). What that kernel wrote is not read-only over this kernel's
+// life, so it is read with ordinary loads, never through the non-coherent path (no ld.global.nc,
+// and no const __restrict__ pointers, which let the compiler choose it). Launch latency and the kernel's own set-up then overlap the
 // previous kernel's end: a right-hand side of 128 x 64 elements every 8.16 us instead of 10.24
 // (8.91 with let_next_start first thing, when the waiting CTAs take room that the running ones'
 // L1 would use). Not while a graph is captured: its nodes start faster than these edges
@@ -145,21 +147,20 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block,
 }
 
 // The controller's per-launch values (buffer index, dt, tolerances) read again late in a
-// stage kernel, through the read-only path: the controller state does not change while a
-// stage kernel runs (the controller kernel writes it between launches), so after the
-// first read on an SM the line comes from L1 instead of an L2 round trip. Asm statements,
-// so the compiler neither merges them with the kernel's first read nor keeps that value
-// live in registers in between.
+// stage kernel. The controller, which writes them, is another kernel: the state does not change
+// after wait_for_previous, and after the first read on an SM the line comes from L1. Asm
+// statements, so the compiler neither merges them with the kernel's first read nor keeps that
+// value live in registers in between.
 struct CtrlReload {
   int cur;
   double dt, atol, rtol;
 };
 __device__ __forceinline__ CtrlReload ctrl_reload(const CtrlState* c) {
   CtrlReload r;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(r.cur) : "l"(&c->cur));
-  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(r.dt) : "l"(&c->dt));
-  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(r.atol) : "l"(&c->atol));
-  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(r.rtol) : "l"(&c->rtol));
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(r.cur) : "l"(&c->cur));
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(r.dt) : "l"(&c->dt));
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(r.atol) : "l"(&c->atol));
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(r.rtol) : "l"(&c->rtol));
   return r;
 }
 

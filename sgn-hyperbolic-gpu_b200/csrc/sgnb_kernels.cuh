@@ -115,9 +115,9 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // Read-only views of the stage inputs of one launch.
 struct StageIn {
-  const double* __restrict__ in;  // MODE_RHS, MODE_FSAL
-  const double* __restrict__ u;
-  const double* __restrict__ k;   // MODE_STAGE, MODE_CAND: the derivative added to u
+  const double* in;  // MODE_RHS, MODE_FSAL
+  const double* u;
+  const double* k;   // MODE_STAGE, MODE_CAND: the derivative added to u
   double acoef, dt;
 };
 
@@ -548,7 +548,7 @@ __device__ __forceinline__ void fused_tile(const RhsConsts& C, const RhsConsts& 
       if (okk[u]) {
         if (SGNB_INB(gof[u], Nd) && SGNB_INB(sof[u], TE * NPP)) cp_async8(&(&S.H[0][0])[sof[u]], C.Hnod + gof[u]);
       }
-    const double* __restrict__ src = AXPY ? I.u : I.in;
+    const double* src = AXPY ? I.u : I.in;
 #pragma unroll
     for (int v = 0; v < NV; ++v)
 #pragma unroll
@@ -779,10 +779,10 @@ __device__ __forceinline__ void fused_tile(const RhsConsts& C, const RhsConsts& 
       // the passes; one field at a time, with all of its loads in flight
       const CtrlReload rc = ctrl_reload(A.ctrl);
       const double dt = rc.dt;
-      const double* __restrict__ u0 = A.U[rc.cur];
-      const double* __restrict__ k1 = A.K1[rc.cur];
-      const double* __restrict__ k2 = A.K2;
-      const double* __restrict__ part = A.K3;
+      const double* u0 = A.U[rc.cur];
+      const double* k1 = A.K1[rc.cur];
+      const double* k2 = A.K2;
+      const double* part = A.K3;
       double* __restrict__ un_out = A.U[rc.cur ^ 1];
       double* __restrict__ part_out = A.K3;
       double* __restrict__ k4_out = A.K1[rc.cur ^ 1];

@@ -360,8 +360,8 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     dt = A.ctrl->dt;
     acoef = A.coef * dt;
   }
-  const double* __restrict__ src = MODE == MODE_RHS ? A.in : (MODE == MODE_FSAL ? pick(A.U, cur ^ 1) : pick(A.U, cur));
-  const double* __restrict__ kin = AXPY ? (A.kin_k2 ? A.K2 : pick(A.K1, cur)) : nullptr;
+  const double* src = MODE == MODE_RHS ? A.in : (MODE == MODE_FSAL ? pick(A.U, cur ^ 1) : pick(A.U, cur));
+  const double* kin = AXPY ? (A.kin_k2 ? A.K2 : pick(A.K1, cur)) : nullptr;
 
   int tid;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
@@ -435,7 +435,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   constexpr int NE = MODE == MODE_FSAL ? NV : 1;
   double2 eu[NE][LPF];
   if constexpr (MODE == MODE_FSAL) {
-    const double* __restrict__ u0 = pick(A.U, cur) + row0 + kp;
+    const double* u0 = pick(A.U, cur) + row0 + kp;
 #pragma unroll
     for (int v = 0; v < NV; ++v)
 #pragma unroll
@@ -666,7 +666,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   if constexpr (MODE == MODE_CAND) {
     // k3 is used up here: the candidate uNew = u + dt (2/9 k1 + 1/3 k2 + 4/9 k3) and the part
     // 7/24 k1 + 1/4 k2 + 1/3 k3 of the embedded solution leave instead (rk.cpp:106-121)
-    const double* __restrict__ k1 = pick(A.K1, cur) + row0 + kp;
+    const double* k1 = pick(A.K1, cur) + row0 + kp;
     double* __restrict__ un = pick(A.U, cur ^ 1) + row0 + kp;
     double* __restrict__ pe = A.K3 + row0 + kp;
     // a rolled loop over the fields (unrolled, warps waited for instructions), the next field's
@@ -710,9 +710,9 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     const bool outLo = C.edgeL != nullptr && ex0 == 0 && wx == 0;
     const bool outHi = C.edgeR != nullptr && ex0 + wx * LROW + RXv == Nx;
     if (RXv > 0 && (outLo || outHi)) {
-      const double* __restrict__ u0 = pick(A.U, cur);
-      const double* __restrict__ k1 = pick(A.K1, cur);
-      const double* __restrict__ k2 = A.K2;
+      const double* u0 = pick(A.U, cur);
+      const double* k1 = pick(A.K1, cur);
+      const double* k2 = A.K2;
       for (int q = lane; q < 2 * NV * NP; q += 32) {
         const int side = q / (NV * NP), r = q - side * NV * NP, t = r % NP, v = r / NP;
         if (side == 0 ? !outLo : !outHi) continue;
@@ -731,7 +731,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     // scaled embedded error (rk.cpp:118-128) of the row, then of the tile
     const CtrlReload rc = ctrl_reload(A.ctrl);
     double esum = 0.0, emax = 0.0;
-    const double* __restrict__ pe = A.K3 + row0 + kp;
+    const double* pe = A.K3 + row0 + kp;
     double2 p[LPF], np[LPF];
     auto load = [&](int v, double2 (&x)[LPF]) {
 #pragma unroll

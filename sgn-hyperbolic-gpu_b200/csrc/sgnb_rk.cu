@@ -91,7 +91,6 @@ __device__ __forceinline__ bool controller_core(CtrlState* cg, const Row& row, l
   __shared__ double prevPow;
   constexpr int W = sizeof(CtrlState) / 8;
   static_assert(sizeof(CtrlState) % 8 == 0 && W <= kCtrlThreads, "copied by one word per thread");
-  wait_for_previous();
   if (cg->done) return false;
   const int t = threadIdx.x;
   CtrlState* const c = &state;
@@ -155,6 +154,7 @@ __device__ __forceinline__ bool controller_block(CtrlState* c, const double* par
 
 __global__ void __launch_bounds__(kCtrlThreads) k_controller(CtrlState* c, const double* partials,
                                                              int nblk, long long n) {
+  wait_for_previous();
   controller_block(c, partials, nblk, n);
 }
 
@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kCtrlThreads) k_controller(CtrlState* c, const
 __global__ void __launch_bounds__(kCtrlThreads) k_controller_loop(CtrlState* c, const double* partials,
                                                                   int nblk, long long n,
                                                                   cudaGraphConditionalHandle loop) {
+  wait_for_previous();
   const bool running = controller_block(c, partials, nblk, n);
   if (threadIdx.x == 0) cudaGraphSetConditional(loop, running ? 1u : 0u);
 }
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(kCtrlThreads) k_controller_loop(CtrlState* c, 
 __global__ void __launch_bounds__(kCtrlThreads) k_controller_batch_loop(
     CtrlState* ctrls, const double* const* partials, const int* nblk, const long long* n,
     int* counters, cudaGraphConditionalHandle loop) {
+  wait_for_previous();
   const int i = blockIdx.x;
   const bool goes_on = controller_block(ctrls + i, partials[i], nblk[i], n[i]);
   if (threadIdx.x != 0) return;
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(kCtrlThreads) k_controller_batch_loop(
 // other devices: peer loads) in slab order, as one list.
 __global__ void __launch_bounds__(kCtrlThreads) k_controller_slabs(CtrlState* c, const SlabPartials L,
                                                                    long long n) {
+  wait_for_previous();
   controller_core(
       c,
       [&](long long b) {
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(kCtrlThreads) k_controller_slabs(CtrlState* c,
 __global__ void __launch_bounds__(kCtrlThreads) k_controller_batch(CtrlState* ctrls,
                                                                    const double* const* partials,
                                                                    const int* nblk, const long long* n) {
+  wait_for_previous();
   const int i = blockIdx.x;
   controller_block(ctrls + i, partials[i], nblk[i], n[i]);
 }
