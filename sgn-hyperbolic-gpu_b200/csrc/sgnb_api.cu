@@ -918,6 +918,9 @@ struct sgnb_batch {
   LineConsts* dconsts = nullptr;       // [n]
   RhsConsts* dconstsM = nullptr;       // [n], mixed batches
   bool mixed = false;                  // every instance SGNB_MIXED (else SGNB_FP64_FAST)
+  // one instance after the other, each through its own loop: the batched kernels take one set of
+  // FR tables for all instances, in the fast mode with the reflection symmetry
+  bool one_by_one = false;
   StageArgs* dargs = nullptr;          // [n]
   StageArgs* hargs = nullptr;          // pinned host mirror
   StageArgsM* dargsM = nullptr;        // [n], mixed batches
@@ -1089,17 +1092,17 @@ int batch_prepare(sgnb_batch* b) {
 // graph launch up to 4096 attempts (a bound on one launch; the host then relaunches).
 int batch_run(sgnb_batch* b) {
   constexpr long long kAttemptsPerLaunch = 4096;
-  bool sym = true;
-  for (const sgnb_ctx* c : b->ctx) sym = sym && c->C.sym;
-  if (!b->mixed && !sym) {
-    // caller-given FR tables without the reflection symmetry that the batched kernels need:
-    // one instance after the other, each through its own loop
+  if (b->one_by_one) {
+    b->launches = 0;
     for (int i = 0; i < b->n; ++i) {
       sgnb_ctx* c = b->ctx[i];
+      const CtrlState own = *c->hctrl;  // the instance's own runs' (its attempt log)
       *c->hctrl = b->hctrl[i];
-      if (int rc = run_loop(c)) return bfail(b, rc, c->err);
+      const int rc = run_loop(c);
       b->hctrl[i] = *c->hctrl;
-      b->launches = c->launches;
+      *c->hctrl = own;
+      if (rc) return bfail(b, rc, c->err);
+      b->launches += c->launches;
     }
     return SGNB_OK;
   }
@@ -1476,6 +1479,9 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
   for (int i = 0; i < n; ++i) {
     int rc = sgnb_create(&descs[i], &b->ctx[i]);
     if (rc) { sgnb_batch_destroy(b); return rc; }
+    const RhsConsts &C0 = b->ctx[0]->C, &C = b->ctx[i]->C;
+    b->one_by_one = b->one_by_one || (!b->mixed && !C.sym) || std::memcmp(C.D, C0.D, sizeof(C.D)) != 0 ||
+                    std::memcmp(C.gLp, C0.gLp, sizeof(C.gLp)) != 0 || std::memcmp(C.gRp, C0.gRp, sizeof(C.gRp)) != 0;
   }
   cudaSetDevice(b->device);
   auto bail = [&](cudaError_t e, const char* what) {
