@@ -1479,6 +1479,10 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
   for (int i = 0; i < n; ++i) {
     int rc = sgnb_create(&descs[i], &b->ctx[i]);
     if (rc) { sgnb_batch_destroy(b); return rc; }
+    if (b->ctx[i]->tab.gauss) {
+      sgnb_batch_destroy(b);
+      return bfail(nullptr, SGNB_ERR_UNSUPPORTED, "batched instances use GLL points");
+    }
     const RhsConsts &C0 = b->ctx[0]->C, &C = b->ctx[i]->C;
     b->one_by_one = b->one_by_one || (!b->mixed && !C.sym) || std::memcmp(C.D, C0.D, sizeof(C.D)) != 0 ||
                     std::memcmp(C.gLp, C0.gLp, sizeof(C.gLp)) != 0 || std::memcmp(C.gRp, C0.gRp, sizeof(C.gRp)) != 0;

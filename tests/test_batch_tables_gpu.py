@@ -1,5 +1,5 @@
 """A batch whose instances bring their own FR tables: every instance runs its own scheme, as it does
-alone."""
+alone, and instances whose face rows are not those of GLL points are refused."""
 from __future__ import annotations
 
 import numpy as np
@@ -41,3 +41,11 @@ def test_each_instance_has_its_own_tables(precision, first):
             assert (stats[i].accepted, stats[i].rejected, stats[i].dtLast) == (st.accepted, st.rejected, st.dtLast)
             launches += st.kernel_launches
         assert all(s.kernel_launches == launches for s in stats)
+
+
+def test_interpolating_face_rows_are_refused():
+    t = sgnb.fr_tables()
+    t["lL"] = np.array([1.0, 1e-3, 0.0, 0.0, 0.0])
+    kw = dict(Nx=6, Ny=4, Lx=7.5, Ly=5.0, c=9.0, bathy_kind=sgnb.BATHY_NONE)
+    with pytest.raises(sgnb.SgnbError, match="GLL"):
+        sgnb.SGNBatch([dict(kw), dict(kw, tables=t)])
