@@ -180,9 +180,10 @@ int sgnb_adj_create(sgnb_ctx* c, long long nsteps, const double* dts, int ngauge
   a->gnodes.assign(gauge_nodes, gauge_nodes + ngauges);
   const long long S = c->ntot, Nd = c->Nd, ne = (long long)c->desc.Nx * c->desc.Ny;
   const long long segStates = (a->K < nsteps) ? a->K : nsteps;
+  constexpr size_t kAlign = 32;  // the states start at a multiple of 256 bytes: row copies need 16
   size_t total = nsteps + (size_t)ngauges + 2 * (size_t)nsteps * (ngauges > 0 ? ngauges : 1) +
                  ((size_t)a->nseg + segStates + 9) * S + vjp_scratch_doubles(Nd, ne) +
-                 stat_doubles(c) + sizeof(CtrlState) / sizeof(double) + 8;
+                 stat_doubles(c) + sizeof(CtrlState) / sizeof(double) + 8 + kAlign;
   cudaError_t e = cudaMalloc(&a->block, total * sizeof(double));
   if (e != cudaSuccess) { delete a; return afail(c, SGNB_ERR_NOMEM, "sgnb_adj_create: cudaMalloc"); }
   double* p = a->block;
@@ -191,6 +192,7 @@ int sgnb_adj_create(sgnb_ctx* c, long long nsteps, const double* dts, int ngauge
   a->gnodes_dev = reinterpret_cast<long long*>(p); p += ngauges;
   a->eta_dev = p; p += (size_t)nsteps * (ngauges > 0 ? ngauges : 1);
   a->etab_dev = p; p += (size_t)nsteps * (ngauges > 0 ? ngauges : 1);
+  p = a->block + ((size_t)(p - a->block) + kAlign - 1) / kAlign * kAlign;
   a->ckpt = p; p += (size_t)a->nseg * S;
   a->seg = p; p += (size_t)segStates * S;
   for (double** q : {&a->u[0], &a->u[1], &a->k1, &a->k2, &a->k3, &a->lam, &a->acc, &a->y3b, &a->y2b}) {
