@@ -301,6 +301,17 @@ void fill_consts(sgnb_ctx* c) {
   C.bulk = d.Nx % 2 == 0 && !(sw && sw[0] == '0');
 }
 
+cudaError_t prepare_fp64(const sgnb_ctx* c, bool ghost) {
+  return c->precision == SGNB_FP64_FAST ? dev::prepare_fused_fast(c->C, ghost) : dev::prepare_fused_exact(c->C, ghost);
+}
+// The kernels with slab edges: at creation for a slab, else when a context is first given ghosts.
+cudaError_t prepare_ghosts(sgnb_ctx* c) {
+  if (c->ghost_ready) return cudaSuccess;
+  const cudaError_t e = prepare_fp64(c, true);
+  c->ghost_ready = e == cudaSuccess;
+  return e;
+}
+
 // The device-side loop: a CUDA graph whose one node is a WHILE conditional node; its body
 // is one attempt (stages 2, 3, the end-point stage, the controller), and the controller
 // sets the condition. One graph launch runs attempts until the run is done or attemptCap
@@ -555,11 +566,6 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
     if (e != cudaSuccess) { cuda_fail(c, e, "cudaMalloc(traces)"); g_create_error = c->err; return bail(SGNB_ERR_NOMEM); }
   }
   fill_consts(c);
-  // only the kernels that this context launches: raising a kernel's shared memory loads its code
-  e = c->mixed ? dev::prepare_fused_mixed()
-               : (c->precision == SGNB_FP64_FAST ? dev::prepare_fused_fast(c->C) : dev::prepare_fused_exact(c->C));
-  if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
-
   const size_t sbytes = (size_t)c->ntot * sizeof(double);
   // stage derivatives are FP32 in the mixed mode; K2 and K3 are allocated as one block so
   // that together they always hold an FP64 state (scratch for sgnb_rhs_host)
@@ -576,6 +582,10 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   if (e != cudaSuccess) { cuda_fail(c, e, "cudaMalloc(stage)"); g_create_error = c->err; return bail(SGNB_ERR_NOMEM); }
   c->K3 = (char*)c->K2 + kbytes;
   build_tile_maps(c);
+  // only the kernels that this context launches: raising a kernel's shared memory loads its code
+  e = c->mixed ? dev::prepare_fused_mixed(c->C, c->mapsM.ok) : prepare_fp64(c, false);
+  if (e == cudaSuccess && d->Nx_global > 0 && !c->mixed) e = prepare_ghosts(c);
+  if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
   e = cudaMemset(c->U[0], 0, sbytes);
   // error partials: one row per tile of the kernels that this context runs
   c->nblk = !c->mixed && !c->tab.gauss
@@ -963,6 +973,11 @@ int bfail(sgnb_batch* b, int code, const std::string& msg) {
 // One batched stage launch of either arithmetic mode.
 cudaError_t batch_launch(sgnb_batch* b, int mode, int shape, int blocks, int kin_k2, double coef);
 
+// The kernels of one launch configuration: raises their shared memory, which loads their code.
+cudaError_t batch_kernels(const sgnb_batch* b, int shape, int blocks) {
+  return b->mixed ? dev::prepare_mixed_batch(blocks) : dev::prepare_fused_batch(shape, blocks);
+}
+
 BatchArgs batch_args(sgnb_batch* b, int shape, int kin_k2, double coef) {
   BatchArgs B{};
   B.tables = b->ctx[0]->C.eo;
@@ -1167,6 +1182,8 @@ int sgnb_set_ghosts(sgnb_ctx* c, const double* ghostL, const double* ghostR) {
   if (!c) return fail(c, SGNB_ERR_INVALID, "NULL context");
   if (c->tab.gauss) return fail(c, SGNB_ERR_UNSUPPORTED, "Gauss points run on whole meshes");
   if (c->mixed) return fail(c, SGNB_ERR_UNSUPPORTED, "slab edges run in the FP64 modes");
+  if (int rc = set_device(c)) return rc;
+  if (ghostL || ghostR) SGNB_CU(c, prepare_ghosts(c));
   c->C.ghostL = ghostL;
   c->C.ghostR = ghostR;
   if (c->chunk) {  // captured launches hold the old constants
@@ -1255,6 +1272,7 @@ int sgnb_slab_stage(sgnb_ctx* c, int stage, const double* ghostL, const double* 
   if ((edgeL && !ghostL) || (edgeR && !ghostR))
     return fail(c, SGNB_ERR_INVALID, "an edge output needs the neighbour's ghost input");
   if (int rc = set_device(c)) return rc;
+  if (ghostL || ghostR) SGNB_CU(c, prepare_ghosts(c));
   cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
   if (c->chunk) {  // captured launches hold other constants
     cudaGraphExecDestroy(c->chunk);
@@ -1493,7 +1511,7 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
     sgnb_batch_destroy(b);
     return bfail(nullptr, e == cudaErrorMemoryAllocation ? SGNB_ERR_NOMEM : SGNB_ERR_CUDA, m);
   };
-  cudaError_t e = b->mixed ? dev::prepare_mixed_batch() : dev::prepare_fused_batch();
+  cudaError_t e = batch_kernels(b, 0, 0);
   if (e != cudaSuccess) return bail(e, "kernel attributes");
   e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evRead, cudaEventDisableTiming);
@@ -1600,6 +1618,8 @@ sgnb_ctx* sgnb_batch_instance(sgnb_batch* b, int i) {
 int sgnb_batch_set_config(sgnb_batch* b, int shape, int blocks) {
   if (!b || shape < 0 || shape > 2 || blocks < 0) return bfail(b, SGNB_ERR_INVALID, "shape 0..2, blocks >= 0");
   if (b->mixed && shape != 0) return bfail(b, SGNB_ERR_UNSUPPORTED, "mixed batches use tile shape 0");
+  SGNB_BCU(b, cudaSetDevice(b->device));
+  SGNB_BCU(b, batch_kernels(b, shape, blocks));
   b->shape = shape;
   b->blocks = blocks;
   return SGNB_OK;
@@ -1694,7 +1714,8 @@ int sgnb_batch_autotune(sgnb_batch* b, const double* dt0, int reps, double* ms_o
         }
         return e;
       };
-      cudaError_t e = run(1);
+      cudaError_t e = batch_kernels(b, sh, blocks);
+      if (e == cudaSuccess) e = run(1);
       if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
       if (e == cudaSuccess) e = run(reps);
       if (e == cudaSuccess) e = cudaEventRecord(e1, b->stream);

@@ -42,6 +42,7 @@ struct sgnb_ctx {
   static constexpr long long kLogCap = 1 << 16;
   cudaGraphExec_t chunk = nullptr;
   int chunkLen = 0;
+  bool ghost_ready = false;  // the kernels with slab edges are loaded
   cudaEvent_t evRead = nullptr;
   long long launches = 0;  // kernels launched by the last integration
   long long pendingMaxAccepted = 0;  // set by sgnb_integrate_steps

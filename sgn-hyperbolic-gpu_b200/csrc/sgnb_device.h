@@ -360,7 +360,7 @@ struct CellGrid {
 namespace dev {
 // Batched mixed-precision launch: `blocks` persistent CTAs, or one CTA per tile (0).
 cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaStream_t s);
-cudaError_t prepare_mixed_batch();
+cudaError_t prepare_mixed_batch(int blocks);
 
 // Out-of-range access counts of the checked build, per translation unit.
 cudaError_t read_oob_exact(unsigned long long* out, bool reset);
@@ -415,18 +415,21 @@ cudaError_t launch_gauges_back(double* lam, const long long* nodes, int ng, cons
 cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
 cudaError_t launch_line(int mode, const RhsConsts& C, const StageArgs& A, cudaStream_t s);
-cudaError_t prepare_line();
-cudaError_t prepare_fused_exact(const RhsConsts& C);
-cudaError_t prepare_fused_fast(const RhsConsts& C);
+// Raise the shared memory of a context's kernels (its friction and point set; ghost: those with
+// slab edges), which loads their code.
+cudaError_t prepare_line(const RhsConsts& C, bool ghost);
+cudaError_t prepare_fused_exact(const RhsConsts& C, bool ghost);
+cudaError_t prepare_fused_fast(const RhsConsts& C, bool ghost);
 cudaError_t launch_fused_mixed(int mode, const RhsConsts& C, const StageArgsM& A,
                                cudaStream_t s, const TileMapsM* M = nullptr);
-cudaError_t prepare_fused_mixed();
+// tma: the stages that add k take their tiles by tensor maps (whole tiles, no friction)
+cudaError_t prepare_fused_mixed(const RhsConsts& C, bool tma);
 int fused_grid_blocks(int Nx, int Ny);
 // Batched launch (fast mode): tile shape shape_id (0: 6x4 elements, 1: 12x2, 2: 24x1);
 // `blocks` persistent CTAs looping over the work list, or one CTA per tile when blocks == 0.
 cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchArgs& B,
                                cudaStream_t s);
-cudaError_t prepare_fused_batch();
+cudaError_t prepare_fused_batch(int shape_id, int blocks);
 int batch_tile_tx(int shape_id);
 int batch_tile_ty(int shape_id);
 int line_grid_blocks(int Nx, int Ny);

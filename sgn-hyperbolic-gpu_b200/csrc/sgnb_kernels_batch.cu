@@ -97,30 +97,24 @@ cudaError_t launch_fused_batch(int mode, int shape_id, int blocks, const BatchAr
 int batch_tile_tx(int shape_id) { return LROW * (shape_id == 1 ? 2 : (shape_id == 2 ? 4 : 1)); }
 int batch_tile_ty(int shape_id) { return shape_id == 1 ? 2 : (shape_id == 2 ? 1 : 4); }
 
-template <int MODE, int WX>
-static cudaError_t prepare_mode() {
+template <int WX, bool PERSIST>
+static cudaError_t prepare_form() {
   const int bytes = (int)sizeof(typename LineTile<WX>::Smem);
-  cudaError_t e = cudaFuncSetAttribute(k_line_batch<MODE, WX, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_line_batch<MODE, WX, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
-template <int WX>
-static cudaError_t prepare_shape() {
-  cudaError_t e = prepare_mode<MODE_RHS, WX>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE, WX>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL, WX>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_CAND, WX>();
+  const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_line_batch<MODE_RHS, WX, PERSIST>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_batch<MODE_STAGE, WX, PERSIST>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_batch<MODE_FSAL, WX, PERSIST>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_batch<MODE_CAND, WX, PERSIST>, at, bytes);
   return e;
 }
 
-cudaError_t prepare_fused_batch() {
-  cudaError_t e = prepare_shape<1>();
-  if (e == cudaSuccess) e = prepare_shape<2>();
-  if (e == cudaSuccess) e = prepare_shape<4>();
-  return e;
+cudaError_t prepare_fused_batch(int shape_id, int blocks) {
+  switch (shape_id) {
+    case 0: return blocks > 0 ? prepare_form<1, true>() : prepare_form<1, false>();
+    case 1: return blocks > 0 ? prepare_form<2, true>() : prepare_form<2, false>();
+    case 2: return blocks > 0 ? prepare_form<4, true>() : prepare_form<4, false>();
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 // The checked build's out-of-range count of this translation unit's kernels (reset: then

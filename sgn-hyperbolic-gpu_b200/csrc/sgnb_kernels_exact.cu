@@ -33,26 +33,20 @@ cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A,
   }
 }
 
-template <int MODE>
-static cudaError_t prepare_mode() {
+template <bool FRIC, bool GHOST>
+static cudaError_t prepare_lines() {
   const size_t bytes = sizeof(LineTile<1, true>::Smem);
-  cudaError_t e = raise_smem(k_line_exact<MODE, false, false>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE, true, false>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE, false, true>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE, true, true>, bytes);
+  cudaError_t e = raise_smem(k_line_exact<MODE_RHS, FRIC, GHOST>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_STAGE, FRIC, GHOST>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_CAND, FRIC, GHOST>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_FSAL, FRIC, GHOST>, bytes);
   return e;
 }
 
-cudaError_t prepare_fused_exact(const RhsConsts& C) {
-  if (C.gauss) {
-    const cudaError_t g = prepare_variant<false>();
-    return g == cudaSuccess ? prepare_variant<true>() : g;
-  }
-  cudaError_t e = prepare_mode<MODE_RHS>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_CAND>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL>();
-  return e;
+cudaError_t prepare_fused_exact(const RhsConsts& C, bool ghost) {
+  if (C.gauss) return C.manning ? prepare_variant<true>() : prepare_variant<false>();
+  if (C.manning) return ghost ? prepare_lines<true, true>() : prepare_lines<true, false>();
+  return ghost ? prepare_lines<false, true>() : prepare_lines<false, false>();
 }
 int fused_grid_blocks(int Nx, int Ny) { return ((Nx + 7) / 8) * ((Ny + 3) / 4); }
 size_t fused_smem_bytes() { return sizeof(Tile<8, 4, true>::Smem); }

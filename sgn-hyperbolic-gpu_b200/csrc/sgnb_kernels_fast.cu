@@ -20,10 +20,9 @@ cudaError_t launch_fused_fast(int mode, const RhsConsts& C, const StageArgs& A, 
     default: return cudaErrorInvalidValue;
   }
 }
-cudaError_t prepare_fused_fast(const RhsConsts& C) {
-  if (!C.gauss) return C.sym ? prepare_line() : prepare_fused_exact(C);
-  const cudaError_t e = prepare_variant<false>();
-  return e == cudaSuccess ? prepare_variant<true>() : e;
+cudaError_t prepare_fused_fast(const RhsConsts& C, bool ghost) {
+  if (!C.gauss) return C.sym ? prepare_line(C, ghost) : prepare_fused_exact(C, ghost);
+  return C.manning ? prepare_variant<true>() : prepare_variant<false>();
 }
 
 // The checked build's out-of-range count of this translation unit's kernels (reset: then

@@ -36,23 +36,20 @@ int line_grid_blocks(int Nx, int Ny) {
   return ((Nx + L::TX - 1) / L::TX) * ((Ny + L::TY - 1) / L::TY);
 }
 
-template <int MODE>
-static cudaError_t prepare_mode() {
+template <bool FRIC, bool GHOST>
+static cudaError_t prepare_variant() {
   const int bytes = (int)sizeof(typename LineTile<1>::Smem);
   const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(k_line<MODE, false, false>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, false>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, false, true>, at, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE, true, true>, at, bytes);
+  cudaError_t e = cudaFuncSetAttribute(k_line<MODE_RHS, FRIC, GHOST>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE_STAGE, FRIC, GHOST>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE_FSAL, FRIC, GHOST>, at, bytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line<MODE_CAND, FRIC, GHOST>, at, bytes);
   return e;
 }
 
-cudaError_t prepare_line() {
-  cudaError_t e = prepare_mode<MODE_RHS>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_STAGE>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_FSAL>();
-  if (e == cudaSuccess) e = prepare_mode<MODE_CAND>();
-  return e;
+cudaError_t prepare_line(const RhsConsts& C, bool ghost) {
+  if (C.manning) return ghost ? prepare_variant<true, true>() : prepare_variant<true, false>();
+  return ghost ? prepare_variant<false, true>() : prepare_variant<false, false>();
 }
 
 // The checked build's out-of-range count of this translation unit's kernels (reset: then

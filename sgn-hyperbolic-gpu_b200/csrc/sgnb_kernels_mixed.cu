@@ -55,33 +55,30 @@ cudaError_t launch_fused_mixed(int mode, const RhsConsts& C, const StageArgsM& A
   }
 }
 
-template <bool FRIC, bool FULL = false>
-static cudaError_t prepare_mixed_fric() {
-  const int bytes = (int)sizeof(mix::Smem);
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(mix::k_mixed<mix::MODE_RHS, FRIC, FULL>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(mix::k_mixed<mix::MODE_STAGE, FRIC, FULL>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(mix::k_mixed<mix::MODE_CAND, FRIC, FULL>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
-    return e;
-  return cudaFuncSetAttribute(mix::k_mixed<mix::MODE_FSAL, FRIC, FULL>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+template <class K>
+static cudaError_t raise_smem(K* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(mix::Smem));
 }
 
-cudaError_t prepare_fused_mixed() {
-  cudaError_t e = prepare_mixed_fric<false>();
-  if (e == cudaSuccess) e = prepare_mixed_fric<false, true>();
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(mix::k_mixed_tma<mix::MODE_STAGE>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(mix::Smem));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(mix::k_mixed_tma<mix::MODE_CAND>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(mix::Smem));
-  return e == cudaSuccess ? prepare_mixed_fric<true>() : e;
+template <bool FRIC, bool FULL>
+static cudaError_t prepare_variant(bool tma) {
+  cudaError_t e = raise_smem(mix::k_mixed<mix::MODE_RHS, FRIC, FULL>);
+  if (e == cudaSuccess) e = raise_smem(mix::k_mixed<mix::MODE_FSAL, FRIC, FULL>);
+  if (tma) {
+    if (e == cudaSuccess) e = raise_smem(mix::k_mixed_tma<mix::MODE_STAGE>);
+    if (e == cudaSuccess) e = raise_smem(mix::k_mixed_tma<mix::MODE_CAND>);
+  } else {
+    if (e == cudaSuccess) e = raise_smem(mix::k_mixed<mix::MODE_STAGE, FRIC, FULL>);
+    if (e == cudaSuccess) e = raise_smem(mix::k_mixed<mix::MODE_CAND, FRIC, FULL>);
+  }
+  return e;
+}
+
+// The kernels that launch_m picks for this mesh.
+cudaError_t prepare_fused_mixed(const RhsConsts& C, bool tma) {
+  if (C.manning) return prepare_variant<true, false>(false);
+  if (C.Nx % mix::TX == 0 && C.Ny % mix::TY == 0) return prepare_variant<false, true>(tma);
+  return prepare_variant<false, false>(false);
 }
 
 template <int MODE>
@@ -105,23 +102,16 @@ cudaError_t launch_mixed_batch(int mode, int blocks, const BatchArgsM& B, cudaSt
   }
 }
 
-template <int MODE>
-static cudaError_t prepare_mb() {
-  const int bytes = (int)sizeof(mix::Smem);
-  cudaError_t e = cudaFuncSetAttribute(mix::k_mixed_batch<MODE, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(mix::k_mixed_batch<MODE, false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
-cudaError_t prepare_mixed_batch() {
-  cudaError_t e = prepare_mb<mix::MODE_RHS>();
-  if (e == cudaSuccess) e = prepare_mb<mix::MODE_STAGE>();
-  if (e == cudaSuccess) e = prepare_mb<mix::MODE_CAND>();
-  if (e == cudaSuccess) e = prepare_mb<mix::MODE_FSAL>();
+template <bool PERSIST>
+static cudaError_t prepare_batch() {
+  cudaError_t e = raise_smem(mix::k_mixed_batch<mix::MODE_RHS, PERSIST>);
+  if (e == cudaSuccess) e = raise_smem(mix::k_mixed_batch<mix::MODE_STAGE, PERSIST>);
+  if (e == cudaSuccess) e = raise_smem(mix::k_mixed_batch<mix::MODE_CAND, PERSIST>);
+  if (e == cudaSuccess) e = raise_smem(mix::k_mixed_batch<mix::MODE_FSAL, PERSIST>);
   return e;
 }
+
+cudaError_t prepare_mixed_batch(int blocks) { return blocks > 0 ? prepare_batch<true>() : prepare_batch<false>(); }
 
 }  // namespace dev
 }  // namespace sgnb
