@@ -11,8 +11,8 @@
 // states are recomputed from its checkpoint; then, step by step backwards, the stage
 // derivatives k1, k2 are recomputed and the three right-hand-side VJPs of the step run
 // (sgnb_adjoint.cu), carrying the state cotangent and accumulating the cotangents of
-// the depth statics. The statics' cotangents map back to the element means through the
-// transpose of the interpolant on the host.
+// the nodal depths and their gradients, which map back to the element means through the
+// transpose of the interpolant on the device (sgnb_cells.cu).
 #include "sgnb_ctx.h"
 
 #include <cmath>
@@ -42,7 +42,6 @@ struct sgnb_adj {
   CtrlState* ctrl = nullptr;
   VjpArgs V{};
   GatherArgs G{};
-  size_t statBytes = 0;       // accumulators (contiguous from G.Hacc)
 };
 
 namespace {
@@ -87,36 +86,12 @@ void carve_vjp(VjpArgs& V, double*& p, long long Nd, long long ne) {
   for (int d = 0; d < 2; ++d)
     for (int f = 0; f < 2; ++f) { V.Sn[d][f] = p; p += 25 * ne; }
 }
-size_t stat_doubles(const sgnb_ctx* c) {
-  const long long ne = (long long)c->desc.Nx * c->desc.Ny;
-  return 3 * (size_t)c->Nd + 10 * (size_t)ne + 5 * (size_t)(c->desc.Nx + c->desc.Ny);
-}
+size_t stat_doubles(const sgnb_ctx* c) { return 3 * (size_t)c->Nd; }
 void carve_stats(GatherArgs& G, double*& p, const sgnb_ctx* c) {
-  const long long ne = (long long)c->desc.Nx * c->desc.Ny;
   G.Hacc = p; p += c->Nd;
   G.Hxacc = p; p += c->Nd;
   G.Hyacc = p; p += c->Nd;
-  G.HfXacc = p; p += 5 * ne;
-  G.HfYacc = p; p += 5 * ne;
-  G.HfXEndacc = p; p += 5 * c->desc.Ny;
-  G.HfYEndacc = p; p += 5 * c->desc.Nx;
 }
-// device statics accumulators -> host Bathymetry of cotangents
-cudaError_t download_stats(const sgnb_ctx* c, const GatherArgs& G, Bathymetry& bar) {
-  const long long ne = (long long)c->desc.Nx * c->desc.Ny;
-  bar.Hnod.resize(c->Nd); bar.Hx.resize(c->Nd); bar.Hy.resize(c->Nd);
-  bar.HfX.resize(5 * ne); bar.HfY.resize(5 * ne);
-  bar.HfXEnd.resize(5 * (size_t)c->desc.Ny); bar.HfYEnd.resize(5 * (size_t)c->desc.Nx);
-  std::vector<double> all(stat_doubles(c));
-  cudaError_t e = cudaMemcpy(all.data(), G.Hacc, all.size() * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return e;
-  const double* p = all.data();
-  auto take = [&](std::vector<double>& v) { std::memcpy(v.data(), p, v.size() * sizeof(double)); p += v.size(); };
-  take(bar.Hnod); take(bar.Hx); take(bar.Hy); take(bar.HfX); take(bar.HfY);
-  take(bar.HfXEnd); take(bar.HfYEnd);
-  return cudaSuccess;
-}
-
 CellGrid grid_of(const sgnb_ctx* c) {
   CellGrid g{};
   g.Nx = c->desc.Nx; g.Ny = c->desc.Ny;
@@ -362,16 +337,17 @@ int sgnb_rhs_vjp(sgnb_ctx* c, const double* U, const double* Rbar, double* Ubar,
   G.ybar = nullptr; G.uacc = Ubd; G.lam = nullptr; G.init = 1;
   if (e == cudaSuccess) e = dev::launch_vjp_rhs(c->C, tables_of(c), V, G, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(Ubar, Ubd, S * sizeof(double), cudaMemcpyDeviceToHost, s);
-  Bathymetry bar;
+  auto down = [&](double* host, const double* dev) {
+    if (e == cudaSuccess && host)
+      e = cudaMemcpyAsync(host, dev, Nd * sizeof(double), cudaMemcpyDeviceToHost, s);
+  };
+  down(Hnod_bar, G.Hacc); down(Hx_bar, G.Hxacc); down(Hy_bar, G.Hyacc);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) e = download_stats(c, G, bar);
   cudaFree(block);
   if (e != cudaSuccess) return afail(c, SGNB_ERR_CUDA, std::string("sgnb_rhs_vjp: ") + cudaGetErrorName(e));
-  auto out = [](const std::vector<double>& v, double* o) {
-    if (o) std::memcpy(o, v.data(), v.size() * sizeof(double));
-  };
-  out(bar.Hnod, Hnod_bar); out(bar.Hx, Hx_bar); out(bar.Hy, Hy_bar); out(bar.HfX, HfX_bar);
-  out(bar.HfY, HfY_bar); out(bar.HfXEnd, HfXEnd_bar); out(bar.HfYEnd, HfYEnd_bar);
+  // the face depths cancel in R
+  auto none = [](double* o, long long n) { if (o) std::memset(o, 0, n * sizeof(double)); };
+  none(HfX_bar, 5 * ne); none(HfY_bar, 5 * ne); none(HfXEnd_bar, 5LL * c->desc.Ny); none(HfYEnd_bar, 5LL * c->desc.Nx);
   return SGNB_OK;
 }
 

@@ -151,15 +151,11 @@ __global__ void __launch_bounds__(64) k_cells_back_gauges(const long long* __res
   Hb[node] = h;
 }
 
-// Gradient of one mean: the weights of its cell at every point that the interpolant is sampled
-// at around it, in a fixed order. A point of element (ex, ey) touches the cells of the
-// elements beside it only, so 3 x 3 elements hold every contribution (2 of a direction where
-// the mesh has only two elements along it). One warp per mean, lanes over the points.
+// Gradient of one mean: the weights of its cell at every node around it, in a fixed order. A node
+// of element (ex, ey) touches the cells of the elements beside it only, so 3 x 3 elements hold
+// every contribution (2 of a direction where the mesh has only two elements along it). One warp
+// per mean, lanes over the nodes.
 __global__ void __launch_bounds__(256) k_cells_back(const CellGrid g, const double* __restrict__ Hb,
-                                                    const double* __restrict__ HfXb,
-                                                    const double* __restrict__ HfYb,
-                                                    const double* __restrict__ HfXEndb,
-                                                    const double* __restrict__ HfYEndb,
                                                     double* __restrict__ grad) {
   const int cell = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (cell >= g.Nx * g.Ny) return;
@@ -179,17 +175,10 @@ __global__ void __launch_bounds__(256) k_cells_back(const CellGrid g, const doub
     for (int dx = 0; dx < nx3; ++dx) {
       const int ex = (ci + dx - 1 + g.Nx) % g.Nx, ey = (cj + dy - 1 + g.Ny) % g.Ny;
       const long long e = ex + (long long)g.Nx * ey;
-      // lanes 0..24 the element's nodes; then its left and bottom edge nodes, and the domain's
-      // far edges where the element lies on them
+      // lanes 0..24 the element's nodes (the face depths cancel in R: their cotangents are zero)
       if (lane < NPP) {
         const int b = lane / NP, a = lane - NP * b;
         add(node_x(g, ex, a), node_y(g, ey, b), Hb[e * NPP + lane]);
-      }
-      if (lane < NP) {
-        add(ex * g.hx, node_y(g, ey, lane), HfXb[e * NP + lane]);
-        add(node_x(g, ex, lane), ey * g.hy, HfYb[e * NP + lane]);
-        if (ex == g.Nx - 1) add(g.Nx * g.hx, node_y(g, ey, lane), HfXEndb[ey * NP + lane]);
-        if (ey == g.Ny - 1) add(node_x(g, ex, lane), g.Ny * g.hy, HfYEndb[ex * NP + lane]);
       }
     }
 #pragma unroll
@@ -216,8 +205,7 @@ cudaError_t launch_cells_back(const CellGrid& g, const GatherArgs& G, const doub
   const long long Nd = 25LL * g.Nx * g.Ny;
   k_cells_back_nodes<<<blocks_of(Nd), 256, 0, s>>>(g, G.Hacc, lam, G.Hxacc, G.Hyacc, Hb);
   if (ng > 0) k_cells_back_gauges<<<(unsigned)((ng + 63) / 64), 64, 0, s>>>(gauges, ng, nsteps, etab, Hb);
-  k_cells_back<<<blocks_of(32LL * g.Nx * g.Ny), 256, 0, s>>>(g, Hb, G.HfXacc, G.HfYacc, G.HfXEndacc,
-                                                            G.HfYEndacc, grad);
+  k_cells_back<<<blocks_of(32LL * g.Nx * g.Ny), 256, 0, s>>>(g, Hb, grad);
   return cudaGetLastError();
 }
 

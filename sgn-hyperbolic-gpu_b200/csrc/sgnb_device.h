@@ -331,10 +331,6 @@ struct GatherArgs {
   double* Hacc;
   double* Hxacc;
   double* Hyacc;
-  double* HfXacc;
-  double* HfYacc;
-  double* HfXEndacc;
-  double* HfYEndacc;
 };
 
 // Work list of a batched mixed-precision launch (8x4 tiles), as BatchArgs.
