@@ -925,7 +925,7 @@ struct sgnb_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
   std::vector<sgnb_ctx*> ctx;          // per-instance buffers and statics
-  LineConsts* dconsts = nullptr;       // [n]
+  LineConsts* dconsts = nullptr;       // [n], FP64 batches
   RhsConsts* dconstsM = nullptr;       // [n], mixed batches
   bool mixed = false;                  // every instance SGNB_MIXED (else SGNB_FP64_FAST)
   // one instance after the other, each through its own loop: the batched kernels take one set of
@@ -1515,8 +1515,8 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
   if (e != cudaSuccess) return bail(e, "kernel attributes");
   e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->evRead, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc(&b->dconsts, n * sizeof(LineConsts));
-  if (e == cudaSuccess) e = cudaMalloc(&b->dconstsM, n * sizeof(RhsConsts));
+  if (e == cudaSuccess)
+    e = b->mixed ? cudaMalloc(&b->dconstsM, n * sizeof(RhsConsts)) : cudaMalloc(&b->dconsts, n * sizeof(LineConsts));
   if (e == cudaSuccess) e = cudaMalloc(&b->dargs, n * sizeof(StageArgs));
   if (e == cudaSuccess) e = cudaMallocHost(&b->hargs, n * sizeof(StageArgs));
   if (e == cudaSuccess) e = cudaMalloc(&b->dargsM, n * sizeof(StageArgsM));
@@ -1536,8 +1536,8 @@ int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out) {
     hcM[i] = b->ctx[i]->C;
     ht[i] = b->ctx[i]->ntot;
   }
-  e = cudaMemcpy(b->dconsts, hc.data(), n * sizeof(LineConsts), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->dconstsM, hcM.data(), n * sizeof(RhsConsts), cudaMemcpyHostToDevice);
+  e = b->mixed ? cudaMemcpy(b->dconstsM, hcM.data(), n * sizeof(RhsConsts), cudaMemcpyHostToDevice)
+               : cudaMemcpy(b->dconsts, hc.data(), n * sizeof(LineConsts), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->dntot, ht.data(), n * sizeof(long long), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return bail(e, "batch upload");
   std::vector<long long> maxTiles(n, 0);

@@ -217,23 +217,6 @@ __device__ __forceinline__ double flux_normal(const TC& C, const double* U,
   return hn * (DIR == 0 ? q.u : q.v) + hydro(C, U[0], Hloc) + hp;
 }
 
-// Directional flux: fluxX (DIR 0) or fluxY (DIR 1), src/physics/sgn_flux2d.h:89-116.
-template <bool EXACT, int DIR, class TC>
-__device__ __forceinline__ void flux(const TC& C, const double* U, const Prim<EXACT>& q,
-                                     double Hloc, double* F) {
-  const double hn = DIR == 0 ? U[1] : U[2];  // normal discharge
-  F[0] = hn;
-  if constexpr (DIR == 0) {
-    F[1] = flux_normal<EXACT, DIR>(C, U, q, Hloc);
-    F[2] = hn * q.v;
-  } else {
-    F[1] = hn * q.u;
-    F[2] = flux_normal<EXACT, DIR>(C, U, q, Hloc);
-  }
-  F[3] = hn * q.w;
-  F[4] = hn * (q.p + C.c2);
-}
-
 // |normal velocity| + sqrt(max(g h + p + c^2, 0)), src/physics/sgn_flux2d.h:73-86.
 template <bool EXACT, int DIR, class TC>
 __device__ __forceinline__ double wave_speed(const TC& C, const double* U,

@@ -49,7 +49,6 @@ cudaError_t prepare_fused_exact(const RhsConsts& C, bool ghost) {
   return ghost ? prepare_lines<false, true>() : prepare_lines<false, false>();
 }
 int fused_grid_blocks(int Nx, int Ny) { return ((Nx + 7) / 8) * ((Ny + 3) / 4); }
-size_t fused_smem_bytes() { return sizeof(Tile<8, 4, true>::Smem); }
 // The checked build's out-of-range count of this translation unit's kernels (reset: then
 // zero it); cudaErrorNotSupported in the normal build.
 cudaError_t read_oob_exact(unsigned long long* out, bool reset) {

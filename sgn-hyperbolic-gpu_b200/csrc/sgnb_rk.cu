@@ -200,15 +200,6 @@ __global__ void __launch_bounds__(kCtrlThreads) k_controller_slabs(CtrlState* c,
       L.start[L.ns], n);
 }
 
-// Batched controller: block i runs instance i's controller on its own partials.
-__global__ void __launch_bounds__(kCtrlThreads) k_controller_batch(CtrlState* ctrls,
-                                                                   const double* const* partials,
-                                                                   const int* nblk, const long long* n) {
-  wait_for_previous();
-  const int i = blockIdx.x;
-  controller_block(ctrls + i, partials[i], nblk[i], n[i]);
-}
-
 struct QW {
   double w[5];
 };
@@ -275,12 +266,6 @@ cudaError_t launch_controller_batch_loop(CtrlState* ctrls, const double* const* 
 cudaError_t launch_controller_slabs(CtrlState* c, const SlabPartials& L, long long n,
                                     cudaStream_t s) {
   return launch_dependent(k_controller_slabs, dim3(1), dim3(kCtrlThreads), 0, s, c, L, n);
-}
-
-cudaError_t launch_controller_batch(CtrlState* ctrls, const double* const* partials,
-                                    const int* nblk, const long long* n, int ninst,
-                                    cudaStream_t s) {
-  return launch_dependent(k_controller_batch, dim3(ninst), dim3(kCtrlThreads), 0, s, ctrls, partials, nblk, n);
 }
 
 // ---- rk4Step (src/solver/rk.cpp:23-38) -------------------------------------------------
