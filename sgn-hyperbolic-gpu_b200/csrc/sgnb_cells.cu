@@ -6,6 +6,7 @@
 // Per gradient evaluation the host versions took about 60 ms on 256 x 128 elements (evaluation,
 // 26 MB of pageable uploads and as much back, a serial scatter); these kernels take tens of
 // microseconds, and only the means, eta0 and the two gradients cross the bus.
+#include "sgnb_checked.cuh"
 #include "sgnb_device.h"
 
 namespace sgnb {
@@ -13,6 +14,14 @@ namespace dev {
 
 namespace {
 constexpr int NP = 5, NPP = 25;
+
+// p[i] of n values (the checked build: 0 out of range).
+__device__ __forceinline__ double at(const double* p, [[maybe_unused]] long long i, [[maybe_unused]] long long n) {
+  return SGNB_INB(i, n) ? p[i] : 0.0;
+}
+__device__ __forceinline__ void put(double* p, [[maybe_unused]] long long i, [[maybe_unused]] long long n, double v) {
+  if (SGNB_INB(i, n)) p[i] = v;
+}
 
 // The four cells and the position (tx, ty) between their centres at (x, y): the index
 // arithmetic of the host's interpolant.
@@ -39,8 +48,9 @@ __device__ __forceinline__ CellAt cell_at(const CellGrid& g, double x, double y)
 }
 __device__ __forceinline__ double depth_at(const CellGrid& g, const double* m, double x, double y) {
   const CellAt c = cell_at(g, x, y);
-  const double v00 = m[c.i0 + g.Nx * c.j0], v10 = m[c.i1 + g.Nx * c.j0];
-  const double v01 = m[c.i0 + g.Nx * c.j1], v11 = m[c.i1 + g.Nx * c.j1];
+  const int n = g.Nx * g.Ny;
+  const double v00 = at(m, c.i0 + g.Nx * c.j0, n), v10 = at(m, c.i1 + g.Nx * c.j0, n);
+  const double v01 = at(m, c.i0 + g.Nx * c.j1, n), v11 = at(m, c.i1 + g.Nx * c.j1, n);
   const double lo = v00 + c.tx * (v10 - v00);
   const double hi = v01 + c.tx * (v11 - v01);
   return lo + c.ty * (hi - lo);
@@ -62,28 +72,28 @@ __global__ void __launch_bounds__(256) k_cells_depth(const CellGrid g, const dou
   const int e = (int)(i / NPP), n = (int)(i - (long long)e * NPP);
   const int ey = e / g.Nx, ex = e - ey * g.Nx, b = n / NP, a = n - NP * b;
   const double h = depth_at(g, means, node_x(g, ex, a), node_y(g, ey, b));
-  H[i] = h;
-  u0[i] = h + eta0[i];
+  put(H, i, Nd, h);
+  put(u0, i, 5 * Nd, h + at(eta0, i, Nd));
 #pragma unroll
-  for (int v = 1; v < 5; ++v) u0[v * Nd + i] = 0.0;
+  for (int v = 1; v < 5; ++v) put(u0, v * Nd + i, 5 * Nd, 0.0);
 }
 
 // Nodal depth gradients: the GLL derivative along each line over J; one thread per node.
 __global__ void __launch_bounds__(256) k_cells_gradient(const CellGrid g, const double* __restrict__ H,
                                                         double* __restrict__ Hx, double* __restrict__ Hy) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 25LL * g.Nx * g.Ny) return;
+  const long long Nd = 25LL * g.Nx * g.Ny;
+  if (i >= Nd) return;
   const long long e = i / NPP;
   const int n = (int)(i - e * NPP), b = n / NP, a = n - NP * b;
-  const double* He = H + e * NPP;
   double sx = 0.0, sy = 0.0;
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
-    sx += g.D[a * NP + k] * He[k + NP * b];
-    sy += g.D[b * NP + k] * He[a + NP * k];
+    sx += g.D[a * NP + k] * at(H, e * NPP + k + NP * b, Nd);
+    sy += g.D[b * NP + k] * at(H, e * NPP + a + NP * k, Nd);
   }
-  Hx[i] = sx / (0.5 * g.hx);
-  Hy[i] = sy / (0.5 * g.hy);
+  put(Hx, i, Nd, sx / (0.5 * g.hx));
+  put(Hy, i, Nd, sy / (0.5 * g.hy));
 }
 
 // Face depths: left and bottom edges of every element (5 Nx Ny each), then the right and top
@@ -95,15 +105,15 @@ __global__ void __launch_bounds__(256) k_cells_faces(const CellGrid g, const dou
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nf) {
     const int e = (int)(i / NP), s = (int)(i - (long long)e * NP), ey = e / g.Nx, ex = e - ey * g.Nx;
-    HfX[i] = depth_at(g, m, ex * g.hx, node_y(g, ey, s));
-    HfY[i] = depth_at(g, m, node_x(g, ex, s), ey * g.hy);
+    put(HfX, i, nf, depth_at(g, m, ex * g.hx, node_y(g, ey, s)));
+    put(HfY, i, nf, depth_at(g, m, node_x(g, ex, s), ey * g.hy));
     return;
   }
   i -= nf;
   if (i < NP * g.Ny) {
-    HfXEnd[i] = depth_at(g, m, g.Nx * g.hx, node_y(g, (int)(i / NP), (int)(i % NP)));
+    put(HfXEnd, i, NP * g.Ny, depth_at(g, m, g.Nx * g.hx, node_y(g, (int)(i / NP), (int)(i % NP))));
   } else if ((i -= NP * g.Ny) < NP * g.Nx) {
-    HfYEnd[i] = depth_at(g, m, node_x(g, (int)(i / NP), (int)(i % NP)), g.Ny * g.hy);
+    put(HfYEnd, i, NP * g.Nx, depth_at(g, m, node_x(g, (int)(i / NP), (int)(i % NP)), g.Ny * g.hy));
   }
 }
 
@@ -116,24 +126,23 @@ __global__ void __launch_bounds__(256) k_cells_back_nodes(const CellGrid g, cons
                                                           const double* __restrict__ Hyb,
                                                           double* __restrict__ out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 25LL * g.Nx * g.Ny) return;
+  const long long Nd = 25LL * g.Nx * g.Ny;
+  if (i >= Nd) return;
   const long long e = i / NPP;
   const int n = (int)(i - e * NPP), b = n / NP, a = n - NP * b;
-  const double* gx = Hxb + e * NPP;
-  const double* gy = Hyb + e * NPP;
   double sx = 0.0, sy = 0.0;
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
-    sx += g.D[k * NP + a] * gx[k + NP * b];
-    sy += g.D[k * NP + b] * gy[a + NP * k];
+    sx += g.D[k * NP + a] * at(Hxb, e * NPP + k + NP * b, Nd);
+    sy += g.D[k * NP + b] * at(Hyb, e * NPP + a + NP * k, Nd);
   }
-  out[i] = (Hb[i] + lam[i]) + (sx / (0.5 * g.hx) + sy / (0.5 * g.hy));
+  put(out, i, Nd, (at(Hb, i, Nd) + at(lam, i, Nd)) + (sx / (0.5 * g.hx) + sy / (0.5 * g.hy)));
 }
 
 // eta = h - H at the gauges: the cotangents of a gauge's records leave its node's depth, in
 // step order. One thread per gauge; the first of several gauges at one node takes all of them.
-__global__ void __launch_bounds__(64) k_cells_back_gauges(const long long* __restrict__ nodes, int ng,
-                                                          long long nsteps,
+__global__ void __launch_bounds__(64) k_cells_back_gauges(const long long Nd, const long long* __restrict__ nodes,
+                                                          int ng, long long nsteps,
                                                           const double* __restrict__ etab,
                                                           double* __restrict__ Hb) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -144,10 +153,11 @@ __global__ void __launch_bounds__(64) k_cells_back_gauges(const long long* __res
   int last = q;
   for (int p = q + 1; p < ng; ++p)
     if (nodes[p] == node) last = p;
+  if (!SGNB_INB(node, Nd)) return;
   double h = Hb[node];
   for (long long n = 0; n < nsteps; ++n)
     for (int p = q; p <= last; ++p)
-      if (nodes[p] == node) h -= etab[n * ng + p];
+      if (nodes[p] == node) h -= at(etab, n * ng + p, nsteps * ng);
   Hb[node] = h;
 }
 
@@ -178,7 +188,7 @@ __global__ void __launch_bounds__(256) k_cells_back(const CellGrid g, const doub
       // lanes 0..24 the element's nodes (the face depths cancel in R: their cotangents are zero)
       if (lane < NPP) {
         const int b = lane / NP, a = lane - NP * b;
-        add(node_x(g, ex, a), node_y(g, ey, b), Hb[e * NPP + lane]);
+        add(node_x(g, ex, a), node_y(g, ey, b), at(Hb, e * NPP + lane, 25LL * g.Nx * g.Ny));
       }
     }
 #pragma unroll
@@ -188,6 +198,23 @@ __global__ void __launch_bounds__(256) k_cells_back(const CellGrid g, const doub
 
 unsigned blocks_of(long long n) { return (unsigned)((n + 255) / 256); }
 }  // namespace
+
+// The checked build's out-of-range count of this translation unit's kernels (reset: then
+// zero it); cudaErrorNotSupported in the normal build.
+cudaError_t read_oob_cells(unsigned long long* out, bool reset) {
+#ifdef SGNB_CHECKED
+  cudaError_t e = cudaMemcpyFromSymbol(out, g_sgnb_oob, sizeof(*out));
+  if (e == cudaSuccess && reset) {
+    const unsigned long long z = 0;
+    e = cudaMemcpyToSymbol(g_sgnb_oob, &z, sizeof(z));
+  }
+  return e;
+#else
+  *out = 0;
+  (void)reset;
+  return cudaErrorNotSupported;
+#endif
+}
 
 cudaError_t launch_cells_statics(const CellGrid& g, const double* means, const double* eta0, double* Hnod,
                                  double* Hx, double* Hy, double* HfX, double* HfY, double* HfXEnd,
@@ -204,7 +231,7 @@ cudaError_t launch_cells_back(const CellGrid& g, const GatherArgs& G, const doub
                               double* Hb, double* grad, cudaStream_t s) {
   const long long Nd = 25LL * g.Nx * g.Ny;
   k_cells_back_nodes<<<blocks_of(Nd), 256, 0, s>>>(g, G.Hacc, lam, G.Hxacc, G.Hyacc, Hb);
-  if (ng > 0) k_cells_back_gauges<<<(unsigned)((ng + 63) / 64), 64, 0, s>>>(gauges, ng, nsteps, etab, Hb);
+  if (ng > 0) k_cells_back_gauges<<<(unsigned)((ng + 63) / 64), 64, 0, s>>>(Nd, gauges, ng, nsteps, etab, Hb);
   k_cells_back<<<blocks_of(32LL * g.Nx * g.Ny), 256, 0, s>>>(g, Hb, grad);
   return cudaGetLastError();
 }

@@ -365,6 +365,7 @@ cudaError_t read_oob_line(unsigned long long* out, bool reset);
 cudaError_t read_oob_batch(unsigned long long* out, bool reset);
 cudaError_t read_oob_mixed(unsigned long long* out, bool reset);
 cudaError_t read_oob_adjoint(unsigned long long* out, bool reset);
+cudaError_t read_oob_cells(unsigned long long* out, bool reset);
 
 // The fast mode's reciprocal (fn 0) and square root (fn 1) elementwise, for tests.
 cudaError_t launch_fast_math(int fn, const double* x, double* y, long long n, cudaStream_t s);
