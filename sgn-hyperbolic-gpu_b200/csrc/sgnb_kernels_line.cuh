@@ -524,9 +524,13 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   if (bulk) {
     bool landed = RXv == 0;
     for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
-    // the copies did not complete: NaN, so that the launch's results are non-finite and the
-    // controller ends the run with that error
-    if (!landed) uc[0] = __longlong_as_double(0x7ff8000000000000LL);
+    if (!landed) {
+      // the copies did not complete: as long again, so that none lands after this CTA has left its
+      // shared memory, and NaN, so that the launch's results are non-finite and the controller
+      // ends the run with that error
+      for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
+      uc[0] = __longlong_as_double(0x7ff8000000000000LL);
+    }
   }
   if constexpr (MODE == MODE_CAND) __syncthreads();  // the stash's address
   else if constexpr (AXPY) __syncwarp();             // the lanes' own copies

@@ -558,8 +558,10 @@ __device__ __forceinline__ void mixed_tile(const TC& C, const TB& Tb, const TA& 
         bool landed = false;
         for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
         if (!landed) {
-          // the copies did not complete: this thread's state items become NaN, so the
-          // launch's results are non-finite and the controller ends the run with that error
+          // the copies did not complete: as long again, so that none lands after this CTA has left
+          // its shared memory; this thread's state items become NaN, so the launch's results are
+          // non-finite and the controller ends the run with that error
+          for (int it = 0; it < kTmaTries && !landed; ++it) landed = mbar_try_wait(mbar, 0);
           const double nan = __longlong_as_double(0x7ff8000000000000LL);
 #pragma unroll
           for (int v = 0; v < NV; ++v)
