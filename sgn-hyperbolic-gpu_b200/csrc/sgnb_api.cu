@@ -1183,8 +1183,10 @@ int sgnb_set_ghosts(sgnb_ctx* c, const double* ghostL, const double* ghostR) {
   if (!c) return fail(c, SGNB_ERR_INVALID, "NULL context");
   if (c->tab.gauss) return fail(c, SGNB_ERR_UNSUPPORTED, "Gauss points run on whole meshes");
   if (c->mixed) return fail(c, SGNB_ERR_UNSUPPORTED, "slab edges run in the FP64 modes");
-  if (int rc = set_device(c)) return rc;
-  if (ghostL || ghostR) SGNB_CU(c, prepare_ghosts(c));
+  if ((ghostL || ghostR) && !c->ghost_ready) {
+    if (int rc = set_device(c)) return rc;
+    SGNB_CU(c, prepare_ghosts(c));
+  }
   c->C.ghostL = ghostL;
   c->C.ghostR = ghostR;
   if (c->chunk) {  // captured launches hold the old constants
