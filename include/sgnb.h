@@ -316,7 +316,9 @@ int sgnb_write_vtk(sgnb_ctx* ctx, const char* path);
  * CUDA graph whose WHILE conditional node repeats one attempt of every still-running
  * instance until all are done). All
  * instances of a batch run in one arithmetic mode: SGNB_FP64_FAST (tile shapes 6x4, 12x2,
- * 24x1) or SGNB_MIXED (8x4 tiles). Instance i is an ordinary context
+ * 24x1) or SGNB_MIXED (8x4 tiles). A launch takes one set of FR tables: instances that bring
+ * different ones (or, in the fast mode, ones without the reflection symmetry of the GLL tables)
+ * run one after another. Instance i is an ordinary context
  * (sgnb_batch_instance) for upload / download / diagnostics between runs. */
 typedef struct sgnb_batch sgnb_batch;
 int sgnb_batch_create(const sgnb_desc* descs, int n, sgnb_batch** out);

@@ -32,7 +32,8 @@
 //         IEEE division by the Jacobians, face traces formed as 0.0 + v exactly like the
 //         reference's sum over unit GLL interpolation rows; bit-identical to the CPU;
 //   FAST  (sgnb_kernels_fast.cu, -fmad=true): reciprocal of h and of the Jacobians,
-//         FMA contraction, redundant work removed; agrees to round-off (<1e-13 rel).
+//         FMA contraction, redundant work removed; agrees to round-off (relative 1e-13 per field
+//         where elements are of order one; the rounding of the hydrostatic flux grows with 1/J).
 #pragma once
 
 #include <cstdint>

@@ -1,7 +1,9 @@
 // sgnb_kernels_fast.cu -- the fast arithmetic mode's dispatch, its Gauss-point kernels and the
 // slab packs. Built with -fmad=true: FMA contraction, reciprocals of h and of the Jacobians.
-// Agrees with the reference to round-off (relative 1e-13 per field is the test bound). The
-// kernels on GLL points are in sgnb_kernels_line.cu.
+// Agrees with the reference to round-off: one rounding of the hydrostatic flux, times the
+// differentiation matrix over J, relative to a field's largest value (1e-13 per field on meshes of
+// elements of order one, 2e-13 at J = 0.01). The kernels on GLL points are in
+// sgnb_kernels_line.cu.
 #define SGNB_EXACT false
 #include "sgnb_kernels_inst.cuh"
 

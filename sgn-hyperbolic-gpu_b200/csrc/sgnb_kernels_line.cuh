@@ -12,8 +12,8 @@
 //
 // The arithmetic is arranged for the fast mode:
 //   * every flux component is the normal velocity times a state component, F = u_n U_v (plus
-//     the hydrostatic term and c^2 h u_n where they belong), so a line keeps u_n and reads one
-//     field at a time from shared memory;
+//     the hydrostatic term in the normal discharge; h u_n (p + c^2) in hp), so a line keeps u_n and
+//     reads one field at a time from shared memory;
 //   * the Rusanov flux minus the element's own face flux is half the flux difference of the
 //     two traces plus the dissipation, in which the face depth cancels (both traces take the
 //     same one): no face depths are read;
@@ -22,15 +22,17 @@
 //     lifts splits into an even and an odd half (29 operations instead of 35);
 //   * each pass adds its own direction's sources, so no pass differentiates the depth along
 //     the other direction, and h_n and H_n of the hp equation share one derivative.
-// What bounds it. At 1024 x 512 elements a right-hand side takes 0.227 ms (5.1 TB/s, 79 % of a
-// plain copy's rate), the second, third and end-point stage 0.320, 0.508 and 0.476 ms (5.2, 5.4
-// and 4.6 TB/s); the kernels before these took 0.408, 0.497, 0.497 and 0.981 ms (the end point
-// then read four inputs twice). What is left is latency: HBM, FP64 issue (59 % busy in the
-// right-hand side) and shared memory (66 %) are all within 1.5x of their limits. The
-// right-hand side and the end point run four CTAs of 128 registers per SM (at three 0.247 and
-// 0.503 ms); the stages that add k run three (at four 0.358 and 0.556 ms: their halos read two
-// arrays, whose sectors only stay in L1 if shared memory leaves it more than 24 KB). Tiles of
-// 2 x 2 or 4 x 1 warps are slower (second stage 0.334 and 0.349 ms).
+// What bounds it. At 1024 x 512 elements a right-hand side takes 0.224 ms (5.1 TB/s, 80 % of a
+// plain copy's rate), the second, third and end-point stage 0.321, 0.515 and 0.508 ms (5.2, 5.3
+// and 4.3 TB/s; the end point 0.49 to 0.51 from GPU to GPU); kernels with one warp per GLL line took
+// 0.408, 0.497, 0.497 and 0.981 ms (the end point then read four inputs twice). What is left is
+// latency: HBM, FP64 issue (62 % busy in the right-hand side) and shared memory (65 %) are all
+// within 1.6x of their limits. The right-hand side and the end point run four CTAs of 128
+// registers per SM, the stages that add k three: their halos read two arrays, whose sectors only
+// stay in L1 if shared memory leaves it more than 24 KB. (Before the derivatives acted on
+// differences, which costs 1 %: right-hand side and end point at three CTAs 0.247 and 0.503 ms, at
+// four 0.227 and 0.476; the stages at four 0.358 and 0.556, at three 0.320 and 0.508; tiles of
+// 2 x 2 or 4 x 1 warps 0.334 and 0.349 ms in the second stage.)
 #pragma once
 
 #include "sgnb_kernels.cuh"

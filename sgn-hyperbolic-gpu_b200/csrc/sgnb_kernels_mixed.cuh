@@ -28,12 +28,13 @@
 // error estimate promote them to FP64).
 //
 // Layout and work decomposition are those of sgnb_kernels.cuh (8 x 4 element tiles, 5 warps,
-// lane = element, warp = GLL line); shared memory is 56.3 KB, so 3 CTAs fit per SM.
+// lane = element, warp = GLL line); shared memory is 58.2 KB, so 3 CTAs fit per SM.
 //
 // What bounds it: instruction latency and the conversions between the two precisions (XU pipe). At
 // 1024 x 512 elements, ms per launch: right-hand side 0.393, second stage 0.425, third stage with
 // the candidate 0.577, end point 0.606; with the candidate formed by the end point, from four arrays
-// at every own and halo node, 0.425 and 0.789. Storing the k1..k3 part of the embedded solution
+// at every own and halo node, 0.425 and 0.789 (whole attempts 1.01 to 1.10 times as fast, 64 x 32 to
+// 1399 x 700 elements, most on meshes of partial tiles). Storing the k1..k3 part of the embedded solution
 // instead of k3 took 0.62 and 0.58. The third stage prefetches its epilogue's k1 to L2 (0.592
 // without); the same for all that the end point's epilogue reads cost it 0.03 ms.
 #pragma once
