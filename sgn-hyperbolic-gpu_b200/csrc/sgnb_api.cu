@@ -299,6 +299,7 @@ void fill_consts(sgnb_ctx* c) {
   }
   const char* sw = std::getenv("SGNB_TMA");
   C.bulk = d.Nx % 2 == 0 && !(sw && sw[0] == '0');
+  C.columns = d.Nx_global == 0 && dev::exact_columns(d.Nx, d.Ny);
 }
 
 cudaError_t prepare_fp64(const sgnb_ctx* c, bool ghost) {
@@ -588,8 +589,9 @@ int sgnb_create(const sgnb_desc* d, sgnb_ctx** out) {
   if (e != cudaSuccess) { cuda_fail(c, e, "kernel attributes"); g_create_error = c->err; return bail(SGNB_ERR_CUDA); }
   e = cudaMemset(c->U[0], 0, sbytes);
   // error partials: one row per tile of the kernels that this context runs
-  c->nblk = !c->mixed && !c->tab.gauss
-                ? dev::line_grid_blocks(d->Nx, d->Ny) : dev::fused_grid_blocks(d->Nx, d->Ny);
+  if (c->mixed || c->tab.gauss) c->nblk = dev::fused_grid_blocks(d->Nx, d->Ny);
+  else if (c->precision == SGNB_FP64_FAST && c->C.sym) c->nblk = dev::line_grid_blocks(d->Nx, d->Ny);
+  else c->nblk = dev::exact_grid_blocks(c->C);
   c->ndiag = 592;
   if (e == cudaSuccess) e = cudaMalloc(&c->partials, 3 * (size_t)c->nblk * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&c->diag, (size_t)c->ndiag * sizeof(double));

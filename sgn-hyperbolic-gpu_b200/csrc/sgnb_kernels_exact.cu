@@ -7,12 +7,38 @@
 
 namespace sgnb {
 namespace dev {
+// Tiles of the two shapes (LineTile): 6 x 4 elements, and 2 x 12 (COL).
+template <bool COL>
+static dim3 tiles(int Nx, int Ny) {
+  using L = LineTile<1, true, COL>;
+  return dim3((Nx + L::TX - 1) / L::TX, (Ny + L::TY - 1) / L::TY);
+}
+// Rows of six waste lanes where Nx is a little more than a multiple of six: on meshes up to 14
+// elements wide 2 x 12 tiles can be fewer by a fifth and more. Their halo is larger and a warp's row
+// takes three copies, so they are taken only where a launch then also needs fewer waves of the
+// CTAs that are resident at once (three per SM). us per launch, rhs / stages 2, 3, end point:
+// 8 x 4096 elements on rows 123 / 114 139 171, on columns 94 / 97 119 142; 14 x 1500: 70 / 65 79 100
+// and 55 / 51 65 79; within one wave, 8 x 256: 23.7 / 19.7 21.8 29.2 and 25.6 / 20.9 24.4 32.5; 10
+// x 2048, where columns are fewer by a sixth: rows 69 / 64 76 93.
+bool exact_columns(int Nx, int Ny) {
+  constexpr long long kResident = 3 * 148;
+  const dim3 rt = tiles<false>(Nx, Ny), ct = tiles<true>(Nx, Ny);
+  const long long r = (long long)rt.x * rt.y, c = (long long)ct.x * ct.y;
+  return 10 * c <= 8 * r && (c + kResident - 1) / kResident < (r + kResident - 1) / kResident;
+}
+int exact_grid_blocks(const RhsConsts& C) {
+  const dim3 g = C.columns ? tiles<true>(C.Nx, C.Ny) : tiles<false>(C.Nx, C.Ny);
+  return (int)(g.x * g.y);
+}
+
+template <int MODE, bool FRIC, bool GHOST, bool COL>
+static cudaError_t launch_form(const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
+  return launch_dependent(k_line_exact<MODE, FRIC, GHOST, COL>, tiles<COL>(C.Nx, C.Ny), dim3(LTHR),
+                          sizeof(typename LineTile<1, true, COL>::Smem), s, C, A, (int)bulk_rows(C, A));
+}
 template <int MODE, bool FRIC, bool GHOST>
 static cudaError_t launch_variant(const RhsConsts& C, const StageArgs& A, cudaStream_t s) {
-  using L = LineTile<1, true>;
-  const dim3 grid((C.Nx + L::TX - 1) / L::TX, (C.Ny + L::TY - 1) / L::TY);
-  return launch_dependent(k_line_exact<MODE, FRIC, GHOST>, grid, dim3(LTHR), sizeof(typename L::Smem), s, C, A,
-                          (int)bulk_rows(C, A));
+  return C.columns ? launch_form<MODE, FRIC, GHOST, true>(C, A, s) : launch_form<MODE, FRIC, GHOST, false>(C, A, s);
 }
 
 template <int MODE>
@@ -33,20 +59,24 @@ cudaError_t launch_fused_exact(int mode, const RhsConsts& C, const StageArgs& A,
   }
 }
 
-template <bool FRIC, bool GHOST>
-static cudaError_t prepare_lines() {
-  const size_t bytes = sizeof(LineTile<1, true>::Smem);
-  cudaError_t e = raise_smem(k_line_exact<MODE_RHS, FRIC, GHOST>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_STAGE, FRIC, GHOST>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_CAND, FRIC, GHOST>, bytes);
-  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_FSAL, FRIC, GHOST>, bytes);
+template <bool FRIC, bool GHOST, bool COL>
+static cudaError_t prepare_form() {
+  const size_t bytes = sizeof(typename LineTile<1, true, COL>::Smem);
+  cudaError_t e = raise_smem(k_line_exact<MODE_RHS, FRIC, GHOST, COL>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_STAGE, FRIC, GHOST, COL>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_CAND, FRIC, GHOST, COL>, bytes);
+  if (e == cudaSuccess) e = raise_smem(k_line_exact<MODE_FSAL, FRIC, GHOST, COL>, bytes);
   return e;
+}
+template <bool FRIC, bool GHOST>
+static cudaError_t prepare_lines(const RhsConsts& C) {
+  return C.columns ? prepare_form<FRIC, GHOST, true>() : prepare_form<FRIC, GHOST, false>();
 }
 
 cudaError_t prepare_fused_exact(const RhsConsts& C, bool ghost) {
   if (C.gauss) return C.manning ? prepare_variant<true>() : prepare_variant<false>();
-  if (C.manning) return ghost ? prepare_lines<true, true>() : prepare_lines<true, false>();
-  return ghost ? prepare_lines<false, true>() : prepare_lines<false, false>();
+  if (C.manning) return ghost ? prepare_lines<true, true>(C) : prepare_lines<true, false>(C);
+  return ghost ? prepare_lines<false, true>(C) : prepare_lines<false, false>(C);
 }
 int fused_grid_blocks(int Nx, int Ny) { return ((Nx + 7) / 8) * ((Ny + 3) / 4); }
 // The checked build's out-of-range count of this translation unit's kernels (reset: then

@@ -8,7 +8,8 @@
 // and synchronises once, when its tile has landed and every warp has formed its stage inputs.
 // With the lanes over 32 elements and one warp per line instead (as the Gauss-point kernels of
 // sgnb_kernels.cuh), two of the eight cycles a warp took per instruction were waits at the
-// barriers between the passes.
+// barriers between the passes. On narrow meshes the exact mode's warps hold three rows of two
+// elements instead (COL; the rule and its figures are in sgnb_kernels_exact.cu).
 //
 // The arithmetic is arranged for the fast mode:
 //   * every flux component is the normal velocity times a state component, F = u_n U_v (plus
@@ -49,11 +50,13 @@ constexpr int LTHR = 32 * LWARPS;
 // stride:
 //   U[v][i * 25 + a + 5 b]        node (a, b) of tile element i = ix + TX iy
 //   U[v][TN + 5 * slot + t]       slots left [TY], right [TY], bottom [TX], top [TX]
-template <int WX_, bool EXACT_ = false>
+// COL: a warp's six elements are three rows of two, the tile 2 x 12 elements.
+template <int WX_, bool EXACT_ = false, bool COL = false>
 struct LineTile {
   static constexpr int WX = WX_, WY = LWARPS / WX_;
-  static constexpr int TX = LROW * WX, TY = WY;
-  static_assert(WX * WY == LWARPS, "four warps");
+  static constexpr int WR = COL ? 3 : 1, WC = LROW / WR;  // rows of a warp, elements of such a row
+  static constexpr int TX = WC * WX, TY = WR * WY;
+  static_assert(WX * WY == LWARPS && (!COL || WX == 1), "four warps");
   static constexpr int NHALO = 2 * TY + 2 * TX;
   static constexpr int TN = TX * TY * NPP;        // nodes per tile
   static constexpr int US = TN + NHALO * NP;      // field stride of U
@@ -345,12 +348,13 @@ __device__ __forceinline__ void line_terms(const TC& C, const TE_& T, const doub
 // One tile. The CTA holds its stash (S.stash, written before or visible after the first barrier
 // here) in the modes that use one. bulk: rows start 16-byte aligned in every buffer (Nx even) and come and go by the bulk
 // copy engine; otherwise value by value.
-template <int MODE, int WX, bool FRIC, bool GHOST, bool EXACT = false, class TC, class TE_, class TA>
+template <int MODE, int WX, bool FRIC, bool GHOST, bool EXACT = false, bool COL = false, class TC, class TE_, class TA>
 __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A, int bx, int by,
                                           long long blk, const bool bulk,
-                                          typename LineTile<WX, EXACT>::Smem& S) {
-  using L = LineTile<WX, EXACT>;
+                                          typename LineTile<WX, EXACT, COL>::Smem& S) {
+  using L = LineTile<WX, EXACT, COL>;
   constexpr int TX = L::TX, TY = L::TY, NHALO = L::NHALO, TN = L::TN, US = L::US;
+  constexpr int WR = L::WR, WC = L::WC, WRUN = WC * NPP;  // nodes of one row of a warp
   constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND;
 
   // ---- controller state -----------------------------------------------------------
@@ -368,12 +372,13 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   int tid;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
   const int w = tid >> 5, lane = tid & 31;
-  const int wx = WX == 1 ? 0 : w % WX, iy = WX == 1 ? w : w / WX;  // this warp's row of the tile
+  const int wx = WX == 1 ? 0 : w % WX, iy0 = WR * (WX == 1 ? w : w / WX);  // this warp's (first) row of the tile
   const int Nx = C.Nx, Ny = C.Ny;
   const long long Nd = C.Nd;
   const int ex0 = bx * TX, ey0 = by * TY;
   const int TXv = min(TX, Nx - ex0), TYv = min(TY, Ny - ey0);
-  const int RXv = iy < TYv ? max(0, min(LROW, TXv - wx * LROW)) : 0;  // elements of the row in the mesh
+  // elements of the warp's row in the mesh, and such rows
+  const int RXv = iy0 < TYv ? max(0, min(WC, TXv - wx * LROW)) : 0, RYv = COL ? min(WR, TYv - iy0) : 1;
   bool ghostL = false, ghostR = false;
   if constexpr (GHOST) {
     ghostL = C.ghostL != nullptr && ex0 == 0;
@@ -381,20 +386,28 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   }
   const bool wallL = C.bcx && ex0 == 0 && !ghostL, wallR = C.bcx && ex0 + TXv == Nx && !ghostR;
   const bool wallB = C.bcy && ey0 == 0, wallT = C.bcy && ey0 + TYv == Ny;
-  const int row0 = (ex0 + wx * LROW + Nx * (ey0 + iy)) * NPP;  // the row's first node in a field (Nd < 2^31)
-  const int s0 = (wx * LROW + TX * iy) * NPP;                  // and in the tile
-  const int rowv = RXv * NPP;                                  // its nodes in the mesh
+  const int row0 = (ex0 + wx * LROW + Nx * (ey0 + iy0)) * NPP;  // the row's first node in a field (Nd < 2^31)
+  const int s0 = (wx * LROW + TX * iy0) * NPP;                  // and in the tile
+  const int rowv = RXv * NPP;                                   // its nodes in the mesh
+  const int next_row = Nx * NPP;                                // to the same node one row up
+  // column and row in the tile of the warp's element e
+  auto el_x = [&](int e) { return COL ? e % WC : wx * LROW + e; };
+  auto el_y = [&](int e) { return COL ? iy0 + e / WC : iy0; };
 
   // ---- the row's own nodes ------------------------------------------------------------
   const unsigned mbar = smem_addr(&S.mbar[w]);
   double* const ks = &S.G[0][0];  // the stage derivative, until the passes
-  // pair m of a field: nodes kp + 2 LPL m and the next one, where in[m] (and two[m])
+  // pair m of a field: the warp's nodes kp + 2 LPL m and the next one, where in[m] (and two[m]); in
+  // the mesh it is step(m) from the first pair (COL: pair m is in row m, 2 LPL nodes long)
+  static_assert(!COL || WRUN == 2 * LPL, "a pair per row");
   const int kp = 2 * lane;
+  auto step = [&](int m) { return COL ? m * next_row : 2 * LPL * m; };
   bool in[LPF], two[LPF];
 #pragma unroll
   for (int m = 0; m < LPF; ++m) {
-    in[m] = lane < LPL && kp + 2 * LPL * m < rowv;
-    two[m] = kp + 2 * LPL * m + 1 < rowv;
+    const int k = COL ? kp : kp + 2 * LPL * m;
+    in[m] = lane < LPL && k < rowv && (!COL || m < RYv);
+    two[m] = k + 1 < rowv;
   }
   if (bulk) {
     constexpr int NROW = NV + 1 + (AXPY ? NV : 0);
@@ -402,27 +415,35 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     if (lane == 0) {
       mbar_init(mbar);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      mbar_expect_tx(mbar, NROW * bytes);
+      mbar_expect_tx(mbar, RXv > 0 ? NROW * RYv * bytes : 0u);
     }
     __syncwarp();
-    if (lane < NROW && RXv > 0) {
-      int g = row0;
+    auto copy = [&](int f, int r) {  // array f's row r
+      const int sr = s0 + r * WRUN;
+      int g = row0 + r * next_row;
       if (!SGNB_INB(g, Nd - rowv + 1)) g = 0;
-      if (lane < NV) bulk_load(smem_addr(&S.U[lane][s0]), src + lane * Nd + g, bytes, mbar);
-      else if (lane == NV) bulk_load(smem_addr(&S.H[s0]), C.Hnod + g, bytes, mbar);
-      else bulk_load(smem_addr(ks + (lane - NV - 1) * TN + s0), kin + (lane - NV - 1) * Nd + g, bytes, mbar);
+      if (f < NV) bulk_load(smem_addr(&S.U[f][sr]), src + f * Nd + g, bytes, mbar);
+      else if (f == NV) bulk_load(smem_addr(&S.H[sr]), C.Hnod + g, bytes, mbar);
+      else bulk_load(smem_addr(ks + (f - NV - 1) * TN + sr), kin + (f - NV - 1) * Nd + g, bytes, mbar);
+    };
+    if constexpr (COL) {
+      for (int q = lane; q < NROW * RYv; q += 32)
+        if (RXv > 0) copy(q % NROW, q / NROW);
+    } else if (lane < NROW && RXv > 0) {
+      copy(lane, 0);
     }
     // what the epilogue reads starts its way to L2
     if constexpr (MODE == MODE_CAND || MODE == MODE_FSAL) {
-      const int f = lane - 16;  // lanes that copy no row
-      if (f >= 0 && f < NV && RXv > 0 && SGNB_INB(row0, Nd - rowv + 1))
-        bulk_prefetch((MODE == MODE_CAND ? pick(A.K1, cur) : A.K3) + f * Nd + row0, bytes);
+      const int q = COL ? lane : lane - 16;  // (lanes that copy no row)
+      const int f = COL ? q % NV : q, r = COL ? q / NV : 0, g = row0 + r * next_row;
+      if (f >= 0 && f < NV && r < RYv && RXv > 0 && SGNB_INB(g, Nd - rowv + 1))
+        bulk_prefetch((MODE == MODE_CAND ? pick(A.K1, cur) : A.K3) + f * Nd + g, bytes);
     }
   } else {
 #pragma unroll
     for (int m = 0; m < (LRUN + 31) / 32; ++m) {
-      const int k = lane + 32 * m, g = row0 + k;
-      if (k < rowv && SGNB_INB(g, Nd)) {
+      const int k = lane + 32 * m, r = COL ? k / WRUN : 0, kr = k - r * WRUN, g = row0 + r * next_row + kr;
+      if (kr < rowv && r < RYv && SGNB_INB(g, Nd)) {
         cp_async8(&S.H[s0 + k], C.Hnod + g);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -443,7 +464,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
 #pragma unroll
       for (int m = 0; m < LPF; ++m) {
         eu[v][m] = make_double2(0.0, 0.0);
-        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) eu[v][m] = load_pair(u0 + v * Nd + 2 * LPL * m, bulk, two[m]);
+        if (in[m] && SGNB_INB(row0 + kp + step(m), Nd)) eu[v][m] = load_pair(u0 + v * Nd + step(m), bulk, two[m]);
       }
   }
   // ---- nodes across the tile's edges: one (slot, transverse node) per thread, five fields ---
@@ -497,10 +518,10 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   // exact mode: the depths of the faces at both ends of this lane's two lines
   const int ce = kColumnLane[lane] >> 3, cj = kColumnLane[lane] & 7;  // column pass: element, line
   double fy0 = 0.0, fy1 = 0.0, fx0 = 0.0, fx1 = 0.0;
+  auto in_mesh = [&](int e) { return COL ? el_x(e) < TXv && el_y(e) < TYv : e < RXv; };
   if constexpr (EXACT) {
-    const int ey = ey0 + iy;
-    if (lane < LROW * NP && ce < RXv) {
-      const int ex = ex0 + wx * LROW + ce;
+    if (lane < LROW * NP && in_mesh(ce)) {
+      const int ex = ex0 + el_x(ce), ey = ey0 + el_y(ce);
       const bool end = C.bcy && ey + 1 == Ny;
       const long long f0 = ((long long)ex + (long long)Nx * ey) * NP + cj;
       const long long f1 = end ? (long long)ex * NP + cj
@@ -508,8 +529,8 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       if (SGNB_INB(f0, Nd / NP)) fy0 = C.HfY[f0];
       if (SGNB_INB(f1, end ? (long long)Nx * NP : Nd / NP)) fy1 = (end ? C.HfYEnd : C.HfY)[f1];
     }
-    if (lane < LROW * NP && lane / NP < RXv) {
-      const int ex = ex0 + wx * LROW + lane / NP, t = lane % NP;
+    if (lane < LROW * NP && in_mesh(lane / NP)) {
+      const int ex = ex0 + el_x(lane / NP), ey = ey0 + el_y(lane / NP), t = lane % NP;
       const bool end = ex + 1 == Nx && (C.bcx || ghostR);
       const long long f0 = ((long long)ex + (long long)Nx * ey) * NP + t;
       const long long f1 = end ? (long long)ey * NP + t
@@ -520,7 +541,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   }
 
   // ---- this warp's row has landed; stage input u + (c dt) k in place; then the whole tile ---
-  const bool cvalid = lane < LROW * NP && ce < RXv;
+  const bool cvalid = lane < LROW * NP && in_mesh(ce);
   double* const uc = &S.U[0][s0 + ce * NPP + cj];
   if (!bulk) cp_async_wait_all();
   if (bulk) {
@@ -578,8 +599,8 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
 
   // ---- column pass: y-lines ----------------------------------------------------------
   if (cvalid) {
+    const int ix = el_x(ce), iy = el_y(ce);
     const bool mlo = iy == 0 && wallB, mhi = iy + 1 >= TYv && wallT;
-    const int ix = wx * LROW + ce;
     const double* const lo = mlo ? uc : (iy > 0 ? uc - TX * NPP + NP * (NP - 1) : &S.U[0][TN + (2 * TY + ix) * NP + cj]);
     const double* const hi = mhi ? uc + NP * (NP - 1)
                                  : (iy + 1 < TYv ? uc + TX * NPP : &S.U[0][TN + (2 * TY + TX + ix) * NP + cj]);
@@ -613,8 +634,8 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   let_next_start();
   // ---- row pass: x-lines, completes dU --------------------------------------------------
   {
-    const int e = lane / NP, j = lane - NP * e, ix = wx * LROW + e;
-    if (lane < LROW * NP && e < RXv) {
+    const int e = lane / NP, j = lane - NP * e, ix = el_x(e), iy = el_y(e);
+    if (lane < LROW * NP && in_mesh(e)) {
       const int o = s0 + NP * lane;
       const double* const u = &S.U[0][o];
       const bool mlo = ix == 0 && wallL, mhi = ix + 1 >= TXv && wallR;
@@ -657,15 +678,16 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   if constexpr (MODE != MODE_CAND) {
     double* __restrict__ outp = MODE == MODE_FSAL ? pick(A.K1, cur ^ 1) : A.out;
     if (bulk_out) {
-      if (lane < NV && RXv > 0 && SGNB_INB(row0, Nd - rowv + 1))
-        bulk_store(outp + lane * Nd + row0, smem_addr(&S.G[lane][s0]), (unsigned)rowv * sizeof(double));
+      const int f = COL ? lane % NV : lane, r = COL ? lane / NV : 0, g = row0 + r * next_row;
+      if (f < NV && r < RYv && RXv > 0 && SGNB_INB(g, Nd - rowv + 1))
+        bulk_store(outp + f * Nd + g, smem_addr(&S.G[f][s0 + r * WRUN]), (unsigned)rowv * sizeof(double));
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v)
 #pragma unroll
         for (int m = 0; m < LPF; ++m)
-          if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd))
-            store_pair(outp + v * Nd + row0 + kp + 2 * LPL * m, *(const double2*)&S.G[v][s0 + kp + 2 * LPL * m],
+          if (in[m] && SGNB_INB(row0 + kp + step(m), Nd))
+            store_pair(outp + v * Nd + row0 + kp + step(m), *(const double2*)&S.G[v][s0 + kp + 2 * LPL * m],
                        false, two[m]);
     }
   }
@@ -681,7 +703,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     auto load = [&](int v, double2 (&x)[LPF]) {
 #pragma unroll
       for (int m = 0; m < LPF; ++m)
-        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) x[m] = load_pair(k1 + v * Nd + 2 * LPL * m, bulk, two[m]);
+        if (in[m] && SGNB_INB(row0 + kp + step(m), Nd)) x[m] = load_pair(k1 + v * Nd + step(m), bulk, two[m]);
     };
     load(0, nb);
     stash_put_wait();
@@ -703,9 +725,9 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
         x.y = fsal_finish(a[m].y, fsal_part(b[m].y, c[m].y), k3.y, dt);
         p.x = emb_part(b[m].x, c[m].x, k3.x);
         p.y = emb_part(b[m].y, c[m].y, k3.y);
-        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) {
-          store_pair(un + v * Nd + 2 * LPL * m, x, bulk, two[m]);
-          store_pair(pe + v * Nd + 2 * LPL * m, p, bulk, two[m]);
+        if (in[m] && SGNB_INB(row0 + kp + step(m), Nd)) {
+          store_pair(un + v * Nd + step(m), x, bulk, two[m]);
+          store_pair(pe + v * Nd + step(m), p, bulk, two[m]);
         }
       }
     }
@@ -719,13 +741,14 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       const double* u0 = pick(A.U, cur);
       const double* k1 = pick(A.K1, cur);
       const double* k2 = A.K2;
-      for (int q = lane; q < 2 * NV * NP; q += 32) {
-        const int side = q / (NV * NP), r = q - side * NV * NP, t = r % NP, v = r / NP;
+      for (int q = lane; q < 2 * NV * NP * RYv; q += 32) {
+        const int row = q / (2 * NV * NP), qr = q - row * 2 * NV * NP;
+        const int side = qr / (NV * NP), r = qr - side * NV * NP, t = r % NP, v = r / NP;
         if (side == 0 ? !outLo : !outHi) continue;
         const int at = side == 0 ? NP * t : (RXv - 1) * NPP + NP - 1 + NP * t;
-        const long long g = (long long)v * Nd + row0 + at;
-        const double kout = S.G[v][s0 + at];
-        const long long ge = (long long)v * Ny * NP + (long long)(ey0 + iy) * NP + t;
+        const long long g = (long long)v * Nd + row0 + row * next_row + at;
+        const double kout = S.G[v][s0 + row * WRUN + at];
+        const long long ge = (long long)v * Ny * NP + (long long)(ey0 + iy0 + row) * NP + t;
         if (!SGNB_INB(g, NV * Nd) || !SGNB_INB(ge, (long long)NV * Ny * NP)) continue;
         (side == 0 ? C.edgeL : C.edgeR)[ge] =
             MODE == MODE_STAGE ? stage_axpy(u0[g], 0.75 * dt, kout)
@@ -742,7 +765,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     auto load = [&](int v, double2 (&x)[LPF]) {
 #pragma unroll
       for (int m = 0; m < LPF; ++m)
-        if (in[m] && SGNB_INB(row0 + kp + 2 * LPL * m, Nd)) x[m] = load_pair(pe + v * Nd + 2 * LPL * m, bulk, two[m]);
+        if (in[m] && SGNB_INB(row0 + kp + step(m), Nd)) x[m] = load_pair(pe + v * Nd + step(m), bulk, two[m]);
     };
     load(0, np);
     stash_put_wait();
@@ -785,7 +808,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
     else errors([](double e, double sc) { return sc >= kNormal ? e * fast_rcp(sc) : e / sc; });
     reduce_error<LWARPS>(esum, emax, esum != esum, S.red, A.partials, blk);
   }
-  if (bulk_out && lane < NV) bulk_store_wait();  // shared memory is read out
+  if (bulk_out && lane < NV * WR) bulk_store_wait();  // shared memory is read out
   if (bulk) {
     // a persistent CTA's next tile: its copies write what this one read and wrote, and its
     // warps initialise their barriers again
@@ -813,14 +836,14 @@ __global__ void __launch_bounds__(LTHR, (kLineCtas<MODE, 1>))
 
 // The exact mode's: the reference's operation order and IEEE divisions in the same tiles. Three
 // CTAs per SM (62 KB with the sixth field of column results).
-template <int MODE, bool FRIC, bool GHOST>
+template <int MODE, bool FRIC, bool GHOST, bool COL>
 __global__ void __launch_bounds__(LTHR, 3) k_line_exact(const RhsConsts C, const StageArgs A, const int bulk) {
   extern __shared__ __align__(128) unsigned char smem_line_exact[];
-  auto& S = *reinterpret_cast<typename LineTile<1, true>::Smem*>(smem_line_exact);
+  auto& S = *reinterpret_cast<typename LineTile<1, true, COL>::Smem*>(smem_line_exact);
   if (kStash<MODE> && threadIdx.x < 32) stash_alloc(&S.stash);
   wait_for_previous();
-  line_tile<MODE, 1, FRIC, GHOST, true>(C, C, A, blockIdx.x, blockIdx.y,
-                                        (long long)blockIdx.y * gridDim.x + blockIdx.x, bulk != 0, S);
+  line_tile<MODE, 1, FRIC, GHOST, true, COL>(C, C, A, blockIdx.x, blockIdx.y,
+                                             (long long)blockIdx.y * gridDim.x + blockIdx.x, bulk != 0, S);
   if constexpr (kStash<MODE>) {
     __syncthreads();
     if (threadIdx.x < 32) stash_free(S.stash);
