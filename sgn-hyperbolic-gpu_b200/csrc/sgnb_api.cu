@@ -299,7 +299,7 @@ void fill_consts(sgnb_ctx* c) {
   }
   const char* sw = std::getenv("SGNB_TMA");
   C.bulk = d.Nx % 2 == 0 && !(sw && sw[0] == '0');
-  C.columns = d.Nx_global == 0 && dev::exact_columns(d.Nx, d.Ny);
+  C.form = dev::exact_form(d.Nx, d.Ny, d.Nx_global > 0);
 }
 
 cudaError_t prepare_fp64(const sgnb_ctx* c, bool ghost) {

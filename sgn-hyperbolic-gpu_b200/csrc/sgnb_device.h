@@ -71,7 +71,7 @@ struct RhsConsts {
   int sym;
   int bulk;       // bulk row copies: the rows of FP64 buffers start and end at multiples of 16
                   // bytes (Nx even)
-  int columns;    // the exact line kernels on tiles of 2 x 12 elements instead of 6 x 4
+  int form;       // the exact line kernels' form for this mesh (exact_form)
 };
 
 // What the line kernels (fast mode) take of RhsConsts.
@@ -256,6 +256,7 @@ struct StageArgs {
   double coef;        // MODE_STAGE, MODE_CAND: 0.5 or 0.75
   const CtrlState* ctrl;
   double* partials;   // MODE_FSAL: 3 doubles per CTA (sum r^2, max |r|, NaN count)
+  int cand, pad_;     // MODE_STAGES: the third stage, with the candidate
 };
 
 // Whether the rows of every buffer of a launch can move by bulk copies: aligned rows (C.bulk) in
@@ -431,8 +432,9 @@ cudaError_t prepare_fused_batch(int shape_id, int blocks);
 int batch_tile_tx(int shape_id);
 int batch_tile_ty(int shape_id);
 int line_grid_blocks(int Nx, int Ny);
-// The exact line kernels' tile shape for a mesh, and the error partials of a right-hand side.
-bool exact_columns(int Nx, int Ny);
+// The exact line kernels' form for a mesh (slab: one of a decomposed one), and the number of its
+// tiles.
+int exact_form(int Nx, int Ny, bool slab);
 int exact_grid_blocks(const RhsConsts& C);
 // rk4Step: c->dt = dts[i], and the final update u += dt/6 (k1 + 2 k2 + 2 k3 + k4) over n values
 cudaError_t launch_rk4_set_dt(CtrlState* c, const double* dts, long long i, cudaStream_t s);

@@ -63,7 +63,9 @@ enum : int {
   // third stage of a BS3(2) attempt: k3 = R(u + 3/4 dt k2) is used up in the launch that forms
   // it; the candidate uNew = u + dt (2/9 k1 + 1/3 k2 + 4/9 k3) goes to the spare state buffer
   // and the part 7/24 k1 + 1/4 k2 + 1/3 k3 of the embedded solution to the K3 buffer
-  MODE_CAND = 3
+  MODE_CAND = 3,
+  // MODE_STAGE or MODE_CAND, as StageArgs::cand says (the exact mode's line kernels)
+  MODE_STAGES = 4
 };
 
 // A tile of TX x TY = 32 elements (TX in 4, 8, 16) and its shared-memory layout.

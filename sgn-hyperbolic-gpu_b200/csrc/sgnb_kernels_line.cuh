@@ -128,7 +128,7 @@ __device__ __forceinline__ auto pick(const P& p, int c) { return c ? p[1] : p[0]
 // memory in 4.1 and 2.6 of the 10 and 8 cycles a warp took per instruction.)
 constexpr unsigned kStashCols = 128;
 template <int MODE>
-constexpr bool kStash = MODE == MODE_CAND || MODE == MODE_FSAL;
+constexpr bool kStash = MODE == MODE_CAND || MODE == MODE_STAGES || MODE == MODE_FSAL;
 __device__ __forceinline__ void stash_alloc(unsigned* smem) {  // one warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(smem)),
                "r"(kStashCols)
@@ -355,7 +355,10 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
   using L = LineTile<WX, EXACT, COL>;
   constexpr int TX = L::TX, TY = L::TY, NHALO = L::NHALO, TN = L::TN, US = L::US;
   constexpr int WR = L::WR, WC = L::WC, WRUN = WC * NPP;  // nodes of one row of a warp
-  constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND;
+  constexpr bool AXPY = MODE == MODE_STAGE || MODE == MODE_CAND || MODE == MODE_STAGES;
+  constexpr bool MAYBE_CAND = MODE == MODE_CAND || MODE == MODE_STAGES;
+  bool cand = MODE == MODE_CAND;  // the candidate leaves
+  if constexpr (MODE == MODE_STAGES) cand = A.cand != 0;
 
   // ---- controller state -----------------------------------------------------------
   int cur = 0;
@@ -433,11 +436,11 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       copy(lane, 0);
     }
     // what the epilogue reads starts its way to L2
-    if constexpr (MODE == MODE_CAND || MODE == MODE_FSAL) {
+    if ((MAYBE_CAND && cand) || MODE == MODE_FSAL) {
       const int q = COL ? lane : lane - 16;  // (lanes that copy no row)
       const int f = COL ? q % NV : q, r = COL ? q / NV : 0, g = row0 + r * next_row;
       if (f >= 0 && f < NV && r < RYv && RXv > 0 && SGNB_INB(g, Nd - rowv + 1))
-        bulk_prefetch((MODE == MODE_CAND ? pick(A.K1, cur) : A.K3) + f * Nd + g, bytes);
+        bulk_prefetch((MAYBE_CAND ? pick(A.K1, cur) : A.K3) + f * Nd + g, bytes);
     }
   } else {
 #pragma unroll
@@ -555,7 +558,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       uc[0] = __longlong_as_double(0x7ff8000000000000LL);
     }
   }
-  if constexpr (MODE == MODE_CAND) __syncthreads();  // the stash's address
+  if constexpr (MAYBE_CAND) __syncthreads();  // the stash's address
   else if constexpr (AXPY) __syncwarp();             // the lanes' own copies
   if constexpr (AXPY) {
     // in the linear order of the row (no bank conflicts, 16 bytes per access), the next field's
@@ -582,7 +585,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
         if (in[m])
           *(double2*)&S.U[v][s0 + kp + 2 * LPL * m] =
               make_double2(stage_axpy(xv[m].x, acoef, yv[m].x), stage_axpy(xv[m].y, acoef, yv[m].y));
-      if constexpr (MODE == MODE_CAND) {
+      if (MAYBE_CAND && cand) {
         __syncwarp();
         const unsigned st = S.stash + ((unsigned)w << 21) + 4 * LPF * v;
         stash_put(st, xv);
@@ -670,12 +673,12 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
       }
     }
   }
-  const bool bulk_out = bulk && MODE != MODE_CAND;
+  const bool bulk_out = bulk && !cand;
   if (bulk_out) asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   __syncwarp();
 
   // ---- results ---------------------------------------------------------------------
-  if constexpr (MODE != MODE_CAND) {
+  if (!(MAYBE_CAND && cand)) {
     double* __restrict__ outp = MODE == MODE_FSAL ? pick(A.K1, cur ^ 1) : A.out;
     if (bulk_out) {
       const int f = COL ? lane % NV : lane, r = COL ? lane / NV : 0, g = row0 + r * next_row;
@@ -691,7 +694,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
                        false, two[m]);
     }
   }
-  if constexpr (MODE == MODE_CAND) {
+  if (MAYBE_CAND && cand) {
     // k3 is used up here: the candidate uNew = u + dt (2/9 k1 + 1/3 k2 + 4/9 k3) and the part
     // 7/24 k1 + 1/4 k2 + 1/3 k3 of the embedded solution leave instead (rk.cpp:106-121)
     const double* k1 = pick(A.K1, cur) + row0 + kp;
@@ -751,8 +754,7 @@ __device__ __forceinline__ void line_tile(const TC& C, const TE_& T, const TA& A
         const long long ge = (long long)v * Ny * NP + (long long)(ey0 + iy0 + row) * NP + t;
         if (!SGNB_INB(g, NV * Nd) || !SGNB_INB(ge, (long long)NV * Ny * NP)) continue;
         (side == 0 ? C.edgeL : C.edgeR)[ge] =
-            MODE == MODE_STAGE ? stage_axpy(u0[g], 0.75 * dt, kout)
-                               : fsal_finish(u0[g], fsal_part(k1[g], k2[g]), kout, dt);
+            cand ? fsal_finish(u0[g], fsal_part(k1[g], k2[g]), kout, dt) : stage_axpy(u0[g], 0.75 * dt, kout);
       }
     }
   }
@@ -834,10 +836,13 @@ __global__ void __launch_bounds__(LTHR, (kLineCtas<MODE, 1>))
   }
 }
 
-// The exact mode's: the reference's operation order and IEEE divisions in the same tiles. Three
-// CTAs per SM (62 KB with the sixth field of column results).
-template <int MODE, bool FRIC, bool GHOST, bool COL>
-__global__ void __launch_bounds__(LTHR, 3) k_line_exact(const RhsConsts C, const StageArgs A, const int bulk) {
+// The exact mode's: the reference's operation order and IEEE divisions in the same tiles. At most
+// three CTAs per SM fit (62 KB with the sixth field of column results); CTAS: the number that the
+// registers are set for. Such a kernel is 115 to 140 KB of instructions, executed once per warp, and
+// an attempt's kernels put each other's out of the instruction caches: both stages are one kernel
+// (MODE_STAGES; 200 x 100 elements, an attempt: 221 us with two, 211 with one).
+template <int MODE, bool FRIC, bool GHOST, bool COL, int CTAS>
+__global__ void __launch_bounds__(LTHR, CTAS) k_line_exact(const RhsConsts C, const StageArgs A, const int bulk) {
   extern __shared__ __align__(128) unsigned char smem_line_exact[];
   auto& S = *reinterpret_cast<typename LineTile<1, true, COL>::Smem*>(smem_line_exact);
   if (kStash<MODE> && threadIdx.x < 32) stash_alloc(&S.stash);
